@@ -189,6 +189,11 @@ const char* ncn_last_cuda_error(void);
 /* Library version (major*100 + minor). */
 int ncn_version(void);
 
+/* Copies L weight vectors of `cols` fp32 values each (device pointers in the host array `weights`, one per stage) into
+ * one [L][cols] buffer, by one launch per 32 of them: what ncn_net_fwd / ncn_net_bwd take as W.
+ * No counterpart in the reference (its stages read their weights one by one). */
+int ncn_gather_weights(const float* const* weights, int L, int64_t cols, float* out, void* stream);
+
 /* The NCN_* environment switches (kernel selection for A/B measurements: NCN_LANES, NCN_LANES_PIPE, NCN_FWD_DUAL, NCN_BWD_DUAL, NCN_NO_PAIR, NCN_NO_FEAT, NCN_EXACT_TANH, ...) are read once,
  * when the library is loaded, and launch plans are remembered per argument set.  This call reads the
  * switches again and forgets the remembered plans.  Not thread-safe against concurrent launches.

@@ -61,6 +61,7 @@ SIGNATURES = {
     "ncn_net_supported": (c_int, [c_int64] * 3 + [c_int] * 6),
     "ncn_bwd_workspace_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 4),
     "ncn_ckpt_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 3),
+    "ncn_gather_weights": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_void_p]),
     "ncn_device_status": (c_int, []),
     "ncn_status_string": (c_char_p, [c_int]),
     "ncn_last_cuda_error": (c_char_p, []),
@@ -69,6 +70,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_torch_ext = None
 
 
 class NCNError(RuntimeError):
@@ -105,3 +107,19 @@ def check(fn: str, status: int) -> None:
     if status == 7:
         text += " (" + lib.ncn_last_cuda_error().decode() + ")"
     raise NCNError(fn, status, text)
+
+
+def native():
+    """The extension module with the autograd nodes (csrc/ncn_torch.cpp), which calls the same library."""
+    global _torch_ext
+    if _torch_ext is None:
+        load()  # the library first: its absence has the clearer message
+        try:
+            from . import _ncn_torch
+        except ImportError as e:
+            raise RuntimeError(
+                f"the extension module _ncn_torch cannot be loaded ({e}): build it with `python -m ncn_cuda_b200.build`. "
+                "This package has no CPU or eager fallback."
+            ) from e
+        _torch_ext = _ncn_torch
+    return _torch_ext

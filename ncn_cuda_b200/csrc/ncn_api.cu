@@ -887,6 +887,20 @@ static int stage_bwd_generic(const void* y, const void* ya, const void* dy, cons
   return reduce_dw(p.partials, dW, g.grid, 2 * (int)E, 0, (cudaStream_t)stream);
 }
 
+// ---- one [L][cols] buffer out of L weight vectors: the pointers travel in the parameter block, 32 to a launch
+constexpr int kGatherMax = 32;
+struct GatherParams {
+  const float* src[kGatherMax];
+  float* out;
+  int cols, total;
+};
+__global__ void gather_weights_kernel(const GatherParams p) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += gridDim.x * blockDim.x) {
+    const int l = i / p.cols;
+    p.out[i] = p.src[l][i - l * p.cols];
+  }
+}
+
 static size_t workspace_floats(const DevInfo& dev, int64_t E, int L) {
   return (size_t)dev.sms * 32 * 2 * (size_t)E * (size_t)(L < 1 ? 1 : L);
 }
@@ -971,6 +985,26 @@ int ncn_net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, 
   if (plan_rows(false, B, (int)N, n_cache, L, dtype, flags, 0, false, dev, ACT_TANH, pl) != NCN_OK) return 0;
   if (plan_rows(true, B, (int)N, n_cache, L, dtype, flags, n_ck, false, dev, ACT_TANH, pl) != NCN_OK) return 0;
   return 1;
+}
+
+int ncn_gather_weights(const float* const* weights, int L, int64_t cols, float* out, void* stream) {
+  if (!weights || !out) return NCN_ERR_NULL;
+  if (L < 1 || cols < 1 || cols > (1 << 25)) return NCN_ERR_SHAPE;
+  for (int l0 = 0; l0 < L; l0 += kGatherMax) {
+    GatherParams p{};
+    const int cnt = L - l0 < kGatherMax ? L - l0 : kGatherMax;
+    for (int l = 0; l < cnt; ++l) {
+      if (!weights[l0 + l]) return NCN_ERR_NULL;
+      p.src[l] = weights[l0 + l];
+    }
+    p.out = out + (int64_t)l0 * cols;
+    p.cols = (int)cols;
+    p.total = cnt * (int)cols;
+    const int blocks = (p.total + 255) / 256;
+    gather_weights_kernel<<<blocks > 64 ? 64 : blocks, p.total < 256 ? (p.total + 31) / 32 * 32 : 256, 0, (cudaStream_t)stream>>>(p);
+  }
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? NCN_OK : cuda_fail(e);
 }
 
 int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya, float* ckpt, int ckpt_every,

@@ -1,0 +1,478 @@
+// PyTorch autograd nodes of the NCN operators (extension module _ncn_torch).
+//
+// What the reference does in Python -- one autograd.Function per stage and a loop over the stages
+// (ncn_cuda/ncn_pytorch_wrapper_v2.py:9-50, 107-144) -- is one C++ node per call here: a fused net
+// (or a stack of residual ones) or a chain of stages, with the C ABI of include/ncn_b200.h below it.
+//
+// Why native: at small batches the host is the bound.  A training step of a 1024 x 1024 net runs 59 us
+// of kernels; through Python autograd functions, ctypes and torch.stack / unbind it took 294 us.
+// A chain of stages keeps its inner activations in one node, so that the engine hands over once per
+// direction instead of once per stage, and the weights of a net are gathered by one small kernel and
+// their gradients returned as views of one buffer.
+//
+// Saved tensors go through SavedVariable, so in-place changes, saved-tensor hooks and a second backward
+// without retain_graph behave as for any autograd operator.  Without gradients no state is stored.
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/extension.h>
+
+#include <mutex>
+#include <string>
+#include <vector>
+
+#include "../../include/ncn_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::edge_list;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+// A non-zero status as the NCNError of _lib.py; also from the engine's threads, which do not hold the GIL.
+void check_status(const char* fn, int status) {
+  if (status == NCN_OK) return;
+  py::gil_scoped_acquire gil;
+  try {
+    py::module_::import("ncn_cuda_b200._lib").attr("check")(fn, status);
+  } catch (py::error_already_set& e) {
+    e.restore();
+    python_error err;
+    err.persist();
+    throw err;
+  }
+}
+
+void check_activations(const Tensor& x, const Tensor& xa) {
+  if (!x.is_cuda()) throw std::runtime_error("NCN kernels run on CUDA tensors only; there is no CPU path in this package");
+  if (x.dim() != 3) throw py::value_error("expected [B, N, E] tensors");
+  if (xa.sizes() != x.sizes() || xa.scalar_type() != x.scalar_type() || xa.device() != x.device())
+    throw py::value_error("x, xa (and the cotangents) must agree in shape, dtype and device");
+  if (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16)
+    throw py::type_error(std::string("NCN kernels take float32 or bfloat16 tensors, got ") + c10::toString(x.scalar_type()));
+}
+
+int dtype_code(const Tensor& t) { return t.scalar_type() == at::kBFloat16 ? NCN_BF16 : NCN_F32; }
+
+// The weights as the kernels take them: fp32, contiguous, on the activations' device.
+Tensor plain_weights(const Tensor& W, int64_t numel, const at::Device& dev) {
+  if (W.numel() != numel)
+    throw py::value_error("weight has " + std::to_string(W.numel()) + " elements, expected " + std::to_string(numel));
+  if (W.scalar_type() == at::kFloat && W.is_contiguous() && W.device() == dev) return W;
+  return W.detach().to(dev, at::kFloat).contiguous();
+}
+
+void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+
+Tensor cotangent(const Tensor& g, const Tensor& like) {
+  return g.defined() ? g.contiguous() : at::zeros_like(like, at::MemoryFormat::Contiguous);
+}
+
+bool wants_grad(const Tensor& x, const Tensor& xa, const variable_list& ws) {
+  if (!at::GradMode::is_enabled()) return false;
+  if (x.requires_grad() || xa.requires_grad()) return true;
+  for (const Tensor& w : ws)
+    if (w.requires_grad()) return true;
+  return false;
+}
+
+struct NcnNode : public Node {
+  at::IntArrayRef shape() const { return shape_; }
+  std::vector<int64_t> shape_;          // [B, N, E]
+  at::TensorOptions options_;           // of the activations
+  std::vector<std::vector<int64_t>> wshape_;
+  std::vector<at::TensorOptions> wopt_;  // of the weights as the caller holds them
+
+  void attach(const Tensor& x, const Tensor& xa, const variable_list& ws) {
+    edge_list e;
+    e.reserve(2 + ws.size());
+    e.push_back(torch::autograd::impl::gradient_edge(x));
+    e.push_back(torch::autograd::impl::gradient_edge(xa));
+    for (const Tensor& w : ws) {
+      e.push_back(torch::autograd::impl::gradient_edge(w));
+      wshape_.push_back(w.sizes().vec());
+      wopt_.push_back(w.options());
+    }
+    set_next_edges(std::move(e));
+    shape_ = x.sizes().vec();
+    options_ = x.options();
+  }
+  // the caller's cotangents, zeros where none arrived
+  void incoming(const variable_list& g, Tensor& dy, Tensor& dya) const {
+    const Tensor& any = g[0].defined() ? g[0] : g[1];
+    if (any.defined()) {
+      dy = cotangent(g[0], any);
+      dya = cotangent(g[1], any);
+    } else {
+      dy = at::zeros(shape_, options_);
+      dya = at::zeros(shape_, options_);
+    }
+  }
+  // The gradient of weight k, `offset` floats into the buffer of all of them.  A tensor over the same storage, put
+  // together by hand: narrow + view cost 4 us for each weight in the engine's thread.
+  Tensor weight_grad(const Tensor& all, int64_t offset, size_t k) const {
+    Tensor g = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(all.storage()), all.key_set(), all.dtype());
+    g.unsafeGetTensorImpl()->set_storage_offset(offset);
+    g.unsafeGetTensorImpl()->set_sizes_contiguous(wshape_[k]);
+    if (wopt_[k].dtype() != at::kFloat || wopt_[k].device() != all.device())
+      g = g.to(wopt_[k].device(), c10::typeMetaToScalarType(wopt_[k].dtype()));
+    return g;
+  }
+};
+
+
+// ---------------------------------------------------------------- fused nets
+// `layers` nets of L stages each (more than one only as residual layers), every net one kernel per direction.
+struct FusedCfg {
+  double alpha;
+  int act, n, C, first, L, layers, every, dt;
+  bool recompute, residual, tape;
+  int flags() const { return (residual ? NCN_RESIDUAL : 0) | (recompute ? NCN_RECOMPUTE : 0) | (tape ? NCN_TAPE : 0); }
+};
+
+struct FusedNode : public NcnNode {
+  FusedCfg c{};
+  bool gathered = false;                       // W was put together from one tensor per stage
+  SavedVariable W;                             // [layers, L, 2E]
+  std::vector<SavedVariable> s0, s1, ckpt;     // per layer: what the backward starts from, stored states
+
+  std::string name() const override { return "NCNNetBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    W.reset_data();
+    for (auto* v : {&s0, &s1, &ckpt})
+      for (SavedVariable& t : *v) t.reset_data();
+  }
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    at::NoGradGuard no_grad;
+    Tensor dy, dya;
+    incoming(g, dy, dya);
+    const c10::cuda::OptionalCUDAGuard guard(dy.device());
+    const int64_t B = shape_[0], N = shape_[1], E = shape_[2];
+    const Tensor w = plain_weights(W.unpack(), (int64_t)c.layers * c.L * 2 * E, dy.device());
+    const Tensor dW = at::empty({(int64_t)c.layers * c.L * 2 * E}, dy.options().dtype(at::kFloat));
+    const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, c.L, c.dt);
+    const Tensor ws = at::empty({(int64_t)ws_bytes}, dy.options().dtype(at::kByte));
+    void* const st = stream_of(dy);
+    for (int k = c.layers - 1; k >= 0; --k) {
+      Tensor a, b, ck;
+      if (!c.tape) {
+        // the only layer whose saved tensors can be the node's own outputs is the last one
+        const bool own = !c.recompute && k == c.layers - 1;
+        a = own ? s0[k].unpack(shared_from_this()) : s0[k].unpack();
+        b = own ? s1[k].unpack(shared_from_this()) : s1[k].unpack();
+      }
+      if (!ckpt.empty()) ck = ckpt[k].unpack();
+      Tensor dx = at::empty(shape_, options_), dxa = at::empty(shape_, options_);
+      check_status("ncn_net_bwd",
+                   ncn_net_bwd(a.defined() ? a.data_ptr() : nullptr, b.defined() ? b.data_ptr() : nullptr, dy.data_ptr(),
+                               dya.data_ptr(), w.const_data_ptr<float>() + (int64_t)k * c.L * 2 * E, dx.data_ptr(),
+                               dxa.data_ptr(), nullptr, nullptr, dW.mutable_data_ptr<float>() + (int64_t)k * c.L * 2 * E,
+                               ck.defined() ? ck.const_data_ptr<float>() : nullptr, c.every, ws.data_ptr(), ws_bytes, B, N, E,
+                               c.n, c.C, c.first, c.L, c.alpha, c.act, c.dt, c.flags(), 0, st));
+      dy = std::move(dx);
+      dya = std::move(dxa);
+    }
+    variable_list out;
+    out.reserve(num_outputs());
+    out.push_back(std::move(dy));
+    out.push_back(std::move(dya));
+    if (!gathered) {
+      out.push_back(weight_grad(dW, 0, 0));
+    } else {
+      for (size_t l = 0; l < wshape_.size(); ++l) out.push_back(weight_grad(dW, (int64_t)l * 2 * E, l));
+    }
+    return out;
+  }
+};
+
+// All stages' weights in one buffer, by one launch for up to 32 of them.
+Tensor gather_weights(const variable_list& ws, int64_t E, const Tensor& x) {
+  const int64_t L = (int64_t)ws.size();
+  Tensor W = at::empty({L * 2 * E}, x.options().dtype(at::kFloat));
+  std::vector<Tensor> keep;
+  std::vector<const float*> ptr;
+  keep.reserve(L);
+  ptr.reserve(L);
+  for (const Tensor& w : ws) {
+    keep.push_back(plain_weights(w, 2 * E, x.device()));
+    ptr.push_back(keep.back().const_data_ptr<float>());
+  }
+  check_status("ncn_gather_weights", ncn_gather_weights(ptr.data(), (int)L, 2 * E, W.mutable_data_ptr<float>(), stream_of(x)));
+  return W;
+}
+
+std::tuple<Tensor, Tensor> fused_forward(const Tensor& x_in, const Tensor& xa_in, const variable_list& ws, bool gathered,
+                                         FusedCfg c) {
+  const bool grad = wants_grad(x_in, xa_in, ws);
+  const c10::cuda::OptionalCUDAGuard guard(x_in.device());
+  std::shared_ptr<FusedNode> node;
+  if (grad) {
+    node = std::shared_ptr<FusedNode>(new FusedNode(), torch::autograd::deleteNode);
+    node->attach(x_in, xa_in, ws);
+  }
+  Tensor y, ya;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor x = x_in.contiguous(), xa = xa_in.contiguous();
+    const int64_t B = x.size(0), N = x.size(1), E = x.size(2);
+    c.dt = dtype_code(x);
+    const Tensor W = gathered ? gather_weights(ws, E, x) : plain_weights(ws[0], (int64_t)c.layers * c.L * 2 * E, x.device());
+    if (!grad) {  // nothing will be walked back: no states are stored
+      c.every = 0;
+      c.tape = c.recompute = false;
+    }
+    const int flags = (c.residual ? NCN_RESIDUAL : 0) | (c.tape ? NCN_TAPE : 0);
+    const size_t ck_bytes = ncn_ckpt_bytes(B, N, E, c.L, c.every, flags);
+    void* const st = stream_of(x);
+    Tensor in = x, ina = xa;
+    for (int k = 0; k < c.layers; ++k) {
+      y = at::empty_like(x);
+      ya = at::empty_like(xa);
+      Tensor ck;
+      if (ck_bytes) ck = at::empty({(int64_t)(ck_bytes / 4)}, x.options().dtype(at::kFloat));
+      check_status("ncn_net_fwd",
+                   ncn_net_fwd(in.data_ptr(), ina.data_ptr(), W.const_data_ptr<float>() + (int64_t)k * c.L * 2 * E, y.data_ptr(),
+                               ya.data_ptr(), ck.defined() ? ck.mutable_data_ptr<float>() : nullptr, c.every, B, N, E, c.n, c.C,
+                               c.first, c.L, c.alpha, c.act, c.dt, flags, st));
+      if (grad) {
+        if (c.recompute) {
+          node->s0.emplace_back(k == 0 && x.is_same(x_in) ? x_in : in, false);
+          node->s1.emplace_back(k == 0 && xa.is_same(xa_in) ? xa_in : ina, false);
+        } else if (!c.tape && k + 1 < c.layers) {
+          node->s0.emplace_back(y, false);
+          node->s1.emplace_back(ya, false);
+        }
+        if (ck.defined()) node->ckpt.emplace_back(ck, false);
+      }
+      in = y;
+      ina = ya;
+    }
+    if (grad) {
+      node->c = c;
+      node->gathered = gathered;
+      node->W = SavedVariable(!gathered && W.is_same(ws[0]) ? ws[0] : W, false);
+    }
+  }
+  if (grad) {
+    torch::autograd::set_history(y, node);
+    torch::autograd::set_history(ya, node);
+    if (!c.tape && !c.recompute) {
+      node->s0.emplace_back(y, true);
+      node->s1.emplace_back(ya, true);
+    }
+  }
+  return {y, ya};
+}
+
+// ---------------------------------------------------------------- chains of stages
+enum Keep : int { KEEP_OUTPUT = 0, KEEP_INPUT = 1, KEEP_MID = 2 };  // set_stage_backward in ncn_pytorch_wrapper_v2.py
+
+struct ChainCfg {
+  double alpha;
+  int act, n, C, first, L, keep, dt;
+};
+
+struct ChainNode : public NcnNode {
+  ChainCfg c{};
+  std::vector<SavedVariable> y, ya, mid, W;  // per stage
+  SavedVariable x0, xa0, ctxlen;
+  bool has_ctx = false;
+
+  std::string name() const override { return has_ctx ? "NCNContextBackward" : "NCNStagesBackward"; }
+  void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    for (auto* v : {&y, &ya, &mid, &W})
+      for (SavedVariable& t : *v) t.reset_data();
+    x0.reset_data();
+    xa0.reset_data();
+    ctxlen.reset_data();
+  }
+  variable_list apply(variable_list&& g) override {
+    std::lock_guard<std::mutex> lock(mutex_);
+    at::NoGradGuard no_grad;
+    Tensor dy, dya;
+    incoming(g, dy, dya);
+    const c10::cuda::OptionalCUDAGuard guard(dy.device());
+    const int64_t B = shape_[0], N = shape_[1], E = shape_[2];
+    const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, 1, c.dt);
+    const Tensor ws = at::empty({(int64_t)ws_bytes}, dy.options().dtype(at::kByte));
+    const Tensor dW = at::empty({(int64_t)c.L * 2 * E}, dy.options().dtype(at::kFloat));
+    const size_t mid_bytes = c.keep == KEEP_MID ? ncn_stage_mid_bytes(B, N, E, c.n, c.dt) : 0;
+    const Tensor cl = has_ctx ? ctxlen.unpack() : Tensor();
+    void* const st = stream_of(dy);
+    auto out_of = [&](std::vector<SavedVariable>& v, int l) {
+      return l == c.L - 1 ? v[l].unpack(shared_from_this()) : v[l].unpack();
+    };
+    for (int l = c.L - 1; l >= 0; --l) {
+      const Tensor w = plain_weights(W[l].unpack(), 2 * E, dy.device());
+      const Tensor yl = out_of(y, l), yal = out_of(ya, l);
+      Tensor dx = at::empty(shape_, options_), dxa = at::empty(shape_, options_);
+      float* const dwl = dW.mutable_data_ptr<float>() + (int64_t)l * 2 * E;
+      const float* const wp = w.const_data_ptr<float>();
+      const int module_l = c.first + l;
+      if (has_ctx) {
+        check_status("ncn_stage_bwd_ctx",
+                     ncn_stage_bwd_ctx(yl.data_ptr(), yal.data_ptr(), dy.data_ptr(), dya.data_ptr(), wp, cl.const_data_ptr<int>(),
+                                       dx.data_ptr(), dxa.data_ptr(), nullptr, nullptr, dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n,
+                                       c.C, module_l, c.alpha, c.act, c.dt, st));
+      } else if (c.keep == KEEP_INPUT) {
+        const Tensor xl = l == 0 ? x0.unpack() : y[l - 1].unpack(), xal = l == 0 ? xa0.unpack() : ya[l - 1].unpack();
+        const Tensor xc = xl.contiguous(), xac = xal.contiguous();
+        check_status("ncn_stage_bwd_saved",
+                     ncn_stage_bwd_saved(xc.data_ptr(), xac.data_ptr(), yl.data_ptr(), yal.data_ptr(), dy.data_ptr(), dya.data_ptr(),
+                                         wp, dx.data_ptr(), dxa.data_ptr(), dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n, c.C,
+                                         module_l, c.alpha, c.act, c.dt, st));
+      } else if (mid_bytes) {
+        const Tensor m = mid[l].unpack();
+        check_status("ncn_stage_bwd_mid",
+                     ncn_stage_bwd_mid(yl.data_ptr(), yal.data_ptr(), m.data_ptr(), mid_bytes, dy.data_ptr(), dya.data_ptr(), wp,
+                                       dx.data_ptr(), dxa.data_ptr(), dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n, c.C, module_l,
+                                       c.alpha, c.act, c.dt, st));
+      } else {
+        check_status("ncn_stage_bwd",
+                     ncn_stage_bwd(yl.data_ptr(), yal.data_ptr(), dy.data_ptr(), dya.data_ptr(), wp, dx.data_ptr(), dxa.data_ptr(),
+                                   nullptr, nullptr, dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n, c.C, module_l, c.alpha, c.act,
+                                   c.dt, st));
+      }
+      dy = std::move(dx);
+      dya = std::move(dxa);
+    }
+    variable_list out;
+    out.reserve(num_outputs());
+    out.push_back(std::move(dy));
+    out.push_back(std::move(dya));
+    for (size_t l = 0; l < wshape_.size(); ++l) out.push_back(weight_grad(dW, (int64_t)l * 2 * E, l));
+    return out;
+  }
+};
+
+std::tuple<Tensor, Tensor> chain_forward(const Tensor& x_in, const Tensor& xa_in, const variable_list& ws, const Tensor& ctx_in,
+                                         ChainCfg c) {
+  const bool grad = wants_grad(x_in, xa_in, ws);
+  const c10::cuda::OptionalCUDAGuard guard(x_in.device());
+  std::shared_ptr<ChainNode> node;
+  if (grad) {
+    node = std::shared_ptr<ChainNode>(new ChainNode(), torch::autograd::deleteNode);
+    node->attach(x_in, xa_in, ws);
+  }
+  Tensor y, ya;
+  {
+    at::AutoDispatchBelowADInplaceOrView below;
+    const Tensor x = x_in.contiguous(), xa = xa_in.contiguous();
+    const int64_t B = x.size(0), N = x.size(1), E = x.size(2);
+    c.dt = dtype_code(x);
+    Tensor ctx;
+    if (ctx_in.defined()) {
+      if (ctx_in.numel() != B)
+        throw py::value_error("ctxlen has " + std::to_string(ctx_in.numel()) + " entries for " + std::to_string(B) + " batch rows");
+      ctx = ctx_in.to(x.device(), at::kInt).contiguous();
+    }
+    const size_t mid_bytes = grad && !ctx.defined() && c.keep == KEEP_MID ? ncn_stage_mid_bytes(B, N, E, c.n, c.dt) : 0;
+    void* const st = stream_of(x);
+    Tensor in = x, ina = xa;
+    for (int l = 0; l < c.L; ++l) {
+      const Tensor w = plain_weights(ws[l], 2 * E, x.device());
+      const float* const wp = w.const_data_ptr<float>();
+      const int module_l = c.first + l;
+      y = at::empty_like(x);
+      ya = at::empty_like(xa);
+      if (ctx.defined()) {
+        check_status("ncn_stage_fwd_ctx",
+                     ncn_stage_fwd_ctx(in.data_ptr(), ina.data_ptr(), wp, ctx.const_data_ptr<int>(), y.data_ptr(), ya.data_ptr(), B,
+                                       N, E, c.n, c.C, module_l, c.alpha, c.act, c.dt, st));
+      } else if (mid_bytes) {
+        Tensor m = at::empty({(int64_t)(mid_bytes / 4)}, x.options().dtype(at::kFloat));
+        check_status("ncn_stage_fwd_mid",
+                     ncn_stage_fwd_mid(in.data_ptr(), ina.data_ptr(), wp, y.data_ptr(), ya.data_ptr(), m.data_ptr(), mid_bytes, B, N,
+                                       E, c.n, c.C, module_l, c.alpha, c.act, c.dt, st));
+        node->mid.emplace_back(m, false);
+      } else {
+        check_status("ncn_stage_fwd", ncn_stage_fwd(in.data_ptr(), ina.data_ptr(), wp, y.data_ptr(), ya.data_ptr(), B, N, E, c.n,
+                                                    c.C, module_l, c.alpha, c.act, c.dt, st));
+      }
+      if (grad) {
+        node->W.emplace_back(w.is_same(ws[l]) ? ws[l] : w, false);
+        if (l + 1 < c.L) {
+          node->y.emplace_back(y, false);
+          node->ya.emplace_back(ya, false);
+        }
+      }
+      in = y;
+      ina = ya;
+    }
+    if (grad) {
+      node->c = c;
+      if (c.keep == KEEP_INPUT) {
+        node->x0 = SavedVariable(x_in, false);
+        node->xa0 = SavedVariable(xa_in, false);
+      }
+      if (ctx.defined()) {
+        node->ctxlen = SavedVariable(ctx, false);
+        node->has_ctx = true;
+      }
+    }
+  }
+  if (grad) {
+    torch::autograd::set_history(y, node);
+    torch::autograd::set_history(ya, node);
+    node->y.emplace_back(y, true);
+    node->ya.emplace_back(ya, true);
+  }
+  return {y, ya};
+}
+
+// ---------------------------------------------------------------- Python entry points
+std::tuple<Tensor, Tensor> py_net(const Tensor& x, const Tensor& xa, const Tensor& W, double alpha, int act, int n, int C, int first,
+                                  int L, int layers, bool recompute, int every, bool tape, bool residual) {
+  check_activations(x, xa);
+  py::gil_scoped_release nogil;
+  return fused_forward(x, xa, {W}, false, FusedCfg{alpha, act, n, C, first, L, layers, every, 0, recompute, residual, tape});
+}
+
+std::tuple<Tensor, Tensor> py_stages(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
+                                     int first, int keep) {
+  check_activations(x, xa);
+  py::gil_scoped_release nogil;
+  return chain_forward(x, xa, ws, Tensor(), ChainCfg{alpha, act, n, C, first, (int)ws.size(), keep, 0});
+}
+
+std::tuple<Tensor, Tensor> py_stage_ctx(const Tensor& x, const Tensor& xa, const Tensor& W, const Tensor& ctxlen, double alpha, int act,
+                                        int n, int C, int module_l) {
+  check_activations(x, xa);
+  py::gil_scoped_release nogil;
+  return chain_forward(x, xa, {W}, ctxlen, ChainCfg{alpha, act, n, C, module_l, 1, KEEP_OUTPUT, 0});
+}
+
+// A net given as one weight tensor per stage: fused where the library covers the shape, else stage by stage.
+std::tuple<Tensor, Tensor> py_net_list(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
+                                       bool recompute, int every, bool tape, int keep) {
+  check_activations(x, xa);
+  py::gil_scoped_release nogil;
+  const int L = (int)ws.size();
+  bool fused = false;
+  if (act != 3) {  // leaky-relu has per-stage kernels only
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    const int flags = (recompute ? NCN_RECOMPUTE : 0) | (tape ? NCN_TAPE : 0);
+    fused = ncn_net_supported(x.size(0), x.size(1), x.size(2), n, C, L, dtype_code(x), flags, every) != 0;
+  }
+  if (fused) return fused_forward(x, xa, ws, true, FusedCfg{alpha, act, n, C, 0, L, 1, every, 0, recompute, false, tape});
+  return chain_forward(x, xa, ws, Tensor(), ChainCfg{alpha, act, n, C, 0, L, keep, 0});
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_ncn_torch, m) {
+  m.doc() = "autograd nodes of the NCN operators over the C ABI of libncn_b200.so";
+  m.def("net", &py_net);
+  m.def("net_list", &py_net_list);
+  m.def("stages", &py_stages);
+  m.def("stage_ctx", &py_stage_ctx);
+}

@@ -21,7 +21,7 @@ from typing import Sequence, Tuple
 import torch
 from torch import nn
 
-from . import ops
+from . import _lib, ops
 
 # Longest chain of steps rebuilt by the reversible inverse before the backward restarts from a
 # stored state.  Each inverse step grows earlier rounding by 1/0.9; 16 steps keep fp32
@@ -61,47 +61,21 @@ def stage_backward_plan(dtype, n_cache: int) -> str:
     return "mid" if dtype == torch.float32 else "input"
 
 
-class NCNFunction(torch.autograd.Function):
+_KEEP = {"output": 0, "input": 1, "mid": 2}  # enum Keep of csrc/ncn_torch.cpp
+
+
+class NCNFunction:
     """One stage (ncn_cuda/ncn_pytorch_wrapper_v2.py:9-50).  Saves the stage OUTPUT and rebuilds the
     input by the reversible inverse, as the reference does; for stages of more than
-    MAX_INVERSE_STEPS steps it keeps more (see set_stage_backward)."""
+    MAX_INVERSE_STEPS steps it keeps more (see set_stage_backward).  The autograd node is native
+    (csrc/ncn_torch.cpp)."""
 
     @staticmethod
-    def forward(ctx, x, xa, W, alpha, activation, n_cache, n_head, module_l):
-        ctx.keep = stage_backward_plan(x.dtype, n_cache)
-        if ctx.keep == "mid":
-            yi, ya, mid = ops.stage_fwd_mid(x, xa, W, alpha, activation, n_cache, n_head, module_l)
-            if mid is None:
-                ctx.keep = "output"
-                ctx.save_for_backward(yi, ya, W)
-            else:
-                ctx.save_for_backward(yi, ya, W, mid)
-        else:
-            yi, ya = ops.stage_fwd(x, xa, W, alpha, activation, n_cache, n_head, module_l)
-            if ctx.keep == "input":
-                ctx.save_for_backward(yi, ya, W, x, xa)
-            else:
-                ctx.save_for_backward(yi, ya, W)
-        ctx.alpha = alpha
-        ctx.activation = activation
-        ctx.n_cache = n_cache
-        ctx.n_head = n_head
-        ctx.module_l = module_l
-        return yi, ya
-
-    @staticmethod
-    def backward(ctx, dyi, dya):
-        cfg = (ctx.alpha, ctx.activation, ctx.n_cache, ctx.n_head, ctx.module_l)
-        if ctx.keep == "input":
-            (yi, ya, W, x, xa) = ctx.saved_tensors
-            dx, dxa, dW = ops.stage_bwd_saved(x, xa, yi, ya, dyi, dya, W, *cfg)
-        elif ctx.keep == "mid":
-            (yi, ya, W, mid) = ctx.saved_tensors
-            dx, dxa, dW = ops.stage_bwd_mid(yi, ya, mid, dyi, dya, W, *cfg)
-        else:
-            (yi, ya, W) = ctx.saved_tensors
-            dx, dxa, dW = ops.stage_bwd(yi, ya, dyi, dya, W, *cfg)
-        return dx, dxa, dW.to(W.dtype), None, None, None, None, None
+    def apply(x, xa, W, alpha, activation, n_cache, n_head, module_l):
+        keep = _KEEP[stage_backward_plan(x.dtype, n_cache)]
+        return _lib.native().stages(
+            x, xa, [W], alpha, ops.activation_code(activation), n_cache, n_head, module_l, keep
+        )
 
 
 def fused_ncn_cuda_v2(
@@ -118,24 +92,16 @@ def fused_ncn_cuda_v2(
     return yi, ya
 
 
-class NCNContextFunction(torch.autograd.Function):
+class NCNContextFunction:
     """One stage with a context length per batch row: the step-count rule of the reference's earlier
     Triton operator (ncn_triton/ncn_triton_old.py:285-359 `FusedLinearChunkNCNFunction`, kernels
     :52-124, :141-283) on the stage index map of torch_ref.  Saves the stage output, like NCNFunction."""
 
     @staticmethod
-    def forward(ctx, x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l):
-        yi, ya = ops.stage_fwd_ctx(x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l)
-        ctx.save_for_backward(yi, ya, W, torch.as_tensor(ctxlen).to(device=x.device, dtype=torch.int32))
-        ctx.cfg = (alpha, activation, n_cache, n_head, module_l)
-        return yi, ya
-
-    @staticmethod
-    def backward(ctx, dyi, dya):
-        yi, ya, W, ctxlen = ctx.saved_tensors
-        alpha, activation, n_cache, n_head, module_l = ctx.cfg
-        dx, dxa, dW = ops.stage_bwd_ctx(yi, ya, dyi, dya, W, ctxlen, alpha, activation, n_cache, n_head, module_l)
-        return dx, dxa, dW.to(W.dtype), None, None, None, None, None, None
+    def apply(x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l):
+        return _lib.native().stage_ctx(
+            x, xa, W, torch.as_tensor(ctxlen), alpha, ops.activation_code(activation), n_cache, n_head, module_l
+        )
 
 
 def fused_ncn_cuda_ctxlen(x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l):
@@ -179,40 +145,17 @@ def plan_backward(dtype, n_cache: int, num_modules: int, residual: bool, backwar
     return False, (every if num_modules > every else 0), tape
 
 
-class NCNNetFunction(torch.autograd.Function):
-    """All stages of a net in one forward and one backward kernel.  W: [L, 2E]."""
+class NCNNetFunction:
+    """All stages of a net in one forward and one backward kernel.  W: [L, 2E].  The autograd node is
+    native (csrc/ncn_torch.cpp); it keeps what plan_backward says, and nothing where no gradient is asked for."""
 
     @staticmethod
-    def forward(ctx, x, xa, W, alpha, activation, n_cache, n_head, first_module, backward_mode, residual):
+    def apply(x, xa, W, alpha, activation, n_cache, n_head, first_module, backward_mode, residual):
         recompute, every, tape = plan_backward(x.dtype, n_cache, W.shape[0], residual, backward_mode)
-        y, ya, ckpt = ops.net_fwd(x, xa, W, alpha, activation, n_cache, n_head, first_module, every, residual, tape)
-        # The stored states go through save_for_backward like the other saved tensors: autograd
-        # frees them after the backward and raises its usual error on a second backward without
-        # retain_graph, instead of a backward that silently finds no stored state.
-        if tape:
-            ctx.save_for_backward(W, ckpt)  # the stored states are all the backward reads
-        elif recompute:
-            ctx.save_for_backward(x, xa, W, ckpt)
-        else:
-            ctx.save_for_backward(y, ya, W, ckpt)
-        ctx.cfg = (alpha, activation, n_cache, n_head, first_module, every, recompute, residual, tape)
-        return y, ya
-
-    @staticmethod
-    def backward(ctx, dy, dya):
-        alpha, activation, n_cache, n_head, first_module, every, recompute, residual, tape = ctx.cfg
-        if tape:
-            W, ckpt = ctx.saved_tensors
-            s0 = s1 = None
-        else:
-            s0, s1, W, ckpt = ctx.saved_tensors
-        if ckpt is None and (tape or (every > 0 and not recompute and W.shape[0] > every)):
-            raise RuntimeError("the stored states of this net forward are gone; cannot run its backward")
-        dx, dxa, dW = ops.net_bwd(
-            s0, s1, dy, dya, W, alpha, activation, n_cache, n_head, first_module,
-            ckpt=ckpt, ckpt_every=every, recompute=recompute, residual=residual, tape=tape,
+        return _lib.native().net(
+            x, xa, W, alpha, ops.activation_code(activation), n_cache, n_head, first_module, W.shape[0], 1, recompute, every,
+            tape, residual,
         )
-        return dx, dxa, dW.to(W.dtype), None, None, None, None, None, None, None
 
 
 def fused_ncn_net(x, xa, W, alpha, activation, n_cache, n_head, first_module=0, backward_mode="auto", residual=False):
@@ -221,19 +164,16 @@ def fused_ncn_net(x, xa, W, alpha, activation, n_cache, n_head, first_module=0, 
 
 
 def _net_forward(x, xa, weights: Sequence[torch.Tensor], alpha, activation_nr, n_cache, n_head, backward_mode):
-    """Shared by the two net modules: fused when the library covers the shape, else stage by stage."""
+    """Shared by the net modules: one kernel per direction when the library covers the shape, else one per stage."""
     L = len(weights)
-    fused = False
-    if L > 0 and x.is_cuda and ops.activation_code(activation_nr) != ops.LEAKY_RELU:  # leaky-relu: per-stage kernels
+    if L == 0:
+        return x, xa
+    act = ops.activation_code(activation_nr)
+    recompute, every, tape = (False, 0, False)
+    if act != ops.LEAKY_RELU:  # leaky-relu: per-stage kernels
         recompute, every, tape = plan_backward(x.dtype, n_cache, L, False, backward_mode)
-        flags = (ops.NCN_RECOMPUTE if recompute else 0) | (ops.NCN_TAPE if tape else 0)
-        fused = ops.net_supported(x, n_cache, n_head, L, flags, every)
-    if fused:
-        W = torch.stack([w.reshape(-1) for w in weights])
-        return fused_ncn_net(x, xa, W, alpha, activation_nr, n_cache, n_head, 0, backward_mode)
-    for module_nr in range(L):
-        x, xa = fused_ncn_cuda_v2(x, xa, weights[module_nr], alpha, activation_nr, n_cache, n_head, module_nr)
-    return x, xa
+    keep = _KEEP[stage_backward_plan(x.dtype, n_cache)]
+    return _lib.native().net_list(x, xa, weights, alpha, act, n_cache, n_head, recompute, every, tape, keep)
 
 
 class NCNModuleCuda(nn.Module):

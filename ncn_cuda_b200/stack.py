@@ -12,8 +12,8 @@ import torch
 import torch.distributed as dist
 from torch import nn
 
-from . import ops
-from .ncn_pytorch_wrapper_v2 import fused_ncn_net
+from . import _lib, ops
+from .ncn_pytorch_wrapper_v2 import plan_backward
 
 
 class NCNResidualStack(nn.Module):
@@ -40,12 +40,14 @@ class NCNResidualStack(nn.Module):
         self.weight = nn.Parameter(torch.empty(num_layers, num_modules, 2 * embed_dim).normal_(0.0, std))
 
     def forward(self, x, xa):
-        for k in range(self.num_layers):
-            x, xa = fused_ncn_net(
-                x, xa, self.weight[k], self.alpha, self.activation_nr, self.n_cache, self.n_head, 0, self.backward_mode,
-                True
-            )
-        return x, xa
+        if self.num_layers == 0:
+            return x, xa
+        # every layer in one autograd node: no select / accumulate launches for the slices of the weight
+        recompute, every, tape = plan_backward(x.dtype, self.n_cache, self.num_modules, True, self.backward_mode)
+        return _lib.native().net(
+            x, xa, self.weight, self.alpha, self.activation_nr, self.n_cache, self.n_head, 0, self.num_modules,
+            self.num_layers, recompute, every, tape, True,
+        )
 
 
 def shard_rows(B: int, rank: int, world: int) -> Tuple[int, int]:

@@ -1,0 +1,103 @@
+"""The native autograd nodes: what autograd promises of any operator (one backward per graph, in-place checks, absent
+cotangents, other weight types) and the weight gather at the edges of its launches."""
+import pytest
+import torch
+
+from oracle import ncn_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ncn():
+    import ncn_cuda_b200 as m
+    return m
+
+
+def _case(kind, L):
+    # fused: one feature per position; chain: several features, stage by stage
+    B, N, E, C, n = (3, 64, 1, 1, 4) if kind == "fused" else (2, 64, 16, 2, 8)
+    x, xa, ws, dy, dya = O.make_inputs(11, B, N, E, L, 0.2, dya_zero=False)
+    net = (B, N, E, C, n)
+    return net, x, xa, ws, dy, dya
+
+
+def _run(ncn, case, train=True, wdtype=torch.float32):
+    (B, N, E, C, n), x, xa, ws, dy, dya = case
+    xd, xad = (t.cuda().requires_grad_(train) for t in (x, xa))
+    wd = [w.cuda().to(wdtype).requires_grad_(train) for w in ws]
+    net = ncn.NCNNetTestCuda(0.9, "tanh", n, C, len(ws), wd)
+    return xd, xad, wd, net, dy.cuda(), dya.cuda()
+
+
+@pytest.mark.parametrize("kind", ["fused", "chain"])
+@pytest.mark.parametrize("L", [1, 3, 33])  # 33: one more than a gather launch takes
+def test_against_oracle_and_without_gradients(ncn, kind, L):
+    case = _case(kind, L)
+    (B, N, E, C, n), x, xa, ws, dy, dya = case
+    xd, xad, wd, net, dyd, dyad = _run(ncn, case)
+    y, ya = net(xd, xad)
+    got = [y, ya, *torch.autograd.grad((y, ya), (xd, xad, *wd), (dyd, dyad))]
+    want = O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, "tanh", n, C)
+    # both sides round in every one of the n * L steps that a value passes, each by a few units of 2^-24 at most: a sum that
+    # grows at worst linearly in the steps, above 1e-5 from 42 steps on (the 132 steps of L = 33)
+    tol = max(1e-5, 4 * n * L * 2.0 ** -24)
+    for a, b in zip(got, [*want[:4], *want[4]]):
+        assert O.rel_err(a.detach(), b) < tol
+    with torch.no_grad():  # nothing stored, the same numbers
+        y2, ya2 = net(xd, xad)
+    assert not y2.requires_grad and torch.equal(y, y2) and torch.equal(ya, ya2)
+
+
+@pytest.mark.parametrize("kind", ["fused", "chain"])
+def test_autograd_semantics(ncn, kind):
+    case = _case(kind, 3)
+    xd, xad, wd, net, dyd, dyad = _run(ncn, case)
+    ins = (xd, xad, *wd)
+    y, ya = net(xd, xad)
+    # a cotangent that never arrives is zero
+    a = torch.autograd.grad(y, ins, dyd, retain_graph=True)
+    b = torch.autograd.grad((y, ya), ins, (dyd, torch.zeros_like(dyad)))
+    assert all(torch.equal(p, q) for p, q in zip(a, b))
+    with pytest.raises(RuntimeError, match="second time"):
+        torch.autograd.grad(y, ins, dyd)
+    # the backward starts from the output: changing it in place is noticed
+    y, ya = net(xd, xad)
+    y.data_ptr()
+    with torch.no_grad():
+        y.mul_(2.0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(y, ins, dyd)
+    # expanded cotangents and non-contiguous inputs
+    xt = xd.detach().transpose(0, 1).contiguous().transpose(0, 1).requires_grad_()
+    y, ya = net(xt, xad)
+    (y.sum() + ya.sum()).backward()
+    ref = torch.autograd.grad(net(xd, xad), (xd,), (torch.ones_like(y), torch.ones_like(y)))[0]
+    assert torch.equal(xt.grad, ref)
+
+
+def test_bf16_weights_get_bf16_gradients(ncn):
+    case = _case("fused", 3)
+    xd, xad, wd, net, dyd, dyad = _run(ncn, case, wdtype=torch.bfloat16)
+    y, ya = net(xd, xad)
+    g = torch.autograd.grad((y, ya), wd, (dyd, dyad))
+    net32 = ncn.NCNNetTestCuda(0.9, "tanh", 4, 1, 3, [w.detach().float().requires_grad_() for w in wd])
+    y, ya = net32(xd, xad)
+    g32 = torch.autograd.grad((y, ya), net32.weights, (dyd, dyad))
+    assert all(p.dtype == torch.bfloat16 and torch.equal(p, q.to(torch.bfloat16)) for p, q in zip(g, g32))
+
+
+def test_residual_stack_is_one_node_of_all_layers(ncn):
+    """Layer by layer (fused_ncn_net on slices of the weight) gives the same numbers."""
+    B, N, n, L, layers = 5, 1024, 4, 3, 3
+    x, xa, _, dy, dya = (t if not torch.is_tensor(t) else t.cuda() for t in O.make_inputs(12, B, N, 1, L, 0.25, dya_zero=False))
+    stack = ncn.NCNResidualStack(layers, 0.9, "tanh", n, 1, L, 1, w_std=0.5).cuda()
+    for mode in ("tape", "recompute"):
+        stack.backward_mode = mode
+        xs, xas = x.clone().requires_grad_(), xa.clone().requires_grad_()
+        one = torch.autograd.grad(stack(xs, xas), (xs, xas, stack.weight), (dy, dya))
+        y, ya = xs, xas
+        for k in range(layers):
+            y, ya = ncn.fused_ncn_net(y, ya, stack.weight[k], 0.9, 0, n, 1, 0, mode, True)
+        many = torch.autograd.grad((y, ya), (xs, xas, stack.weight), (dy, dya))
+        assert all(torch.equal(p, q) for p, q in zip(one, many))
