@@ -722,7 +722,7 @@ static void fill_stage(StageParams& p, int64_t B, int64_t N, int64_t E, int n, i
 }
 
 // ---- register-tiled multi-feature stage kernels (ncn_feat.cuh)
-typedef cudaError_t (*FeatLaunchFn)(int, int, int, const FeatParamsX&, int, int, cudaStream_t, int*);
+typedef cudaError_t (*FeatLaunchFn)(int, int, int, int, const FeatParams&, int, int, cudaStream_t, int*);
 
 static FeatLaunchFn feat_fn(int n, bool bwd) {
   switch (n) {
@@ -735,50 +735,44 @@ static FeatLaunchFn feat_fn(int n, bool bwd) {
   }
 }
 
-static FeatLaunchFn feat_mid_fn(int n) {
-  switch (n) {
-    case 16: return launch_feat_fwdm_n16;
-    case 32: return launch_feat_fwdm_n32;
-    default: return nullptr;
-  }
-}
-
-static FeatLaunchFn feat_saved_fn(int n) {
-  switch (n) {
-    case 16: return launch_feat_bwds_n16;
-    case 32: return launch_feat_bwds_n32;
-    default: return nullptr;
-  }
-}
-
 static long long gcd_ll(long long a, long long b) {
   while (b) { const long long t = a % b; a = b; b = t; }
   return a;
 }
 
+// What a launch needs beyond the tensors every stage has.
+struct FeatExtra {
+  const void* xin[2] = {nullptr, nullptr};  // saved stage input
+  int saved = 0;
+  float* mid = nullptr;
+  int mid_end = 0;
+  const int* ctxlen = nullptr;
+};
+
 // NCN_OK: launched.  NCN_ERR_UNSUPPORTED: no such kernel for these arguments (the caller falls
 // back to the shared-memory kernels); anything else is an error.
 static int launch_feat(bool bwd, const void* const* in, void* const* out, const float* W, float* partials, int64_t B,
                        int64_t N, int64_t E, int n, int C, int module_l, double alpha, int activation, int dtype,
-                       const DevInfo& dev, cudaStream_t st, int* grid_out, const void* x_saved = nullptr,
-                       const void* xa_saved = nullptr, int saved = 0, float* mid = nullptr, int mid_end = 0) {
+                       const DevInfo& dev, cudaStream_t st, int* grid_out, const FeatExtra& ex = FeatExtra()) {
   const int d = (int)(E / C);
-  const int gpw = feat_groups_per_warp(n, d);
-  FeatLaunchFn fn = saved ? feat_saved_fn(n) : (mid && !bwd) ? feat_mid_fn(n) : feat_fn(n, bwd);
-  if (saved && saved != 3 && (!aligned16(x_saved) || !aligned16(xa_saved))) return NCN_ERR_UNSUPPORTED;
-  if (mid && !aligned16(mid)) return NCN_ERR_UNSUPPORTED;
-  if (gpw == 0 || fn == nullptr || map_act(activation) == ACT_LEAKY) return NCN_ERR_UNSUPPORTED;
+  const int lanes = feat_lanes(d), rows = feat_rows(n, lanes);
+  const FeatLaunchFn fn = feat_fn(n, bwd);
+  if (fn == nullptr || rows == 0 || rows > kFeatMaxRows) return NCN_ERR_UNSUPPORTED;
+  if (n < 16 && (ex.saved || ex.mid)) return NCN_ERR_UNSUPPORTED;
+  // bf16 storage with context lengths: the exact tanh of the shared-memory kernels
+  if (ex.ctxlen && dtype != DT_F32) return NCN_ERR_UNSUPPORTED;
   if (env_switches().no_feat) return NCN_ERR_UNSUPPORTED;  // tuning experiments: force the shared-memory kernels
-  const int act = fused_act(map_act(activation), dtype);
-  for (int q = 0; q < (bwd ? 4 : 2); ++q)
-    if (!aligned16(in[q])) return NCN_ERR_UNSUPPORTED;  // (null, where a mode does not read a tensor, counts as aligned)
-  for (int q = 0; q < (bwd ? 4 : 2); ++q)
-    if (out[q] && !aligned16(out[q])) return NCN_ERR_UNSUPPORTED;
-  FeatParamsX p{};
+  const int act = feat_bf16_exact_tanh(n, d) ? map_act(activation) : fused_act(map_act(activation), dtype);
+  for (int q = 0; q < (bwd ? 4 : 2); ++q)  // (null, where a mode does not read or write a tensor, counts as aligned)
+    if (!aligned16(in[q]) || !aligned16(out[q])) return NCN_ERR_UNSUPPORTED;
+  if (!aligned16(ex.xin[0]) || !aligned16(ex.xin[1]) || !aligned16(ex.mid)) return NCN_ERR_UNSUPPORTED;
+  const int gpw = feat_groups_per_warp(n, lanes);
+  FeatParams p{};
   for (int q = 0; q < 4; ++q) { p.in[q] = in[q]; p.out[q] = out[q]; }
-  p.xin[0] = x_saved; p.xin[1] = xa_saved;
-  p.saved = saved;
-  p.mid = mid; p.mid_end = mid_end; p.bne = B * N * E;
+  p.xin[0] = ex.xin[0]; p.xin[1] = ex.xin[1];
+  p.saved = ex.saved;
+  p.mid = ex.mid; p.mid_end = ex.mid_end; p.bne = B * N * E;
+  p.ctxlen = ex.ctxlen;
   p.W = W;
   p.partials = partials;
   p.B = B; p.N = (int)N; p.E = (int)E; p.C = C;
@@ -788,40 +782,48 @@ static int launch_feat(bool bwd, const void* const* in, void* const* out, const 
   p.stride = stage_stride(module_l, p.m);
   p.alpha = (float)alpha;
   p.oma = (float)(1.0 - alpha);
-  // few groups (the reference's own bench has 128): smaller CTAs, so that the warps spread over all SMs
-  const long long want_warps = p.units * C;
-  int wpc = kFeatWarps;
-  while (wpc > 1 && want_warps < (long long)dev.sms * wpc) wpc /= 2;
-  const int threads = wpc * 32;
+  const long long want_teams = p.units * C;
+  const int team = feat_team(rows, bwd, want_teams, dev.sms);
+  // few groups (the reference's own bench has 128): smaller CTAs, so that the teams spread over all SMs
+  int tpc = kFeatWarps / team;
+  while (tpc > 1 && want_teams < (long long)dev.sms * tpc) tpc /= 2;
+  const int threads = tpc * team * 32;
   // resident CTAs per SM of this kernel: asked once per (kernel, device, CTA size)
-  struct Seen { FeatLaunchFn fn; int d, act, dtype, threads, dev, occ; };
+  struct Seen {
+    FeatLaunchFn fn;
+    int d, team, act, dtype, saved, ctx, threads, dev, occ;
+    bool same(const Seen& o) const {
+      return fn == o.fn && d == o.d && team == o.team && act == o.act && dtype == o.dtype && saved == o.saved && ctx == o.ctx &&
+             threads == o.threads && dev == o.dev;
+    }
+  };
   static std::mutex mu;
   static std::vector<Seen> seen;
-  int occ = -1;
+  Seen key{fn, d, team, act, dtype, p.saved, p.ctxlen != nullptr, threads, dev.dev, -1};
   {
     std::lock_guard<std::mutex> lk(mu);
     for (const Seen& q : seen)
-      if (q.fn == fn && q.d == d && q.act == act && q.dtype == dtype && q.threads == threads && q.dev == dev.dev) { occ = q.occ; break; }
+      if (q.same(key)) { key.occ = q.occ; break; }
   }
   cudaError_t e = cudaSuccess;
-  if (occ < 0) {
-    occ = 0;
-    e = fn(d, act, dtype, p, 0, threads, nullptr, &occ);
+  if (key.occ < 0) {
+    key.occ = 0;
+    e = fn(d, team, act, dtype, p, 0, threads, nullptr, &key.occ);
     if (e == cudaErrorNotSupported) return NCN_ERR_UNSUPPORTED;
     if (e != cudaSuccess) return cuda_fail(e);
     std::lock_guard<std::mutex> lk(mu);
     if (seen.size() >= 128) seen.clear();
-    seen.push_back(Seen{fn, d, act, dtype, threads, dev.dev, occ});
+    seen.push_back(key);
   }
-  if (occ < 1) return NCN_ERR_UNSUPPORTED;
-  if (occ > 32) occ = 32;
-  // one warp per (head, unit) at most, a whole number of warps per head
-  long long grid = (want_warps + wpc - 1) / wpc;
+  if (key.occ < 1) return NCN_ERR_UNSUPPORTED;
+  const int occ = key.occ > 32 ? 32 : key.occ;
+  // one team per (head, unit) at most, a whole number of teams per head
+  long long grid = (want_teams + tpc - 1) / tpc;
   if (grid > (long long)dev.sms * occ) grid = (long long)dev.sms * occ;
-  const long long q = C / gcd_ll(C, wpc);
+  const long long q = C / gcd_ll(C, tpc);
   grid = (grid + q - 1) / q * q;
   if (grid > (long long)dev.sms * 32) return NCN_ERR_UNSUPPORTED;  // more heads than the workspace covers
-  e = fn(d, act, dtype, p, (int)grid, threads, st, nullptr);
+  e = fn(d, team, act, dtype, p, (int)grid, threads, st, nullptr);
   if (e != cudaSuccess) return cuda_fail(e);
   if (grid_out) *grid_out = (int)grid;
   return NCN_OK;
@@ -1227,9 +1229,12 @@ int ncn_stage_bwd_saved(const void* x, const void* xa, const void* y, const void
   {
     const void* fin[4] = {replay_all ? nullptr : y, replay_all ? nullptr : ya, dy, dya};
     void* fout[4] = {dx, dxa, nullptr, nullptr};
+    FeatExtra ex;
+    ex.xin[0] = x; ex.xin[1] = xa;
+    ex.saved = replay_all ? 2 : 1;
     int fgrid = 0;
     rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
-                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, x, xa, replay_all ? 2 : 1);
+                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex);
     if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream);
     if (rc != NCN_ERR_UNSUPPORTED) return rc;
   }
@@ -1264,8 +1269,10 @@ int ncn_stage_fwd_mid(const void* x, const void* xa, const float* W, void* y, vo
   {
     const void* fin[4] = {x, xa, nullptr, nullptr};
     void* fout[4] = {y, ya, nullptr, nullptr};
+    FeatExtra ex;
+    ex.mid = static_cast<float*>(mid); ex.mid_end = mid_end;
     rc = launch_feat(false, fin, fout, W, nullptr, B, N, E, n_cache, n_head, module_l, alpha, activation, dtype, dev,
-                     (cudaStream_t)stream, nullptr, nullptr, nullptr, 0, static_cast<float*>(mid), mid_end);
+                     (cudaStream_t)stream, nullptr, ex);
     if (rc != NCN_ERR_UNSUPPORTED) return rc;
   }
   return stage_fwd_generic(x, xa, W, nullptr, y, ya, B, N, E, n_cache, n_head, module_l, alpha, activation, dtype, dev,
@@ -1294,10 +1301,12 @@ int ncn_stage_bwd_mid(const void* y, const void* ya, const void* mid, size_t mid
   {
     const void* fin[4] = {mid_end ? nullptr : y, mid_end ? nullptr : ya, dy, dya};
     void* fout[4] = {dx, dxa, nullptr, nullptr};
+    FeatExtra ex;
+    ex.saved = 3;
+    ex.mid = const_cast<float*>(static_cast<const float*>(mid)); ex.mid_end = mid_end;
     int fgrid = 0;
     rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
-                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, nullptr, nullptr, 3,
-                     const_cast<float*>(static_cast<const float*>(mid)), mid_end);
+                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex);
     if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream);
     if (rc != NCN_ERR_UNSUPPORTED) return rc;
   }
@@ -1315,6 +1324,15 @@ int ncn_stage_fwd_ctx(const void* x, const void* xa, const float* W, const int* 
   if (!x || !xa || !W || !ctxlen || !y || !ya) return NCN_ERR_NULL;
   DevInfo dev;
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
+  {
+    const void* fin[4] = {x, xa, nullptr, nullptr};
+    void* fout[4] = {y, ya, nullptr, nullptr};
+    FeatExtra ex;
+    ex.ctxlen = ctxlen;
+    rc = launch_feat(false, fin, fout, W, nullptr, B, N, E, n_cache, n_head, module_l, alpha, activation, dtype, dev,
+                     (cudaStream_t)stream, nullptr, ex);
+    if (rc != NCN_ERR_UNSUPPORTED) return rc;
+  }
   return stage_fwd_generic(x, xa, W, ctxlen, y, ya, B, N, E, n_cache, n_head, module_l, alpha, activation, dtype, dev,
                            stream);
 }
@@ -1331,6 +1349,17 @@ int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void*
   DevInfo dev;
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
   if (!workspace || workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float)) return NCN_ERR_WORKSPACE;
+  {
+    const void* fin[4] = {y, ya, dy, dya};
+    void* fout[4] = {dx, dxa, x_rec, xa_rec};
+    FeatExtra ex;
+    ex.ctxlen = ctxlen;
+    int fgrid = 0;
+    rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
+                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex);
+    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream);
+    if (rc != NCN_ERR_UNSUPPORTED) return rc;
+  }
   return stage_bwd_generic(y, ya, dy, dya, W, ctxlen, dx, dxa, x_rec, xa_rec, dW, static_cast<float*>(workspace), B, N, E,
                            n_cache, n_head, module_l, alpha, activation, dtype, dev, stream);
 }

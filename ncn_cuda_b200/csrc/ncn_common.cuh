@@ -39,7 +39,7 @@ constexpr float kCoverM = 0.1f / 0.9f;
 
 // ACT_TANH_FAST is internal: tanh through the one-instruction tanh.approx.f32 (relative error 2^-11),
 // used for bf16 storage, whose 2e-2 tolerance it does not threaten; it halves the special-function work.
-// ACT_LEAKY runs on the shared-memory stage kernels only (ncn_generic.cuh).
+// ACT_LEAKY runs on the per-stage kernels only (ncn_feat.cuh, ncn_generic.cuh).
 enum Act : int { ACT_TANH = 0, ACT_RELU = 1, ACT_SIGMOID = 2, ACT_LINEAR = 3, ACT_TANH_FAST = 4, ACT_LEAKY = 5 };
 enum DType : int { DT_F32 = 0, DT_BF16 = 1 };
 
@@ -340,6 +340,16 @@ struct ActForm<ACT_RELU> {
   }
 };
 template <>
+struct ActForm<ACT_LEAKY> {
+  static constexpr double sT = 1.0, f0 = 0.0, f1 = 1.0, ds = 1.0;
+  static __device__ __forceinline__ float2 r(float2 ts) {
+    return make_float2(act_fwd<ACT_LEAKY>(ts.x), act_fwd<ACT_LEAKY>(ts.y));
+  }
+  static __device__ __forceinline__ float2 gt(float2 g, float2 ts, float2) {
+    return make_float2(ts.x >= 0.0f ? g.x : 0.01f * g.x, ts.y >= 0.0f ? g.y : 0.01f * g.y);
+  }
+};
+template <>
 struct ActForm<ACT_LINEAR> {
   static constexpr double sT = 1.0, f0 = 0.0, f1 = 1.0, ds = 1.0;
   static __device__ __forceinline__ float2 r(float2 ts) { return ts; }
@@ -363,6 +373,14 @@ __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG
     if constexpr (BATCH == 1) {
 #pragma unroll
       for (int i = 0; i < NG; ++i) r[i] = make_float2(rcp_approx(d[i].x), rcp_approx(d[i].y));
+    } else if constexpr (NG == 3) {  // one reciprocal of the product of all three
+      const float2 P01 = __fmul2_rn(d[0], d[1]);
+      const float2 PP = __fmul2_rn(P01, d[2]);
+      const float2 R = make_float2(rcp_approx(PP.x), rcp_approx(PP.y));
+      const float2 i01 = __fmul2_rn(d[2], R);
+      r[2] = __fmul2_rn(P01, R);
+      r[0] = __fmul2_rn(d[1], i01);
+      r[1] = __fmul2_rn(d[0], i01);
     } else if constexpr (NG == 2 || BATCH == 2) {
 #pragma unroll
       for (int b = 0; b < NG; b += 2) {
@@ -420,6 +438,16 @@ constexpr double bwd_DX(int k, double f0) {
     CA -= kCd * f0 * cpow(kMd, i);
   }
   return DX;
+}
+
+// Steps group g of row b takes.  With per-row context lengths (the reference's earlier Triton kernels,
+// ncn_triton/ncn_triton_old.py:91-96, 189-192) a group counts its members g*n .. g*n+n-1 against the
+// row's length: groups that lie before it take all n steps, the group it cuts takes the steps of the
+// members before it, groups beyond it take none (their positions pass through unchanged).
+__device__ __forceinline__ int group_steps(const int* ctxlen, long long b, int g, int n) {
+  if (ctxlen == nullptr) return n;
+  const long long left = (long long)ctxlen[b] - (long long)g * n;
+  return left <= 0 ? 0 : (left < n ? (int)left : n);
 }
 
 // weights of one stage as the step code wants them

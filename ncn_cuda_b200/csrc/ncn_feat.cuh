@@ -7,28 +7,24 @@
 // torch_ref/ncn_pytorch.py:74-94 (step) and torch_ref/ncn_pytorch_invertible.py:97-111, 164-172
 // (inverse, gradient).
 //
-// One warp owns one group (or several small ones) for all its n_cache steps:
+// A TEAM of W warps owns one group (or, with W = 1, several small ones) for all its n_cache steps:
 //   lane = (slot, sub): LD = d / KF lanes share a position, each holding KF contiguous features;
-//   the 32 / LD slots of the warp hold the positions, P = n_cache * LD / 32 per lane (position
-//   i = r * SEG + s for slot s, r < P), or several groups side by side when n_cache < 32 / LD.
-// Per step the row x_j reaches every lane by KF shuffles, the dot products over the features are
-// lane-local sums plus log2(LD) exchanges, and no shared memory or barrier is involved.  The
-// kernels are bound by the special-function unit (two instructions per element and step for tanh)
-// like the one-feature kernels.
+//   the 32 / LD slots of a warp hold positions, P per lane; warp t of the team holds rows
+//   t P .. t P + P-1, and position i = row * SEG + slot.
+// Two things per step cross the lanes: the row x_j reaches everyone, and the backward's column sums
+// (one value per feature) reach the lanes of position j.  Within a warp x_j goes by shuffles; between
+// the warps of a team both go through a few hundred bytes of shared memory, double-buffered, behind ONE
+// team barrier per step: the column sums of a step are picked up after the barrier of the next one,
+// which is when H_j is needed first.
+//
+// What bounds them: with few groups (4 sequences = 128 groups of the reference's shape) the chain of
+// instructions of a step, which a team of four warps shortens (4 x 256 x 128, groups of 32: forward
+// 17.8 -> 13.4 us, backward 34 -> 22 us against one warp per group); with many groups the backward's four
+// streams of 1024 elements leave room for two warps per scheduler (issue slots half busy), and smaller
+// tiles per warp pay the step's shared part more often than their occupancy returns (see FeatTune).
 #pragma once
 #include "ncn_common.cuh"
-
-// Reciprocals of the tanh / sigmoid taken together over the feature pairs of a position (act_r_all,
-// ncn_common.cuh): 0 = one special-function reciprocal per value.
-#ifndef NCN_FEAT_FWD_BATCH
-#define NCN_FEAT_FWD_BATCH 4
-#endif
-#ifndef NCN_FEAT_BWD_BATCH
-#define NCN_FEAT_BWD_BATCH 0
-#endif
-#ifndef NCN_FEAT_UNROLL
-#define NCN_FEAT_UNROLL 1
-#endif
+#include "ncn_feat_launch.h"
 
 namespace ncn {
 
@@ -37,18 +33,14 @@ struct FeatParams {
   void* out[4];       // fwd: y, ya ; bwd: dx, dxa, x_rec|null, xa_rec|null
   const float* W;     // [2E]
   float* partials;    // bwd: [gridDim.x][2E]
+  const int* ctxlen;  // [B] context length per batch row, or null
   long long B;
   long long units;    // B * mg work units per head
-  int N, E, C, m, mg, stride;  // mg = ceil(m / groups per warp)
+  int N, E, C, m, mg, stride;  // mg = ceil(m / groups per team)
   float alpha, oma;
-};
-// Parameters of the kernels with a saved stage input or stored states.  A type of its own: the default kernels
-// keep the 128-byte FeatParams (with these fields inside it the default backward, which never reads them, ran
-// 4 % slower: the compiler's schedule at 249 registers is that easily disturbed).
-struct FeatParamsX : FeatParams {
   const void* xin[2]; // bwd with the stage input saved: x, xa
   float* mid;         // fp32 states after every 16th step: state k, stream s at mid + (2k + s) * bne, in the
-                      // element order of the activations (fwd with MID: written; bwd with saved == 3: read)
+                      // element order of the activations (fwd: written if not null; bwd with saved == 3: read)
   long long bne;      // elements per activation tensor
   int saved;          // bwd: 1 = the first half of the steps is replayed from the saved input; 2 = all steps are
                       // (y, ya are not read: bf16 storage); 3 = the states the forward stored in `mid` replace
@@ -56,20 +48,60 @@ struct FeatParamsX : FeatParams {
   int mid_end;        // the state after the LAST step is stored / read as well (bf16 storage: y, ya are not read)
 };
 
-template <int NC, int LD, int KF>
+template <int NC, int LD, int KF, int W>
 struct FeatGeom {
   static_assert(KF % 2 == 0 && 32 % LD == 0, "features are processed in pairs");
   static constexpr int D = LD * KF;
   static constexpr int SLOTS = 32 / LD;
-  static constexpr int P = NC >= SLOTS ? NC / SLOTS : 1;  // positions per lane
-  static constexpr int SEG = NC >= SLOTS ? SLOTS : NC;    // slots of one group
-  static constexpr int GPW = SLOTS / SEG;                 // groups per warp
+  static constexpr int ROWS = NC >= SLOTS ? NC / SLOTS : 1;  // rows of SLOTS positions in a group
+  static constexpr int P = ROWS / W;                         // positions per lane
+  static constexpr int SEG = NC >= SLOTS ? SLOTS : NC;       // slots of one group
+  static constexpr int GPW = SLOTS / SEG;                    // groups per warp (1 unless W = 1)
   static constexpr int KP = KF / 2;
-  static_assert(P * SEG == NC, "n_cache must be a power of two");
+  static constexpr int XS = GPW * D;                         // floats of one x_j buffer
+  static constexpr int TEAMS = kFeatWarps / W;
+  static_assert(ROWS * SEG == NC, "n_cache must be a power of two");
+  static_assert(P * W == ROWS && kFeatWarps % W == 0, "the team divides the rows");
 };
-constexpr int kFeatWarps = 8;  // warps per CTA
-constexpr int kFeatBwdUnroll = NCN_FEAT_UNROLL;  // backward step loop; 2 measured 10-40 % slower (register spills, code size)
+
+// CTAs per SM the register budget is set for, and the reciprocals of tanh / sigmoid that share one special-function
+// reciprocal (act_r_all, ncn_common.cuh; 0 = one each; the forward takes four).  Measured (us): backward of 1024 x 256 x
+// 128, groups of 32 (four rows per lane): two CTAs, batches of two 1064, single 1098; two rows per lane, three CTAs,
+// single 1125, two CTAs 1269, four CTAs (spills) 1592.  1024 x 512 x 256, groups of 16 (two rows): batches of two 2346,
+// single 2279; forward with three CTAs 1188, four 1136.  2048 x 256 x 128, groups of 8 (one row): backward with three CTAs
+// 766, four 702, five 950; forward with four CTAs 348, six 326.
+template <int P>
+struct FeatTune {
+  static constexpr int fwd_blocks = P >= 4 ? 3 : P == 1 ? 6 : 4;
+  static constexpr int bwd_blocks = P >= 4 ? 2 : P == 1 ? 4 : 3;
+  static constexpr int bwd_batch = P >= 4 ? 2 : 0;
+};
+// One row per lane and few steps: the steps are unrolled, which makes the powers of the decay and the lane numbers
+// constants; per step they cost as much as an element otherwise (2048 x 256 x 128, groups of 8, heads of 8: forward 396
+// -> 377 us, backward 756 -> 706).  With several lanes per position the backward's body is too long for eight copies (heads
+// of 32: 755 us against 700).
+constexpr bool feat_unrolled(int n, int p, int w) { return p == 1 && w == 1 && n <= 8; }
+constexpr bool feat_bwd_unrolled(int n, int p, int w, int lanes) { return feat_unrolled(n, p, w) && (n <= 4 || lanes == 1); }
 constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
+
+// m^k and m^-k: x = m^k X in the forward, x = m^-k X in the reverse sweep (k steps done), so that the
+// decay of the two streams costs no instruction per element (as in ncn_common.cuh, but without the
+// constant offsets, whose cancellation would cost accuracy over 32 steps).
+struct FeatPowers {
+  float pos[33], neg[33];
+};
+constexpr FeatPowers feat_powers() {
+  FeatPowers t{};
+  double a = 1.0, b = 1.0;
+  for (int k = 0; k <= 32; ++k) {
+    t.pos[k] = (float)a;
+    t.neg[k] = (float)b;
+    a *= kMd;
+    b /= kMd;
+  }
+  return t;
+}
+static __constant__ FeatPowers kPow = feat_powers();
 
 __device__ __forceinline__ float2 shfl2(float2 v, int src) {
   return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
@@ -81,89 +113,260 @@ __device__ __forceinline__ float red_sub(float v) {
   for (int o = 1; o < LD; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
-// sum over the SEG slots of a group (lanes LD apart), every lane gets the result
-template <int LD, int SEG>
-__device__ __forceinline__ float red_slots(float v) {
-#pragma unroll
-  for (int o = LD; o < LD * SEG; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
 
+// KF contiguous features.  Rows of 6 (d = 24, 48) start on 8-byte (bf16: 4-byte) boundaries only.
 template <int KF, typename T>
 __device__ __forceinline__ void ld_feat(const T* p, float2 (&v)[KF / 2]) {
-  float t[KF];
-  ld_vec<KF>(p, t);
+  if constexpr (KF % 4 != 0) {
 #pragma unroll
-  for (int q = 0; q < KF / 2; ++q) v[q] = make_float2(t[2 * q], t[2 * q + 1]);
+    for (int q = 0; q < KF / 2; ++q) {
+      float t[2];
+      ld_vec<2>(p + 2 * q, t);
+      v[q] = make_float2(t[0], t[1]);
+    }
+  } else {
+    float t[KF];
+    ld_vec<KF>(p, t);
+#pragma unroll
+    for (int q = 0; q < KF / 2; ++q) v[q] = make_float2(t[2 * q], t[2 * q + 1]);
+  }
 }
 template <int KF, typename T>
 __device__ __forceinline__ void st_feat(T* p, const float2 (&v)[KF / 2]) {
-  float t[KF];
+  if constexpr (KF % 4 != 0) {
 #pragma unroll
-  for (int q = 0; q < KF / 2; ++q) { t[2 * q] = v[q].x; t[2 * q + 1] = v[q].y; }
-  st_vec<KF>(p, t);
+    for (int q = 0; q < KF / 2; ++q) {
+      const float t[2] = {v[q].x, v[q].y};
+      st_vec<2>(p + 2 * q, t);
+    }
+  } else {
+    float t[KF];
+#pragma unroll
+    for (int q = 0; q < KF / 2; ++q) { t[2 * q] = v[q].x; t[2 * q + 1] = v[q].y; }
+    st_vec<KF>(p, t);
+  }
+}
+template <int KF>
+__device__ __forceinline__ void st_feat_scaled(float* p, const float2 (&v)[KF / 2], float s) {
+  float2 t[KF / 2];
+#pragma unroll
+  for (int q = 0; q < KF / 2; ++q) t[q] = __fmul2_rn(v[q], f2(s));
+  st_feat<KF, float>(p, t);
 }
 
-// Work split shared by both directions: warp -> head c (fixed for the whole kernel, so the
-// weights and the weight-gradient sums of a lane stay in registers), units of that head.
-struct FeatWarp {
-  int c;
-  long long first, step;
+template <int W>
+__device__ __forceinline__ void team_sync(int team) {
+  if constexpr (W == 1) {
+    __syncwarp();
+  } else {
+    asm volatile("bar.sync %0, %1;" ::"r"(team + 1), "n"(W * 32) : "memory");
+  }
+}
+
+// Position of a thread in the work split shared by both directions.  A team serves one head for the
+// whole kernel, so the weights and the weight-gradient sums of a lane stay in registers.
+template <typename G, int LD, int W>
+struct FeatThread {
+  int lane, warp, team, wt;  // wt: warp of the team
+  int sub, gw, s;            // lane of the position, group of the warp, slot of the group
+  int c;                     // head
+  long long first, step;     // units
+  __device__ __forceinline__ explicit FeatThread(const FeatParams& p) {
+    lane = threadIdx.x & 31;
+    warp = threadIdx.x >> 5;
+    team = warp / W;
+    wt = warp - team * W;
+    sub = lane & (LD - 1);
+    const int slot = lane / LD;
+    gw = slot / G::SEG;
+    s = slot - gw * G::SEG;
+    const int tpc = (int)(blockDim.x >> 5) / W;
+    const long long gt = (long long)blockIdx.x * tpc + team;
+    const long long tt = (long long)gridDim.x * tpc;  // a multiple of C (launch plan)
+    c = (int)(gt % p.C);
+    first = gt / p.C;
+    step = tt / p.C;
+  }
+  __device__ __forceinline__ int pos(int r) const { return (wt * G::P + r) * G::SEG + s; }  // position of row r
+  // row index of step j inside a lane of the warp that owns it, -1 in the other warps of the team
+  __device__ __forceinline__ int local_row(int j) const {
+    const int row = j / G::SEG - wt * G::P;
+    return (unsigned)row < (unsigned)G::P ? row : -1;
+  }
 };
-__device__ __forceinline__ FeatWarp feat_warp(const FeatParams& p) {
-  const long long wg = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const long long tw = (long long)gridDim.x * (blockDim.x >> 5);  // a multiple of C (launch plan)
-  FeatWarp w;
-  w.c = (int)(wg % p.C);
-  w.first = wg / p.C;
-  w.step = tw / p.C;
-  return w;
+
+// r of the activation for the feature pairs of a position.  BATCH > 1: shared reciprocals.
+template <int ACT, int KP, int BATCH>
+__device__ __forceinline__ void feat_act(const float2 (&ts)[KP], float2 (&rr)[KP]) {
+  if constexpr (KP >= 2 && BATCH > 1) {
+    act_r_all<ACT, KP, BATCH>(ts, rr);
+  } else {
+#pragma unroll
+    for (int q = 0; q < KP; ++q) rr[q] = ActForm<ACT>::r(ts[q]);
+  }
+}
+
+// Shared-memory exchange of KF features.  Conditional accesses are single predicated instructions: written as
+// branches they split the step's basic block, and the scheduler could not overlap what lies on either side
+// (backward of a two-warp team 1195 -> 1126 us at 1024 x 256 x 128).
+__device__ __forceinline__ void sts_if(bool on, uint32_t a, float2 v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\t@p st.shared.v2.f32 [%0], {%1, %2};\n\t}" ::"r"(a), "f"(v.x), "f"(v.y), "r"((int)on)
+               : "memory");
+}
+__device__ __forceinline__ void sts_if(bool on, uint32_t a, float2 v, float2 w) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p st.shared.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"r"(a), "f"(v.x), "f"(v.y),
+               "f"(w.x), "f"(w.y), "r"((int)on)
+               : "memory");
+}
+__device__ __forceinline__ void sts_if(bool on, uint32_t a, float v) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p st.shared.f32 [%0], %1;\n\t}" ::"r"(a), "f"(v), "r"((int)on) : "memory");
+}
+template <int KF>
+__device__ __forceinline__ void sts_row_if(bool on, uint32_t a, const float2 (&v)[KF / 2]) {
+  if constexpr (KF % 4 == 0) {
+#pragma unroll
+    for (int q = 0; q < KF / 2; q += 2) sts_if(on, a + 8u * q, v[q], v[q + 1]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < KF / 2; ++q) sts_if(on, a + 8u * q, v[q]);
+  }
+}
+template <int KF>
+__device__ __forceinline__ void lds_row(uint32_t a, float2 (&v)[KF / 2]) {
+  if constexpr (KF % 4 == 0) {
+#pragma unroll
+    for (int q = 0; q < KF / 2; q += 2)
+      asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(v[q].x), "=f"(v[q].y), "=f"(v[q + 1].x), "=f"(v[q + 1].y)
+                   : "r"(a + 8u * q)
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int q = 0; q < KF / 2; ++q) asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v[q].x), "=f"(v[q].y) : "r"(a + 8u * q) : "memory");
+  }
+}
+template <int KF>
+__device__ __forceinline__ void lds_row_if(bool on, uint32_t a, float2 (&v)[KF / 2]) {  // v keeps its value where !on
+  if constexpr (KF % 4 == 0) {
+#pragma unroll
+    for (int q = 0; q < KF / 2; q += 2)
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %5, 0;\n\t@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+                   : "+f"(v[q].x), "+f"(v[q].y), "+f"(v[q + 1].x), "+f"(v[q + 1].y)
+                   : "r"(a + 8u * q), "r"((int)on)
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int q = 0; q < KF / 2; ++q)
+      asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %3, 0;\n\t@p ld.shared.v2.f32 {%0, %1}, [%2];\n\t}"
+                   : "+f"(v[q].x), "+f"(v[q].y)
+                   : "r"(a + 8u * q), "r"((int)on)
+                   : "memory");
+  }
+}
+
+// The lanes of position j hand its row to the team.
+template <int P, int KP, int KF>
+__device__ __forceinline__ void publish_row(uint32_t dst, const float2 (&X)[P][KP], int rj, bool mine) {
+  float2 v[KP];
+#pragma unroll
+  for (int q = 0; q < KP; ++q) {
+    v[q] = X[0][q];
+#pragma unroll
+    for (int r = 1; r < P; ++r)
+      if (rj == r) v[q] = X[r][q];
+  }
+  sts_row_if<KF>(mine, dst, v);
+}
+// The same as a branch: the forward is short of issue slots rather than of overlap, and the selects of four rows cost
+// more than the branch (1024 x 256 x 128, groups of 32: 540 against 571 us).
+template <int P, int KP, int KF>
+__device__ __forceinline__ void publish_row_branch(float* dst, const float2 (&X)[P][KP], int rj, bool mine) {
+  if (mine) {
+#pragma unroll
+    for (int r = 0; r < P; ++r)
+      if (rj == r) st_feat<KF, float>(dst, X[r]);
+  }
+}
+
+// One forward step (k = steps done, x = m^k X, a = m^k A): xj is the row of position j in the same scale.
+//   Ts = sT (alpha x_i + sim_i x_j) ;  A <- A + c m^-(k+1) F ;  X <- X + c A
+template <int LD, int KP, int P, int ACT, bool MASK>
+__device__ __forceinline__ void feat_forward_step(float2 (&X)[P][KP], float2 (&A)[P][KP], const float2 (&xj)[KP],
+                                                  const float2 (&Wi)[KP], const float2 (&Wj)[KP], float alpha, int k, bool on) {
+  using F = ActForm<ACT>;
+  constexpr float sT = (float)F::sT;
+  const float mk = kPow.pos[k], imk1 = kPow.neg[k + 1];
+  const float2 al = f2(alpha * sT * mk);
+  const float ss = sT * mk * mk;
+  const float2 c1 = f2((float)(kCd * F::f1) * imk1);
+  [[maybe_unused]] const float2 c0 = f2((float)(kCd * F::f0) * imk1);
+  float2 accj = f2(0.0f);
+#pragma unroll
+  for (int q = 0; q < KP; ++q) accj = __ffma2_rn(xj[q], Wj[q], accj);
+  const float cj = accj.x + accj.y;
+#pragma unroll
+  for (int r = 0; r < P; ++r) {
+    float2 acc = f2(0.0f);
+#pragma unroll
+    for (int q = 0; q < KP; ++q) acc = __ffma2_rn(X[r][q], Wi[q], acc);
+    const float2 sim = f2(red_sub<LD>(acc.x + acc.y + cj) * ss);
+    float2 ts[KP], rr[KP];
+#pragma unroll
+    for (int q = 0; q < KP; ++q) ts[q] = __ffma2_rn(sim, xj[q], __fmul2_rn(X[r][q], al));
+    feat_act<ACT, KP, 4>(ts, rr);
+    if (!MASK || on) {
+#pragma unroll
+      for (int q = 0; q < KP; ++q) {
+        if constexpr (F::f0 != 0.0) A[r][q] = __fadd2_rn(A[r][q], c0);
+        A[r][q] = __ffma2_rn(rr[q], c1, A[r][q]);
+        X[r][q] = __ffma2_rn(A[r][q], f2(kC), X[r][q]);
+      }
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------------------ forward
-// MID: the fp32 state after every 16th step is also written to p.mid, for a backward whose inverse
-// chains then never exceed 16 steps.
-template <int NC, int LD, int KF, int ACT, typename T, bool MID = false, typename PT = FeatParams>
-__global__ void __launch_bounds__(kFeatWarps * 32) feat_fwd_kernel(const PT p) {
-  using G = FeatGeom<NC, LD, KF>;
-  using F = ActForm<ACT>;
-  constexpr int P = G::P, SEG = G::SEG, KP = G::KP;
-  constexpr float sT = (float)F::sT;
-  constexpr float cf0 = (float)(kCd * F::f0), cf1 = (float)(kCd * F::f1);
-  const int lane = threadIdx.x & 31;
-  const int sub = lane & (LD - 1), slot = lane / LD;
-  const int gw = slot / SEG, s = slot - gw * SEG;
-  const FeatWarp fw = feat_warp(p);
+// p.mid: the fp32 state after every 16th step is also written, for a backward whose inverse chains then
+// never exceed 16 steps.  p.ctxlen: a group takes group_steps() steps; MASK where groups with different
+// numbers of steps share a warp.
+template <int NC, int LD, int KF, int W, int ACT, typename T, bool MASK>
+__global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF, W>::P>::fwd_blocks) feat_fwd_kernel(const FeatParams p) {
+  using G = FeatGeom<NC, LD, KF, W>;
+  constexpr int P = G::P, KP = G::KP, SEG = G::SEG;
+  __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
+  const FeatThread<G, LD, W> th(p);
   const T* gx = static_cast<const T*>(p.in[0]);
   const T* ga = static_cast<const T*>(p.in[1]);
   T* gy = static_cast<T*>(p.out[0]);
   T* gya = static_cast<T*>(p.out[1]);
+  float* const xrow = &xs[th.team][0][th.gw * G::D + th.sub * KF];
 
-  // this lane's weights, with (1 - alpha) and the activation's argument scale folded in
-  float2 Wi[KP], Wj[KP];
+  float2 Wi[KP], Wj[KP];  // (1 - alpha) folded in
   {
-    const float* wi = p.W + fw.c * G::D + sub * KF;
+    const float* wi = p.W + th.c * G::D + th.sub * KF;
     const float* wj = wi + p.E;
-    const float f = p.oma * sT;
 #pragma unroll
     for (int q = 0; q < KP; ++q) {
-      Wi[q] = make_float2(wi[2 * q] * f, wi[2 * q + 1] * f);
-      Wj[q] = make_float2(wj[2 * q] * f, wj[2 * q + 1] * f);
+      Wi[q] = make_float2(wi[2 * q] * p.oma, wi[2 * q + 1] * p.oma);
+      Wj[q] = make_float2(wj[2 * q] * p.oma, wj[2 * q + 1] * p.oma);
     }
   }
-  const float2 alpha_s = f2(p.alpha * sT);
+  int shift[P];  // (i * stride) mod m
+#pragma unroll
+  for (int r = 0; r < P; ++r) shift[r] = (int)((long long)th.pos(r) * p.stride % p.m);
+  int par = 0;
 
-  for (long long u = fw.first; u < p.units; u += fw.step) {
+  for (long long u = th.first; u < p.units; u += th.step) {
     const long long b = u / p.mg;
-    const int g = (int)(u - b * p.mg) * G::GPW + gw;
-    const bool valid = g < p.m;
+    const int g = (int)(u - b * p.mg) * G::GPW + th.gw;
+    const bool valid = G::GPW == 1 || g < p.m;
     float2 X[P][KP], A[P][KP];
     long long off[P];
 #pragma unroll
     for (int r = 0; r < P; ++r) {
-      const int i = r * SEG + s;
-      const int blk = (int)(((long long)g + (long long)i * p.stride) % p.m);
-      off[r] = ((b * p.N + (long long)blk * NC + i) * p.E) + fw.c * G::D + sub * KF;
+      int blk = g + shift[r];
+      if (blk >= p.m) blk -= p.m;
+      off[r] = ((b * p.N + (long long)blk * NC + th.pos(r)) * p.E) + th.c * G::D + th.sub * KF;
       if (valid) {
         ld_feat<KF, T>(gx + off[r], X[r]);
         ld_feat<KF, T>(ga + off[r], A[r]);
@@ -172,67 +375,59 @@ __global__ void __launch_bounds__(kFeatWarps * 32) feat_fwd_kernel(const PT p) {
         for (int q = 0; q < KP; ++q) X[r][q] = A[r][q] = f2(0.0f);
       }
     }
-    [[maybe_unused]] auto store_mid = [&](int done) {  // the state after `done` steps, for the backward (MID)
-      if constexpr (MID) {
-        if (valid) {
-          float* mx = p.mid + (long long)(2 * (done / 16 - 1)) * p.bne;
+    int steps = NC, tsteps = NC;  // of this lane's group, of the team
+    if (G::GPW == 1 || MASK) {
+      if (p.ctxlen != nullptr) {
+        steps = valid ? group_steps(p.ctxlen, b, g, NC) : 0;
+        tsteps = MASK ? (int)__reduce_max_sync(0xffffffffu, (unsigned)steps) : steps;
+      }
+    }
+    auto run_step = [&](int j) {
+      float2 xj[KP];
+      // x_j by shuffles where several lanes share a position (2048 x 256 x 128, groups of 8: 4 heads 334 against 342 us
+      // through shared memory; 16 heads, one lane per position, 420 against 387)
+      if constexpr (W == 1 && P == 1 && LD > 1) {
+        const int src = (th.gw * SEG + j) * LD + th.sub;
 #pragma unroll
-          for (int r = 0; r < P; ++r) {
-            st_feat<KF, float>(mx + off[r], X[r]);
-            st_feat<KF, float>(mx + p.bne + off[r], A[r]);
-          }
+        for (int q = 0; q < KP; ++q) xj[q] = shfl2(X[0][q], src);
+      } else {
+        const int rj = th.local_row(j);
+        float* const xb = xrow + par * G::XS;
+        par ^= 1;
+        publish_row_branch<P, KP, KF>(xb, X, rj, rj >= 0 && th.s == (j & (SEG - 1)));
+        team_sync<W>(th.team);
+        ld_feat<KF, float>(xb, xj);
+      }
+      feat_forward_step<LD, KP, P, ACT, MASK>(X, A, xj, Wi, Wj, p.alpha, j, j < steps);
+      if (NC >= 16 && p.mid != nullptr && ((j + 1) & 15) == 0 && (j + 1 < NC || p.mid_end) && valid) {
+        float* mx = p.mid + (long long)(2 * ((j + 1) / 16 - 1)) * p.bne;
+        const float sc = kPow.pos[j + 1];
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+          st_feat_scaled<KF>(mx + off[r], X[r], sc);
+          st_feat_scaled<KF>(mx + p.bne + off[r], A[r], sc);
         }
       }
     };
+    if constexpr (feat_unrolled(NC, P, W)) {
 #pragma unroll
-    for (int rj = 0; rj < P; ++rj) {
+      for (int j = 0; j < NC; ++j) {
+        if ((G::GPW == 1 || MASK) && j >= tsteps) break;
+        run_step(j);
+      }
+    } else {
 #pragma unroll 1
-      for (int sj = 0; sj < SEG; ++sj) {
-        const int src = (gw * SEG + sj) * LD + sub;
-        float2 xj[KP];
-        float2 accj = f2(0.0f);
-#pragma unroll
-        for (int q = 0; q < KP; ++q) {
-          xj[q] = shfl2(X[rj][q], src);
-          accj = __ffma2_rn(xj[q], Wj[q], accj);
-        }
-        const float cj = accj.x + accj.y;
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-          float2 acc = f2(0.0f);
-#pragma unroll
-          for (int q = 0; q < KP; ++q) acc = __ffma2_rn(X[r][q], Wi[q], acc);
-          const float2 sim = f2(red_sub<LD>(acc.x + acc.y + cj));  // sT (1-alpha)(x_i.Wi + x_j.Wj)
-          // the forward is bound by the special-function unit: the reciprocals of a position's feature
-          // pairs come from one reciprocal of their product
-          float2 ts[KP], rr[KP];
-#pragma unroll
-          for (int q = 0; q < KP; ++q) ts[q] = __ffma2_rn(sim, xj[q], __fmul2_rn(X[r][q], alpha_s));
-          if constexpr (KP >= 2 && NCN_FEAT_FWD_BATCH > 1) {
-            act_r_all<ACT, KP, NCN_FEAT_FWD_BATCH>(ts, rr);
-          } else {
-#pragma unroll
-            for (int q = 0; q < KP; ++q) rr[q] = F::r(ts[q]);
-          }
-#pragma unroll
-          for (int q = 0; q < KP; ++q) {
-            A[r][q] = __ffma2_rn(rr[q], f2(cf1), __ffma2_rn(A[r][q], f2(kM), f2(cf0)));
-            X[r][q] = __ffma2_rn(A[r][q], f2(kC), __fmul2_rn(X[r][q], f2(kM)));
-          }
-        }
-        if constexpr (MID && SEG > 16) {  // a boundary of 16 steps inside this run of SEG steps
-          const int done = rj * SEG + sj + 1;
-          if ((done & 15) == 0 && (done < NC || p.mid_end)) store_mid(done);
-        }
-      }
-      if constexpr (MID && SEG <= 16) {  // boundaries of 16 steps fall between two runs (rj is unrolled: known at compile time)
-        const int done = (rj + 1) * SEG;
-        if ((done & 15) == 0 && (done < NC || p.mid_end)) store_mid(done);
-      }
+      for (int j = 0; j < tsteps; ++j) run_step(j);
     }
     if (valid) {
+      const float2 sc = f2(kPow.pos[steps]);
 #pragma unroll
       for (int r = 0; r < P; ++r) {
+#pragma unroll
+        for (int q = 0; q < KP; ++q) {
+          X[r][q] = __fmul2_rn(X[r][q], sc);
+          A[r][q] = __fmul2_rn(A[r][q], sc);
+        }
         st_feat<KF, T>(gy + off[r], X[r]);
         st_feat<KF, T>(gya + off[r], A[r]);
       }
@@ -250,29 +445,32 @@ __global__ void __launch_bounds__(kFeatWarps * 32) feat_fwd_kernel(const PT p) {
 //     gx_i = m gy_i + alpha gT_i + gs_i Wi
 //     gx_j += Wj sum_i gs_i + sum_i sim_i gT_i          (position j in its role as x_j)
 //     dWi += sum_i gs_i x_i ;  dWj += (sum_i gs_i) x_j
+// With k inverse steps done x = m^-k X, a = m^-k A, gy = m^k H, ga = m^k Gv; in these variables the
+// step is (q = m^-(k+1), gT = c ds m^k gt)
+//     X <- X - c A ;  Ts = sT (alpha q X_i + q^2 (X_i.Wi + X_j.Wj) X_j) ;  A <- A - c m^k F
+//     Gv <- Gv + c H ;  g_i = (c ds / m) q gt_i.X_j ;  H_i <- H_i + (alpha c ds / m) gt_i + g_i Wi
+//     H_j += sum_i [ g_i Wj + (c ds / m) q (X_i.Wi + X_j.Wj) gt_i ] ;  dWi += g_i X_i ;  dWj += g_i X_j
 // The weight gradient is summed per lane over all its groups, then over the slots of the warp
 // (fixed shuffle tree), the warps of the CTA that serve the same head (warp order) and the CTAs
 // (dw_reduce_kernel): a fixed order for a given launch shape.
 //
-// SAVED: the caller also kept the stage INPUT.  Every inverse step grows earlier rounding by 1/m, so
-// a chain of NC = 32 steps from the output alone leaves the gradients at 1e-5 of their size; here
-// the state half way is rebuilt exactly by running the forward over the first NC/2 steps from the
+// REPLAY (saved = 1, 2): the caller also kept the stage INPUT.  Every inverse step grows earlier rounding
+// by 1/m, so a chain of NC = 32 steps from the output alone leaves the gradients at 1e-5 of their size;
+// here the state half way is rebuilt exactly by running the forward over the first NC/2 steps from the
 // input, so that no inverse chain is longer than NC/2 steps.  With bf16 storage (p.saved == 2) the
 // end state is replayed too: an inverse started from rounded outputs would amplify their rounding.
-template <int NC, int LD, int KF, int ACT, typename T, bool SAVED = false, typename PT = FeatParams>
-__global__ void __launch_bounds__(kFeatWarps * 32) feat_bwd_kernel(const PT p) {
-  using G = FeatGeom<NC, LD, KF>;
+template <int NC, int LD, int KF, int W, int ACT, typename T, bool REPLAY, bool MASK>
+__global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF, W>::P>::bwd_blocks) feat_bwd_kernel(const FeatParams p) {
+  using G = FeatGeom<NC, LD, KF, W>;
   using F = ActForm<ACT>;
   constexpr int P = G::P, SEG = G::SEG, KP = G::KP, D = G::D;
   constexpr float sT = (float)F::sT;
-  constexpr float cds = (float)(kCd * F::ds);                 // gT = cds * gt
-  constexpr float af0 = (float)(-kCd * F::f0 / kMd), af1 = (float)(-kCd * F::f1 / kMd);
-  constexpr float ff0 = (float)(kCd * F::f0), ff1 = (float)(kCd * F::f1);  // forward replay (SAVED)
+  constexpr float cdsm = (float)(kCd * F::ds / kMd);
+  constexpr bool COLS_SHFL = W == 1 && P == 1 && NC <= 4;  // (longer chains: 702 us by shared memory, 714 by shuffles)
+  __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
+  __shared__ __align__(16) float cs[G::TEAMS][2][W][G::XS];
   __shared__ float sdw[kFeatWarps][2][D];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int sub = lane & (LD - 1), slot = lane / LD;
-  const int gw = slot / SEG, s = slot - gw * SEG;
-  const FeatWarp fw = feat_warp(p);
+  const FeatThread<G, LD, W> th(p);
   const T* g_y = static_cast<const T*>(p.in[0]);
   const T* g_ya = static_cast<const T*>(p.in[1]);
   const T* g_dy = static_cast<const T*>(p.in[2]);
@@ -281,10 +479,24 @@ __global__ void __launch_bounds__(kFeatWarps * 32) feat_bwd_kernel(const PT p) {
   T* g_dxa = static_cast<T*>(p.out[1]);
   T* g_xr = static_cast<T*>(p.out[2]);
   T* g_xar = static_cast<T*>(p.out[3]);
+  const int frow = th.gw * D + th.sub * KF;
+  const uint32_t xrow = smem_u32(&xs[th.team][0][frow]);
+  const uint32_t crow = smem_u32(&cs[th.team][0][0][frow]);
+
+  // Column sums over the slots: halving exchange (each round a lane keeps one half of its values and
+  // receives the partner's sums for that half), then the remaining slots by plain exchanges.
+  constexpr int HALV = KF == 6 ? 1 : ilog2(KF);
+  constexpr int ROUNDS = HALV < ilog2(SEG) ? HALV : ilog2(SEG);
+  constexpr int LEFT = KF >> ROUNDS;  // values a lane still holds
+  int cfirst = 0;                     // the first of them
+#pragma unroll
+  for (int t = 0; t < ROUNDS; ++t) cfirst += ((th.s >> t) & 1) * (KF >> (t + 1));
+  const uint32_t ccol = crow + 4u * (uint32_t)(th.wt * G::XS + cfirst);
+  const bool cwriter = (th.s >> ROUNDS) == 0;
 
   float2 Wi[KP], Wj[KP];  // (1 - alpha) folded in
   {
-    const float* wi = p.W + fw.c * D + sub * KF;
+    const float* wi = p.W + th.c * D + th.sub * KF;
     const float* wj = wi + p.E;
 #pragma unroll
     for (int q = 0; q < KP; ++q) {
@@ -292,64 +504,60 @@ __global__ void __launch_bounds__(kFeatWarps * 32) feat_bwd_kernel(const PT p) {
       Wj[q] = make_float2(wj[2 * q] * p.oma, wj[2 * q + 1] * p.oma);
     }
   }
-  const float2 alpha_s = f2(p.alpha * sT);
-  const float2 alpha_g = f2(p.alpha * cds);
+  const float2 alpha_g = f2(p.alpha * cdsm);
+  int shift[P];  // (i * stride) mod m
+#pragma unroll
+  for (int r = 0; r < P; ++r) shift[r] = (int)((long long)th.pos(r) * p.stride % p.m);
   float2 dwi[KP], dwj[KP];  // without the factor (1 - alpha)
 #pragma unroll
   for (int q = 0; q < KP; ++q) dwi[q] = dwj[q] = f2(0.0f);
+  int par = 0;
 
-  for (long long u = fw.first; u < p.units; u += fw.step) {
+  for (long long u = th.first; u < p.units; u += th.step) {
     const long long b = u / p.mg;
-    const int g = (int)(u - b * p.mg) * G::GPW + gw;
-    const bool valid = g < p.m;
+    const int g = (int)(u - b * p.mg) * G::GPW + th.gw;
+    const bool valid = G::GPW == 1 || g < p.m;
     float2 X[P][KP], A[P][KP], H[P][KP], Gv[P][KP];
     long long off[P];
+    // (stored end state or full replay: y, ya are not read)
+    const bool from_output = !(REPLAY && p.saved == 2) && !(p.saved == 3 && p.mid_end);
 #pragma unroll
     for (int r = 0; r < P; ++r) {
-      const int i = r * SEG + s;
-      const int blk = (int)(((long long)g + (long long)i * p.stride) % p.m);
-      off[r] = ((b * p.N + (long long)blk * NC + i) * p.E) + fw.c * D + sub * KF;
+      int blk = g + shift[r];
+      if (blk >= p.m) blk -= p.m;
+      off[r] = ((b * p.N + (long long)blk * NC + th.pos(r)) * p.E) + th.c * D + th.sub * KF;
+#pragma unroll
+      for (int q = 0; q < KP; ++q) X[r][q] = A[r][q] = H[r][q] = Gv[r][q] = f2(0.0f);
       if (valid) {
-        bool from_output = true;  // (stored end state or full replay: y, ya are not read)
-        if constexpr (SAVED) from_output = !(p.saved == 2 || (p.saved == 3 && p.mid_end));
         if (from_output) {
           ld_feat<KF, T>(g_y + off[r], X[r]);
           ld_feat<KF, T>(g_ya + off[r], A[r]);
         }
         ld_feat<KF, T>(g_dy + off[r], H[r]);
         ld_feat<KF, T>(g_dya + off[r], Gv[r]);
-        if constexpr (SAVED) {
-          // the stored state is needed half a stage from now: towards L2 already (one lane per 128-byte line)
-          if (p.saved == 3 && (sub & (128 / (KF * 4) - 1)) == 0) {
-            const float* mx = p.mid + off[r];
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(mx));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(mx + p.bne));
-          }
+        // the stored state is needed half a stage from now: towards L2 already
+        if (NC > 16 && p.saved == 3 && (th.sub & 3) == 0) {
+          const float* mx = p.mid + off[r];
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(mx));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(mx + p.bne));
         }
-      } else {
-#pragma unroll
-        for (int q = 0; q < KP; ++q) X[r][q] = A[r][q] = H[r][q] = Gv[r][q] = f2(0.0f);
       }
     }
-    // SAVED: the steps go in two runs of NC / 2; what replaces the rebuilt state (stored by the forward, or replayed
-    // from the saved input) is dealt with between the runs, outside the step loop.  Otherwise one run of NC steps.
-    constexpr int RUN = SAVED ? NC / 2 : NC;
+    int steps = NC, tsteps = NC;  // of this lane's group, of the team
+    if (G::GPW == 1 || MASK) {
+      if (p.ctxlen != nullptr) {
+        steps = valid ? group_steps(p.ctxlen, b, g, NC) : 0;
+        tsteps = MASK ? (int)__reduce_max_sync(0xffffffffu, (unsigned)steps) : steps;
+      }
+    }
+    // The steps go in runs of RUN; what replaces the rebuilt state (stored by the forward, or replayed from
+    // the saved input) is dealt with between the runs, outside the step loop.  A run ends in true scale.
+    constexpr int RUN = REPLAY ? NC / 2 : NC > 16 ? 16 : NC;
 #pragma unroll 1
-    for (int j0 = NC - 1; j0 >= 0; j0 -= RUN) {
-      if constexpr (SAVED) {
-        const int j = j0;  // the state wanted is the one after step j0
-        if (p.saved == 3) {
-          // the state after step j as the forward stored it
-          if (((j + 1) & 15) == 0 && (j + 1 < NC || p.mid_end) && valid) {
-            const float* mx = p.mid + (long long)(2 * ((j + 1) / 16 - 1)) * p.bne;
-#pragma unroll
-            for (int r = 0; r < P; ++r) {
-              ld_feat<KF, float>(mx + off[r], X[r]);
-              ld_feat<KF, float>(mx + p.bne + off[r], A[r]);
-            }
-          }
-        } else if (j == NC / 2 - 1 || (j == NC - 1 && p.saved == 2)) {
-          // the state after step j, exactly: the forward over steps 0..j from the saved input
+    for (int j0 = tsteps - 1; j0 >= 0; j0 -= j0 % RUN + 1) {
+      if (REPLAY) {
+        if (j0 == NC / 2 - 1 || p.saved == 2) {
+          // the state after step j0, exactly: the forward over steps 0..j0 from the saved input
           const T* g_x = static_cast<const T*>(p.xin[0]);
           const T* g_xa = static_cast<const T*>(p.xin[1]);
           if (valid) {
@@ -360,147 +568,215 @@ __global__ void __launch_bounds__(kFeatWarps * 32) feat_bwd_kernel(const PT p) {
             }
           }
 #pragma unroll 1
-          for (int jf = 0; jf <= j; ++jf) {
-            const int rf = jf / SEG, sf = jf - rf * SEG;
-            const int srcf = (gw * SEG + sf) * LD + sub;
+          for (int jf = 0; jf <= j0; ++jf) {
+            const int rf = th.local_row(jf);
+            const uint32_t xb = xrow + 4u * (uint32_t)(par * G::XS);
+            par ^= 1;
+            publish_row<P, KP, KF>(xb, X, rf, rf >= 0 && th.s == (jf & (SEG - 1)));
+            team_sync<W>(th.team);
             float2 xf[KP];
-            float2 accf = f2(0.0f);
+            lds_row<KF>(xb, xf);
+            feat_forward_step<LD, KP, P, ACT, false>(X, A, xf, Wi, Wj, p.alpha, jf, true);
+          }
+          const float2 sc = f2(kPow.pos[j0 + 1]);
+#pragma unroll
+          for (int r = 0; r < P; ++r)
 #pragma unroll
             for (int q = 0; q < KP; ++q) {
-              float2 v = X[0][q];
-#pragma unroll
-              for (int r = 1; r < P; ++r)
-                if (rf == r) v = X[r][q];
-              xf[q] = shfl2(v, srcf);
-              accf = __ffma2_rn(xf[q], Wj[q], accf);
+              X[r][q] = __fmul2_rn(X[r][q], sc);
+              A[r][q] = __fmul2_rn(A[r][q], sc);
             }
-            const float cf = accf.x + accf.y;
+        }
+      } else if (NC >= 16 && p.saved == 3) {
+        // the state after step j0 as the forward stored it
+        if (((j0 + 1) & 15) == 0 && (j0 + 1 < NC || p.mid_end) && valid) {
+          const float* mx = p.mid + (long long)(2 * ((j0 + 1) / 16 - 1)) * p.bne;
 #pragma unroll
-            for (int r = 0; r < P; ++r) {
-              float2 acc = f2(0.0f);
-#pragma unroll
-              for (int q = 0; q < KP; ++q) acc = __ffma2_rn(X[r][q], Wi[q], acc);
-              const float2 sim_s = f2(red_sub<LD>(acc.x + acc.y + cf) * sT);
-#pragma unroll
-              for (int q = 0; q < KP; ++q) {
-                const float2 rr = F::r(__ffma2_rn(sim_s, xf[q], __fmul2_rn(X[r][q], alpha_s)));
-                A[r][q] = __ffma2_rn(rr, f2(ff1), __ffma2_rn(A[r][q], f2(kM), f2(ff0)));
-                X[r][q] = __ffma2_rn(A[r][q], f2(kC), __fmul2_rn(X[r][q], f2(kM)));
-              }
-            }
+          for (int r = 0; r < P; ++r) {
+            ld_feat<KF, float>(mx + off[r], X[r]);
+            ld_feat<KF, float>(mx + p.bne + off[r], A[r]);
           }
         }
       }
-#pragma unroll kFeatBwdUnroll
-    for (int j = j0; j > j0 - RUN; --j) {
-      // one body for every step: the row index of x_j inside a lane (rj) is a run-time value,
-      // resolved by selects, so that the code stays small enough for the instruction cache
-      const int rj = j / SEG, sj = j - rj * SEG;
-      const int src = (gw * SEG + sj) * LD + sub;
-      const bool is_j = (s == sj);
-      // the step's input x for every position, then the row x_j
+      const int jend = j0 - j0 % RUN;
+      // first step of this lane's group in the run (MASK: groups of a warp start at different steps)
+      const int jtop = MASK && steps - 1 < j0 ? steps - 1 : j0;
+      int rprev = -1;  // row and slot test of the step whose column sums are still in `cs`
+      bool sprev = false;
+      auto take_columns = [&]() {  // H_j += the team's column sums of the previous step (buffer par ^ 1)
+        const bool mine = rprev >= 0 && sprev;
+        const uint32_t cb = crow + 4u * (uint32_t)((par ^ 1) * W * G::XS);
+        float2 add[KP];
+#pragma unroll
+        for (int q = 0; q < KP; ++q) add[q] = f2(0.0f);
+        lds_row_if<KF>(mine, cb, add);
+#pragma unroll
+        for (int w = 1; w < W; ++w) {
+          float2 t[KP];
+#pragma unroll
+          for (int q = 0; q < KP; ++q) t[q] = f2(0.0f);
+          lds_row_if<KF>(mine, cb + 4u * (uint32_t)(w * G::XS), t);
+#pragma unroll
+          for (int q = 0; q < KP; ++q) add[q] = __fadd2_rn(add[q], t[q]);
+        }
+#pragma unroll
+        for (int r = 0; r < P; ++r)
+#pragma unroll
+          for (int q = 0; q < KP; ++q)
+            if (P == 1 || rprev == r) H[r][q] = __fadd2_rn(H[r][q], add[q]);
+      };
+      auto run_step = [&](int j, int kk) {  // kk steps of the run done
+        const bool on = !MASK || j <= jtop;
+        const int k = MASK ? (on ? jtop - j : 0) : kk;
+        const float mk = kPow.pos[k], iq = kPow.neg[k + 1];
+        if (on) {
+#pragma unroll
+          for (int r = 0; r < P; ++r)
+#pragma unroll
+            for (int q = 0; q < KP; ++q) X[r][q] = __ffma2_rn(A[r][q], f2(-kC), X[r][q]);
+        }
+        const int rj = th.local_row(j);
+        const bool sj = on && th.s == (j & (SEG - 1));
+        float2 xj[KP];
+        if constexpr (W == 1) {  // (shuffles: shorter than the way through shared memory)
+          if constexpr (!COLS_SHFL) {
+            team_sync<W>(th.team);
+            take_columns();
+          }
+          const int src = (th.gw * SEG + (j & (SEG - 1))) * LD + th.sub;
+#pragma unroll
+          for (int q = 0; q < KP; ++q) {
+            float2 v = X[0][q];
+#pragma unroll
+            for (int r = 1; r < P; ++r)
+              if (rj == r) v = X[r][q];
+            xj[q] = shfl2(v, src);
+          }
+        } else {
+          const uint32_t xb = xrow + 4u * (uint32_t)(par * G::XS);
+          publish_row<P, KP, KF>(xb, X, rj, rj >= 0 && th.s == (j & (SEG - 1)));
+          team_sync<W>(th.team);
+          take_columns();
+          lds_row<KF>(xb, xj);
+        }
+        float2 accj = f2(0.0f);
+#pragma unroll
+        for (int q = 0; q < KP; ++q) accj = __ffma2_rn(xj[q], Wj[q], accj);
+        const float cj = accj.x + accj.y;
+        const float2 al = f2(p.alpha * sT * iq);
+        const float ss = sT * iq * iq, sg = cdsm * iq;
+        const float2 a1 = f2((float)(-kCd * F::f1) * mk);
+        [[maybe_unused]] const float2 a0 = f2((float)(-kCd * F::f0) * mk);
+        float gs[P];
+        float2 uu[KP];  // sum_i sim_i gT_i of this lane's positions, per feature
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+          float2 acc = f2(0.0f);
+#pragma unroll
+          for (int q = 0; q < KP; ++q) acc = __ffma2_rn(X[r][q], Wi[q], acc);
+          const float sim = red_sub<LD>(acc.x + acc.y + cj);
+          const float2 sim_s = f2(sim * ss), simg = f2(sim * sg);
+          float2 ts[KP], rr[KP];
+#pragma unroll
+          for (int q = 0; q < KP; ++q) ts[q] = __ffma2_rn(sim_s, xj[q], __fmul2_rn(X[r][q], al));
+          feat_act<ACT, KP, FeatTune<P>::bwd_batch>(ts, rr);
+          float2 gacc = f2(0.0f);
+#pragma unroll
+          for (int q = 0; q < KP; ++q) {
+            const float2 gap = __ffma2_rn(f2(kC), H[r][q], Gv[r][q]);
+            const float2 gt = F::gt(gap, ts[q], rr[q]);
+            gacc = __ffma2_rn(gt, xj[q], gacc);
+            uu[q] = r == 0 ? __fmul2_rn(simg, gt) : __ffma2_rn(simg, gt, uu[q]);
+            if (on) {
+              if constexpr (F::f0 != 0.0) A[r][q] = __fadd2_rn(A[r][q], a0);
+              A[r][q] = __ffma2_rn(rr[q], a1, A[r][q]);
+              Gv[r][q] = gap;
+              H[r][q] = __ffma2_rn(gt, alpha_g, H[r][q]);  // gs_i Wi is added below
+            }
+          }
+          gs[r] = red_sub<LD>(gacc.x + gacc.y) * sg;
+        }
+        float sl = 0.0f;
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+          const float2 gsv = f2(gs[r]);
+          sl += gs[r];
+          if (on) {
+#pragma unroll
+            for (int q = 0; q < KP; ++q) {
+              H[r][q] = __ffma2_rn(gsv, Wi[q], H[r][q]);
+              dwi[q] = __ffma2_rn(gsv, X[r][q], dwi[q]);
+            }
+          }
+        }
+        float v[KF];
+#pragma unroll
+        for (int q = 0; q < KP; ++q) {
+          if (on) dwj[q] = __ffma2_rn(f2(sl), xj[q], dwj[q]);
+          const float2 t = __ffma2_rn(f2(sl), Wj[q], uu[q]);  // + sum_i gs_i Wj
+          v[2 * q] = t.x; v[2 * q + 1] = t.y;
+        }
+#pragma unroll
+        for (int t = 0; t < ROUNDS; ++t) {
+          const int half = KF >> (t + 1);
+          const bool up = ((th.s >> t) & 1) != 0;
+#pragma unroll
+          for (int i = 0; i < half; ++i) {
+            const float keep = up ? v[i + half] : v[i];
+            const float send = up ? v[i] : v[i + half];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, LD << t);
+          }
+        }
+#pragma unroll
+        for (int o = LD << ROUNDS; o < LD * SEG; o <<= 1)
+#pragma unroll
+          for (int i = 0; i < LEFT; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+        if constexpr (COLS_SHFL) {  // straight to the lanes of position j
+          const int base = th.lane - ((th.s & ((1 << ROUNDS) - 1)) * LD);
+          float col[KF];
+#pragma unroll
+          for (int f = 0; f < KF; ++f) {
+            int owner = 0;  // slot bits of the lane that ends up with feature f
+#pragma unroll
+            for (int t = 0; t < ROUNDS; ++t) owner |= ((f / (KF >> (t + 1))) & 1) << t;
+            col[f] = __shfl_sync(0xffffffffu, v[f % LEFT], base + owner * LD);
+          }
+#pragma unroll
+          for (int q = 0; q < KP; ++q)
+            if (sj) H[0][q] = __fadd2_rn(H[0][q], make_float2(col[2 * q], col[2 * q + 1]));
+        } else {
+#pragma unroll
+          for (int i = 0; i < LEFT; ++i) sts_if(cwriter, ccol + 4u * (uint32_t)(par * W * G::XS + i), v[i]);
+          rprev = rj;
+          sprev = sj;
+          par ^= 1;
+        }
+      };
+      if constexpr (feat_bwd_unrolled(NC, P, W, LD)) {
+#pragma unroll
+        for (int kk = 0; kk < NC; ++kk) {
+          if ((G::GPW == 1 || MASK) && kk > j0) break;
+          run_step(j0 - kk, kk);
+        }
+      } else {
+#pragma unroll 1
+        for (int j = j0; j >= jend; --j) run_step(j, j0 - j);
+      }
+      if constexpr (!COLS_SHFL) {
+        team_sync<W>(th.team);
+        take_columns();
+      }
+      // true scale: k steps done
+      const float2 up = f2(kPow.neg[jtop - jend + 1]), dn = f2(kPow.pos[jtop - jend + 1]);
 #pragma unroll
       for (int r = 0; r < P; ++r)
 #pragma unroll
-        for (int q = 0; q < KP; ++q) X[r][q] = __ffma2_rn(A[r][q], f2(-kCoverM), __fmul2_rn(X[r][q], f2(kInvM)));
-      float2 xj[KP];
-      float2 accj = f2(0.0f);
-#pragma unroll
-      for (int q = 0; q < KP; ++q) {
-        float2 v = X[0][q];
-#pragma unroll
-        for (int r = 1; r < P; ++r)
-          if (rj == r) v = X[r][q];
-        xj[q] = shfl2(v, src);
-        accj = __ffma2_rn(xj[q], Wj[q], accj);
-      }
-      const float cj = accj.x + accj.y;
-      float gs[P];
-      float u[KF];  // sum_i sim_i gT_i of this lane's positions, per feature
-#pragma unroll
-      for (int k = 0; k < KF; ++k) u[k] = 0.0f;
-#pragma unroll
-      for (int r = 0; r < P; ++r) {
-        float2 acc = f2(0.0f);
-#pragma unroll
-        for (int q = 0; q < KP; ++q) acc = __ffma2_rn(X[r][q], Wi[q], acc);
-        const float sim = red_sub<LD>(acc.x + acc.y + cj);
-        const float2 sim_s = f2(sim * sT), simg = f2(sim * cds);
-        float2 gacc = f2(0.0f);
-        float2 tsv[KP], rrv[KP];
-#pragma unroll
-        for (int q = 0; q < KP; ++q) tsv[q] = __ffma2_rn(sim_s, xj[q], __fmul2_rn(X[r][q], alpha_s));
-        if constexpr (KP >= 2 && NCN_FEAT_BWD_BATCH > 1) {
-          act_r_all<ACT, KP, NCN_FEAT_BWD_BATCH>(tsv, rrv);
-        } else {
-#pragma unroll
-          for (int q = 0; q < KP; ++q) rrv[q] = F::r(tsv[q]);
-        }
-#pragma unroll
         for (int q = 0; q < KP; ++q) {
-          const float2 ts = tsv[q];
-          const float2 rr = rrv[q];
-          A[r][q] = __ffma2_rn(rr, f2(af1), __ffma2_rn(A[r][q], f2(kInvM), f2(af0)));
-          const float2 gap = __ffma2_rn(f2(kC), H[r][q], Gv[r][q]);
-          const float2 gt = F::gt(gap, ts, rr);
-          Gv[r][q] = __fmul2_rn(gap, f2(kM));
-          H[r][q] = __ffma2_rn(gt, alpha_g, __fmul2_rn(H[r][q], f2(kM)));  // gs_i Wi is added below
-          gacc = __ffma2_rn(gt, xj[q], gacc);
-          const float2 uu = __ffma2_rn(simg, gt, make_float2(u[2 * q], u[2 * q + 1]));
-          u[2 * q] = uu.x; u[2 * q + 1] = uu.y;
+          X[r][q] = __fmul2_rn(X[r][q], up);
+          A[r][q] = __fmul2_rn(A[r][q], up);
+          H[r][q] = __fmul2_rn(H[r][q], dn);
+          Gv[r][q] = __fmul2_rn(Gv[r][q], dn);
         }
-        gs[r] = red_sub<LD>(gacc.x + gacc.y) * cds;  // gT_i . x_j
-      }
-      float sl = 0.0f;
-#pragma unroll
-      for (int r = 0; r < P; ++r) {
-        const float2 gsv = f2(gs[r]);
-        sl += gs[r];
-#pragma unroll
-        for (int q = 0; q < KP; ++q) {
-          H[r][q] = __ffma2_rn(gsv, Wi[q], H[r][q]);
-          dwi[q] = __ffma2_rn(gsv, X[r][q], dwi[q]);
-        }
-      }
-      const float S = red_slots<LD, SEG>(sl);
-      // column sums over the group's slots: halving exchange (each round a lane keeps one half of
-      // its values and receives the partner's sums for that half), then the owners hand every
-      // feature's total to the lanes of position j
-      constexpr int ROUNDS = (KF < SEG) ? ilog2(KF) : ilog2(SEG);
-      constexpr int LEFT = KF >> ROUNDS;  // values a lane still holds
-#pragma unroll
-      for (int t = 0; t < ROUNDS; ++t) {
-        const int half = KF >> (t + 1);
-        const bool up = ((s >> t) & 1) != 0;
-#pragma unroll
-        for (int i = 0; i < half; ++i) {
-          const float keep = up ? u[i + half] : u[i];
-          const float send = up ? u[i] : u[i + half];
-          u[i] = keep + __shfl_xor_sync(0xffffffffu, send, LD << t);
-        }
-      }
-      if constexpr (LEFT == 1) {
-#pragma unroll
-        for (int o = LD << ROUNDS; o < LD * SEG; o <<= 1) u[0] += __shfl_xor_sync(0xffffffffu, u[0], o);
-      }
-      const int base = lane - ((s & ((1 << ROUNDS) - 1)) * LD);
-      float col[KF];
-#pragma unroll
-      for (int f = 0; f < KF; ++f) {
-        int owner = 0;  // slot bits of the lane that ends up with feature f
-#pragma unroll
-        for (int t = 0; t < ROUNDS; ++t) owner |= ((f / (KF >> (t + 1))) & 1) << t;
-        col[f] = __shfl_sync(0xffffffffu, u[f % LEFT], base + owner * LD);
-      }
-#pragma unroll
-      for (int q = 0; q < KP; ++q) {
-        const float2 add = __ffma2_rn(f2(S), Wj[q], make_float2(col[2 * q], col[2 * q + 1]));
-#pragma unroll
-        for (int r = 0; r < P; ++r)
-          if (is_j && rj == r) H[r][q] = __fadd2_rn(H[r][q], add);
-        if (is_j) dwj[q] = __ffma2_rn(f2(S), xj[q], dwj[q]);
-      }
-    }
     }  // runs
     if (valid) {
 #pragma unroll
@@ -526,24 +802,24 @@ __global__ void __launch_bounds__(kFeatWarps * 32) feat_bwd_kernel(const PT p) {
       dwj[q].y += __shfl_xor_sync(0xffffffffu, dwj[q].y, o);
     }
   }
-  if (slot == 0) {
+  if (th.lane < LD) {
 #pragma unroll
     for (int q = 0; q < KP; ++q) {
-      sdw[warp][0][sub * KF + 2 * q] = dwi[q].x * p.oma;
-      sdw[warp][0][sub * KF + 2 * q + 1] = dwi[q].y * p.oma;
-      sdw[warp][1][sub * KF + 2 * q] = dwj[q].x * p.oma;
-      sdw[warp][1][sub * KF + 2 * q + 1] = dwj[q].y * p.oma;
+      sdw[th.warp][0][th.sub * KF + 2 * q] = dwi[q].x * p.oma;
+      sdw[th.warp][0][th.sub * KF + 2 * q + 1] = dwi[q].y * p.oma;
+      sdw[th.warp][1][th.sub * KF + 2 * q] = dwj[q].x * p.oma;
+      sdw[th.warp][1][th.sub * KF + 2 * q + 1] = dwj[q].y * p.oma;
     }
   }
   __syncthreads();
-  const int nwarp = blockDim.x >> 5;
+  const int nwarp = blockDim.x >> 5, tpc = nwarp / W;
   for (int idx = threadIdx.x; idx < 2 * p.E; idx += blockDim.x) {
     const int which = idx / p.E, f = idx - which * p.E;
     const int c = f / D, k = f - c * D;
     float acc = 0.0f;
     for (int w = 0; w < nwarp; ++w) {
-      const long long wg = (long long)blockIdx.x * nwarp + w;
-      if ((int)(wg % p.C) == c) acc += sdw[w][which][k];
+      const long long gt = (long long)blockIdx.x * tpc + w / W;
+      if ((int)(gt % p.C) == c) acc += sdw[w][which][k];
     }
     p.partials[(long long)blockIdx.x * 2 * p.E + idx] = acc;
   }

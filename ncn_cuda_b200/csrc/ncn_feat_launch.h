@@ -6,12 +6,15 @@
 
 namespace ncn {
 
-struct FeatParamsX;  // FeatParams plus what the kernels with a saved stage input or stored states take
+struct FeatParams;
 
-#define NCN_DECL(n)                                                                                          \
-  cudaError_t launch_feat_fwd_n##n(int d, int act, int dtype, const FeatParamsX& p, int grid, int threads,     \
-                                   cudaStream_t st, int* occ);                                                                 \
-  cudaError_t launch_feat_bwd_n##n(int d, int act, int dtype, const FeatParamsX& p, int grid, int threads,     \
+constexpr int kFeatWarps = 4;  // warps per CTA
+
+// team: warps per group (feat_team)
+#define NCN_DECL(n)                                                                                                   \
+  cudaError_t launch_feat_fwd_n##n(int d, int team, int act, int dtype, const FeatParams& p, int grid, int threads,   \
+                                   cudaStream_t st, int* occ);                                                        \
+  cudaError_t launch_feat_bwd_n##n(int d, int team, int act, int dtype, const FeatParams& p, int grid, int threads,   \
                                    cudaStream_t st, int* occ);
 NCN_DECL(2)
 NCN_DECL(4)
@@ -19,25 +22,46 @@ NCN_DECL(8)
 NCN_DECL(16)
 NCN_DECL(32)
 #undef NCN_DECL
-// the backward that also takes the saved stage input (inverse chains of n_cache / 2 steps)
-cudaError_t launch_feat_bwds_n16(int d, int act, int dtype, const FeatParamsX& p, int grid, int threads, cudaStream_t st,
-                                 int* occ);
-cudaError_t launch_feat_bwds_n32(int d, int act, int dtype, const FeatParamsX& p, int grid, int threads, cudaStream_t st,
-                                 int* occ);
-// the forward that also stores the state after every 16th step
-cudaError_t launch_feat_fwdm_n16(int d, int act, int dtype, const FeatParamsX& p, int grid, int threads, cudaStream_t st,
-                                 int* occ);
-cudaError_t launch_feat_fwdm_n32(int d, int act, int dtype, const FeatParamsX& p, int grid, int threads, cudaStream_t st,
-                                 int* occ);
 
-// groups a warp works on side by side for (n_cache, d); 0 if there is no kernel
-inline int feat_groups_per_warp(int n, int d) {
-  if (n != 2 && n != 4 && n != 8 && n != 16 && n != 32) return 0;
-  if (d != 2 && d != 4 && d != 8 && d != 16 && d != 32 && d != 64 && d != 128) return 0;
-  if (n * d > 1024) return 0;
-  const int ld = d <= 8 ? 1 : d / 8;
-  const int slots = 32 / ld;
-  return n >= slots ? 1 : slots / n;
+// lanes that share a position of d features (8 features per lane, 6 for 24 and 48); 0: no kernel
+constexpr int feat_lanes(int d) {
+  switch (d) {
+    case 2: case 4: case 8: return 1;
+    case 16: return 2;
+    case 24: case 32: return 4;
+    case 48: case 64: return 8;
+    case 128: return 16;
+    default: return 0;
+  }
+}
+// rows of 32 / lanes positions in a group of n; 0: no kernel
+constexpr int feat_rows(int n, int lanes) { return lanes == 0 ? 0 : n * lanes <= 32 ? 1 : n * lanes / 32; }
+// groups a warp works on side by side
+constexpr int feat_groups_per_warp(int n, int lanes) { return n * lanes >= 32 ? 1 : 32 / (n * lanes); }
+
+// bf16 storage: heads of 24 and 48 features and tiles of more than 1024 elements keep the exact tanh that the
+// shared-memory kernels take (dW 7e-7 off the fp64 result, 5e-6 with tanh.approx).
+constexpr bool feat_bf16_exact_tanh(int n, int d) { return d == 24 || d == 48 || n * d > 1024; }
+
+// Warps per group.  The widest share (four rows per lane, as few warps as that takes) does the least work per element:
+// the step's shared part is paid once per warp.  Larger teams shorten a step: taken while all groups' teams together
+// leave the SMs at no more than this many warps.  Measured (us, start = one warp per group always; 256 tokens of 128
+// features in 4 heads, groups of 32):  4 sequences forward 17.7 -> 13.4 (W = 4), backward 34.0 -> 21.8 (W = 4); 16
+// sequences forward 19.5 -> 18.0 (W = 4), backward W = 4 40.1, W = 2 32.5, W = 1 36.2; 32 sequences (14 warps per SM with
+// W = 2) backward W = 2 57, W = 1 50.
+constexpr int kFeatMaxRows = 8;
+constexpr int kFeatTeamFwd = 16, kFeatTeamBwd = 8;
+constexpr int feat_team_min(int rows) { return rows <= 4 ? 1 : rows / 4; }
+constexpr int feat_team_max(int rows) { return rows < kFeatWarps ? rows : kFeatWarps; }
+// team sizes there are kernels for
+constexpr bool feat_team_ok(int rows, bool bwd, int w) {
+  if (w < feat_team_min(rows) || w > feat_team_max(rows)) return false;
+  return bwd || w == feat_team_min(rows) || w == feat_team_max(rows);
+}
+inline int feat_team(int rows, bool bwd, long long groups, int sms) {
+  for (int w = feat_team_max(rows); w > feat_team_min(rows); w /= 2)
+    if (feat_team_ok(rows, bwd, w) && groups * w <= (long long)sms * (bwd ? kFeatTeamBwd : kFeatTeamFwd)) return w;
+  return feat_team_min(rows);
 }
 
 }  // namespace ncn

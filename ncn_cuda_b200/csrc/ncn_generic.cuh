@@ -61,16 +61,6 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
-// Steps group g of row b takes.  With per-row context lengths (the reference's earlier Triton kernels,
-// ncn_triton/ncn_triton_old.py:91-96, 189-192) a group counts its members g*n .. g*n+n-1 against the
-// row's length: groups that lie before it take all n steps, the group it cuts takes the steps of the
-// members before it, groups beyond it take none (their positions pass through unchanged).
-__device__ __forceinline__ int group_steps(const int* ctxlen, long long b, int g, int n) {
-  if (ctxlen == nullptr) return n;
-  const long long left = (long long)ctxlen[b] - (long long)g * n;
-  return left <= 0 ? 0 : (left < n ? (int)left : n);
-}
-
 // element offset of (row b, position pos, feature f)
 __device__ __forceinline__ long long elem_off(long long b, int pos, int f, int N, int E) {
   return (b * N + pos) * (long long)E + f;

@@ -1,0 +1,114 @@
+"""Register-tiled kernels for several features per position: every team size (warps per group), rows of 6 features per
+lane, several small groups per warp, ragged group counts, context lengths and leaky-relu, against the fp64 oracle."""
+import pytest
+import torch
+
+from oracle import ncn_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+ALPHA = 0.9
+# (B, N, heads, d, n): teams of 4, 2 and 1 warps (small to larger batches of the same shape), eight rows per group, groups
+# side by side in a warp with a last warp that is partly empty, heads of 24 and 48 features
+SHAPES = [
+    (3, 256, 4, 32, 32),
+    (12, 256, 4, 32, 32),
+    (160, 96, 4, 32, 32),
+    (2, 96, 2, 64, 32),
+    (40, 96, 8, 48, 32),
+    (5, 80, 1, 128, 16),
+    (5, 96, 2, 24, 32),
+    (5, 72, 2, 24, 8),
+    (5, 60, 3, 8, 4),
+    (5, 10, 2, 2, 2),
+    (300, 48, 5, 4, 16),
+]
+
+
+def _case(B, N, heads, d, seed=0):
+    g = torch.Generator().manual_seed(seed)
+    E = heads * d
+
+    def r(s):
+        return torch.randn(B, N, E, generator=g) * s
+
+    return r(1.0), r(0.25), torch.randn(2 * E, generator=g) * d**-0.5, r(1.0), r(0.25)
+
+
+def _oracle(fn, x, xa, W, dy, dya):
+    leaves = [t.double().requires_grad_(True) for t in (x, xa, W)]
+    y, ya = fn(*leaves)
+    return [y.detach(), ya.detach(), *torch.autograd.grad((y, ya), leaves, (dy.double(), dya.double()))]
+
+
+def _check(got, want, tol):
+    for name, a, b in zip(("y", "ya", "dx", "dxa", "dW"), got, want):
+        err = (a.double().cpu() - b).abs().max() / b.abs().max()
+        assert err <= tol, f"{name}: {err:.2e} > {tol:.0e}"
+
+
+@pytest.mark.parametrize("activation", ["tanh", "linear"])
+@pytest.mark.parametrize("B,N,heads,d,n", SHAPES)
+def test_stage(B, N, heads, d, n, activation):
+    import ncn_cuda_b200 as ncn
+
+    x, xa, W, dy, dya = _case(B, N, heads, d)
+    want = _oracle(lambda a, b, w: O.stage_forward(a, b, w, ALPHA, activation, n, heads, 2), x, xa, W, dy, dya)
+    leaves = [t.cuda().requires_grad_(True) for t in (x, xa, W)]
+    y, ya = ncn.fused_ncn_cuda_v2(*leaves, ALPHA, ncn.ops.ACTIVATION_CODES[activation], n, heads, 2)
+    grads = torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda()))
+    _check((y, ya, *grads), want, 1e-5)  # no inverse chain is longer than 16 steps
+
+
+@pytest.mark.parametrize("B,N,heads,d,n", SHAPES)
+def test_context_lengths(B, N, heads, d, n):
+    import ncn_cuda_b200 as ncn
+
+    x, xa, W, dy, dya = _case(B, N, heads, d, seed=1)
+    ctx = torch.randint(0, N + 3, (B,), generator=torch.Generator().manual_seed(2), dtype=torch.int32)
+    ctx[0] = 0
+    ctx[-1] = N
+    want = _oracle(lambda a, b, w: O.stage_forward_ctxlen(a, b, w, ctx, ALPHA, "tanh", n, heads, 1), x, xa, W, dy, dya)
+    leaves = [t.cuda().requires_grad_(True) for t in (x, xa, W)]
+    y, ya = ncn.fused_ncn_cuda_ctxlen(*leaves, ctx.cuda(), ALPHA, 0, n, heads, 1)
+    grads = torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda()))
+    # the walk back from the output: rounding grows by 1 / 0.9 per step, 29-fold over 32 steps
+    _check((y, ya, *grads), want, 1e-5 if n <= 16 else 3e-5)
+
+
+@pytest.mark.parametrize("n,d", [(4, 8), (16, 24)])
+def test_padding_is_not_read_into_the_results(n, d):
+    """Groups beyond a row's length take no step: what stands there (NaN, as in memory never written) stays there."""
+    import ncn_cuda_b200 as ncn
+
+    B, N, heads = 3, 8 * n, 2
+    x, xa, W, dy, dya = _case(B, N, heads, d, seed=3)
+    ctx = torch.tensor([n, 3 * n, 8 * n], dtype=torch.int32)
+    w = W.cuda().requires_grad_(True)
+    out = []
+    for fill in (0.0, float("nan")):
+        a, b = x.clone(), xa.clone()
+        for i in range(B):
+            a[i, ctx[i] :] = fill
+            b[i, ctx[i] :] = fill
+        a, b = a.cuda().requires_grad_(True), b.cuda().requires_grad_(True)
+        y, ya = ncn.fused_ncn_cuda_ctxlen(a, b, w, ctx.cuda(), ALPHA, 0, n, heads, 0)
+        gx, gxa, gw = torch.autograd.grad((y, ya), (a, b, w), (dy.cuda(), dya.cuda()))
+        out.append((y, gx, gxa, gw))
+    for i in range(B):
+        for p, q in zip(out[0][:3], out[1][:3]):
+            assert torch.equal(p[i, : ctx[i]], q[i, : ctx[i]])
+    assert torch.equal(out[0][3], out[1][3])
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,d", [(8, 16), (16, 32)])
+def test_leaky_relu(n, d, dtype):
+    from ncn_cuda_b200 import ops
+
+    B, N, heads = 4, 6 * n, 2
+    x, xa, W, _, _ = _case(B, N, heads, d, seed=4)
+    x, xa = x.to(dtype), xa.to(dtype)
+    y, ya = ops.stage_fwd(x.cuda(), xa.cuda(), W.cuda(), ALPHA, 3, n, heads, 1)
+    Y, YA = O.stage_forward(x.double(), xa.double(), W.double(), ALPHA, "leaky-relu", n, heads, 1)
+    _check((y, ya), (Y, YA), 1e-5 if dtype == torch.float32 else 2e-2)
