@@ -505,9 +505,10 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
     }
   }
   const float2 alpha_g = f2(p.alpha * cdsm);
-  int shift[P];  // (i * stride) mod m
-#pragma unroll
-  for (int r = 0; r < P; ++r) shift[r] = (int)((long long)th.pos(r) * p.stride % p.m);
+  // Block of row r: g + (i * stride) mod m, i = i_0 + r SEG.  The offsets are formed again where they are used: kept over
+  // the steps they would cost the four-row kernels registers that are not there (1024 x 256 x 128, groups of 32: 1084 ->
+  // 1067 us).
+  const int shift0 = (int)((long long)th.pos(0) * p.stride % p.m), shift1 = (int)((long long)SEG * p.stride % p.m);
   float2 dwi[KP], dwj[KP];  // without the factor (1 - alpha)
 #pragma unroll
   for (int q = 0; q < KP; ++q) dwi[q] = dwj[q] = f2(0.0f);
@@ -515,29 +516,38 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
 
   for (long long u = th.first; u < p.units; u += th.step) {
     const long long b = u / p.mg;
-    const int g = (int)(u - b * p.mg) * G::GPW + th.gw;
+    int g = (int)(u - b * p.mg) * G::GPW + th.gw;
     const bool valid = G::GPW == 1 || g < p.m;
     float2 X[P][KP], A[P][KP], H[P][KP], Gv[P][KP];
-    long long off[P];
+    auto offsets = [&](long long (&off)[P]) {
+      asm volatile("" : "+r"(g));  // (or the compiler keeps the first result after all)
+      int blk = g + shift0;
+      if (blk >= p.m) blk -= p.m;
+#pragma unroll
+      for (int r = 0; r < P; ++r) {
+        off[r] = ((b * p.N + (long long)blk * NC + th.pos(r)) * p.E) + th.c * D + th.sub * KF;
+        blk += shift1;
+        if (blk >= p.m) blk -= p.m;
+      }
+    };
     // (stored end state or full replay: y, ya are not read)
     const bool from_output = !(REPLAY && p.saved == 2) && !(p.saved == 3 && p.mid_end);
+    long long off0[P];
+    offsets(off0);
 #pragma unroll
     for (int r = 0; r < P; ++r) {
-      int blk = g + shift[r];
-      if (blk >= p.m) blk -= p.m;
-      off[r] = ((b * p.N + (long long)blk * NC + th.pos(r)) * p.E) + th.c * D + th.sub * KF;
 #pragma unroll
       for (int q = 0; q < KP; ++q) X[r][q] = A[r][q] = H[r][q] = Gv[r][q] = f2(0.0f);
       if (valid) {
         if (from_output) {
-          ld_feat<KF, T>(g_y + off[r], X[r]);
-          ld_feat<KF, T>(g_ya + off[r], A[r]);
+          ld_feat<KF, T>(g_y + off0[r], X[r]);
+          ld_feat<KF, T>(g_ya + off0[r], A[r]);
         }
-        ld_feat<KF, T>(g_dy + off[r], H[r]);
-        ld_feat<KF, T>(g_dya + off[r], Gv[r]);
+        ld_feat<KF, T>(g_dy + off0[r], H[r]);
+        ld_feat<KF, T>(g_dya + off0[r], Gv[r]);
         // the stored state is needed half a stage from now: towards L2 already
         if (NC > 16 && p.saved == 3 && (th.sub & 3) == 0) {
-          const float* mx = p.mid + off[r];
+          const float* mx = p.mid + off0[r];
           asm volatile("prefetch.global.L2 [%0];" ::"l"(mx));
           asm volatile("prefetch.global.L2 [%0];" ::"l"(mx + p.bne));
         }
@@ -561,6 +571,8 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
           const T* g_x = static_cast<const T*>(p.xin[0]);
           const T* g_xa = static_cast<const T*>(p.xin[1]);
           if (valid) {
+            long long off[P];
+            offsets(off);
 #pragma unroll
             for (int r = 0; r < P; ++r) {
               ld_feat<KF, T>(g_x + off[r], X[r]);
@@ -570,12 +582,24 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
 #pragma unroll 1
           for (int jf = 0; jf <= j0; ++jf) {
             const int rf = th.local_row(jf);
-            const uint32_t xb = xrow + 4u * (uint32_t)(par * G::XS);
-            par ^= 1;
-            publish_row<P, KP, KF>(xb, X, rf, rf >= 0 && th.s == (jf & (SEG - 1)));
-            team_sync<W>(th.team);
             float2 xf[KP];
-            lds_row<KF>(xb, xf);
+            if constexpr (W == 1) {  // (bf16, 1024 x 256 x 128, groups of 32: 1553 us, through shared memory 1702)
+              const int src = (th.gw * SEG + (jf & (SEG - 1))) * LD + th.sub;
+#pragma unroll
+              for (int q = 0; q < KP; ++q) {
+                float2 v = X[0][q];
+#pragma unroll
+                for (int r = 1; r < P; ++r)
+                  if (rf == r) v = X[r][q];
+                xf[q] = shfl2(v, src);
+              }
+            } else {
+              const uint32_t xb = xrow + 4u * (uint32_t)(par * G::XS);
+              par ^= 1;
+              publish_row<P, KP, KF>(xb, X, rf, rf >= 0 && th.s == (jf & (SEG - 1)));
+              team_sync<W>(th.team);
+              lds_row<KF>(xb, xf);
+            }
             feat_forward_step<LD, KP, P, ACT, false>(X, A, xf, Wi, Wj, p.alpha, jf, true);
           }
           const float2 sc = f2(kPow.pos[j0 + 1]);
@@ -591,6 +615,8 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
         // the state after step j0 as the forward stored it
         if (((j0 + 1) & 15) == 0 && (j0 + 1 < NC || p.mid_end) && valid) {
           const float* mx = p.mid + (long long)(2 * ((j0 + 1) / 16 - 1)) * p.bne;
+          long long off[P];
+          offsets(off);
 #pragma unroll
           for (int r = 0; r < P; ++r) {
             ld_feat<KF, float>(mx + off[r], X[r]);
@@ -779,6 +805,8 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
         }
     }  // runs
     if (valid) {
+      long long off[P];
+      offsets(off);
 #pragma unroll
       for (int r = 0; r < P; ++r) {
         st_feat<KF, T>(g_dx + off[r], H[r]);
