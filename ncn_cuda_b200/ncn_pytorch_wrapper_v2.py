@@ -64,18 +64,53 @@ def stage_backward_plan(dtype, n_cache: int) -> str:
 _KEEP = {"output": 0, "input": 1, "mid": 2}  # enum Keep of csrc/ncn_torch.cpp
 
 
-class NCNFunction:
+class NCNFunction(torch.autograd.Function):
     """One stage (ncn_cuda/ncn_pytorch_wrapper_v2.py:9-50).  Saves the stage OUTPUT and rebuilds the
     input by the reversible inverse, as the reference does; for stages of more than
-    MAX_INVERSE_STEPS steps it keeps more (see set_stage_backward).  The autograd node is native
-    (csrc/ncn_torch.cpp)."""
+    MAX_INVERSE_STEPS steps it keeps more (see set_stage_backward).  `apply` goes to the native node of
+    csrc/ncn_torch.cpp, which does the same with less host work; a subclass keeps forward and backward."""
 
-    @staticmethod
-    def apply(x, xa, W, alpha, activation, n_cache, n_head, module_l):
+    @classmethod
+    def apply(cls, *args):
+        if cls is not NCNFunction:
+            return super().apply(*args)
+        x, xa, W, alpha, activation, n_cache, n_head, module_l = args
         keep = _KEEP[stage_backward_plan(x.dtype, n_cache)]
         return _lib.native().stages(
             x, xa, [W], alpha, ops.activation_code(activation), n_cache, n_head, module_l, keep
         )
+
+    @staticmethod
+    def forward(ctx, x, xa, W, alpha, activation, n_cache, n_head, module_l):
+        ctx.keep = stage_backward_plan(x.dtype, n_cache)
+        if ctx.keep == "mid":
+            yi, ya, mid = ops.stage_fwd_mid(x, xa, W, alpha, activation, n_cache, n_head, module_l)
+            if mid is None:
+                ctx.keep = "output"
+                ctx.save_for_backward(yi, ya, W)
+            else:
+                ctx.save_for_backward(yi, ya, W, mid)
+        else:
+            yi, ya = ops.stage_fwd(x, xa, W, alpha, activation, n_cache, n_head, module_l)
+            if ctx.keep == "input":
+                ctx.save_for_backward(yi, ya, W, x, xa)
+            else:
+                ctx.save_for_backward(yi, ya, W)
+        ctx.cfg = (alpha, activation, n_cache, n_head, module_l)
+        return yi, ya
+
+    @staticmethod
+    def backward(ctx, dyi, dya):
+        if ctx.keep == "input":
+            (yi, ya, W, x, xa) = ctx.saved_tensors
+            dx, dxa, dW = ops.stage_bwd_saved(x, xa, yi, ya, dyi, dya, W, *ctx.cfg)
+        elif ctx.keep == "mid":
+            (yi, ya, W, mid) = ctx.saved_tensors
+            dx, dxa, dW = ops.stage_bwd_mid(yi, ya, mid, dyi, dya, W, *ctx.cfg)
+        else:
+            (yi, ya, W) = ctx.saved_tensors
+            dx, dxa, dW = ops.stage_bwd(yi, ya, dyi, dya, W, *ctx.cfg)
+        return dx, dxa, dW.to(W.dtype), None, None, None, None, None
 
 
 def fused_ncn_cuda_v2(
@@ -92,16 +127,34 @@ def fused_ncn_cuda_v2(
     return yi, ya
 
 
-class NCNContextFunction:
+class NCNContextFunction(torch.autograd.Function):
     """One stage with a context length per batch row: the step-count rule of the reference's earlier
     Triton operator (ncn_triton/ncn_triton_old.py:285-359 `FusedLinearChunkNCNFunction`, kernels
-    :52-124, :141-283) on the stage index map of torch_ref.  Saves the stage output, like NCNFunction."""
+    :52-124, :141-283) on the stage index map of torch_ref.  Saves the stage output, like NCNFunction,
+    and like there `apply` goes to the native node."""
 
-    @staticmethod
-    def apply(x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l):
+    @classmethod
+    def apply(cls, *args):
+        if cls is not NCNContextFunction:
+            return super().apply(*args)
+        x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l = args
         return _lib.native().stage_ctx(
             x, xa, W, torch.as_tensor(ctxlen), alpha, ops.activation_code(activation), n_cache, n_head, module_l
         )
+
+    @staticmethod
+    def forward(ctx, x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l):
+        yi, ya = ops.stage_fwd_ctx(x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l)
+        ctx.save_for_backward(yi, ya, W, torch.as_tensor(ctxlen).to(device=x.device, dtype=torch.int32))
+        ctx.cfg = (alpha, activation, n_cache, n_head, module_l)
+        return yi, ya
+
+    @staticmethod
+    def backward(ctx, dyi, dya):
+        yi, ya, W, ctxlen = ctx.saved_tensors
+        alpha, activation, n_cache, n_head, module_l = ctx.cfg
+        dx, dxa, dW = ops.stage_bwd_ctx(yi, ya, dyi, dya, W, ctxlen, alpha, activation, n_cache, n_head, module_l)
+        return dx, dxa, dW.to(W.dtype), None, None, None, None, None, None
 
 
 def fused_ncn_cuda_ctxlen(x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l):
@@ -145,17 +198,52 @@ def plan_backward(dtype, n_cache: int, num_modules: int, residual: bool, backwar
     return False, (every if num_modules > every else 0), tape
 
 
-class NCNNetFunction:
-    """All stages of a net in one forward and one backward kernel.  W: [L, 2E].  The autograd node is
-    native (csrc/ncn_torch.cpp); it keeps what plan_backward says, and nothing where no gradient is asked for."""
+class NCNNetFunction(torch.autograd.Function):
+    """All stages of a net in one forward and one backward kernel.  W: [L, 2E].  `apply` goes to the native
+    node of csrc/ncn_torch.cpp, which keeps what plan_backward says, and nothing where no gradient is asked for."""
 
-    @staticmethod
-    def apply(x, xa, W, alpha, activation, n_cache, n_head, first_module, backward_mode, residual):
+    @classmethod
+    def apply(cls, *args):
+        if cls is not NCNNetFunction:
+            return super().apply(*args)
+        x, xa, W, alpha, activation, n_cache, n_head, first_module, backward_mode, residual = args
         recompute, every, tape = plan_backward(x.dtype, n_cache, W.shape[0], residual, backward_mode)
         return _lib.native().net(
             x, xa, W, alpha, ops.activation_code(activation), n_cache, n_head, first_module, W.shape[0], 1, recompute, every,
             tape, residual,
         )
+
+    @staticmethod
+    def forward(ctx, x, xa, W, alpha, activation, n_cache, n_head, first_module, backward_mode, residual):
+        recompute, every, tape = plan_backward(x.dtype, n_cache, W.shape[0], residual, backward_mode)
+        y, ya, ckpt = ops.net_fwd(x, xa, W, alpha, activation, n_cache, n_head, first_module, every, residual, tape)
+        # The stored states go through save_for_backward like the other saved tensors: autograd
+        # frees them after the backward and raises its usual error on a second backward without
+        # retain_graph, instead of a backward that silently finds no stored state.
+        if tape:
+            ctx.save_for_backward(W, ckpt)  # the stored states are all the backward reads
+        elif recompute:
+            ctx.save_for_backward(x, xa, W, ckpt)
+        else:
+            ctx.save_for_backward(y, ya, W, ckpt)
+        ctx.cfg = (alpha, activation, n_cache, n_head, first_module, every, recompute, residual, tape)
+        return y, ya
+
+    @staticmethod
+    def backward(ctx, dy, dya):
+        alpha, activation, n_cache, n_head, first_module, every, recompute, residual, tape = ctx.cfg
+        if tape:
+            W, ckpt = ctx.saved_tensors
+            s0 = s1 = None
+        else:
+            s0, s1, W, ckpt = ctx.saved_tensors
+        if ckpt is None and (tape or (every > 0 and not recompute and W.shape[0] > every)):
+            raise RuntimeError("the stored states of this net forward are gone; cannot run its backward")
+        dx, dxa, dW = ops.net_bwd(
+            s0, s1, dy, dya, W, alpha, activation, n_cache, n_head, first_module,
+            ckpt=ckpt, ckpt_every=every, recompute=recompute, residual=residual, tape=tape,
+        )
+        return dx, dxa, dW.to(W.dtype), None, None, None, None, None, None, None
 
 
 def fused_ncn_net(x, xa, W, alpha, activation, n_cache, n_head, first_module=0, backward_mode="auto", residual=False):

@@ -53,6 +53,14 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
         _lib.load()
 
 
+def test_operators_are_autograd_functions():
+    import ncn_cuda_b200 as ncn
+
+    for f in (ncn.NCNFunction, ncn.NCNContextFunction, ncn.NCNNetFunction):
+        assert issubclass(f, torch.autograd.Function)
+        assert {"forward", "backward"} <= set(vars(f))
+
+
 def test_cpu_tensors_are_rejected():
     import ncn_cuda_b200 as ncn
 

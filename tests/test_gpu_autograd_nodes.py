@@ -14,9 +14,9 @@ def ncn():
     return m
 
 
-def _case(kind, L):
-    # fused: one feature per position; chain: several features, stage by stage
-    B, N, E, C, n = (3, 64, 1, 1, 4) if kind == "fused" else (2, 64, 16, 2, 8)
+def _case(kind, L, n=None):
+    # fused: one feature per position; chain, ctx: several features, stage by stage
+    B, N, E, C, n = (3, 64, 1, 1, n or 4) if kind == "fused" else (2, 64, 16, 2, n or 8)
     x, xa, ws, dy, dya = O.make_inputs(11, B, N, E, L, 0.2, dya_zero=False)
     net = (B, N, E, C, n)
     return net, x, xa, ws, dy, dya
@@ -101,3 +101,43 @@ def test_residual_stack_is_one_node_of_all_layers(ncn):
             y, ya = ncn.fused_ncn_net(y, ya, stack.weight[k], 0.9, 0, n, 1, 0, mode, True)
         many = torch.autograd.grad((y, ya), (xs, xas, stack.weight), (dy, dya))
         assert all(torch.equal(p, q) for p, q in zip(one, many))
+
+
+def _calls(ncn, kind, case):
+    """The call under test on (x, xa, *ws), and the same through the Function's own forward and backward."""
+    (B, N, E, C, n), *_ = case
+
+    def general(f):
+        return type("Subclass", (f,), {})
+
+    ctx = torch.tensor([B, N - 3] + [N] * (B - 2), dtype=torch.int32)
+    if kind == "fused":
+        return (lambda x, xa, *ws: ncn.NCNNetTestCuda(0.9, "tanh", n, C, len(ws), ws)(x, xa),
+                lambda x, xa, *ws: general(ncn.NCNNetFunction).apply(x, xa, torch.stack(ws), 0.9, 0, n, C, 0, "auto", False))
+    if kind == "ctx":
+        return (lambda x, xa, *ws: ncn.fused_ncn_cuda_ctxlen(x, xa, ws[0], ctx, 0.9, "tanh", n, C, 1),
+                lambda x, xa, *ws: general(ncn.NCNContextFunction).apply(x, xa, ws[0], ctx, 0.9, 0, n, C, 1))
+
+    def stages(x, xa, *ws):
+        for l, w in enumerate(ws):
+            x, xa = general(ncn.NCNFunction).apply(x, xa, w, 0.9, "tanh", n, C, l)
+        return x, xa
+
+    return lambda x, xa, *ws: ncn.NCNNetTestCuda(0.9, "tanh", n, C, len(ws), ws)(x, xa), stages
+
+
+@pytest.mark.parametrize("kind,keep", [("fused", "auto"), ("chain", "output"), ("chain", "input"), ("chain", "mid"), ("ctx", "auto")])
+def test_functions_have_a_forward_and_a_backward_of_their_own(ncn, kind, keep):
+    """NCNFunction and its like are autograd Functions; what `apply` answers natively is what they compute."""
+    case = _case(kind, 1 if kind == "ctx" else 3, n=32 if keep != "auto" else None)
+    _, x, xa, ws, dy, dya = case
+    prev = ncn.set_stage_backward(keep)
+    try:
+        out = []
+        for call in _calls(ncn, kind, case):
+            leaves = [t.cuda().requires_grad_() for t in (x, xa, *ws)]
+            y, ya = call(*leaves)
+            out.append([y, ya, *torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda()))])
+    finally:
+        ncn.set_stage_backward(prev)
+    assert all(torch.equal(p, q) for p, q in zip(*out))
