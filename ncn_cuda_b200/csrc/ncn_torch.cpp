@@ -18,9 +18,11 @@
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/extension.h>
 
 #include <mutex>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -430,30 +432,41 @@ std::tuple<Tensor, Tensor> chain_forward(const Tensor& x_in, const Tensor& xa_in
 }
 
 // ---------------------------------------------------------------- Python entry points
-std::tuple<Tensor, Tensor> py_net(const Tensor& x, const Tensor& xa, const Tensor& W, double alpha, int act, int n, int C, int first,
+// What an entry returns where the Python Function (ncn_pytorch_wrapper_v2.py) has to take the call: nothing.
+using Result = std::optional<std::tuple<Tensor, Tensor>>;
+
+// A call the native nodes must not answer.  Under torch.jit.trace the kernels leave no trace of themselves, and the
+// graph would hold the allocations of their results alone; the Function is recorded as a whole.
+bool needs_function() { return torch::jit::tracer::isTracing(); }
+
+Result py_net(const Tensor& x, const Tensor& xa, const Tensor& W, double alpha, int act, int n, int C, int first,
                                   int L, int layers, bool recompute, int every, bool tape, bool residual) {
+  if (needs_function()) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   return fused_forward(x, xa, {W}, false, FusedCfg{alpha, act, n, C, first, L, layers, every, 0, recompute, residual, tape});
 }
 
-std::tuple<Tensor, Tensor> py_stages(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
+Result py_stages(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
                                      int first, int keep) {
+  if (needs_function()) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   return chain_forward(x, xa, ws, Tensor(), ChainCfg{alpha, act, n, C, first, (int)ws.size(), keep, 0});
 }
 
-std::tuple<Tensor, Tensor> py_stage_ctx(const Tensor& x, const Tensor& xa, const Tensor& W, const Tensor& ctxlen, double alpha, int act,
+Result py_stage_ctx(const Tensor& x, const Tensor& xa, const Tensor& W, const Tensor& ctxlen, double alpha, int act,
                                         int n, int C, int module_l) {
+  if (needs_function()) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   return chain_forward(x, xa, {W}, ctxlen, ChainCfg{alpha, act, n, C, module_l, 1, KEEP_OUTPUT, 0});
 }
 
 // A net given as one weight tensor per stage: fused where the library covers the shape, else stage by stage.
-std::tuple<Tensor, Tensor> py_net_list(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
+Result py_net_list(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
                                        bool recompute, int every, bool tape, int keep) {
+  if (needs_function()) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   const int L = (int)ws.size();

@@ -68,7 +68,8 @@ class NCNFunction(torch.autograd.Function):
     """One stage (ncn_cuda/ncn_pytorch_wrapper_v2.py:9-50).  Saves the stage OUTPUT and rebuilds the
     input by the reversible inverse, as the reference does; for stages of more than
     MAX_INVERSE_STEPS steps it keeps more (see set_stage_backward).  `apply` goes to the native node of
-    csrc/ncn_torch.cpp, which does the same with less host work; a subclass keeps forward and backward."""
+    csrc/ncn_torch.cpp, which does the same with less host work; forward and backward stand for the calls that
+    the node declines (needs_function there) and for subclasses."""
 
     @classmethod
     def apply(cls, *args):
@@ -76,9 +77,10 @@ class NCNFunction(torch.autograd.Function):
             return super().apply(*args)
         x, xa, W, alpha, activation, n_cache, n_head, module_l = args
         keep = _KEEP[stage_backward_plan(x.dtype, n_cache)]
-        return _lib.native().stages(
+        out = _lib.native().stages(
             x, xa, [W], alpha, ops.activation_code(activation), n_cache, n_head, module_l, keep
         )
+        return super().apply(*args) if out is None else out
 
     @staticmethod
     def forward(ctx, x, xa, W, alpha, activation, n_cache, n_head, module_l):
@@ -138,9 +140,10 @@ class NCNContextFunction(torch.autograd.Function):
         if cls is not NCNContextFunction:
             return super().apply(*args)
         x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l = args
-        return _lib.native().stage_ctx(
+        out = _lib.native().stage_ctx(
             x, xa, W, torch.as_tensor(ctxlen), alpha, ops.activation_code(activation), n_cache, n_head, module_l
         )
+        return super().apply(*args) if out is None else out
 
     @staticmethod
     def forward(ctx, x, xa, W, ctxlen, alpha, activation, n_cache, n_head, module_l):
@@ -208,10 +211,11 @@ class NCNNetFunction(torch.autograd.Function):
             return super().apply(*args)
         x, xa, W, alpha, activation, n_cache, n_head, first_module, backward_mode, residual = args
         recompute, every, tape = plan_backward(x.dtype, n_cache, W.shape[0], residual, backward_mode)
-        return _lib.native().net(
+        out = _lib.native().net(
             x, xa, W, alpha, ops.activation_code(activation), n_cache, n_head, first_module, W.shape[0], 1, recompute, every,
             tape, residual,
         )
+        return super().apply(*args) if out is None else out
 
     @staticmethod
     def forward(ctx, x, xa, W, alpha, activation, n_cache, n_head, first_module, backward_mode, residual):
@@ -261,7 +265,16 @@ def _net_forward(x, xa, weights: Sequence[torch.Tensor], alpha, activation_nr, n
     if act != ops.LEAKY_RELU:  # leaky-relu: per-stage kernels
         recompute, every, tape = plan_backward(x.dtype, n_cache, L, False, backward_mode)
     keep = _KEEP[stage_backward_plan(x.dtype, n_cache)]
-    return _lib.native().net_list(x, xa, weights, alpha, act, n_cache, n_head, recompute, every, tape, keep)
+    out = _lib.native().net_list(x, xa, weights, alpha, act, n_cache, n_head, recompute, every, tape, keep)
+    if out is not None:
+        return out
+    flags = (ops.NCN_RECOMPUTE if recompute else 0) | (ops.NCN_TAPE if tape else 0)
+    if act != ops.LEAKY_RELU and x.is_cuda and ops.net_supported(x, n_cache, n_head, L, flags, every):
+        W = torch.stack([w.reshape(-1) for w in weights])
+        return fused_ncn_net(x, xa, W, alpha, activation_nr, n_cache, n_head, 0, backward_mode)
+    for module_nr in range(L):
+        x, xa = fused_ncn_cuda_v2(x, xa, weights[module_nr], alpha, activation_nr, n_cache, n_head, module_nr)
+    return x, xa
 
 
 class NCNModuleCuda(nn.Module):

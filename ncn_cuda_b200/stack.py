@@ -13,7 +13,7 @@ import torch.distributed as dist
 from torch import nn
 
 from . import _lib, ops
-from .ncn_pytorch_wrapper_v2 import plan_backward
+from .ncn_pytorch_wrapper_v2 import fused_ncn_net, plan_backward
 
 
 class NCNResidualStack(nn.Module):
@@ -44,10 +44,17 @@ class NCNResidualStack(nn.Module):
             return x, xa
         # every layer in one autograd node: no select / accumulate launches for the slices of the weight
         recompute, every, tape = plan_backward(x.dtype, self.n_cache, self.num_modules, True, self.backward_mode)
-        return _lib.native().net(
+        out = _lib.native().net(
             x, xa, self.weight, self.alpha, self.activation_nr, self.n_cache, self.n_head, 0, self.num_modules,
             self.num_layers, recompute, every, tape, True,
         )
+        if out is not None:
+            return out
+        for k in range(self.num_layers):
+            x, xa = fused_ncn_net(
+                x, xa, self.weight[k], self.alpha, self.activation_nr, self.n_cache, self.n_head, 0, self.backward_mode, True
+            )
+        return x, xa
 
 
 def shard_rows(B: int, rank: int, world: int) -> Tuple[int, int]:

@@ -141,3 +141,25 @@ def test_functions_have_a_forward_and_a_backward_of_their_own(ncn, kind, keep):
     finally:
         ncn.set_stage_backward(prev)
     assert all(torch.equal(p, q) for p, q in zip(*out))
+
+
+@pytest.mark.parametrize("kind", ["fused", "chain", "ctx", "stack"])
+def test_a_traced_module_computes(ncn, kind):
+    """torch.jit.trace records the operators: the traced module gives other inputs' results, not the memory of the tracing."""
+    case = _case("fused" if kind == "stack" else kind, 1 if kind == "ctx" else 3)
+    _, x, xa, ws, dy, dya = case
+    if kind == "stack":
+        net = ncn.NCNResidualStack(2, 0.9, "tanh", 4, 1, 3, 1, w_std=0.5).cuda()
+    else:
+        class Net(torch.nn.Module):
+            def __init__(self):
+                super().__init__()
+                self.ws = torch.nn.ParameterList(w.cuda() for w in ws)
+
+            def forward(self, a, b):
+                return _calls(ncn, kind, case)[0](a, b, *self.ws)
+
+        net = Net()
+    traced = torch.jit.trace(net, (x.cuda(), xa.cuda()))
+    for p, q in zip(traced(dy.cuda(), dya.cuda()), net(dy.cuda(), dya.cuda())):
+        assert torch.equal(p, q)
