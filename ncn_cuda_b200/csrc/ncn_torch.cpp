@@ -435,13 +435,32 @@ std::tuple<Tensor, Tensor> chain_forward(const Tensor& x_in, const Tensor& xa_in
 // What an entry returns where the Python Function (ncn_pytorch_wrapper_v2.py) has to take the call: nothing.
 using Result = std::optional<std::tuple<Tensor, Tensor>>;
 
-// A call the native nodes must not answer.  Under torch.jit.trace the kernels leave no trace of themselves, and the
-// graph would hold the allocations of their results alone; the Function is recorded as a whole.
-bool needs_function() { return torch::jit::tracer::isTracing(); }
+// Tensors the nodes can take: the memory is the value.  Not those with a forward gradient (the nodes have no
+// forward-mode rule and would drop it), nor wrappers of functorch or of Python subclasses with their own dispatch.
+bool plain(const Tensor& t) {
+  constexpr c10::DispatchKeySet wrapped({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                         c10::DispatchKey::BatchedNestedTensor, c10::DispatchKey::Functionalize,
+                                         c10::DispatchKey::Python});
+  return !t.key_set().has_any(wrapped) && !t._fw_grad(/*level=*/0).defined();
+}
+
+// A call the native nodes must not answer: it goes through the Function, which records, transforms or refuses it as
+// any custom Function is.  Under torch.jit.trace the kernels leave no trace of themselves, and the graph would hold
+// the allocations of their results alone; with a functorch transform or a dispatch mode in effect the nodes would
+// pass it by.
+bool needs_function(const Tensor& x, const Tensor& xa, const variable_list& ws) {
+  const c10::impl::LocalDispatchKeySet tls = c10::impl::tls_local_dispatch_key_set();
+  constexpr c10::DispatchKeySet modes({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::Python});
+  if (torch::jit::tracer::isTracing() || tls.included_.has_any(modes)) return true;
+  if (!plain(x) || !plain(xa)) return true;
+  for (const Tensor& w : ws)
+    if (!plain(w)) return true;
+  return false;
+}
 
 Result py_net(const Tensor& x, const Tensor& xa, const Tensor& W, double alpha, int act, int n, int C, int first,
                                   int L, int layers, bool recompute, int every, bool tape, bool residual) {
-  if (needs_function()) return std::nullopt;
+  if (needs_function(x, xa, {W})) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   return fused_forward(x, xa, {W}, false, FusedCfg{alpha, act, n, C, first, L, layers, every, 0, recompute, residual, tape});
@@ -449,7 +468,7 @@ Result py_net(const Tensor& x, const Tensor& xa, const Tensor& W, double alpha, 
 
 Result py_stages(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
                                      int first, int keep) {
-  if (needs_function()) return std::nullopt;
+  if (needs_function(x, xa, ws)) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   return chain_forward(x, xa, ws, Tensor(), ChainCfg{alpha, act, n, C, first, (int)ws.size(), keep, 0});
@@ -457,7 +476,7 @@ Result py_stages(const Tensor& x, const Tensor& xa, const variable_list& ws, dou
 
 Result py_stage_ctx(const Tensor& x, const Tensor& xa, const Tensor& W, const Tensor& ctxlen, double alpha, int act,
                                         int n, int C, int module_l) {
-  if (needs_function()) return std::nullopt;
+  if (needs_function(x, xa, {W})) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   return chain_forward(x, xa, {W}, ctxlen, ChainCfg{alpha, act, n, C, module_l, 1, KEEP_OUTPUT, 0});
@@ -466,7 +485,7 @@ Result py_stage_ctx(const Tensor& x, const Tensor& xa, const Tensor& W, const Te
 // A net given as one weight tensor per stage: fused where the library covers the shape, else stage by stage.
 Result py_net_list(const Tensor& x, const Tensor& xa, const variable_list& ws, double alpha, int act, int n, int C,
                                        bool recompute, int every, bool tape, int keep) {
-  if (needs_function()) return std::nullopt;
+  if (needs_function(x, xa, ws)) return std::nullopt;
   check_activations(x, xa);
   py::gil_scoped_release nogil;
   const int L = (int)ws.size();

@@ -163,3 +163,29 @@ def test_a_traced_module_computes(ncn, kind):
     traced = torch.jit.trace(net, (x.cuda(), xa.cuda()))
     for p, q in zip(traced(dy.cuda(), dya.cuda()), net(dy.cuda(), dya.cuda())):
         assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("kind", ["fused", "chain", "ctx", "stack"])
+def test_transforms_are_refused(ncn, kind):
+    """No forward-mode rule and no vmap rule: a dual tensor or a functorch transform is an error, never a lost tangent."""
+    import torch.autograd.forward_ad as fwAD
+
+    case = _case("fused" if kind == "stack" else kind, 1 if kind == "ctx" else 3)
+    _, x, xa, ws, *_ = case
+    args = [t.cuda() for t in (x, xa, *ws)]
+    if kind == "stack":
+        net = ncn.NCNResidualStack(2, 0.9, "tanh", 4, 1, 3, 1).cuda()
+        args, call = args[:2], lambda a, b: net(a, b)
+    else:
+        call = _calls(ncn, kind, case)[0]
+    for i in range(len(args)):  # every input and every weight
+        with fwAD.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
+            call(*[fwAD.make_dual(t, torch.ones_like(t)) if i == k else t for k, t in enumerate(args)])
+    first, rest = args[0], args[1:]
+    for transformed in (lambda: torch.func.grad(lambda a: call(a, *rest)[0].sum())(first),
+                        lambda: torch.func.vmap(lambda a: call(a, *rest))(torch.stack([first, first])),
+                        lambda: torch.func.grad(lambda s: (s * call(*args)[0]).sum())(torch.ones((), device="cuda"))):
+        with pytest.raises(RuntimeError, match="setup_context"):
+            transformed()
+    with torch.no_grad():  # with the level left, the same tensors are taken
+        call(*args)
