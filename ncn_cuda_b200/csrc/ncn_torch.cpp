@@ -313,7 +313,12 @@ struct ChainNode : public NcnNode {
     auto out_of = [&](std::vector<SavedVariable>& v, int l) {
       return l == c.L - 1 ? v[l].unpack(shared_from_this()) : v[l].unpack();
     };
-    for (int l = c.L - 1; l >= 0; --l) {
+    // The walk ends at the first stage whose gradient is asked for: at stage 0 where the input's is.
+    const bool inputs = task_should_compute_output(0) || task_should_compute_output(1);
+    int last = 0;
+    if (!inputs)
+      while (last < c.L - 1 && !task_should_compute_output(2 + last)) ++last;
+    for (int l = c.L - 1; l >= last; --l) {
       const Tensor w = plain_weights(W[l].unpack(), 2 * E, dy.device());
       const Tensor yl = out_of(y, l), yal = out_of(ya, l);
       Tensor dx = at::empty(shape_, options_), dxa = at::empty(shape_, options_);
@@ -347,11 +352,12 @@ struct ChainNode : public NcnNode {
       dy = std::move(dx);
       dya = std::move(dxa);
     }
-    variable_list out;
-    out.reserve(num_outputs());
-    out.push_back(std::move(dy));
-    out.push_back(std::move(dya));
-    for (size_t l = 0; l < wshape_.size(); ++l) out.push_back(weight_grad(dW, (int64_t)l * 2 * E, l));
+    variable_list out(2 + wshape_.size());
+    if (inputs) {
+      out[0] = std::move(dy);
+      out[1] = std::move(dya);
+    }
+    for (size_t l = last; l < wshape_.size(); ++l) out[2 + l] = weight_grad(dW, (int64_t)l * 2 * E, l);
     return out;
   }
 };
@@ -359,6 +365,17 @@ struct ChainNode : public NcnNode {
 std::tuple<Tensor, Tensor> chain_forward(const Tensor& x_in, const Tensor& xa_in, const variable_list& ws, const Tensor& ctx_in,
                                          ChainCfg c) {
   const bool grad = wants_grad(x_in, xa_in, ws);
+  if (grad && !x_in.requires_grad() && !xa_in.requires_grad() && !ws[0].requires_grad()) {
+    // Stages that nothing is asked of come first: they run without a node, and store nothing.
+    size_t first = 1;
+    while (!ws[first].requires_grad()) ++first;
+    ChainCfg frozen = c, rest = c;
+    frozen.L = (int)first;
+    rest.L = c.L - (int)first;
+    rest.first = c.first + (int)first;
+    const auto mid = chain_forward(x_in, xa_in, variable_list(ws.begin(), ws.begin() + first), ctx_in, frozen);
+    return chain_forward(std::get<0>(mid), std::get<1>(mid), variable_list(ws.begin() + first, ws.end()), ctx_in, rest);
+  }
   const c10::cuda::OptionalCUDAGuard guard(x_in.device());
   std::shared_ptr<ChainNode> node;
   if (grad) {

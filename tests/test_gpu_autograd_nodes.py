@@ -189,3 +189,35 @@ def test_transforms_are_refused(ncn, kind):
             transformed()
     with torch.no_grad():  # with the level left, the same tensors are taken
         call(*args)
+
+
+@pytest.mark.parametrize("n,keep", [(8, "auto"), (32, "auto"), (32, "input")])
+def test_a_chain_is_walked_as_far_as_gradients_are_asked_for(ncn, n, keep):
+    """Frozen stages before the first trainable one store nothing and have no backward; a gradient of late weights
+    alone walks the late stages alone.  Counted by the tensors saved and unpacked."""
+    case = _case("chain", 3, n)
+    _, x, xa, ws, dy, dya = case
+    call = _calls(ncn, "chain", case)[0]
+
+    def run(trainable, wanted, x_grad=False):
+        packed, unpacked = [], []
+        xd = x.cuda().requires_grad_(x_grad)
+        wd = [w.cuda().requires_grad_(t) for w, t in zip(ws, trainable)]
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: packed.append(t) or t, lambda t: unpacked.append(t) or t):
+            y, ya = call(xd, xa.cuda(), *wd)
+        ins = [wd[i] for i in wanted] + ([xd] if x_grad else [])
+        return torch.autograd.grad((y, ya), ins, (dy.cuda(), dya.cuda())), len(packed), len(unpacked)
+
+    prev = ncn.set_stage_backward(keep)
+    try:
+        full, saved, read = run([True] * 3, [0, 1, 2])
+        late, _, read_late = run([True] * 3, [2])
+        frozen, saved_one, read_one = run([False, False, True], [2])
+        gap, saved_gap, read_gap = run([False, True, False], [1])
+        through, _, read_all = run([False, False, False], [], x_grad=True)
+    finally:
+        ncn.set_stage_backward(prev)
+    assert torch.equal(full[2], late[0]) and torch.equal(full[2], frozen[0]) and torch.equal(full[1], gap[0])
+    extra = 2 if keep == "input" else 0  # the input of the first stage, beside each stage's own tensors
+    assert saved_one - extra == (saved - extra) // 3 and saved_gap - extra == (saved - extra) * 2 // 3
+    assert read_one == read_late == read // 3 and read_gap == read * 2 // 3 and read_all == read
