@@ -15,6 +15,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/engine.h>
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -163,6 +164,7 @@ struct FusedNode : public NcnNode {
     const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, c.L, c.dt);
     const Tensor ws = at::empty({(int64_t)ws_bytes}, dy.options().dtype(at::kByte));
     void* const st = stream_of(dy);
+    const bool release = !torch::autograd::get_current_graph_task_keep_graph();  // (as ChainNode)
     for (int k = c.layers - 1; k >= 0; --k) {
       Tensor a, b, ck;
       if (!c.tape) {
@@ -181,6 +183,10 @@ struct FusedNode : public NcnNode {
                                c.n, c.C, c.first, c.L, c.alpha, c.act, c.dt, c.flags(), 0, st));
       dy = std::move(dx);
       dya = std::move(dxa);
+      if (release) {
+        for (auto* v : {&s0, &s1, &ckpt})
+          if (!v->empty()) (*v)[k].reset_data();
+      }
     }
     variable_list out;
     out.reserve(num_outputs());
@@ -313,6 +319,8 @@ struct ChainNode : public NcnNode {
     auto out_of = [&](std::vector<SavedVariable>& v, int l) {
       return l == c.L - 1 ? v[l].unpack(shared_from_this()) : v[l].unpack();
     };
+    // What a stage kept is released behind it, unless the graph is kept: a node per stage would do the same.
+    const bool release = !torch::autograd::get_current_graph_task_keep_graph();
     // The walk ends at the first stage whose gradient is asked for: at stage 0 where the input's is.
     const bool inputs = task_should_compute_output(0) || task_should_compute_output(1);
     int last = 0;
@@ -351,6 +359,10 @@ struct ChainNode : public NcnNode {
       }
       dy = std::move(dx);
       dya = std::move(dxa);
+      if (release) {
+        for (auto* v : {&y, &ya, &mid, &W})
+          if (!v->empty()) (*v)[l].reset_data();
+      }
     }
     variable_list out(2 + wshape_.size());
     if (inputs) {

@@ -221,3 +221,31 @@ def test_a_chain_is_walked_as_far_as_gradients_are_asked_for(ncn, n, keep):
     extra = 2 if keep == "input" else 0  # the input of the first stage, beside each stage's own tensors
     assert saved_one - extra == (saved - extra) // 3 and saved_gap - extra == (saved - extra) * 2 // 3
     assert read_one == read_late == read // 3 and read_gap == read * 2 // 3 and read_all == read
+
+
+@pytest.mark.parametrize("kind", ["chain", "stack"])
+def test_the_walk_back_releases_what_it_has_used(ncn, kind):
+    """The states of a stage (a layer) are freed behind it, so that the next one's results take their memory."""
+    if kind == "chain":  # 32 steps: each stage keeps its output (2 tensors) and the state half way (2)
+        B, N, E, C, n, L = 64, 256, 64, 2, 32, 4
+        ws = [(torch.randn(2 * E, device="cuda") * 0.1).requires_grad_() for _ in range(L)]
+        net = ncn.NCNNetTestCuda(0.9, "tanh", n, C, L, ws)
+    else:  # each layer keeps two states of 2 tensors
+        B, N, E, n, L = 4096, 1024, 1, 8, 4
+        net = ncn.NCNResidualStack(L, 0.9, "tanh", n, 1, 3, E, w_std=0.2).cuda()
+        ws = [net.weight]
+    one = 4 * B * N * E
+    x, xa, dy, dya = (torch.randn(B, N, E, device="cuda") * s for s in (1.0, 0.25, 1.0, 0.25))
+    x.requires_grad_()
+
+    def rise(**kw):
+        y, ya = net(x, xa)
+        base = torch.cuda.memory_allocated()
+        torch.cuda.reset_peak_memory_stats()
+        torch.autograd.grad((y, ya), [x, *ws], (dy, dya), **kw)
+        return (torch.cuda.max_memory_allocated() - base) / one
+
+    rise()
+    # the results of two stages are alive at a time (4 tensors), and workspace of less than one; against that stands
+    # what the first of the two had kept and nobody else holds
+    assert rise() < 3.5 < 4 < rise(retain_graph=True)
