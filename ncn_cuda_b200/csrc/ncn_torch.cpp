@@ -7,8 +7,8 @@
 // Why native: at small batches the host is the bound.  A training step of a 1024 x 1024 net runs 59 us
 // of kernels; through Python autograd functions, ctypes and torch.stack / unbind it took 294 us.
 // A chain of stages keeps its inner activations in one node, so that the engine hands over once per
-// direction instead of once per stage, and the weights of a net are gathered by one small kernel and
-// their gradients returned as views of one buffer.
+// direction instead of once per stage, and the weights of a fused net are gathered by one small kernel
+// and their gradients returned as views of one buffer (as torch.stack and its backward would).
 //
 // Saved tensors go through SavedVariable, so in-place changes, saved-tensor hooks and a second backward
 // without retain_graph behave as for any autograd operator.  Without gradients no state is stored.
@@ -123,9 +123,12 @@ struct NcnNode : public Node {
     Tensor g = at::detail::make_tensor<c10::TensorImpl>(c10::Storage(all.storage()), all.key_set(), all.dtype());
     g.unsafeGetTensorImpl()->set_storage_offset(offset);
     g.unsafeGetTensorImpl()->set_sizes_contiguous(wshape_[k]);
-    if (wopt_[k].dtype() != at::kFloat || wopt_[k].device() != all.device())
-      g = g.to(wopt_[k].device(), c10::typeMetaToScalarType(wopt_[k].dtype()));
-    return g;
+    return as_weight(std::move(g), k);
+  }
+  // an fp32 gradient in the type and on the device of weight k
+  Tensor as_weight(Tensor g, size_t k) const {
+    if (wopt_[k].dtype() == at::kFloat && wopt_[k].device() == g.device()) return g;
+    return g.to(wopt_[k].device(), c10::typeMetaToScalarType(wopt_[k].dtype()));
   }
 };
 
@@ -312,7 +315,7 @@ struct ChainNode : public NcnNode {
     const int64_t B = shape_[0], N = shape_[1], E = shape_[2];
     const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, 1, c.dt);
     const Tensor ws = at::empty({(int64_t)ws_bytes}, dy.options().dtype(at::kByte));
-    const Tensor dW = at::empty({(int64_t)c.L * 2 * E}, dy.options().dtype(at::kFloat));
+    std::vector<Tensor> dW(c.L);  // a tensor of its own per stage: a weight's .grad holds no other's memory
     const size_t mid_bytes = c.keep == KEEP_MID ? ncn_stage_mid_bytes(B, N, E, c.n, c.dt) : 0;
     const Tensor cl = has_ctx ? ctxlen.unpack() : Tensor();
     void* const st = stream_of(dy);
@@ -330,7 +333,8 @@ struct ChainNode : public NcnNode {
       const Tensor w = plain_weights(W[l].unpack(), 2 * E, dy.device());
       const Tensor yl = out_of(y, l), yal = out_of(ya, l);
       Tensor dx = at::empty(shape_, options_), dxa = at::empty(shape_, options_);
-      float* const dwl = dW.mutable_data_ptr<float>() + (int64_t)l * 2 * E;
+      dW[l] = at::empty(wshape_[l], dy.options().dtype(at::kFloat));
+      float* const dwl = dW[l].mutable_data_ptr<float>();
       const float* const wp = w.const_data_ptr<float>();
       const int module_l = c.first + l;
       if (has_ctx) {
@@ -369,7 +373,7 @@ struct ChainNode : public NcnNode {
       out[0] = std::move(dy);
       out[1] = std::move(dya);
     }
-    for (size_t l = last; l < wshape_.size(); ++l) out[2 + l] = weight_grad(dW, (int64_t)l * 2 * E, l);
+    for (int l = last; l < c.L; ++l) out[2 + l] = as_weight(std::move(dW[l]), l);
     return out;
   }
 };

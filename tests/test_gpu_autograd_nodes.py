@@ -249,3 +249,11 @@ def test_the_walk_back_releases_what_it_has_used(ncn, kind):
     # the results of two stages are alive at a time (4 tensors), and workspace of less than one; against that stands
     # what the first of the two had kept and nobody else holds
     assert rise() < 3.5 < 4 < rise(retain_graph=True)
+
+
+def test_gradients_of_a_chain_have_memory_of_their_own(ncn):
+    """Keeping (or saving) one stage's gradient keeps that one alone."""
+    case = _case("chain", 3)
+    xd, xad, wd, net, dyd, dyad = _run(ncn, case)
+    grads = torch.autograd.grad(net(xd, xad), wd, (dyd, dyad))
+    assert [g.untyped_storage().nbytes() for g in grads] == [4 * w.numel() for w in wd]
