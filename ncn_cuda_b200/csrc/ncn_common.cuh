@@ -122,6 +122,12 @@ __device__ __forceinline__ float rcp_approx(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// The smaller of two values; NaN if either is one (fminf drops it: a NaN argument of tanh came out as tanh = 1).
+__device__ __forceinline__ float min_nan(float a, float b) {
+  float y;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(y) : "f"(a), "f"(b));
+  return y;
+}
 
 // ------------------------------------------------------------------ storage types
 template <typename T>
@@ -361,15 +367,20 @@ struct ActForm<ACT_LINEAR> {
 // BATCH: reciprocals taken from one special-function reciprocal of the product of BATCH values
 // (4: 1.25, 2: 1.5, 1: 2 special-function instructions per position and step; the smaller the batch
 // the fewer multiplies on the FMA pipe).
-template <int ACT, int NG, int BATCH>
+template <int ACT, int NG, int BATCH, bool KEEP_NAN = false>
 __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG]) {
   if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {
     // r_i = 1 / d_i, d_i = 1 + 2^ts_i.  The exponent is capped at 30: beyond it r < 1e-9 (tanh = 1 to the last
-    // bit) and the product of four d stays a normal fp32 number, as does its reciprocal.
+    // bit) and the product of four d stays a normal fp32 number, as does its reciprocal.  A NaN reaches all values that
+    // share its reciprocal.  KEEP_NAN: it may, because they are features of one position, whose dot product it is in
+    // already; the positions of a group need not see each other's NaN, and there the cap drops it (r = 2^-30).
     float2 d[NG];
 #pragma unroll
-    for (int i = 0; i < NG; ++i)
-      d[i] = __fadd2_rn(make_float2(ex2_approx(fminf(ts[i].x, 30.0f)), ex2_approx(fminf(ts[i].y, 30.0f))), f2(1.0f));
+    for (int i = 0; i < NG; ++i) {
+      const float2 e = KEEP_NAN ? make_float2(min_nan(ts[i].x, 30.0f), min_nan(ts[i].y, 30.0f))
+                                : make_float2(fminf(ts[i].x, 30.0f), fminf(ts[i].y, 30.0f));
+      d[i] = __fadd2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), f2(1.0f));
+    }
     if constexpr (BATCH == 1) {
 #pragma unroll
       for (int i = 0; i < NG; ++i) r[i] = make_float2(rcp_approx(d[i].x), rcp_approx(d[i].y));

@@ -112,3 +112,35 @@ def test_leaky_relu(n, d, dtype):
     y, ya = ops.stage_fwd(x.cuda(), xa.cuda(), W.cuda(), ALPHA, 3, n, heads, 1)
     Y, YA = O.stage_forward(x.double(), xa.double(), W.double(), ALPHA, "leaky-relu", n, heads, 1)
     _check((y, ya), (Y, YA), 1e-5 if dtype == torch.float32 else 2e-2)
+
+
+@pytest.mark.parametrize("activation", ["tanh", "sigmoid"])
+@pytest.mark.parametrize("B,N,heads,d,n,ctx", [(2, 96, 2, 32, 32, False), (600, 96, 2, 32, 32, False), (2, 96, 2, 24, 32, False),
+                                               (2, 96, 2, 48, 16, False), (2, 96, 2, 64, 32, False), (2, 64, 2, 32, 8, False),
+                                               (2, 128, 2, 32, 32, True), (2, 64, 2, 8, 4, True), (2, 64, 2, 2, 2, False)])
+def test_nan_goes_where_the_arithmetic_takes_it(B, N, heads, d, n, ctx, activation):
+    """A NaN in a token reaches its whole group (head by head) and nothing else; one in the second stream of the group's
+    first token, which is x_j before it is touched, stays with that token."""
+    import ncn_cuda_b200 as ncn
+
+    act = ncn.ops.ACTIVATION_CODES[activation]
+    x, xa, W, dy, dya = _case(B, N, heads, d, seed=5)
+    x[0, n + 1, 3 % d] = float("nan")
+    xa[1, 2 * n, (5 % d) + d] = float("nan")
+    # (the groups that hold a NaN are complete: the oracle selects between a step and none, and 0 * NaN is NaN there)
+    cl = torch.full((B,), 3 * n + 1, dtype=torch.int32)
+
+    def oracle(a, b, w):
+        if ctx:
+            return O.stage_forward_ctxlen(a, b, w, cl, ALPHA, activation, n, heads, 0)
+        return O.stage_forward(a, b, w, ALPHA, activation, n, heads, 0)
+
+    want = _oracle(oracle, x, xa, W, dy, dya)
+    leaves = [t.cuda().requires_grad_(True) for t in (x, xa, W)]
+    if ctx:
+        y, ya = ncn.fused_ncn_cuda_ctxlen(*leaves, cl.cuda(), ALPHA, act, n, heads, 0)
+    else:
+        y, ya = ncn.fused_ncn_cuda_v2(*leaves, ALPHA, act, n, heads, 0)
+    got = (y, ya, *torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda())))
+    for name, p, q in zip(("y", "ya", "dx", "dxa", "dW"), got, want):
+        assert torch.equal(p.isnan().cpu(), q.isnan()), name
