@@ -35,6 +35,11 @@ struct StageParams {
 
 // longest chain of steps the backward rebuilds by the inverse when it has the stage input or stored states
 constexpr int kSegment = 16;
+// Whether the state after step j of `steps` is stored / read: state j / kSegment.  The end state is one whatever the
+// number of steps.
+__device__ __forceinline__ bool state_is_stored(int j, int steps, int mid_end) {
+  return j + 1 == steps ? mid_end != 0 : (j + 1) % kSegment == 0;
+}
 
 __device__ __forceinline__ float act_rt(int act, float t) {
   switch (act) {
@@ -137,8 +142,8 @@ __global__ void __launch_bounds__(256) stage_fwd_kernel(const StageParams p, con
     const int steps = group_steps(p.ctxlen, b, g, n);
     for (int j = 0; j < steps; ++j) {
       stage_forward_step(p, act, X, A, xj, sim, Wi, Wj, j, lane);
-      if (p.mid != nullptr && (j + 1) % kSegment == 0 && (j + 1 < steps || p.mid_end)) {
-        float* mx = p.mid + (long long)(2 * ((j + 1) / kSegment - 1)) * p.bne;
+      if (p.mid != nullptr && state_is_stored(j, steps, p.mid_end)) {
+        float* mx = p.mid + (long long)(2 * (j / kSegment)) * p.bne;
         for (int i = li; i < n; i += LT) {
           const int pos = (int)(((long long)g + (long long)i * p.stride) % p.m) * n + i;
           const long long off = elem_off(b, pos, c * d, p.N, p.E);
@@ -219,8 +224,8 @@ __global__ void __launch_bounds__(256) stage_bwd_kernel(const StageParams p, con
     const int steps = group_steps(p.ctxlen, b, g, n);
     for (int j = steps - 1; j >= 0; --j) {
       if (p.mid != nullptr) {
-        if ((j + 1) % kSegment == 0 && (j + 1 < steps || p.mid_end)) {  // the state after step j as the forward stored it
-          const float* mx = p.mid + (long long)(2 * ((j + 1) / kSegment - 1)) * p.bne;
+        if (state_is_stored(j, steps, p.mid_end)) {  // the state after step j as the forward stored it
+          const float* mx = p.mid + (long long)(2 * (j / kSegment)) * p.bne;
           for (int i = li; i < n; i += LT) {
             const int pos = (int)(((long long)g + (long long)i * p.stride) % p.m) * n + i;
             const long long off = elem_off(b, pos, c * d, p.N, E);

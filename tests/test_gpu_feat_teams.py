@@ -144,3 +144,19 @@ def test_nan_goes_where_the_arithmetic_takes_it(B, N, heads, d, n, ctx, activati
     got = (y, ya, *torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda())))
     for name, p, q in zip(("y", "ya", "dx", "dxa", "dW"), got, want):
         assert torch.equal(p.isnan().cpu(), q.isnan()), name
+
+
+@pytest.mark.parametrize("n,heads,d", [(8, 2, 24), (8, 1, 1), (24, 2, 5), (20, 1, 16), (32, 1, 40)])
+def test_stored_end_state_of_any_number_of_steps(n, heads, d):
+    """bf16 storage with stored states: the backward starts from the fp32 state after the last step, also where the
+    number of steps is no multiple of 16."""
+    from ncn_cuda_b200 import ops
+
+    B, N = 6, 3 * n
+    x, xa, W, dy, dya = _case(B, N, heads, d, seed=7)
+    x, xa, dy, dya = (t.bfloat16() for t in (x, xa, dy, dya))
+    want = _oracle(lambda a, b, w: O.stage_forward(a, b, w, ALPHA, "tanh", n, heads, 1), x, xa, W, dy, dya)
+    y, ya, mid = ops.stage_fwd_mid(x.cuda(), xa.cuda(), W.cuda(), ALPHA, 0, n, heads, 1)
+    got = (y, ya, *ops.stage_bwd_mid(y, ya, mid, dy.cuda(), dya.cuda(), W.cuda(), ALPHA, 0, n, heads, 1))
+    # results rounded to 2^-9; the weight gradient is not rounded, and its terms start from unrounded states
+    _check(got, want, 2e-2)
