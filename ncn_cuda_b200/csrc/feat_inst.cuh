@@ -8,35 +8,48 @@
 namespace ncn {
 
 template <int LD, int KF, int W, int ACT, typename T>
-static cudaError_t launch_one(const FeatParams& p, int grid, int threads, cudaStream_t st, int* occ) {
-  auto go = [&](auto k) {
+static cudaError_t launch_one(const FeatParamsX& p, int grid, int threads, cudaStream_t st, int* occ) {
+  auto go = [&](auto k, const auto& args) {
     if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, 0);
-    k<<<grid, threads, 0, st>>>(p);
+    k<<<grid, threads, 0, st>>>(args);
     return cudaGetLastError();
   };
-  constexpr bool SEVERAL = feat_groups_per_warp(NCN_NC, LD) > 1;
+  constexpr int P = FeatGeom<NCN_NC, LD, KF, W>::P;
+  constexpr bool SEVERAL = feat_groups_per_warp(NCN_NC, LD) > 1, BF16 = sizeof(T) != 4;
+  const bool ctx = p.ctxlen != nullptr;
+  if (ctx && BF16) return cudaErrorNotSupported;
 #ifdef NCN_BWD
-  if constexpr (SEVERAL && sizeof(T) == 4) {
-    if (p.ctxlen != nullptr) return go(feat_bwd_kernel<NCN_NC, LD, KF, W, ACT, T, false, true>);
-  }
+#define NCN_KERNEL feat_bwd_kernel
+  const bool stored = p.saved == 3;
+  constexpr bool OWN_PLAIN = feat_bwd_own(FM_PLAIN, NCN_NC, P, W, LD, BF16), OWN_STORED = feat_bwd_own(FM_STORED, NCN_NC, P, W, LD, BF16);
   if constexpr (NCN_NC >= 16) {
-    if (p.saved == 1 || p.saved == 2) return go(feat_bwd_kernel<NCN_NC, LD, KF, W, ACT, T, true, false>);
+    if (p.saved == 1) return go(feat_bwd_kernel<NCN_NC, LD, KF, W, ACT, T, FM_REPLAY>, p);
   }
   if (p.saved != 0 && NCN_NC < 16) return cudaErrorNotSupported;
-  if ((SEVERAL || sizeof(T) != 4) && p.ctxlen != nullptr) return cudaErrorNotSupported;
-  return go(feat_bwd_kernel<NCN_NC, LD, KF, W, ACT, T, false, false>);
 #else
-  if constexpr (SEVERAL && sizeof(T) == 4) {
-    if (p.ctxlen != nullptr) return go(feat_fwd_kernel<NCN_NC, LD, KF, W, ACT, T, true>);
-  }
-  if (p.mid != nullptr && NCN_NC < 16) return cudaErrorNotSupported;
-  if ((SEVERAL || sizeof(T) != 4) && p.ctxlen != nullptr) return cudaErrorNotSupported;
-  return go(feat_fwd_kernel<NCN_NC, LD, KF, W, ACT, T, false>);
+#define NCN_KERNEL feat_fwd_kernel
+  const bool stored = p.mid != nullptr;
+  constexpr bool OWN_PLAIN = feat_fwd_own(FM_PLAIN, NCN_NC, P, W, LD, BF16), OWN_STORED = feat_fwd_own(FM_STORED, NCN_NC, P, W, LD, BF16);
+  if (stored && NCN_NC < 16) return cudaErrorNotSupported;
 #endif
+  if constexpr (SEVERAL && !BF16) {
+    if (ctx) return go(NCN_KERNEL<NCN_NC, LD, KF, W, ACT, T, FM_MASK>, p);
+  }
+  if constexpr (OWN_PLAIN) {
+    const FeatParams& plain = p;
+    if (!ctx && !stored) return go(NCN_KERNEL<NCN_NC, LD, KF, W, ACT, T, FM_PLAIN>, plain);
+  }
+  if constexpr (OWN_STORED && NCN_NC >= 16) {
+    if (!ctx && stored) return go(NCN_KERNEL<NCN_NC, LD, KF, W, ACT, T, FM_STORED>, p);
+  }
+  // what is left for the kernel with the branches, where anything is
+  constexpr bool LEFT = !OWN_PLAIN || (!SEVERAL && !BF16) || (NCN_NC >= 16 && !OWN_STORED);
+  if constexpr (LEFT) return go(NCN_KERNEL<NCN_NC, LD, KF, W, ACT, T, FM_ANY>, p);
+  return cudaErrorNotSupported;
 }
 
 template <int LD, int KF, int W>
-static cudaError_t launch_act(int act, int dtype, const FeatParams& p, int grid, int threads, cudaStream_t st, int* occ) {
+static cudaError_t launch_act(int act, int dtype, const FeatParamsX& p, int grid, int threads, cudaStream_t st, int* occ) {
   if (dtype == DT_F32) {
     switch (act) {
       case ACT_TANH: return launch_one<LD, KF, W, ACT_TANH, float>(p, grid, threads, st, occ);
@@ -62,7 +75,7 @@ static cudaError_t launch_act(int act, int dtype, const FeatParams& p, int grid,
 }
 
 template <int LD, int KF>
-static cudaError_t launch_geo(int team, int act, int dtype, const FeatParams& p, int grid, int threads, cudaStream_t st, int* occ) {
+static cudaError_t launch_geo(int team, int act, int dtype, const FeatParamsX& p, int grid, int threads, cudaStream_t st, int* occ) {
 #ifdef NCN_BWD
   constexpr bool BWD = true;
 #else
@@ -89,7 +102,7 @@ static cudaError_t launch_geo(int team, int act, int dtype, const FeatParams& p,
 #define NCN_FN NCN_CAT(launch_feat_fwd_n, NCN_NC)
 #endif
 
-cudaError_t NCN_FN(int d, int team, int act, int dtype, const FeatParams& p, int grid, int threads, cudaStream_t st, int* occ) {
+cudaError_t NCN_FN(int d, int team, int act, int dtype, const FeatParamsX& p, int grid, int threads, cudaStream_t st, int* occ) {
   switch (d) {
     case 2: return launch_geo<1, 2>(team, act, dtype, p, grid, threads, st, occ);
     case 4: return launch_geo<1, 4>(team, act, dtype, p, grid, threads, st, occ);

@@ -722,7 +722,7 @@ static void fill_stage(StageParams& p, int64_t B, int64_t N, int64_t E, int n, i
 }
 
 // ---- register-tiled multi-feature stage kernels (ncn_feat.cuh)
-typedef cudaError_t (*FeatLaunchFn)(int, int, int, int, const FeatParams&, int, int, cudaStream_t, int*);
+typedef cudaError_t (*FeatLaunchFn)(int, int, int, int, const FeatParamsX&, int, int, cudaStream_t, int*);
 
 static FeatLaunchFn feat_fn(int n, bool bwd) {
   switch (n) {
@@ -767,7 +767,7 @@ static int launch_feat(bool bwd, const void* const* in, void* const* out, const 
     if (!aligned16(in[q]) || !aligned16(out[q])) return NCN_ERR_UNSUPPORTED;
   if (!aligned16(ex.xin[0]) || !aligned16(ex.xin[1]) || !aligned16(ex.mid)) return NCN_ERR_UNSUPPORTED;
   const int gpw = feat_groups_per_warp(n, lanes);
-  FeatParams p{};
+  FeatParamsX p{};
   for (int q = 0; q < 4; ++q) { p.in[q] = in[q]; p.out[q] = out[q]; }
   p.xin[0] = ex.xin[0]; p.xin[1] = ex.xin[1];
   p.saved = ex.saved;
@@ -791,15 +791,15 @@ static int launch_feat(bool bwd, const void* const* in, void* const* out, const 
   // resident CTAs per SM of this kernel: asked once per (kernel, device, CTA size)
   struct Seen {
     FeatLaunchFn fn;
-    int d, team, act, dtype, saved, ctx, threads, dev, occ;
+    int d, team, act, dtype, saved, mid, ctx, threads, dev, occ;
     bool same(const Seen& o) const {
-      return fn == o.fn && d == o.d && team == o.team && act == o.act && dtype == o.dtype && saved == o.saved && ctx == o.ctx &&
-             threads == o.threads && dev == o.dev;
+      return fn == o.fn && d == o.d && team == o.team && act == o.act && dtype == o.dtype && saved == o.saved && mid == o.mid &&
+             ctx == o.ctx && threads == o.threads && dev == o.dev;
     }
   };
   static std::mutex mu;
   static std::vector<Seen> seen;
-  Seen key{fn, d, team, act, dtype, p.saved, p.ctxlen != nullptr, threads, dev.dev, -1};
+  Seen key{fn, d, team, act, dtype, p.saved, p.mid != nullptr, p.ctxlen != nullptr, threads, dev.dev, -1};
   {
     std::lock_guard<std::mutex> lk(mu);
     for (const Seen& q : seen)
@@ -1231,7 +1231,7 @@ int ncn_stage_bwd_saved(const void* x, const void* xa, const void* y, const void
     void* fout[4] = {dx, dxa, nullptr, nullptr};
     FeatExtra ex;
     ex.xin[0] = x; ex.xin[1] = xa;
-    ex.saved = replay_all ? 2 : 1;
+    ex.saved = 1;
     int fgrid = 0;
     rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
                      activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex);

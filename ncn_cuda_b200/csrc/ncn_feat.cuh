@@ -23,6 +23,8 @@
 // streams of 1024 elements leave room for two warps per scheduler (issue slots half busy), and smaller
 // tiles per warp pay the step's shared part more often than their occupancy returns (see FeatTune).
 #pragma once
+#include <type_traits>
+
 #include "ncn_common.cuh"
 #include "ncn_feat_launch.h"
 
@@ -33,20 +35,32 @@ struct FeatParams {
   void* out[4];       // fwd: y, ya ; bwd: dx, dxa, x_rec|null, xa_rec|null
   const float* W;     // [2E]
   float* partials;    // bwd: [gridDim.x][2E]
-  const int* ctxlen;  // [B] context length per batch row, or null
   long long B;
   long long units;    // B * mg work units per head
   int N, E, C, m, mg, stride;  // mg = ceil(m / groups per team)
   float alpha, oma;
+};
+// What the kernels beyond the plain call take as well.
+struct FeatParamsX : FeatParams {
+  const int* ctxlen;  // [B] context length per batch row, or null
   const void* xin[2]; // bwd with the stage input saved: x, xa
   float* mid;         // fp32 states after every 16th step: state k, stream s at mid + (2k + s) * bne, in the
                       // element order of the activations (fwd: written if not null; bwd with saved == 3: read)
   long long bne;      // elements per activation tensor
-  int saved;          // bwd: 1 = the first half of the steps is replayed from the saved input; 2 = all steps are
-                      // (y, ya are not read: bf16 storage); 3 = the states the forward stored in `mid` replace
-                      // the rebuilt ones
+  int saved;          // bwd: 1 = the first half of the steps is replayed from the saved input, with bf16 storage all
+                      // steps are (y, ya are not read); 3 = the states the forward stored in `mid` replace the
+                      // rebuilt ones
   int mid_end;        // the state after the LAST step is stored / read as well (bf16 storage: y, ya are not read)
 };
+enum FeatMode : int {
+  FM_ANY,     // context lengths and stored states where the parameters have them (a run-time test)
+  FM_PLAIN,   // neither
+  FM_STORED,  // stored states
+  FM_REPLAY,  // backward: states replayed from the saved stage input
+  FM_MASK     // context lengths, groups with different numbers of steps side by side in a warp
+};
+template <int MODE>
+using FeatArgs = std::conditional_t<MODE == FM_PLAIN, FeatParams, FeatParamsX>;
 
 template <int NC, int LD, int KF, int W>
 struct FeatGeom {
@@ -64,17 +78,14 @@ struct FeatGeom {
   static_assert(P * W == ROWS && kFeatWarps % W == 0, "the team divides the rows");
 };
 
-// CTAs per SM the register budget is set for, and the reciprocals of tanh / sigmoid that share one special-function
-// reciprocal (act_r_all, ncn_common.cuh; 0 = one each; the forward takes four).  Measured (us): backward of 1024 x 256 x
-// 128, groups of 32 (four rows per lane): two CTAs, batches of two 1064, single 1098; two rows per lane, three CTAs,
-// single 1125, two CTAs 1269, four CTAs (spills) 1592.  1024 x 512 x 256, groups of 16 (two rows): batches of two 2346,
-// single 2279; forward with three CTAs 1188, four 1136.  2048 x 256 x 128, groups of 8 (one row): backward with three CTAs
-// 766, four 702, five 950; forward with four CTAs 348, six 326.
+// CTAs per SM the register budget is set for.  Measured (us): backward of 1024 x 256 x 128, groups of 32: four rows per
+// lane, two CTAs 1064; two rows per lane, three CTAs 1125, two CTAs 1269, four CTAs (spills) 1592.  1024 x 512 x 256, groups
+// of 16 (two rows): forward with three CTAs 1188, four 1136.  2048 x 256 x 128, groups of 8 (one row): backward with three
+// CTAs 766, four 702, five 950; forward with four CTAs 348, six 326.
 template <int P>
 struct FeatTune {
   static constexpr int fwd_blocks = P >= 4 ? 3 : P == 1 ? 6 : 4;
   static constexpr int bwd_blocks = P >= 4 ? 2 : P == 1 ? 4 : 3;
-  static constexpr int bwd_batch = P >= 4 ? 2 : 0;
 };
 // One row per lane and few steps: the steps are unrolled, which makes the powers of the decay and the lane numbers
 // constants; per step they cost as much as an element otherwise (2048 x 256 x 128, groups of 8, heads of 8: forward 396
@@ -82,6 +93,42 @@ struct FeatTune {
 // of 32: 755 us against 700).
 constexpr bool feat_unrolled(int n, int p, int w) { return p == 1 && w == 1 && n <= 8; }
 constexpr bool feat_bwd_unrolled(int n, int p, int w, int lanes) { return feat_unrolled(n, p, w) && (n <= 4 || lanes == 1); }
+
+// Which calls have a kernel of their own.  At these register counts a branch that is never taken costs 2 to 10 per cent
+// (it is the schedule of the whole step loop that changes, not the branch), and now and then the kernel with the branches
+// comes out better: taken is what measured faster (us, with the branches -> without).
+//   forward, plain: bf16 1024 x 256 x 128, groups of 32 376 -> 366; 1024 x 512 x 256, groups of 16 855 -> 805; heads of 32,
+//     groups of 8 248 -> 234, fp32 326 -> 323; one row per lane, fp32: heads of 8, groups of 16 173 -> 155.  But fp32,
+//     several rows per lane: 530 -> 536 and 1138 -> 1162; heads of 8, groups of 8 (unrolled) 376 -> 385.
+//   forward with stored states: one row per lane 325 -> 312 (heads of 8, groups of 32); four rows 540 -> 566.
+//   backward, plain: bf16 2024 -> 1889 (groups of 16), 1023 -> 840 (groups of 32), fp32 2270 -> 2200; heads of 16, groups
+//     of 16 (256 x 256 x 128) bf16 169 -> 158.  But fp32 unrolled: 703 -> 710.
+//   backward with stored states: four rows 1070 -> 1033; two rows 575 -> 581, one row 668 -> 678.
+// Small batches (teams of several warps) wait for the chain of a step; one kernel serves all their calls.
+constexpr bool feat_fwd_own(int mode, int n, int p, int w, int lanes, bool bf16) {
+  if (w > 1) return false;
+  if (mode == FM_STORED) return p == 1;
+  return bf16 || (p == 1 && (!feat_unrolled(n, p, w) || lanes >= 4));
+}
+constexpr bool feat_bwd_own(int mode, int n, int p, int w, int lanes, bool bf16) {
+  return w == 1 && (mode == FM_STORED ? p >= 4 : bf16 || !feat_bwd_unrolled(n, p, w, lanes));
+}
+
+// Whether the decay of the two streams is carried as a power of m outside the steps.  It saves one instruction per
+// element pair and stream, and costs a dozen per step and lane for the constants of the step: too many for one row per lane
+// (forward, heads of 16, groups of 16, 256 x 256 x 128: 85 -> 80.5 us without; heads of 8, 1024 x 256 x 64: 161 -> 154.5),
+// and too many registers for the four-row backward with the exact tanh (with the power it spills: stored states 1065 ->
+// 1033 us without, replay 1374 -> 1317; heads of 64, groups of 16, 1024 x 256 x 128: 603 -> 551.  Plain with heads of 32 has
+// room for it: 1029 against 1043; tanh.approx too: 840 against 881; and linear: 767 against 831).
+constexpr bool feat_fwd_scaled(int mode, int n, int p, int w) { return mode == FM_ANY || mode == FM_MASK || p > 1 || w > 1 || feat_unrolled(n, p, w); }
+constexpr bool feat_bwd_scaled(int mode, int p, int w, int lanes, int act) {
+  const bool exact = act == ACT_TANH || act == ACT_SIGMOID;
+  return !(exact && p >= 4 && w == 1 && mode != FM_ANY) || (mode == FM_PLAIN && lanes <= 4);
+}
+// Reciprocals of tanh / sigmoid that share one special-function reciprocal in the backward (act_r_all, ncn_common.cuh; 0 =
+// one each; the forward takes four): context lengths, four rows (64 x 256 x 128): two 85 us, single 86.5; the kernels of
+// their own 1040 -> 1030 with single ones (groups of 32), 1024 x 512 x 256, groups of 16 (two rows): 2346 -> 2279.
+constexpr int feat_bwd_batch(int mode, int p, int w) { return p >= 4 && (w > 1 || mode == FM_ANY) ? 2 : 0; }
 constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
 
 // m^k and m^-k: x = m^k X in the forward, x = m^-k X in the reverse sweep (k steps done), so that the
@@ -188,8 +235,10 @@ struct FeatThread {
     step = tt / p.C;
   }
   __device__ __forceinline__ int pos(int r) const { return (wt * G::P + r) * G::SEG + s; }  // position of row r
-  // row index of step j inside a lane of the warp that owns it, -1 in the other warps of the team
+  // row index of step j inside a lane of the warp that owns it, -1 in the other warps of the team (ALONE: there are none)
+  template <bool ALONE>
   __device__ __forceinline__ int local_row(int j) const {
+    if (ALONE) return j / G::SEG;
     const int row = j / G::SEG - wt * G::P;
     return (unsigned)row < (unsigned)G::P ? row : -1;
   }
@@ -288,14 +337,14 @@ __device__ __forceinline__ void publish_row_branch(float* dst, const float2 (&X)
   }
 }
 
-// One forward step (k = steps done, x = m^k X, a = m^k A): xj is the row of position j in the same scale.
-//   Ts = sT (alpha x_i + sim_i x_j) ;  A <- A + c m^-(k+1) F ;  X <- X + c A
-template <int LD, int KP, int P, int ACT, bool MASK>
+// One forward step (k = steps done; SC: x = m^k X, a = m^k A): xj is the row of position j in the same scale.
+//   Ts = sT (alpha x_i + sim_i x_j) ;  SC: A <- A + c m^-(k+1) F ;  X <- X + c A, else a <- m a + c F ;  x <- m x + c a
+template <int LD, int KP, int P, int ACT, bool MASK, bool SC>
 __device__ __forceinline__ void feat_forward_step(float2 (&X)[P][KP], float2 (&A)[P][KP], const float2 (&xj)[KP],
                                                   const float2 (&Wi)[KP], const float2 (&Wj)[KP], float alpha, int k, bool on) {
   using F = ActForm<ACT>;
   constexpr float sT = (float)F::sT;
-  const float mk = kPow.pos[k], imk1 = kPow.neg[k + 1];
+  const float mk = SC ? kPow.pos[k] : 1.0f, imk1 = SC ? kPow.neg[k + 1] : 1.0f;
   const float2 al = f2(alpha * sT * mk);
   const float ss = sT * mk * mk;
   const float2 c1 = f2((float)(kCd * F::f1) * imk1);
@@ -317,9 +366,14 @@ __device__ __forceinline__ void feat_forward_step(float2 (&X)[P][KP], float2 (&A
     if (!MASK || on) {
 #pragma unroll
       for (int q = 0; q < KP; ++q) {
-        if constexpr (F::f0 != 0.0) A[r][q] = __fadd2_rn(A[r][q], c0);
-        A[r][q] = __ffma2_rn(rr[q], c1, A[r][q]);
-        X[r][q] = __ffma2_rn(A[r][q], f2(kC), X[r][q]);
+        if constexpr (SC) {
+          if constexpr (F::f0 != 0.0) A[r][q] = __fadd2_rn(A[r][q], c0);
+          A[r][q] = __ffma2_rn(rr[q], c1, A[r][q]);
+          X[r][q] = __ffma2_rn(A[r][q], f2(kC), X[r][q]);
+        } else {
+          A[r][q] = __ffma2_rn(rr[q], c1, __ffma2_rn(A[r][q], f2(kM), c0));
+          X[r][q] = __ffma2_rn(A[r][q], f2(kC), __fmul2_rn(X[r][q], f2(kM)));
+        }
       }
     }
   }
@@ -327,12 +381,14 @@ __device__ __forceinline__ void feat_forward_step(float2 (&X)[P][KP], float2 (&A
 
 // ------------------------------------------------------------------------------------------ forward
 // p.mid: the fp32 state after every 16th step is also written, for a backward whose inverse chains then
-// never exceed 16 steps.  p.ctxlen: a group takes group_steps() steps; MASK where groups with different
-// numbers of steps share a warp.
-template <int NC, int LD, int KF, int W, int ACT, typename T, bool MASK>
-__global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF, W>::P>::fwd_blocks) feat_fwd_kernel(const FeatParams p) {
+// never exceed 16 steps.  p.ctxlen: a group takes group_steps() steps.
+template <int NC, int LD, int KF, int W, int ACT, typename T, int MODE>
+__global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF, W>::P>::fwd_blocks) feat_fwd_kernel(const FeatArgs<MODE> p) {
   using G = FeatGeom<NC, LD, KF, W>;
   constexpr int P = G::P, KP = G::KP, SEG = G::SEG;
+  constexpr bool MASK = MODE == FM_MASK, CTX = MASK || (MODE == FM_ANY && G::GPW == 1);
+  constexpr bool MID = NC >= 16 && (MODE == FM_ANY || MODE == FM_STORED);
+  constexpr bool SC = feat_fwd_scaled(MODE, NC, P, W);
   __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
   const FeatThread<G, LD, W> th(p);
   const T* gx = static_cast<const T*>(p.in[0]);
@@ -376,7 +432,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
       }
     }
     int steps = NC, tsteps = NC;  // of this lane's group, of the team
-    if (G::GPW == 1 || MASK) {
+    if constexpr (CTX) {
       if (p.ctxlen != nullptr) {
         steps = valid ? group_steps(p.ctxlen, b, g, NC) : 0;
         tsteps = MASK ? (int)__reduce_max_sync(0xffffffffu, (unsigned)steps) : steps;
@@ -391,28 +447,30 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
 #pragma unroll
         for (int q = 0; q < KP; ++q) xj[q] = shfl2(X[0][q], src);
       } else {
-        const int rj = th.local_row(j);
+        const int rj = th.template local_row<W == 1>(j);
         float* const xb = xrow + par * G::XS;
         par ^= 1;
         publish_row_branch<P, KP, KF>(xb, X, rj, rj >= 0 && th.s == (j & (SEG - 1)));
         team_sync<W>(th.team);
         ld_feat<KF, float>(xb, xj);
       }
-      feat_forward_step<LD, KP, P, ACT, MASK>(X, A, xj, Wi, Wj, p.alpha, j, j < steps);
-      if (NC >= 16 && p.mid != nullptr && ((j + 1) & 15) == 0 && (j + 1 < NC || p.mid_end) && valid) {
-        float* mx = p.mid + (long long)(2 * ((j + 1) / 16 - 1)) * p.bne;
-        const float sc = kPow.pos[j + 1];
+      feat_forward_step<LD, KP, P, ACT, MASK, SC>(X, A, xj, Wi, Wj, p.alpha, j, j < steps);
+      if constexpr (MID) {
+        if (p.mid != nullptr && ((j + 1) & 15) == 0 && (j + 1 < NC || p.mid_end) && valid) {
+          float* mx = p.mid + (long long)(2 * ((j + 1) / 16 - 1)) * p.bne;
+          const float sc = SC ? kPow.pos[j + 1] : 1.0f;
 #pragma unroll
-        for (int r = 0; r < P; ++r) {
-          st_feat_scaled<KF>(mx + off[r], X[r], sc);
-          st_feat_scaled<KF>(mx + p.bne + off[r], A[r], sc);
+          for (int r = 0; r < P; ++r) {
+            st_feat_scaled<KF>(mx + off[r], X[r], sc);
+            st_feat_scaled<KF>(mx + p.bne + off[r], A[r], sc);
+          }
         }
       }
     };
     if constexpr (feat_unrolled(NC, P, W)) {
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        if ((G::GPW == 1 || MASK) && j >= tsteps) break;
+        if (CTX && j >= tsteps) break;
         run_step(j);
       }
     } else {
@@ -424,7 +482,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
 #pragma unroll
       for (int r = 0; r < P; ++r) {
 #pragma unroll
-        for (int q = 0; q < KP; ++q) {
+        for (int q = 0; q < KP && SC; ++q) {
           X[r][q] = __fmul2_rn(X[r][q], sc);
           A[r][q] = __fmul2_rn(A[r][q], sc);
         }
@@ -454,18 +512,26 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
 // (fixed shuffle tree), the warps of the CTA that serve the same head (warp order) and the CTAs
 // (dw_reduce_kernel): a fixed order for a given launch shape.
 //
-// REPLAY (saved = 1, 2): the caller also kept the stage INPUT.  Every inverse step grows earlier rounding
+// Without the power (SC false; see feat_bwd_scaled) X, A, H and Gv are the true values, and m is applied in the step.
+//
+// REPLAY (saved = 1): the caller also kept the stage INPUT.  Every inverse step grows earlier rounding
 // by 1/m, so a chain of NC = 32 steps from the output alone leaves the gradients at 1e-5 of their size;
 // here the state half way is rebuilt exactly by running the forward over the first NC/2 steps from the
-// input, so that no inverse chain is longer than NC/2 steps.  With bf16 storage (p.saved == 2) the
+// input, so that no inverse chain is longer than NC/2 steps.  With bf16 storage the
 // end state is replayed too: an inverse started from rounded outputs would amplify their rounding.
-template <int NC, int LD, int KF, int W, int ACT, typename T, bool REPLAY, bool MASK>
-__global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF, W>::P>::bwd_blocks) feat_bwd_kernel(const FeatParams p) {
+template <int NC, int LD, int KF, int W, int ACT, typename T, int MODE>
+__global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF, W>::P>::bwd_blocks) feat_bwd_kernel(const FeatArgs<MODE> p) {
   using G = FeatGeom<NC, LD, KF, W>;
   using F = ActForm<ACT>;
   constexpr int P = G::P, SEG = G::SEG, KP = G::KP, D = G::D;
+  constexpr bool REPLAY = MODE == FM_REPLAY, MASK = MODE == FM_MASK, CTX = MASK || (MODE == FM_ANY && G::GPW == 1);
+  constexpr bool STORED = NC >= 16 && (MODE == FM_ANY || MODE == FM_STORED);
+  constexpr bool SC = feat_bwd_scaled(MODE, P, W, LD, ACT);
+  // (bf16 with one row per lane comes out slower without the test that is always true: 2048 x 256 x 128, groups of 8 618 ->
+  // 651 us, 256 x 256 x 128, heads of 16, groups of 16 158 -> 163; elsewhere it costs, four rows 1044 -> 1033, fp32 178 -> 175)
+  constexpr bool ALONE = W == 1 && (P > 1 || sizeof(T) == 4);
   constexpr float sT = (float)F::sT;
-  constexpr float cdsm = (float)(kCd * F::ds / kMd);
+  constexpr float cds = (float)(kCd * F::ds), cdsm = (float)(kCd * F::ds / kMd);
   constexpr bool COLS_SHFL = W == 1 && P == 1 && NC <= 4;  // (longer chains: 702 us by shared memory, 714 by shuffles)
   __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
   __shared__ __align__(16) float cs[G::TEAMS][2][W][G::XS];
@@ -504,7 +570,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
       Wj[q] = make_float2(wj[2 * q] * p.oma, wj[2 * q + 1] * p.oma);
     }
   }
-  const float2 alpha_g = f2(p.alpha * cdsm);
+  const float2 alpha_g = f2(p.alpha * (SC ? cdsm : cds));
   // Block of row r: g + (i * stride) mod m, i = i_0 + r SEG.  The offsets are formed again where they are used: kept over
   // the steps they would cost the four-row kernels registers that are not there (1024 x 256 x 128, groups of 32: 1084 ->
   // 1067 us).
@@ -531,7 +597,9 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
       }
     };
     // (stored end state or full replay: y, ya are not read)
-    const bool from_output = !(REPLAY && p.saved == 2) && !(p.saved == 3 && p.mid_end);
+    bool from_output = true;
+    if constexpr (REPLAY) from_output = sizeof(T) == 4;
+    if constexpr (STORED) from_output = !(p.saved == 3 && p.mid_end);
     long long off0[P];
     offsets(off0);
 #pragma unroll
@@ -546,15 +614,17 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
         ld_feat<KF, T>(g_dy + off0[r], H[r]);
         ld_feat<KF, T>(g_dya + off0[r], Gv[r]);
         // the stored state is needed half a stage from now: towards L2 already
-        if (NC > 16 && p.saved == 3 && (th.sub & 3) == 0) {
-          const float* mx = p.mid + off0[r];
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(mx));
-          asm volatile("prefetch.global.L2 [%0];" ::"l"(mx + p.bne));
+        if constexpr (STORED && NC > 16) {
+          if (p.saved == 3 && (th.sub & 3) == 0) {
+            const float* mx = p.mid + off0[r];
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(mx));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(mx + p.bne));
+          }
         }
       }
     }
     int steps = NC, tsteps = NC;  // of this lane's group, of the team
-    if (G::GPW == 1 || MASK) {
+    if constexpr (CTX) {
       if (p.ctxlen != nullptr) {
         steps = valid ? group_steps(p.ctxlen, b, g, NC) : 0;
         tsteps = MASK ? (int)__reduce_max_sync(0xffffffffu, (unsigned)steps) : steps;
@@ -562,11 +632,12 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
     }
     // The steps go in runs of RUN; what replaces the rebuilt state (stored by the forward, or replayed from
     // the saved input) is dealt with between the runs, outside the step loop.  A run ends in true scale.
-    constexpr int RUN = REPLAY ? NC / 2 : NC > 16 ? 16 : NC;
+    constexpr int RUN = REPLAY ? NC / 2 : STORED && NC > 16 ? 16 : NC;
 #pragma unroll 1
     for (int j0 = tsteps - 1; j0 >= 0; j0 -= j0 % RUN + 1) {
-      if (REPLAY) {
-        if (j0 == NC / 2 - 1 || p.saved == 2) {
+      if constexpr (REPLAY) {
+        if (j0 == NC / 2 - 1 || sizeof(T) != 4) {
+          constexpr bool SCF = feat_fwd_scaled(FM_PLAIN, NC, P, W);
           // the state after step j0, exactly: the forward over steps 0..j0 from the saved input
           const T* g_x = static_cast<const T*>(p.xin[0]);
           const T* g_xa = static_cast<const T*>(p.xin[1]);
@@ -581,7 +652,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
           }
 #pragma unroll 1
           for (int jf = 0; jf <= j0; ++jf) {
-            const int rf = th.local_row(jf);
+            const int rf = th.template local_row<ALONE>(jf);
             float2 xf[KP];
             if constexpr (W == 1) {  // (bf16, 1024 x 256 x 128, groups of 32: 1553 us, through shared memory 1702)
               const int src = (th.gw * SEG + (jf & (SEG - 1))) * LD + th.sub;
@@ -600,20 +671,20 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
               team_sync<W>(th.team);
               lds_row<KF>(xb, xf);
             }
-            feat_forward_step<LD, KP, P, ACT, false>(X, A, xf, Wi, Wj, p.alpha, jf, true);
+            feat_forward_step<LD, KP, P, ACT, false, SCF>(X, A, xf, Wi, Wj, p.alpha, jf, true);
           }
           const float2 sc = f2(kPow.pos[j0 + 1]);
 #pragma unroll
           for (int r = 0; r < P; ++r)
 #pragma unroll
-            for (int q = 0; q < KP; ++q) {
+            for (int q = 0; q < KP && SCF; ++q) {
               X[r][q] = __fmul2_rn(X[r][q], sc);
               A[r][q] = __fmul2_rn(A[r][q], sc);
             }
         }
-      } else if (NC >= 16 && p.saved == 3) {
+      } else if constexpr (STORED) {
         // the state after step j0 as the forward stored it
-        if (((j0 + 1) & 15) == 0 && (j0 + 1 < NC || p.mid_end) && valid) {
+        if (p.saved == 3 && ((j0 + 1) & 15) == 0 && (j0 + 1 < NC || p.mid_end) && valid) {
           const float* mx = p.mid + (long long)(2 * ((j0 + 1) / 16 - 1)) * p.bne;
           long long off[P];
           offsets(off);
@@ -654,14 +725,17 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
       auto run_step = [&](int j, int kk) {  // kk steps of the run done
         const bool on = !MASK || j <= jtop;
         const int k = MASK ? (on ? jtop - j : 0) : kk;
-        const float mk = kPow.pos[k], iq = kPow.neg[k + 1];
+        const float mk = SC ? kPow.pos[k] : 1.0f, iq = SC ? kPow.neg[k + 1] : 1.0f;
         if (on) {
 #pragma unroll
           for (int r = 0; r < P; ++r)
 #pragma unroll
-            for (int q = 0; q < KP; ++q) X[r][q] = __ffma2_rn(A[r][q], f2(-kC), X[r][q]);
+            for (int q = 0; q < KP; ++q) {
+              if constexpr (SC) X[r][q] = __ffma2_rn(A[r][q], f2(-kC), X[r][q]);
+              else X[r][q] = __ffma2_rn(A[r][q], f2(-kCoverM), __fmul2_rn(X[r][q], f2(kInvM)));
+            }
         }
-        const int rj = th.local_row(j);
+        const int rj = th.template local_row<ALONE>(j);
         const bool sj = on && th.s == (j & (SEG - 1));
         float2 xj[KP];
         if constexpr (W == 1) {  // (shuffles: shorter than the way through shared memory)
@@ -690,9 +764,9 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
         for (int q = 0; q < KP; ++q) accj = __ffma2_rn(xj[q], Wj[q], accj);
         const float cj = accj.x + accj.y;
         const float2 al = f2(p.alpha * sT * iq);
-        const float ss = sT * iq * iq, sg = cdsm * iq;
-        const float2 a1 = f2((float)(-kCd * F::f1) * mk);
-        [[maybe_unused]] const float2 a0 = f2((float)(-kCd * F::f0) * mk);
+        const float ss = sT * iq * iq, sg = SC ? cdsm * iq : cds;
+        const float2 a1 = f2((float)(-kCd * F::f1 / (SC ? 1.0 : kMd)) * mk);
+        [[maybe_unused]] const float2 a0 = f2((float)(-kCd * F::f0 / (SC ? 1.0 : kMd)) * mk);
         float gs[P];
         float2 uu[KP];  // sum_i sim_i gT_i of this lane's positions, per feature
 #pragma unroll
@@ -705,7 +779,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
           float2 ts[KP], rr[KP];
 #pragma unroll
           for (int q = 0; q < KP; ++q) ts[q] = __ffma2_rn(sim_s, xj[q], __fmul2_rn(X[r][q], al));
-          feat_act<ACT, KP, FeatTune<P>::bwd_batch>(ts, rr);
+          feat_act<ACT, KP, feat_bwd_batch(MODE, P, W)>(ts, rr);
           float2 gacc = f2(0.0f);
 #pragma unroll
           for (int q = 0; q < KP; ++q) {
@@ -713,11 +787,17 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
             const float2 gt = F::gt(gap, ts[q], rr[q]);
             gacc = __ffma2_rn(gt, xj[q], gacc);
             uu[q] = r == 0 ? __fmul2_rn(simg, gt) : __ffma2_rn(simg, gt, uu[q]);
-            if (on) {
-              if constexpr (F::f0 != 0.0) A[r][q] = __fadd2_rn(A[r][q], a0);
-              A[r][q] = __ffma2_rn(rr[q], a1, A[r][q]);
-              Gv[r][q] = gap;
-              H[r][q] = __ffma2_rn(gt, alpha_g, H[r][q]);  // gs_i Wi is added below
+            if (on) {  // (gs_i Wi is added to H below)
+              if constexpr (SC) {
+                if constexpr (F::f0 != 0.0) A[r][q] = __fadd2_rn(A[r][q], a0);
+                A[r][q] = __ffma2_rn(rr[q], a1, A[r][q]);
+                Gv[r][q] = gap;
+                H[r][q] = __ffma2_rn(gt, alpha_g, H[r][q]);
+              } else {
+                A[r][q] = __ffma2_rn(rr[q], a1, __ffma2_rn(A[r][q], f2(kInvM), a0));
+                Gv[r][q] = __fmul2_rn(gap, f2(kM));
+                H[r][q] = __ffma2_rn(gt, alpha_g, __fmul2_rn(H[r][q], f2(kM)));
+              }
             }
           }
           gs[r] = red_sub<LD>(gacc.x + gacc.y) * sg;
@@ -781,7 +861,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
       if constexpr (feat_bwd_unrolled(NC, P, W, LD)) {
 #pragma unroll
         for (int kk = 0; kk < NC; ++kk) {
-          if ((G::GPW == 1 || MASK) && kk > j0) break;
+          if (CTX && kk > j0) break;
           run_step(j0 - kk, kk);
         }
       } else {
@@ -797,7 +877,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
 #pragma unroll
       for (int r = 0; r < P; ++r)
 #pragma unroll
-        for (int q = 0; q < KP; ++q) {
+        for (int q = 0; q < KP && SC; ++q) {
           X[r][q] = __fmul2_rn(X[r][q], up);
           A[r][q] = __fmul2_rn(A[r][q], up);
           H[r][q] = __fmul2_rn(H[r][q], dn);

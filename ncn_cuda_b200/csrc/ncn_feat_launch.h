@@ -6,15 +6,15 @@
 
 namespace ncn {
 
-struct FeatParams;
+struct FeatParamsX;
 
 constexpr int kFeatWarps = 4;  // warps per CTA
 
 // team: warps per group (feat_team)
 #define NCN_DECL(n)                                                                                                   \
-  cudaError_t launch_feat_fwd_n##n(int d, int team, int act, int dtype, const FeatParams& p, int grid, int threads,   \
+  cudaError_t launch_feat_fwd_n##n(int d, int team, int act, int dtype, const FeatParamsX& p, int grid, int threads,   \
                                    cudaStream_t st, int* occ);                                                        \
-  cudaError_t launch_feat_bwd_n##n(int d, int team, int act, int dtype, const FeatParams& p, int grid, int threads,   \
+  cudaError_t launch_feat_bwd_n##n(int d, int team, int act, int dtype, const FeatParamsX& p, int grid, int threads,   \
                                    cudaStream_t st, int* occ);
 NCN_DECL(2)
 NCN_DECL(4)

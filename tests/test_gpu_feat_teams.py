@@ -60,6 +60,34 @@ def test_stage(B, N, heads, d, n, activation):
     _check((y, ya, *grads), want, 1e-5)  # no inverse chain is longer than 16 steps
 
 
+# One warp per group with four, two and one rows per lane, teams of two warps with two rows, heads of 24 and 48, several
+# groups per warp: what a call keeps for its backward chooses among the kernels of each.
+@pytest.mark.parametrize("keep", ["auto", "input", "mid"])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("B,N,heads,d,n", [(160, 96, 4, 32, 32), (12, 256, 4, 32, 32), (160, 96, 4, 16, 32), (40, 96, 8, 48, 32),
+                                           (5, 96, 2, 24, 32), (5, 72, 2, 24, 8), (160, 48, 4, 64, 16), (160, 96, 4, 8, 32),
+                                           (160, 48, 4, 16, 16), (300, 48, 5, 4, 16), (40, 72, 4, 8, 8), (40, 60, 4, 16, 4)])
+def test_kernels_of_a_call(B, N, heads, d, n, dtype, keep):
+    import ncn_cuda_b200 as ncn
+
+    x, xa, W, dy, dya = _case(B, N, heads, d, seed=6)
+    x, xa, dy, dya = (t.to(dtype) for t in (x, xa, dy, dya))
+    want = _oracle(lambda a, b, w: O.stage_forward(a, b, w, ALPHA, "tanh", n, heads, 1), x, xa, W, dy, dya)
+    prev = ncn.set_stage_backward(keep)
+    try:
+        leaves = [t.cuda().requires_grad_(True) for t in (x, xa, W)]
+        y, ya = ncn.fused_ncn_cuda_v2(*leaves, ALPHA, 0, n, heads, 1)
+        got = (y, ya, *torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda())))
+    finally:
+        ncn.set_stage_backward(prev)
+    if keep != "mid" or n >= 16:  # (the states of shorter groups are stored by the shared-memory kernels, with the exact tanh)
+        with torch.no_grad():  # stored states change no result
+            assert torch.equal(y, ncn.fused_ncn_cuda_v2(*leaves, ALPHA, 0, n, heads, 1)[0])
+    # bf16: results rounded to 2^-9; the weight gradient sums terms that carry the rounding and largely cancel
+    _check(got[:4], want[:4], 1e-5 if dtype == torch.float32 else 2e-2)
+    _check([got[4]], [want[4]], 1e-5 if dtype == torch.float32 else 3e-2)
+
+
 @pytest.mark.parametrize("B,N,heads,d,n", SHAPES)
 def test_context_lengths(B, N, heads, d, n):
     import ncn_cuda_b200 as ncn
