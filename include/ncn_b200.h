@@ -114,8 +114,9 @@ int ncn_stage_bwd_mid(const void* y, const void* ya, const void* mid, size_t mid
  * ctxlen[b]: groups before it take all n_cache steps, the group it cuts takes the steps of the members before
  * it, groups at or beyond it take none.  Every position is still read and written: positions of groups that
  * take no step pass through unchanged (y = x, ya = xa; dx = dy, dxa = dya) - the reference leaves them
- * unwritten.  ctxlen[b] >= N gives ncn_stage_fwd / ncn_stage_bwd.  Other arguments as in those calls; these
- * entries always run the shared-memory kernels (any E, n_head, n_cache). */
+ * unwritten.  ctxlen[b] >= N gives ncn_stage_fwd / ncn_stage_bwd.  Other arguments as in those calls
+ * (any E, n_head, n_cache; fp32 runs the register-tiled kernels where they cover the group and head size, the rest
+ * and bf16 the shared-memory kernels). */
 int ncn_stage_fwd_ctx(const void* x, const void* xa, const float* W, const int* ctxlen, void* y, void* ya, int64_t B,
                       int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation, int dtype,
                       void* stream);

@@ -1,8 +1,9 @@
 // Explicit instantiation of the register-tiled multi-feature stage kernels (ncn_feat.cuh) for one
 // n_cache (NCN_NC) and one direction (NCN_BWD defined or not); one translation unit each.
 // Head widths d = 2, 4 (one lane per position), 8, 16, 32, 64, 128 (8 features per lane), 24, 48 (6 per lane), up to
-// kFeatMaxRows rows of positions per group (n_cache * d <= 2048).  Every other shape, and bf16 storage with the exact
-// tanh, stays with the shared-memory kernels of ncn_generic.cuh.
+// kFeatMaxRows rows of positions per group (n_cache * d <= 2048).  Every other shape stays with the shared-memory kernels
+// of ncn_generic.cuh, and so do bf16 storage with context lengths and, where tanh.approx is the rule (feat_bf16_exact_tanh
+// false), bf16 storage with the exact tanh.
 #include "ncn_feat.cuh"
 
 namespace ncn {

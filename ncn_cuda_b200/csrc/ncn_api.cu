@@ -104,7 +104,7 @@ static int map_act(int code) {
     case 0: return ACT_TANH;
     case 1: return ACT_RELU;
     case 2: return ACT_SIGMOID;
-    case 3: return ACT_LEAKY;  // shared-memory stage kernels only
+    case 3: return ACT_LEAKY;  // per-stage kernels only
     default: return ACT_LINEAR;
   }
 }

@@ -40,7 +40,9 @@ constexpr int feat_rows(int n, int lanes) { return lanes == 0 ? 0 : n * lanes <=
 constexpr int feat_groups_per_warp(int n, int lanes) { return n * lanes >= 32 ? 1 : 32 / (n * lanes); }
 
 // bf16 storage: heads of 24 and 48 features and tiles of more than 1024 elements keep the exact tanh that the
-// shared-memory kernels take (dW 7e-7 off the fp64 result, 5e-6 with tanh.approx).
+// shared-memory kernels take; the other shapes take tanh.approx (relative error 2^-11), unless NCN_EXACT_TANH=1 sends them
+// to the shared-memory kernels.  (64 x 256 x 128, groups of 32, replayed from the bf16 input: dW 8e-7 off the fp64 result of the
+// same input for heads of 64, 3.5e-6 for heads of 32.)
 constexpr bool feat_bf16_exact_tanh(int n, int d) { return d == 24 || d == 48 || n * d > 1024; }
 
 // Warps per group.  The widest share (four rows per lane, as few warps as that takes) does the least work per element:

@@ -1,7 +1,9 @@
 """Tensor-level calls into the C ABI (include/ncn_b200.h).
 
 torch is used for device memory and streams only; every function here launches
-kernels of libncn_b200.so on the current stream and returns torch tensors.
+kernels of libncn_b200.so on the current stream and returns torch tensors.  The modules go through the
+native nodes (csrc/ncn_torch.cpp) instead; these functions serve callers without autograd, the Functions' own
+forward and backward, and tests.
 """
 from __future__ import annotations
 

@@ -98,8 +98,8 @@ STAGE_CASES = [
     (1, 64, 128, 4, 32, 1, "tanh"),
     (2, 32, 40, 1, 8, 3, "linear"),    # d = 40 > 32
     (5, 30, 1, 1, 2, 3, "tanh"),       # N % 4 != 0: generic kernel
-    (3, 64, 1, 1, 4, 2, "leaky-relu"),  # general kernels (one feature per position)
-    (2, 64, 32, 4, 8, 1, "leaky-relu"), # general kernels (several features)
+    (3, 64, 1, 1, 4, 2, "leaky-relu"),  # shared-memory kernels (one feature per position)
+    (2, 64, 32, 4, 8, 1, "leaky-relu"), # register-tiled kernels (several features)
 ]
 
 
@@ -131,7 +131,7 @@ def test_stage_bf16(ncn):
     y, ya = ncn.ops.stage_fwd(dev(x), dev(xa), dev(W), 0.9, 0, n, C, l)
     ry, rya = O.stage_forward(x.float(), xa.float(), W, 0.9, "tanh", n, C, l)
     assert O.rel_err(y.float(), ry) < TOLBF and O.rel_err(ya.float(), rya) < TOLBF
-    # multi-feature bf16 through the generic kernel
+    # multi-feature bf16
     x = torch.randn(2, 64, 16).bfloat16(); xa = torch.zeros(2, 64, 16).bfloat16(); W = torch.randn(32) * 0.2
     y, ya = ncn.ops.stage_fwd(dev(x), dev(xa), dev(W), 0.9, 0, 8, 2, 1)
     ry, rya = O.stage_forward(x.float(), xa.float(), W, 0.9, "tanh", 8, 2, 1)
@@ -140,7 +140,7 @@ def test_stage_bf16(ncn):
 
 # ---------------------------------------------------------------- several features per position, register-tiled kernels
 FEAT_CASES = [
-    # B, N, E, C, n, module_l        (d = E / C; covered: d in {2, 4, ..., 128}, n * d <= 1024)
+    # B, N, E, C, n, module_l        (d = E / C; covered: d in {2, 4, ..., 128}, n * d <= 2048)
     (3, 64, 8, 2, 2, 1),       # d = 4, sixteen groups per warp
     (2, 96, 12, 3, 4, 2),      # d = 4, three heads (warps per head not a power of two), m = 24
     (3, 72, 16, 2, 8, 3),      # d = 8, m = 9: the last warp's group slots are partly empty
