@@ -257,3 +257,26 @@ def test_gradients_of_a_chain_have_memory_of_their_own(ncn):
     xd, xad, wd, net, dyd, dyad = _run(ncn, case)
     grads = torch.autograd.grad(net(xd, xad), wd, (dyd, dyad))
     assert [g.untyped_storage().nbytes() for g in grads] == [4 * w.numel() for w in wd]
+
+
+def test_errors_of_the_native_nodes(ncn):
+    """Through the operators and modules: the library's status as NCNError, bad tensors by type."""
+    (_, _, _, C, n), x, xa, ws, _, _ = _case("chain", 2)
+    x, xa, ws = x.cuda(), xa.cuda(), [w.cuda() for w in ws]
+    from ncn_cuda_b200._lib import NCNError
+
+    for bad_n, bad_heads in ((7, C), (n, 3)):
+        with pytest.raises(NCNError, match="bad shape"):
+            ncn.fused_ncn_cuda_v2(x, xa, ws[0], 0.9, 0, bad_n, bad_heads, 0)
+    with pytest.raises(NCNError, match="does not cover"):
+        ncn.fused_ncn_net(x, xa, torch.stack(ws), 0.9, 0, n, C)
+    with pytest.raises(ValueError, match="elements"):
+        ncn.NCNNetTestCuda(0.9, "tanh", n, C, 2, [ws[0], ws[1][:3]])(x, xa)
+    with pytest.raises(ValueError, match="agree"):
+        ncn.fused_ncn_cuda_v2(x, xa[:1], ws[0], 0.9, 0, n, C, 0)
+    with pytest.raises(ValueError, match="entries"):
+        ncn.fused_ncn_cuda_ctxlen(x, xa, ws[0], torch.ones(3), 0.9, 0, n, C, 0)
+    with pytest.raises(TypeError, match="float32 or bfloat16"):
+        ncn.fused_ncn_cuda_v2(x.half(), xa.half(), ws[0], 0.9, 0, n, C, 0)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        ncn.fused_ncn_cuda_v2(x.cpu(), xa.cpu(), ws[0], 0.9, 0, n, C, 0)
