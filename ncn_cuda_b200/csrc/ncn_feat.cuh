@@ -120,8 +120,13 @@ constexpr bool feat_bwd_own(int mode, int n, int p, int w, int lanes, bool bf16)
 // and too many registers for the four-row backward with the exact tanh (with the power it spills: stored states 1065 ->
 // 1033 us without, replay 1374 -> 1317; heads of 64, groups of 16, 1024 x 256 x 128: 603 -> 551.  Plain with heads of 32 has
 // room for it: 1029 against 1043; tanh.approx too: 840 against 881; and linear: 767 against 831).
-constexpr bool feat_fwd_scaled(int mode, int n, int p, int w) { return mode == FM_ANY || mode == FM_MASK || p > 1 || w > 1 || feat_unrolled(n, p, w); }
-constexpr bool feat_bwd_scaled(int mode, int p, int w, int lanes, int act) {
+// Groups of 2 and 4 save next to nothing by it, and the multiplications back to true scale cost them 10 per cent in accuracy.
+constexpr bool feat_fwd_scaled(int mode, int n, int p, int w) {
+  if (n <= 4) return false;
+  return mode == FM_ANY || mode == FM_MASK || p > 1 || w > 1 || feat_unrolled(n, p, w);
+}
+constexpr bool feat_bwd_scaled(int mode, int n, int p, int w, int lanes, int act) {
+  if (n <= 4) return false;
   const bool exact = act == ACT_TANH || act == ACT_SIGMOID;
   return !(exact && p >= 4 && w == 1 && mode != FM_ANY) || (mode == FM_PLAIN && lanes <= 4);
 }
@@ -134,17 +139,20 @@ constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
 // m^k and m^-k: x = m^k X in the forward, x = m^-k X in the reverse sweep (k steps done), so that the
 // decay of the two streams costs no instruction per element (as in ncn_common.cuh, but without the
 // constant offsets, whose cancellation would cost accuracy over 32 steps).
+// The powers are those of 0.9 itself, not of its fp32 value: that one is 2.6e-8 off, the same way in every step (8e-7 of
+// the result after 32 steps, more than all roundings together).
 struct FeatPowers {
   float pos[33], neg[33];
 };
+constexpr double kFeatM = 0.9, kFeatC = 0.1;
 constexpr FeatPowers feat_powers() {
   FeatPowers t{};
   double a = 1.0, b = 1.0;
   for (int k = 0; k <= 32; ++k) {
     t.pos[k] = (float)a;
     t.neg[k] = (float)b;
-    a *= kMd;
-    b /= kMd;
+    a *= kFeatM;
+    b /= kFeatM;
   }
   return t;
 }
@@ -347,8 +355,8 @@ __device__ __forceinline__ void feat_forward_step(float2 (&X)[P][KP], float2 (&A
   const float mk = SC ? kPow.pos[k] : 1.0f, imk1 = SC ? kPow.neg[k + 1] : 1.0f;
   const float2 al = f2(alpha * sT * mk);
   const float ss = sT * mk * mk;
-  const float2 c1 = f2((float)(kCd * F::f1) * imk1);
-  [[maybe_unused]] const float2 c0 = f2((float)(kCd * F::f0) * imk1);
+  const float2 c1 = f2((float)((SC ? kFeatC : kCd) * F::f1) * imk1);
+  [[maybe_unused]] const float2 c0 = f2((float)((SC ? kFeatC : kCd) * F::f0) * imk1);
   float2 accj = f2(0.0f);
 #pragma unroll
   for (int q = 0; q < KP; ++q) accj = __ffma2_rn(xj[q], Wj[q], accj);
@@ -526,12 +534,12 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
   constexpr int P = G::P, SEG = G::SEG, KP = G::KP, D = G::D;
   constexpr bool REPLAY = MODE == FM_REPLAY, MASK = MODE == FM_MASK, CTX = MASK || (MODE == FM_ANY && G::GPW == 1);
   constexpr bool STORED = NC >= 16 && (MODE == FM_ANY || MODE == FM_STORED);
-  constexpr bool SC = feat_bwd_scaled(MODE, P, W, LD, ACT);
+  constexpr bool SC = feat_bwd_scaled(MODE, NC, P, W, LD, ACT);
   // (bf16 with one row per lane comes out slower without the test that is always true: 2048 x 256 x 128, groups of 8 618 ->
   // 651 us, 256 x 256 x 128, heads of 16, groups of 16 158 -> 163; elsewhere it costs, four rows 1044 -> 1033, fp32 178 -> 175)
   constexpr bool ALONE = W == 1 && (P > 1 || sizeof(T) == 4);
   constexpr float sT = (float)F::sT;
-  constexpr float cds = (float)(kCd * F::ds), cdsm = (float)(kCd * F::ds / kMd);
+  constexpr float cds = (float)(kCd * F::ds), cdsm = (float)(kFeatC * F::ds / kFeatM);
   constexpr bool COLS_SHFL = W == 1 && P == 1 && NC <= 4;  // (longer chains: 702 us by shared memory, 714 by shuffles)
   __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
   __shared__ __align__(16) float cs[G::TEAMS][2][W][G::XS];
@@ -765,8 +773,9 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
         const float cj = accj.x + accj.y;
         const float2 al = f2(p.alpha * sT * iq);
         const float ss = sT * iq * iq, sg = SC ? cdsm * iq : cds;
-        const float2 a1 = f2((float)(-kCd * F::f1 / (SC ? 1.0 : kMd)) * mk);
-        [[maybe_unused]] const float2 a0 = f2((float)(-kCd * F::f0 / (SC ? 1.0 : kMd)) * mk);
+        constexpr double ca = SC ? kFeatC : kCd / kMd;
+        const float2 a1 = f2((float)(-ca * F::f1) * mk);
+        [[maybe_unused]] const float2 a0 = f2((float)(-ca * F::f0) * mk);
         float gs[P];
         float2 uu[KP];  // sum_i sim_i gT_i of this lane's positions, per feature
 #pragma unroll

@@ -188,3 +188,21 @@ def test_stored_end_state_of_any_number_of_steps(n, heads, d):
     got = (y, ya, *ops.stage_bwd_mid(y, ya, mid, dy.cuda(), dya.cuda(), W.cuda(), ALPHA, 0, n, heads, 1))
     # results rounded to 2^-9; the weight gradient is not rounded, and its terms start from unrounded states
     _check(got, want, 2e-2)
+
+
+@pytest.mark.parametrize("activation", ["tanh", "linear"])
+@pytest.mark.parametrize("B,d,ctx", [(4, 32, False), (64, 32, False), (16, 64, False), (16, 24, False), (64, 32, True)])
+def test_forward_error_over_32_steps_is_that_of_roundings(B, d, ctx, activation):
+    """Each of 32 steps rounds a value a few times by 2^-25 of its size on average, independently: sqrt(32) * 2^-25 * 2 = 3.4e-7
+    in the mean.  The fp32 value of 0.9 alone, 2.6e-8 off in every step, would add 8e-7."""
+    import ncn_cuda_b200 as ncn
+
+    N, heads, n = 96, 2, 32
+    x, xa, W, dy, dya = _case(B, N, heads, d, seed=8)
+    cl = torch.full((B,), N, dtype=torch.int32)
+    Y, YA = O.stage_forward(x.double(), xa.double(), W.double(), ALPHA, activation, n, heads, 1)
+    act = ncn.ops.ACTIVATION_CODES[activation]
+    args = (x.cuda(), xa.cuda(), W.cuda())
+    y, ya = ncn.fused_ncn_cuda_ctxlen(*args, cl.cuda(), ALPHA, act, n, heads, 1) if ctx else ncn.fused_ncn_cuda_v2(*args, ALPHA, act, n, heads, 1)
+    for got, want in ((y, Y), (ya, YA)):
+        assert (got.double().cpu() - want).norm() / want.norm() < 3.5e-7
