@@ -4,12 +4,27 @@
 
 namespace ncn {
 
+template <int ACT, typename T, bool RAG, bool NANX>
+static cudaError_t launch_form(const LaneParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
+#ifdef NCN_BWD
+  auto k = lane_bwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads, RAG>;
+#else
+  auto k = lane_fwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneFwdBlocks * kLaneThreads / kLaneMaxThreads, RAG, NANX>;
+#endif
+  static SmemGrant granted;
+  cudaError_t e = grant_smem(granted, k, smem);
+  if (e != cudaSuccess) return e;
+  if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, smem);
+  k<<<grid, threads, smem, st>>>(p);
+  return cudaGetLastError();
+}
+
 template <int ACT, typename T>
 static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
 #ifdef NCN_BWD
 #if NCN_NG == 4
   if (p.pipelined) {  // two half-rows per thread, half a stage apart (ncn_lanes_pipe.cuh)
-    auto kp = lanep_bwd_kernel<NCN_NG, ACT, T, kLaneThreads, kLaneBwdBlocks>;
+    auto kp = lanep_bwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads>;
     static SmemGrant granted_p;
     cudaError_t ep = grant_smem(granted_p, kp, smem);
     if (ep != cudaSuccess) return ep;
@@ -18,11 +33,10 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
     return cudaGetLastError();
   }
 #endif
-  auto k = lane_bwd_kernel<NCN_NG, ACT, T, kLaneThreads, kLaneBwdBlocks>;
 #else
 #if NCN_NG == 4
   if (p.pipelined) {  // (A/B runs only: measured slower than lane_fwd_kernel)
-    auto kp = lanep_fwd_kernel<NCN_NG, ACT, T, kLaneThreads, kLaneBwdBlocks>;
+    auto kp = lanep_fwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads>;
     static SmemGrant granted_pf;
     cudaError_t ep = grant_smem(granted_pf, kp, smem);
     if (ep != cudaSuccess) return ep;
@@ -31,14 +45,12 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
     return cudaGetLastError();
   }
 #endif
-  auto k = lane_fwd_kernel<NCN_NG, ACT, T, kLaneThreads, kLaneFwdBlocks>;
 #endif
-  static SmemGrant granted;
-  cudaError_t e = grant_smem(granted, k, smem);
-  if (e != cudaSuccess) return e;
-  if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, smem);
-  k<<<grid, threads, smem, st>>>(p);
-  return cudaGetLastError();
+  if (p.ragged) return launch_form<ACT, T, true, true>(p, grid, threads, smem, st, occ);
+#ifndef NCN_BWD
+  if (p.tpr > kLaneThreads) return launch_form<ACT, T, false, true>(p, grid, threads, smem, st, occ);
+#endif
+  return launch_form<ACT, T, false, false>(p, grid, threads, smem, st, occ);
 }
 
 template <typename T>

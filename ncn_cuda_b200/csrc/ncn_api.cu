@@ -421,7 +421,7 @@ static bool lanep_enabled() { return !env_switches().lanes_pipe_off; }
 static bool lanes_enabled() { return !env_switches().lanes_off; }
 
 struct LanePlan {
-  int threads = 0, R = 0, grid = 0, tpr = 0, ea_max = 0, occ = 0;
+  int threads = 0, R = 0, grid = 0, tpr = 0, thr = 0, ragged = 0, ea_max = 0, occ = 0;
   size_t smem = 0;
   uint32_t off_work = 0, off_res = 0, off_ckpt = 0, off_halo = 0, off_red = 0, off_w = 0, off_bar = 0;
   uint32_t halo_warp_bytes = 0, n_ckpt_slots = 0;
@@ -435,24 +435,57 @@ static int lane_ilog2(long long v) {
   return e;
 }
 
-// The family covers: one feature per position, n in {2,4,8}, m = N/n a power of two with a whole
-// number of warps per row and at most one CTA of threads per row, and stage strides that do not
-// wrap (2^(l-1) < m for every stage), so that every change of stride is a shift by a power of two.
-static bool lane_shape_ok(int64_t N, int64_t E, int n, int C, int l0, int L, int dtype, int* e_needed_max) {
+// What a row looks like to the family.
+struct LaneShape {
+  int tpr, thr;    // threads per row (whole warps), threads that hold blocks
+  bool ragged;
+  int min_blocks;  // fewest blocks a warp holds
+  int e_need;      // log2 of the largest shift
+};
+
+// The family covers: one feature per position, n in {2,4,8}, an even number m = N/n of blocks, at most one CTA of
+// kLaneMaxThreads threads per row, and stage strides that do not wrap (2^(l-1) < m for every stage), so that every change
+// of stride is a shift by a power of two.  Rows of a power of two of blocks that fill whole warps have kernels of their own;
+// the ragged form pays for its idle lanes and takes a row only where the kernels of ncn_pairs.cuh / ncn_rows.cuh are
+// slower all the same (lane_ragged_pays).
+//
+// The line, measured (forward + backward time of the ragged form over theirs; 16.8 M elements, fp32, tanh; thr / tpr is the
+// share of lanes that work):
+//   n = 2  N 528 (0.52) 1.09, 640 (0.62) 1.05, 1040 (0.68) 0.97, 768 (0.75) 0.85, 2000 (0.98) 0.74; more than 2048 positions, where
+//          the others do not fit a row's pairs into a CTA: 0.52 .. 0.89
+//   n = 4  N 720 (0.70) 1.14, 1200 (0.78) 1.13, 2080 (0.81) 1.10, 1328 (0.86) 1.11, 4112 (0.89) 0.94, 480 (0.94) 0.94, 4000 (0.98) 0.95
+//   n = 8  N 640 (0.62) 1.21, 720 (0.70) 1.02, 1328 (0.86) 1.00, 480 (0.94) 0.86; four warps and more: 1600 (0.78) 0.86, 2080 (0.81)
+//          0.62, 3008 (0.98) 0.75, 5008 (0.98) 0.92
+static bool lane_ragged_pays(int n, int thr, int tpr) {
+  if (n == 2) return tpr > 128 || 100 * thr >= 66 * tpr;
+  return (n == 8 && tpr >= 128) || 100 * thr >= 88 * tpr;
+}
+static bool lane_shape_ok(int64_t N, int64_t E, int n, int C, int l0, int L, int dtype, LaneShape* sh) {
   if (E != 1 || C != 1 || lane_fn(n, false) == nullptr) return false;
-  if (N % n != 0) return false;
-  const int64_t m = N / n;
-  if (m <= 0 || (m & (m - 1)) != 0) return false;
-  const int G = lane_groups(n);
-  if (m % (32 * G) != 0 || m / G > kLaneThreads) return false;
+  if (N % n != 0 || N > (1 << 20)) return false;
+  const int m = (int)(N / n), G = lane_groups(n);
+  if (m % 2 != 0) return false;
   const int64_t quantum = dtype == DT_BF16 ? 8 : 4;
   if (N % quantum != 0) return false;
+  sh->thr = (m + G - 1) / G;
+  const int wpr = (sh->thr + 31) / 32;
+  sh->tpr = 32 * wpr;
+  if (sh->tpr > kLaneMaxThreads) return false;
+  sh->ragged = (m & (m - 1)) != 0 || m != sh->tpr * G;
+  sh->min_blocks = 32 * G;
+  if (sh->ragged) {
+    // a single stage stays where a NaN in xa alone reaches no other position of its group
+    if (L < 2 || !lane_ragged_pays(n, sh->thr, sh->tpr)) return false;
+    for (int w = 0; w < wpr; ++w) {  // as LaneShare (ncn_lanes.cuh) deals them
+      const int end = G * ((w + 1) * sh->thr / wpr), vb = (end < m ? end : m) - G * (w * sh->thr / wpr);
+      if (vb < sh->min_blocks) sh->min_blocks = vb;
+    }
+    if (sh->min_blocks < n) return false;
+  }
   const int last = l0 + L - 1;
-  if (last >= 1 && (last - 1) >= lane_ilog2(m)) return false;  // 2^(last-1) >= m: the stride wraps
+  if (last >= 1 && (last - 1) >= 31 - __builtin_clz((unsigned)m) + ((m & (m - 1)) != 0 ? 1 : 0)) return false;  // 2^(last-1) >= m: the stride wraps
   // largest shift: back from the last stride to 0 (2^(last-1)), or the first one up to stride(l0)
-  int emax = -1;
-  if (last >= 1) emax = last - 1;
-  *e_needed_max = emax;
+  sh->e_need = last >= 1 ? last - 1 : -1;
   return true;
 }
 
@@ -531,8 +564,9 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
                       int n_ck, const DevInfo& dev, int act, LanePlan& pl) {
   if (!lanes_enabled()) return NCN_ERR_UNSUPPORTED;
   if (flags & F_RECOMPUTE) return NCN_ERR_UNSUPPORTED;
-  int e_need = -1;
-  if (!lane_shape_ok(N, E, n, C, l0, L, dtype, &e_need)) return NCN_ERR_UNSUPPORTED;
+  LaneShape shape{};
+  if (!lane_shape_ok(N, E, n, C, l0, L, dtype, &shape)) return NCN_ERR_UNSUPPORTED;
+  const int e_need = shape.e_need;
   static std::mutex mu;
   static std::vector<std::pair<LaneKey, std::pair<int, LanePlan>>> cache;
   const LaneKey key{g_plan_epoch.load(), dev.dev, bwd ? 1 : 0, (int)N, n, L, l0, dtype, flags & (F_RESIDUAL | F_TAPE), n_ck, act, (long long)B};
@@ -545,8 +579,8 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
       }
   }
   const int G = lane_groups(n);
-  const int tpr = (int)(N / n) / G;
-  int R = kLaneThreads / tpr;
+  const int tpr = shape.tpr;
+  int R = tpr >= kLaneThreads ? 1 : kLaneThreads / tpr;
   {
     // A CTA is one barrier domain.  With plenty of tiles per CTA, halves of kLaneThreads do better (more,
     // smaller domains per SM drift apart and fill each other's waits: the 12-layer bf16 stack 89.7 -> 84.3 ms);
@@ -559,15 +593,17 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   if ((int64_t)R > B) R = (int)B;
   if (R < 1) R = 1;
   // the register budget allows kLane*Blocks CTAs of kLaneThreads threads: smaller CTAs, more of them
-  const int want_occ = (bwd ? kLaneBwdBlocks : kLaneFwdBlocks) * (kLaneThreads / (R * tpr));
+  const int want_occ = (bwd ? kLaneBwdBlocks : kLaneFwdBlocks) * kLaneThreads / (R * tpr);
   const int cap = lane_ea_cap(n);
   int ea_hi = e_need < cap ? e_need : cap;
-  int ea_lo = lane_ilog2(G) - 1;  // longer shifts through the tile buffer must be multiples of G blocks
+  // longer shifts through the tile buffer must be multiples of G blocks (ragged: even numbers)
+  int ea_lo = shape.ragged ? 0 : lane_ilog2(G) - 1;
+  while (shape.ragged && ea_hi > 0 && ((n - 1) << ea_hi) > shape.min_blocks) --ea_hi;
   if (ea_lo > ea_hi) ea_lo = ea_hi;
   int rc = NCN_ERR_UNSUPPORTED;
   LanePlan best;
   bool have_pipe = false;
-  if (n == 4 && (bwd ? lanep_enabled() : env_switches().lanes_pipe_fwd)) {
+  if (n == 4 && !shape.ragged && (bwd ? lanep_enabled() : env_switches().lanes_pipe_fwd)) {
     LanePlan trial;
     if (lanep_layout(bwd, (int)N, L, dtype, flags, n_ck, R, tpr, e_need, (uint32_t)dev.smem_optin, trial)) {
       int occ = 0;
@@ -588,6 +624,8 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
     if (!lane_layout(bwd, (int)N, n, L, dtype, flags, n_ck, R, tpr, ea, e_need, (uint32_t)dev.smem_optin, trial)) continue;
     int occ = 0;
     LaneParams dummy{};
+    dummy.ragged = shape.ragged ? 1 : 0;
+    dummy.tpr = tpr;
     cudaError_t e = lane_fn(n, bwd)(act, dtype, dummy, 0, trial.threads, trial.smem, nullptr, &occ);
     if (e != cudaSuccess) return cuda_fail(e);
     if (occ < 1) continue;
@@ -597,6 +635,8 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
     if (occ >= want_occ) break;
   }
   if (rc == NCN_OK) {
+    best.thr = shape.thr;
+    best.ragged = shape.ragged ? 1 : 0;
     best.tiles = (B + best.R - 1) / best.R;
     long long grid = (long long)dev.sms * best.occ;
     if (grid > best.tiles) grid = best.tiles;
@@ -612,7 +652,7 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
 }
 
 static void fill_lane(LaneParams& p, const LanePlan& pl) {
-  p.R = pl.R; p.tpr = pl.tpr; p.ea_max = pl.ea_max; p.tiles = pl.tiles;
+  p.R = pl.R; p.tpr = pl.tpr; p.thr = pl.thr; p.ragged = pl.ragged; p.ea_max = pl.ea_max; p.tiles = pl.tiles;
   p.off_work = pl.off_work; p.off_res = pl.off_res; p.off_ckpt = pl.off_ckpt; p.off_halo = pl.off_halo;
   p.off_red = pl.off_red; p.off_w = pl.off_w; p.off_bar = pl.off_bar;
   p.halo_warp_bytes = pl.halo_warp_bytes; p.n_ckpt_slots = pl.n_ckpt_slots;
@@ -1032,6 +1072,12 @@ int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya
     bool lanes = plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, dev, act, lp) == NCN_OK;
     if (lanes && n_ck > 0)
       lanes = plan_lanes(true, B, N, E, n_cache, n_head, first_module, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK;
+    // With tanh.approx the pair forward is as fast on ragged rows of 2 and 8 (1008 x 16.6 K rows, n = 2: 142 us against 148; 3264,
+    // n = 8: 152 against 157), where it fits.
+    if (lanes && lp.ragged && n_ck == 0 && dtype == DT_BF16 && n_cache != 4) {
+      Plan pp;
+      lanes = plan_rows(false, B, (int)N, n_cache, L, dtype, flags, 0, false, dev, act, pp) != NCN_OK || !pp.pair;
+    }
     if (lanes) {
       LaneParams q{};
       q.in[0] = x; q.in[1] = xa;

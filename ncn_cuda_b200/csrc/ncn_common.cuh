@@ -367,13 +367,13 @@ struct ActForm<ACT_LINEAR> {
 // BATCH: reciprocals taken from one special-function reciprocal of the product of BATCH values
 // (4: 1.25, 2: 1.5, 1: 2 special-function instructions per position and step; the smaller the batch
 // the fewer multiplies on the FMA pipe).
-template <int ACT, int NG, int BATCH, bool KEEP_NAN = false>
+// The exponent is capped at 30: beyond it r < 1e-9 (tanh = 1 to the last bit) and the product of four d stays a normal
+// fp32 number, as does its reciprocal.  A NaN reaches all values that share its reciprocal, where these would see it all
+// the same: the features of one position through their dot product, the positions of a group in the reverse sweep, which
+// the NaN joins when its position is x_j.  Without KEEP_NAN the cap drops it (r = 2^-30) and the caller sees to it.
+template <int ACT, int NG, int BATCH, bool KEEP_NAN = true>
 __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG]) {
   if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {
-    // r_i = 1 / d_i, d_i = 1 + 2^ts_i.  The exponent is capped at 30: beyond it r < 1e-9 (tanh = 1 to the last
-    // bit) and the product of four d stays a normal fp32 number, as does its reciprocal.  A NaN reaches all values that
-    // share its reciprocal.  KEEP_NAN: it may, because they are features of one position, whose dot product it is in
-    // already; the positions of a group need not see each other's NaN, and there the cap drops it (r = 2^-30).
     float2 d[NG];
 #pragma unroll
     for (int i = 0; i < NG; ++i) {
@@ -422,31 +422,31 @@ __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG
 }
 
 // forward offsets after k steps: C_k = sum_{i=1..k} c f0 / m^i ; D_k = sum_{i=1..k} c C_i
-constexpr double fwd_C(int k, double f0) {
+constexpr double fwd_C(int k, double f0, double md = kMd, double cd = kCd) {
   double C = 0.0;
-  for (int i = 1; i <= k; ++i) C += kCd * f0 / cpow(kMd, i);
+  for (int i = 1; i <= k; ++i) C += cd * f0 / cpow(md, i);
   return C;
 }
-constexpr double fwd_D(int k, double f0) {
+constexpr double fwd_D(int k, double f0, double md = kMd, double cd = kCd) {
   double C = 0.0, D = 0.0;
   for (int i = 1; i <= k; ++i) {
-    C += kCd * f0 / cpow(kMd, i);
-    D += kCd * C;
+    C += cd * f0 / cpow(md, i);
+    D += cd * C;
   }
   return D;
 }
 // reverse offsets after k inverse steps: x = m^-k (X + DX_k), a = m^-k (A + CA_k)
 //   CA_{k+1} = CA_k - c f0 m^k ;  DX_{k+1} = DX_k - c CA_k
-constexpr double bwd_CA(int k, double f0) {
+constexpr double bwd_CA(int k, double f0, double md = kMd, double cd = kCd) {
   double CA = 0.0;
-  for (int i = 0; i < k; ++i) CA -= kCd * f0 * cpow(kMd, i);
+  for (int i = 0; i < k; ++i) CA -= cd * f0 * cpow(md, i);
   return CA;
 }
-constexpr double bwd_DX(int k, double f0) {
+constexpr double bwd_DX(int k, double f0, double md = kMd, double cd = kCd) {
   double CA = 0.0, DX = 0.0;
   for (int i = 0; i < k; ++i) {
-    DX -= kCd * CA;
-    CA -= kCd * f0 * cpow(kMd, i);
+    DX -= cd * CA;
+    CA -= cd * f0 * cpow(md, i);
   }
   return DX;
 }

@@ -1,4 +1,4 @@
-// Register-resident fused row kernels (one feature per position, power-of-two block count).
+// Register-resident fused row kernels (one feature per position).
 //
 // The kernels of ncn_pairs.cuh send every stream of every position through shared memory at every
 // stage boundary.  Here a thread keeps its share of the row in registers for the whole stack:
@@ -17,6 +17,9 @@
 //   * tanh / sigmoid need r = 1 / (1 + 2^t) per position and step.  The n reciprocals of a group are
 //     taken four at a time from ONE special-function reciprocal of their product (Montgomery's
 //     trick): 1.25 instead of 2 special-function instructions per position and step.
+//
+// Two forms of each kernel: rows of a power of two of blocks that fill their warps, and any even number of blocks (RAG):
+// the last lanes of a warp may then hold nothing, and the length of a warp's share is a run-time value.
 //
 // Stored states (checkpoints) are written straight from registers, in the order [stream][offset][pair of
 // groups of the stage]; that order differs from the one of ncn_pairs.cuh / ncn_rows.cuh, so a forward
@@ -68,13 +71,42 @@ struct LaneBatch {
 };
 
 // ------------------------------------------------------------------ step math (scaled variables of ncn_common.cuh)
-template <int NG, int ACT, int J>
+// The powers of groups of 2 and 4 are those of 0.9 itself: its fp32 value is 2.6e-8 off, the same way in every step, which
+// after 20 steps is more than all roundings together (4096 positions, groups of 4, 6 stages, against fp64: y 6.7e-7 -> 2.2e-7, dx
+// 6.8e-7 -> 2.8e-7).  c is the fp32 value that the steps multiply by (kC): offsets made of another c would not cancel in the
+// inverse.  Groups of 8 keep the powers of the fp32 value: with them the roundings of the constants happen to cancel over long
+// walks back (40 steps from the output: dW within 4e-5 of its size, with those of 0.9 within 1.8e-4).
+template <int NG>
+constexpr double lane_m() { return NG == 8 ? kMd : 0.9; }
+constexpr double kLaneC = kCd;
+template <int NG>
+constexpr double lane_bwd_DX(int k, double f0) { return bwd_DX(k, f0, lane_m<NG>(), kLaneC); }
+
+// The constants of a forward stage as the steps use them, rounded to fp32, and those that undo it.  Groups of 2 and 4: the
+// latter are made of the former and not of the powers, or two independent roundings of m^n would leave a factor that every
+// earlier stage multiplies (32 steps back, groups of 4: dx 2.9e-6 -> 2.6e-6 of its size).
+template <int NG, int ACT>
+struct LaneStage {
+  using F = ActForm<ACT>;
+  static constexpr double m = lane_m<NG>();
+  static constexpr double mN = (double)(float)cpow(m, NG);
+  static constexpr double mNC = (double)(float)(cpow(m, NG) * fwd_C(NG, F::f0, m, kLaneC));
+  static constexpr double mND = (double)(float)(cpow(m, NG) * fwd_D(NG, F::f0, m, kLaneC));
+  static constexpr double cA(int J) { return (double)(float)(kLaneC * F::f1 / cpow(m, J + 1)); }
+  static constexpr bool own = NG != 8;
+  static constexpr double imN = own ? 1.0 / mN : 1.0 / cpow(m, NG);
+  static constexpr double imNDX = own ? (NG * (double)kC * mNC - mND) / mN : bwd_DX(NG, F::f0, m, kLaneC) / cpow(m, NG);
+  static constexpr double imNCA = own ? -mNC / mN : bwd_CA(NG, F::f0, m, kLaneC) / cpow(m, NG);
+  static constexpr double cAr(int J) { return own ? -mN * cA(J) : -kLaneC * F::f1 * cpow(m, NG - 1 - J); }
+};
+
+template <int NG, int ACT, int J, bool NANX>
 struct LFwdSteps {
   static __device__ __forceinline__ void run(float2 (&X)[NG], float2 (&A)[NG], const PairW& w) {
     using F = ActForm<ACT>;
-    constexpr float mk = (float)cpow(kMd, J);
-    constexpr float mkDk = (float)(cpow(kMd, J) * fwd_D(J, F::f0));
-    constexpr float cA = (float)(kCd * F::f1 / cpow(kMd, J + 1));
+    constexpr float mk = (float)cpow(lane_m<NG>(), J);
+    constexpr float mkDk = (float)(cpow(lane_m<NG>(), J) * fwd_D(J, F::f0, lane_m<NG>(), kLaneC));
+    constexpr float cA = (float)LaneStage<NG, ACT>::cA(J);
     float2 xj, P, Q;
     if constexpr (J == 0) {
       xj = X[0];
@@ -90,27 +122,42 @@ struct LFwdSteps {
     float2 ts[NG], r[NG];
 #pragma unroll
     for (int i = 0; i < NG; ++i) ts[i] = ffma2(X[i], P, Q);
-    act_r_all<ACT, NG, LaneBatch<NG>::fwd>(ts, r);
+    act_r_all<ACT, NG, LaneBatch<NG>::fwd, /*KEEP_NAN=*/!NANX>(ts, r);
+    // A NaN that is x_j reaches every position of the group through the constant; one elsewhere stays in its own x, and
+    // joins its a when the results are stored (lane_keep_nan).  |x_j| is never less than a negative constant.
+    float2 c = f2(cA);
+    if constexpr (NANX && ACT == ACT_TANH) c = make_float2(min_nan(cA, fabsf(xj.x)), min_nan(cA, fabsf(xj.y)));
+    if constexpr (NANX && ACT == ACT_SIGMOID) c = make_float2(-min_nan(-cA, fabsf(xj.x)), -min_nan(-cA, fabsf(xj.y)));
 #pragma unroll
     for (int i = 0; i < NG; ++i) {
-      A[i] = ffma2(r[i], f2(cA), A[i]);
+      A[i] = ffma2(r[i], c, A[i]);
       X[i] = ffma2(A[i], f2(kC), X[i]);
     }
-    LFwdSteps<NG, ACT, J + 1>::run(X, A, w);
+    LFwdSteps<NG, ACT, J + 1, NANX>::run(X, A, w);
   }
 };
-template <int NG, int ACT>
-struct LFwdSteps<NG, ACT, NG> {
+template <int NG, int ACT, bool NANX>
+struct LFwdSteps<NG, ACT, NG, NANX> {
   static __device__ __forceinline__ void run(float2 (&)[NG], float2 (&)[NG], const PairW&) {}
 };
 
+// a is NaN where x is (tanh and sigmoid drop it on the way).
 template <int NG, int ACT>
+__device__ __forceinline__ void lane_keep_nan(const float2 (&X)[NG], float2 (&A)[NG]) {
+  if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+      if (X[i].x != X[i].x) A[i].x = X[i].x;
+      if (X[i].y != X[i].y) A[i].y = X[i].y;
+    }
+  }
+}
+
+template <int NG, int ACT, bool NANX = false>
 __device__ __forceinline__ void lane_forward(float2 (&X)[NG], float2 (&A)[NG], const PairW& w) {
   using F = ActForm<ACT>;
-  LFwdSteps<NG, ACT, 0>::run(X, A, w);
-  constexpr float mN = (float)cpow(kMd, NG);
-  constexpr float mNC = (float)(cpow(kMd, NG) * fwd_C(NG, F::f0));
-  constexpr float mND = (float)(cpow(kMd, NG) * fwd_D(NG, F::f0));
+  LFwdSteps<NG, ACT, 0, NANX>::run(X, A, w);
+  constexpr float mN = (float)LaneStage<NG, ACT>::mN, mNC = (float)LaneStage<NG, ACT>::mNC, mND = (float)LaneStage<NG, ACT>::mND;
 #pragma unroll
   for (int i = 0; i < NG; ++i) {
     if constexpr (mND != 0.0f) X[i] = ffma2(X[i], f2(mN), f2(mND)); else X[i] = fmul2(X[i], f2(mN));
@@ -127,15 +174,15 @@ struct LBwdSteps {
                                              const PairWB& w, float2& dwi, float2& dwj) {
     using F = ActForm<ACT>;
     constexpr int k = NG - 1 - J;
-    constexpr double mkd = cpow(kMd, k);
-    constexpr float imk1 = (float)(1.0 / cpow(kMd, k + 1));
-    constexpr float DX1 = (float)bwd_DX(k + 1, F::f0);
-    constexpr float imk1DX1 = (float)(bwd_DX(k + 1, F::f0) / cpow(kMd, k + 1));
-    constexpr float cAr = (float)(-kCd * F::f1 * mkd);
-    constexpr float sTimk1 = (float)(F::sT / cpow(kMd, k + 1));
-    constexpr float cdsm = (float)(kCd * F::ds / kMd);
-    constexpr float K1 = (float)(kCd * F::ds / kMd / cpow(kMd, k + 1));  // c ds / m^(k+2)
-    constexpr float twomk1 = (float)(2.0 * cpow(kMd, k + 1));
+    constexpr double mkd = cpow(lane_m<NG>(), k);
+    constexpr float imk1 = (float)(1.0 / cpow(lane_m<NG>(), k + 1));
+    constexpr float DX1 = (float)lane_bwd_DX<NG>(k + 1, F::f0);
+    constexpr float imk1DX1 = (float)(lane_bwd_DX<NG>(k + 1, F::f0) / cpow(lane_m<NG>(), k + 1));
+    constexpr float cAr = (float)LaneStage<NG, ACT>::cAr(J);
+    constexpr float sTimk1 = (float)(F::sT / cpow(lane_m<NG>(), k + 1));
+    constexpr float cdsm = (float)(kLaneC * F::ds / lane_m<NG>());
+    constexpr float K1 = (float)(kLaneC * F::ds / lane_m<NG>() / cpow(lane_m<NG>(), k + 1));  // c ds / m^(k+2)
+    constexpr float twomk1 = (float)(2.0 * cpow(lane_m<NG>(), k + 1));
     constexpr float mk = (float)mkd;
 #pragma unroll
     for (int i = 0; i < NG; ++i) X[i] = ffma2(f2(-kC), A[i], X[i]);
@@ -189,10 +236,9 @@ __device__ __forceinline__ void lane_backward(float2 (&X)[NG], float2 (&A)[NG], 
                                               const PairWB& w, float2& dwi, float2& dwj) {
   using F = ActForm<ACT>;
   LBwdSteps<NG, ACT, NG - 1>::run(X, A, H, G, w, dwi, dwj);
-  constexpr float imN = (float)(1.0 / cpow(kMd, NG));
-  constexpr float imNDX = (float)(bwd_DX(NG, F::f0) / cpow(kMd, NG));
-  constexpr float imNCA = (float)(bwd_CA(NG, F::f0) / cpow(kMd, NG));
-  constexpr float mN = (float)cpow(kMd, NG);
+  using S = LaneStage<NG, ACT>;
+  constexpr float imN = (float)S::imN, imNDX = (float)S::imNDX, imNCA = (float)S::imNCA;
+  constexpr float mN = (float)cpow(lane_m<NG>(), NG);
 #pragma unroll
   for (int i = 0; i < NG; ++i) {
     if constexpr (imNDX != 0.0f) X[i] = ffma2(X[i], f2(imN), f2(imNDX)); else X[i] = fmul2(X[i], f2(imN));
@@ -201,13 +247,13 @@ __device__ __forceinline__ void lane_backward(float2 (&X)[NG], float2 (&A)[NG], 
     G[i] = fmul2(G[i], f2(mN));
   }
 }
-template <int ACT>
+template <int NG, int ACT>
 __device__ __forceinline__ float lane_dw_scale_i(float oma) {  // (1-alpha) c ds / m
-  return oma * (float)(kCd * ActForm<ACT>::ds / kMd);
+  return oma * (float)(kLaneC * ActForm<ACT>::ds / lane_m<NG>());
 }
 template <int ACT>
 __device__ __forceinline__ float lane_dw_scale_j(float oma) {  // (1-alpha) c ds
-  return oma * (float)(kCd * ActForm<ACT>::ds);
+  return oma * (float)(kLaneC * ActForm<ACT>::ds);
 }
 
 // ------------------------------------------------------------------ exchanges
@@ -225,12 +271,16 @@ __device__ __forceinline__ void cta_sync() { __syncthreads(); }
 
 // Shift of offset o by k = o 2^E blocks: the value of group j comes from D_o index + k (UP = false:
 // from higher threads) or - k (UP = true).  halo_pub / halo_nbr: this warp's and the source
-// neighbour's halo area of the current buffer (shared-window byte addresses).
-template <int NG, int G, int NS, int E, bool UP>
-__device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32_t halo_pub, uint32_t halo_nbr, int lane) {
+// neighbour's halo area of the current buffer (shared-window byte addresses).  RAG: the warp holds vb blocks, an even
+// number of at least (NG-1) 2^E, and its last lanes may hold none; the halo of a shift by k is exchanged by the blocks
+// c < k (UP: c >= vb - k) as in a full warp, with vb in the place of 32 G.
+template <int NG, int G, int NS, int E, bool UP, bool RAG>
+__device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32_t halo_pub, uint32_t halo_nbr, int lane, int vb) {
   constexpr int D = 1 << E;
   constexpr int HS = lane_halo_floats(NG, E);  // floats per stream
-  constexpr int CH = 32 * G;                   // blocks per warp
+  const int CH = RAG ? vb : 32 * G;            // blocks of the warp
+  // block c of the warp is one of the last k / block c + k lies in the next warp, as one of its first k
+  auto tail = [&](int c, int k) { return RAG ? (unsigned)(c - (CH - k)) < (unsigned)k : c >= CH - k; };
   if constexpr (E == 0 && G == 2) {
     // One pair per thread and shifts by k = o blocks.  The pair is published whole (for odd k one value more than
     // the neighbour reads); odd shifts swap the halves of a pair: x <- y of lane +- (k-1)/2, y <- x of lane +- (k+1)/2.
@@ -243,7 +293,7 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
           sts64_if(2 * lane < o, reg + 8u * (uint32_t)lane, V[s][0][o].x, V[s][0][o].y);
         } else {
           const int kb = (CH - o) & ~1;  // first published block, rounded down to a pair
-          sts64_if(2 * lane >= kb, reg + 4u * (uint32_t)(2 * lane - kb), V[s][0][o].x, V[s][0][o].y);
+          sts64_if(2 * lane >= kb && (!RAG || 2 * lane < CH), reg + 4u * (uint32_t)(2 * lane - kb), V[s][0][o].x, V[s][0][o].y);
         }
       }
     }
@@ -260,8 +310,8 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
           if (!UP) {
             n.x = qa > 0 ? __shfl_down_sync(0xffffffffu, v.y, qa) : v.y;
             n.y = __shfl_down_sync(0xffffffffu, v.x, qb);
-            lds32_if(lane + qa >= 32, reg + 4u * (uint32_t)(2 * lane + o - CH), n.x);
-            lds32_if(lane + qb >= 32, reg + 4u * (uint32_t)(2 * lane + o + 1 - CH), n.y);
+            lds32_if(RAG ? tail(2 * lane, o) : lane + qa >= 32, reg + 4u * (uint32_t)(2 * lane + o - CH), n.x);
+            lds32_if(RAG ? tail(2 * lane + 1, o) : lane + qb >= 32, reg + 4u * (uint32_t)(2 * lane + o + 1 - CH), n.y);
           } else {
             n.x = __shfl_up_sync(0xffffffffu, v.y, qb);
             n.y = qa > 0 ? __shfl_up_sync(0xffffffffu, v.x, qa) : v.x;
@@ -273,7 +323,7 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
           if (!UP) {
             n.x = __shfl_down_sync(0xffffffffu, v.x, q);
             n.y = __shfl_down_sync(0xffffffffu, v.y, q);
-            lds64_if(lane + q >= 32, reg + 8u * (uint32_t)(lane + q - 32), n);
+            lds64_if(RAG ? tail(2 * lane, o) : lane + q >= 32, reg + 4u * (uint32_t)(2 * lane + o - CH), n);
           } else {
             n.x = __shfl_up_sync(0xffffffffu, v.x, q);
             n.y = __shfl_up_sync(0xffffffffu, v.y, q);
@@ -300,7 +350,7 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
           if (!UP) {
             sts64_if(c < k, halo_pub + 4u * (uint32_t)(base + c), V[s][p][o].x, V[s][p][o].y);
           } else {
-            sts64_if(c >= CH - k, halo_pub + 4u * (uint32_t)(base + c - (CH - k)), V[s][p][o].x, V[s][p][o].y);
+            sts64_if(tail(c, k), halo_pub + 4u * (uint32_t)(base + c - (CH - k)), V[s][p][o].x, V[s][p][o].y);
           }
         }
       } else {
@@ -310,7 +360,7 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
           if (!UP) {
             sts32_if(c < k, halo_pub + 4u * (uint32_t)(base + c), lane_get<NG, G>(V[s], o, j));
           } else {
-            sts32_if(c >= CH - k, halo_pub + 4u * (uint32_t)(base + c - (CH - k)), lane_get<NG, G>(V[s], o, j));
+            sts32_if(tail(c, k), halo_pub + 4u * (uint32_t)(base + c - (CH - k)), lane_get<NG, G>(V[s], o, j));
           }
         }
       }
@@ -345,9 +395,9 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
         for (int p = 0; p < G / 2; ++p) {
           const int j = 2 * p;
           if (!UP) {
-            const int c = j + k, js = c % G, q = c / G;
+            const int c = j + k, q = c / G;
             float2 h = make_float2(nv[j], nv[j + 1]);
-            lds64_if(lane + q >= 32, halo_nbr + 4u * (uint32_t)(base + G * (lane + q - 32) + js), h);
+            lds64_if(RAG ? tail(c0 + j, k) : lane + q >= 32, halo_nbr + 4u * (uint32_t)(base + c0 + c - CH), h);
             nv[j] = h.x; nv[j + 1] = h.y;
           } else {
             const int c = j - k;
@@ -361,8 +411,8 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
 #pragma unroll
         for (int j = 0; j < G; ++j) {
           if (!UP) {
-            const int c = j + k, js = c % G, q = c / G;
-            lds32_if(lane + q >= 32, halo_nbr + 4u * (uint32_t)(base + G * (lane + q - 32) + js), nv[j]);
+            const int c = j + k, q = c / G;
+            lds32_if(RAG ? tail(c0 + j, k) : lane + q >= 32, halo_nbr + 4u * (uint32_t)(base + c0 + c - CH), nv[j]);
           } else {
             const int c = j - k;
             const int js = ((c % G) + G) % G, q = (js - c) / G;
@@ -376,10 +426,11 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
   }
 }
 
-// Shift by any multiple of G blocks per offset through the tile buffer, viewed as fp32 arrays
-// [stream][offset][m] of the row (row_addr: shared-window byte address of the row's part of it).
-template <int NG, int G, int NS>
-__device__ __forceinline__ void exchange_smem(float2 (&V)[NS][G / 2][NG], uint32_t row_addr, int t, int m, int delta) {
+// Shift by any multiple of G blocks (RAG: any even number) per offset through the tile buffer, viewed as fp32 arrays
+// [stream][offset][m] of the row (row_addr: shared-window byte address of the row's part of it).  blk: first block of the
+// thread, vg: how many of its G blocks exist.
+template <int NG, int G, int NS, bool RAG>
+__device__ __forceinline__ void exchange_smem(float2 (&V)[NS][G / 2][NG], uint32_t row_addr, int blk, int vg, int m, int delta) {
   const int mmask = m - 1;
 #pragma unroll
   for (int s = 0; s < NS; ++s) {
@@ -387,18 +438,29 @@ __device__ __forceinline__ void exchange_smem(float2 (&V)[NS][G / 2][NG], uint32
     for (int o = 1; o < NG; ++o) {
       const uint32_t arr = row_addr + 4u * (uint32_t)((s * NG + o) * m);
 #pragma unroll
-      for (int p = 0; p < G / 2; ++p) sts64(arr + 4u * (uint32_t)(G * t + 2 * p), V[s][p][o].x, V[s][p][o].y);
+      for (int p = 0; p < G / 2; ++p)
+        if (!RAG || 2 * p < vg) sts64(arr + 4u * (uint32_t)(blk + 2 * p), V[s][p][o].x, V[s][p][o].y);
     }
   }
   cta_sync();
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
+  for (int o = 1; o < NG; ++o) {
+    int src;
+    if (RAG) {
+      src = (blk + o * delta) % m;
+      if (src < 0) src += m;
+    } else {
+      src = (blk + o * delta) & mmask;  // multiple of G: the G values stay contiguous
+    }
 #pragma unroll
-    for (int o = 1; o < NG; ++o) {
+    for (int s = 0; s < NS; ++s) {
       const uint32_t arr = row_addr + 4u * (uint32_t)((s * NG + o) * m);
-      const int src = (G * t + o * delta) & mmask;  // multiple of G: the G values stay contiguous
 #pragma unroll
-      for (int p = 0; p < G / 2; ++p) V[s][p][o] = lds64(arr + 4u * (uint32_t)(src + 2 * p));
+      for (int p = 0; p < G / 2; ++p) {
+        int sp = src + 2 * p;
+        if (RAG && sp >= m) sp -= m;
+        if (!RAG || 2 * p < vg) V[s][p][o] = lds64(arr + 4u * (uint32_t)sp);
+      }
     }
   }
   cta_sync();
@@ -413,16 +475,38 @@ struct LaneHalo {
   int parity;
 };
 
+// What a thread holds of its row: blocks blk .. blk + vg - 1 (vg = G, RAG: or less, always an even number).  RAG: the
+// row's `thr` = ceil(m / G) chunks of G blocks are dealt to its warps as evenly as they go, so that no warp is left with
+// fewer blocks than a halo is long; vb blocks to this warp.
+template <int G, bool RAG>
+struct LaneShare {
+  int blk, vg, vb;
+  __device__ __forceinline__ LaneShare(int t, int lane, int wr, int wpr, int thr, int m) {
+    if (RAG) {
+      const int c0 = wr * thr / wpr, c1 = (wr + 1) * thr / wpr;
+      vb = min(m, G * c1) - G * c0;
+      blk = G * (c0 + lane);
+      vg = max(0, min(G, vb - G * lane));
+    } else {
+      blk = G * t;
+      vg = G;
+      vb = 32 * G;
+    }
+  }
+  __device__ __forceinline__ bool any() const { return !RAG || vg > 0; }
+  __device__ __forceinline__ bool pair(int p) const { return !RAG || 2 * p < vg; }
+};
+
 // delta = s_new - s_old (0, or +-2^e).  Shuffle exchange up to 2^ea_max, tile buffer beyond.
-template <int NG, int G, int NS>
+template <int NG, int G, int NS, bool RAG>
 __device__ __forceinline__ void lane_exchange(float2 (&V)[NS][G / 2][NG], int delta, int ea_max, LaneHalo& h, int lane,
-                                              uint32_t row_addr, int t, int m) {
+                                              uint32_t row_addr, const LaneShare<G, RAG>& sh, int m) {
   if (delta == 0) return;
   const bool up = delta < 0;
   const int ad = up ? -delta : delta;
   const int e = 31 - __clz(ad);
   if (e > ea_max) {
-    exchange_smem<NG, G, NS>(V, row_addr, t, m, delta);
+    exchange_smem<NG, G, NS, RAG>(V, row_addr, sh.blk, sh.vg, m, delta);
     return;
   }
   const uint32_t bufa = h.base + (uint32_t)h.parity * h.buf_bytes;
@@ -433,8 +517,8 @@ __device__ __forceinline__ void lane_exchange(float2 (&V)[NS][G / 2][NG], int de
   // one dense switch over (e, direction): a jump table instead of a chain of compares, each of which would be a
   // possibly divergent branch with its own reconvergence point
 #define NCN_LANE_CASE(EE)                                                                                   \
-  case 2 * EE: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, false>(V, pub, nbr, lane); break;      \
-  case 2 * EE + 1: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, true>(V, pub, nbr, lane); break;
+  case 2 * EE: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, false, RAG>(V, pub, nbr, lane, sh.vb); break; \
+  case 2 * EE + 1: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, true, RAG>(V, pub, nbr, lane, sh.vb); break;
   switch (2 * e + (up ? 1 : 0)) {
     NCN_LANE_CASE(0)
     NCN_LANE_CASE(1)
@@ -498,8 +582,8 @@ __device__ __forceinline__ void lane_ld_native(const T* chunk, float2 (&Sv)[G / 
       Sv[p][o] = make_float2(q[ea / EPS][ea % EPS], q[eb / EPS][eb % EPS]);
     }
 }
-template <int NG, int G, typename T>
-__device__ __forceinline__ void lane_st_native(T* chunk, const float2 (&Sv)[G / 2][NG], int t) {
+template <int NG, int G, typename T, bool RAG = false>
+__device__ __forceinline__ void lane_st_native(T* chunk, const float2 (&Sv)[G / 2][NG], int t, int vg = G) {
   using C = LaneChunk<NG, G, T>;
   constexpr int S = C::S, EPS = C::EPS;
   const int r = C::rot(t);
@@ -526,11 +610,14 @@ __device__ __forceinline__ void lane_st_native(T* chunk, const float2 (&Sv)[G / 
       for (int e = 0; e < EPS; ++e) q[i][e] = n[i][e];
   }
 #pragma unroll
-  for (int i = 0; i < S; ++i) st_vec<EPS>(chunk + ((i + r) & (S - 1)) * EPS, q[i]);  // q[i] = slot (i + r) mod S
+  for (int i = 0; i < S; ++i) {
+    const int slot = (i + r) & (S - 1);  // q[i] = slot (i + r) mod S
+    if (!RAG || slot * EPS < vg * NG) st_vec<EPS>(chunk + slot * EPS, q[i]);
+  }
 }
 
 // ------------------------------------------------------------------------------------------ forward
-template <int NG, int ACT, typename T, int MAXT, int MINB>
+template <int NG, int ACT, typename T, int MAXT, int MINB, bool RAG, bool NANX>
 __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
@@ -583,7 +670,8 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p
   halo.warp_dn = r * wpr + (wr == 0 ? wpr - 1 : wr - 1);
   halo.parity = 0;
   const uint32_t xrow = smem_u32(smem + p.off_work) + (uint32_t)r * (uint32_t)(2 * N) * 4u;  // fp32 [2][NG][m] per row
-  const int chunk = r * N + t * (G * NG);  // this thread's positions of the tile
+  const LaneShare<G, RAG> sh(t, lane, wr, wpr, p.thr, m);
+  const int chunk = r * N + sh.blk * NG;  // this thread's positions of the tile
   constexpr float sT = (float)F::sT;
   PairW w;
   w.alpha = f2(p.alpha * sT);
@@ -601,7 +689,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p
 
     const long long row0 = tile * R;
     const int rows = (int)min((long long)R, p.B - row0);
-    const bool active = r < rows;
+    const bool active = r < rows && sh.any();
 
     float2 V[2][G / 2][NG];  // x, xa
     if (active) {
@@ -629,20 +717,24 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p
     for (int l = 0; l < L; ++l) {
       const StageRec rec = rec_next;
       if (l + 1 < L) rec_next = recs[l + 1];
-      lane_exchange<NG, G, 2>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, t, m);
+      lane_exchange<NG, G, 2, RAG>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, sh, m);
       s_cur = rec.s;
       w.owi = f2(rec.owi * sT);
       w.owj = f2(rec.owj * sT);
 #pragma unroll
-      for (int pp = 0; pp < G / 2; ++pp) lane_forward<NG, ACT>(V[0][pp], V[1][pp], w);
+      for (int pp = 0; pp < G / 2; ++pp) lane_forward<NG, ACT, NANX>(V[0][pp], V[1][pp], w);
       if (rec.ck >= 0 && active) {
         // order of a stored state: [stream][offset][pair of groups], a pair = groups 2q, 2q+1 of the stage
-        float2* ck = ckpt + (long long)rec.ck * BN + (row0 + r) * N + (G / 2) * t;
+        float2* ck = ckpt + (long long)rec.ck * BN + (row0 + r) * N + (sh.blk >> 1);
 #pragma unroll
         for (int s = 0; s < 2; ++s)
 #pragma unroll
           for (int o = 0; o < NG; ++o) {
-            if constexpr (G >= 4) {  // a thread's pairs are neighbours in memory: whole 16-byte stores
+            if constexpr (RAG) {  // (m / 2 may be odd: no 16-byte alignment)
+#pragma unroll
+              for (int pp = 0; pp < G / 2; ++pp)
+                if (sh.pair(pp)) ck[(s * NG + o) * (m >> 1) + pp] = V[s][pp][o];
+            } else if constexpr (G >= 4) {  // a thread's pairs are neighbours in memory: whole 16-byte stores
 #pragma unroll
               for (int pp = 0; pp < G / 2; pp += 2)
                 *reinterpret_cast<float4*>(ck + (s * NG + o) * (m >> 1) + pp) =
@@ -653,7 +745,11 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p
           }
       }
     }
-    lane_exchange<NG, G, 2>(V, -s_cur, p.ea_max, halo, lane, xrow, t, m);  // back to stride 0 = native order
+    if constexpr (NANX) {
+#pragma unroll
+      for (int pp = 0; pp < G / 2; ++pp) lane_keep_nan<NG, ACT>(V[0][pp], V[1][pp]);
+    }
+    lane_exchange<NG, G, 2, RAG>(V, -s_cur, p.ea_max, halo, lane, xrow, sh, m);  // back to stride 0 = native order
     if (active) {
       if (residual) {
         float2 xin[G / 2][NG];
@@ -663,8 +759,8 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p
 #pragma unroll
           for (int o = 0; o < NG; ++o) V[0][pp][o] = fadd2(V[0][pp][o], xin[pp][o]);
       }
-      lane_st_native<NG, G, T>(win + chunk, V[0], t);
-      lane_st_native<NG, G, T>(win + RN + chunk, V[1], t);
+      lane_st_native<NG, G, T, RAG>(win + chunk, V[0], t, sh.vg);
+      lane_st_native<NG, G, T, RAG>(win + RN + chunk, V[1], t, sh.vg);
     }
     fence_proxy_async();
     __syncthreads();
@@ -684,7 +780,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p
 // ------------------------------------------------------------------------------------------ backward
 // From the net output (reversible inverse), from stored states (checkpoints, F_TAPE), F_RESIDUAL; no
 // forward replay.
-template <int NG, int ACT, typename T, int MAXT, int MINB>
+template <int NG, int ACT, typename T, int MAXT, int MINB, bool RAG>
 __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
@@ -743,12 +839,13 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
   halo.warp_dn = r * wpr + (wr == 0 ? wpr - 1 : wr - 1);
   halo.parity = 0;
   const uint32_t xrow = smem_u32(smem + p.off_work) + (uint32_t)r * (uint32_t)(4 * N) * 4u;  // fp32 [4][NG][m] per row
-  const int chunk = r * N + t * (G * NG);
+  const LaneShare<G, RAG> sh(t, lane, wr, wpr, p.thr, m);
+  const int chunk = r * N + sh.blk * NG;
   constexpr float sT = (float)F::sT;
   PairWB w;
   w.alpha = f2(p.alpha);
   w.oma = f2(p.oma);
-  const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
+  const float dsi = lane_dw_scale_i<NG, ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
   for (long long tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
@@ -763,7 +860,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
 
     const long long row0 = tile * R;
     const int rows = (int)min((long long)R, p.B - row0);
-    const bool active = r < rows;
+    const bool on_row = r < rows, active = on_row && sh.any();
 
     float2 V[4][G / 2][NG];  // x, xa, gx, ga
 #pragma unroll
@@ -796,23 +893,29 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
     for (int l = L - 1; l >= 0; --l) {
       const StageRec rec = rec_next;
       if (l > 0) rec_next = recs[l - 1];
-      lane_exchange<NG, G, 4>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, t, m);
+      lane_exchange<NG, G, 4, RAG>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, sh, m);
       s_cur = rec.s;
       w.owi = f2(rec.owi);
       w.owj = f2(rec.owj);
       w.owjs = f2(rec.owj * sT);
       if (rec.ck >= 0) {  // a state saved after stage l replaces the rebuilt one
-        const float2* c = sck + rec.ck * RN + r * N + (G / 2) * t;
+        const float2* c = sck + rec.ck * RN + r * N + (sh.blk >> 1);
 #pragma unroll
         for (int s = 0; s < 2; ++s)
 #pragma unroll
           for (int o = 0; o < NG; ++o)
 #pragma unroll
-            for (int pp = 0; pp < G / 2; ++pp) V[s][pp][o] = c[(s * NG + o) * (m >> 1) + pp];
+            for (int pp = 0; pp < G / 2; ++pp)
+              if (sh.pair(pp)) V[s][pp][o] = c[(s * NG + o) * (m >> 1) + pp];
       }
       float2 dwi = f2(0.0f), dwj = f2(0.0f);
 #pragma unroll
-      for (int pp = 0; pp < G / 2; ++pp) lane_backward<NG, ACT>(V[0][pp], V[1][pp], V[2][pp], V[3][pp], w, dwi, dwj);
+      for (int pp = 0; pp < G / 2; ++pp) {
+        // (RAG: a pair of blocks that does not exist computes on leftovers; its sums are dropped)
+        const float2 di = dwi, dj = dwj;
+        lane_backward<NG, ACT>(V[0][pp], V[1][pp], V[2][pp], V[3][pp], w, dwi, dwj);
+        if (!sh.pair(pp)) { dwi = di; dwj = dj; }
+      }
       // ---- weight-gradient partial of this stage: fixed-order warp tree, one slot per warp
       {
         const float di = (dwi.x + dwi.y) * dsi, dj = (dwj.x + dwj.y) * dsj;
@@ -822,10 +925,10 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
         keep += __shfl_xor_sync(0xffffffffu, give, 16);
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) keep += __shfl_xor_sync(0xffffffffu, keep, o);
-        if ((lane & 15) == 0 && active) red[(l * nwarp + warp) * 2 + (hi ? 1 : 0)] += keep;
+        if ((lane & 15) == 0 && on_row) red[(l * nwarp + warp) * 2 + (hi ? 1 : 0)] += keep;
       }
     }
-    lane_exchange<NG, G, 4>(V, -s_cur, p.ea_max, halo, lane, xrow, t, m);  // back to stride 0 = native order
+    lane_exchange<NG, G, 4, RAG>(V, -s_cur, p.ea_max, halo, lane, xrow, sh, m);  // back to stride 0 = native order
     if (active) {
       if (residual) {
         float2 gin[G / 2][NG];
@@ -835,11 +938,11 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
 #pragma unroll
           for (int o = 0; o < NG; ++o) V[2][pp][o] = fadd2(V[2][pp][o], gin[pp][o]);
       }
-      lane_st_native<NG, G, T>(win + chunk, V[2], t);
-      lane_st_native<NG, G, T>(win + RN + chunk, V[3], t);
+      lane_st_native<NG, G, T, RAG>(win + chunk, V[2], t, sh.vg);
+      lane_st_native<NG, G, T, RAG>(win + RN + chunk, V[3], t, sh.vg);
       if (want_rec) {
-        lane_st_native<NG, G, T>(win + 2 * RN + chunk, V[0], t);
-        lane_st_native<NG, G, T>(win + 3 * RN + chunk, V[1], t);
+        lane_st_native<NG, G, T, RAG>(win + 2 * RN + chunk, V[0], t, sh.vg);
+        lane_st_native<NG, G, T, RAG>(win + 3 * RN + chunk, V[1], t, sh.vg);
       }
     }
     fence_proxy_async();

@@ -14,7 +14,9 @@ struct LaneParams {
   long long B;
   long long tiles;
   int N, m, R, L, l0, ckpt_every, flags;
-  int tpr;             // threads per row (m / G), a multiple of 32
+  int tpr;             // threads per row, a multiple of 32
+  int thr;             // of these, the threads that hold blocks (ceil(m / G))
+  int ragged;          // any even number of blocks (else: a power of two that fills the warps)
   int ea_max;          // shifts of up to 2^ea_max blocks per offset use shuffles + halo, longer ones the tile buffer
   float alpha, oma;
   uint32_t off_work, off_res, off_ckpt, off_halo, off_red, off_w, off_bar;
@@ -44,7 +46,9 @@ __host__ __device__ constexpr int lane_halo_pair_base(int o) {
 // constant, so that every halo access is "per-thread base register + immediate".
 constexpr unsigned kPipeSo = 208;
 
-// Block size the kernels are compiled for, and the CTAs per SM their register budget allows.
+// Block size the kernels are compiled for (one row of up to 512 threads), block size of a tile of several rows, and how
+// many CTAs of the latter the register budget allows per SM.
+constexpr int kLaneMaxThreads = 512;
 constexpr int kLaneThreads = 256;
 constexpr int kLaneFwdBlocks = 4;
 constexpr int kLaneBwdBlocks = 2;

@@ -1,0 +1,104 @@
+"""Register-resident row kernels on rows that do not fill their warps, and on rows of 8192 positions: where a warp's
+share ends inside a thread's blocks, inside a warp and just behind one, halos as long as a warp's share, shifts through
+the tile buffer, several rows per CTA, a last tile that is not full.  Tolerances are those of test_gpu_sweep.py: 1e-5 (fp32) of
+the largest value, 2e-5 for the gradients of a walk back over more than 16 steps, 2e-2 (bf16)."""
+import pytest
+import torch
+
+from oracle import ncn_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ncn():
+    import ncn_cuda_b200
+
+    return ncn_cuda_b200
+
+
+def _data(B, N, n, L, dtype, seed):
+    x, xa, ws, dy, dya = O.make_inputs(seed, B, N, 1, L, 1.0 / n, dya_zero=False)
+    xa = torch.randn(B, N, 1, generator=torch.Generator().manual_seed(seed)) * 0.3
+    if dtype != torch.float32:
+        x, xa, dy, dya = (t.bfloat16().float() for t in (x, xa, dy, dya))
+    return x, xa, ws, dy, dya
+
+
+def _step(ncn, x, xa, ws, dy, dya, act, n, mode, dtype, first=0):
+    xd, xad = (t.cuda().to(dtype).requires_grad_() for t in (x, xa))
+    W = torch.stack(ws).cuda().requires_grad_()
+    y, ya = ncn.fused_ncn_net(xd, xad, W, 0.9, ncn.ops.ACTIVATION_CODES[act], n, 1, first_module=first, backward_mode=mode)
+    torch.autograd.backward([y, ya], [dy.cuda().to(dtype), dya.cuda().to(dtype)])
+    ncn.ops.device_status()
+    return [t.float().cpu() for t in (y.detach(), ya.detach(), xd.grad, xad.grad, W.grad)]
+
+
+# (n, N): blocks per row m = N / n in the comment
+SHAPES = [
+    (2, 248), (2, 264), (2, 1040), (2, 4088), (2, 8184), (2, 8192),  # m = 124, 132, 520, 2044, 4092, 4096
+    (4, 240), (4, 520), (4, 1032), (4, 3000), (4, 4104), (4, 8184), (4, 8192),  # m = 60, 130, 258, 750, 1026, 2046, 2048
+    (8, 256), (8, 272), (8, 528), (8, 1040), (8, 3008), (8, 8176), (8, 8192),  # m = 32, 34, 66, 130, 376, 1022, 1024
+]
+STAGES = {2: 9, 4: 6, 8: 4}
+
+
+@pytest.mark.parametrize("n,N", SHAPES)
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rows_of_any_even_number_of_blocks(ncn, n, N, dtype):
+    L = STAGES[n]
+    while 2 ** (L - 2) >= N // n:
+        L -= 1
+    x, xa, ws, dy, dya = _data(7, N, n, L, dtype, N + n)
+    ry, rya, rdx, rdxa, rdW = O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, "tanh", n, 1)
+    got = _step(ncn, x, xa, ws, dy, dya, "tanh", n, "auto", dtype)
+    for name, a, b in zip(("y", "ya", "dx", "dxa", "dW"), got, (ry, rya, rdx, rdxa, torch.stack(list(rdW)))):
+        assert O.rel_err(a, b) < (1e-5 if dtype == torch.float32 else 2e-2), name
+
+
+@pytest.mark.parametrize("n,N,B,act,mode,first", [
+    (4, 1048, 1, "linear", "checkpoint", 0), (4, 1048, 300, "sigmoid", "tape", 0), (4, 2984, 3, "relu", "invert", 2),
+    (8, 1040, 65, "tanh", "tape", 1), (2, 1044, 5, "tanh", "checkpoint", 3), (8, 8192, 2, "tanh", "invert", 0),
+])
+def test_modes_and_first_stages(ncn, n, N, B, act, mode, first):
+    L = {2: 5, 4: 3, 8: 2}[n]
+    x, xa, ws, dy, dya = _data(B, N, n, L, torch.float32, 3 * N + B)
+    ry, rya, rdx, rdxa, rdW = O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, act, n, 1, first_module=first)
+    got = _step(ncn, x, xa, ws, dy, dya, act, n, mode, torch.float32, first)
+    for name, a, b in zip(("y", "ya", "dx", "dxa", "dW"), got, (ry, rya, rdx, rdxa, torch.stack(list(rdW)))):
+        assert O.rel_err(a, b) < 1e-5, name
+
+
+def test_residual_layers_on_such_rows(ncn):
+    n, N, B, layers, L = 8, 1040, 9, 3, 3
+    stack = ncn.NCNResidualStack(layers, 0.9, "tanh", n, 1, L, 1).cuda()
+    W = torch.randn(layers, L, 2, generator=torch.Generator().manual_seed(5)) * n ** -0.5
+    with torch.no_grad():
+        stack.weight.copy_(W.cuda())
+    x, xa, _, dy, dya = _data(B, N, n, L, torch.float32, 77)
+    want = O.stack_fwd_bwd(x, xa, [list(w) for w in W], dy, dya, 0.9, "tanh", n, 1)
+    xd, xad = x.cuda().requires_grad_(), xa.cuda().requires_grad_()
+    y, ya = stack(xd, xad)
+    g = torch.autograd.grad((y, ya), (xd, xad, stack.weight), (dy.cuda(), dya.cuda()))
+    for a, b in zip((y, ya, g[0], g[1]), want[:4]):
+        assert O.rel_err(a.detach().cpu(), b) < 1e-5
+
+
+def test_the_weight_gradient_is_bitwise_repeatable(ncn):
+    x, xa, ws, dy, dya = _data(70, 3000, 4, 5, torch.float32, 11)
+    a, b = (_step(ncn, x, xa, ws, dy, dya, "tanh", 4, "auto", torch.float32) for _ in range(2))
+    assert all(torch.equal(p, q) for p, q in zip(a, b))
+
+
+@pytest.mark.parametrize("n,N", [(4, 1024), (4, 1048), (8, 1024), (8, 1040), (2, 1048)])
+def test_a_nan_reaches_the_groups_that_read_it_and_no_others(ncn, n, N):
+    L = 3
+    x, xa, ws, dy, dya = _data(3, N, n, L, torch.float32, 21)
+    x[1, 37] = float("nan")
+    xa[1, N - 2] = float("nan")
+    want = O.net_forward(x, xa, ws, 0.9, "tanh", n, 1)
+    W = torch.stack(ws).cuda()
+    with torch.no_grad():
+        got = ncn.fused_ncn_net(x.cuda(), xa.cuda(), W, 0.9, 0, n, 1)
+    for a, b in zip(got, want):
+        assert torch.equal(torch.isnan(a).cpu(), torch.isnan(b))
