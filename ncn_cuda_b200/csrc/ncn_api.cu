@@ -12,6 +12,7 @@
 #include "ncn_generic.cuh"
 #include "ncn_rows_launch.h"
 #include "ncn_lanes_launch.h"
+#include "ncn_solo_launch.h"
 #include "ncn_feat.cuh"
 #include "ncn_feat_launch.h"
 
@@ -651,6 +652,108 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   return rc;
 }
 
+// ---- one group per thread (ncn_solo.cuh)
+struct SoloPlan {
+  int threads = 0, R = 0, grid = 0, occ = 0;
+  size_t smem = 0;
+  uint32_t off_res = 0, off_red = 0, off_w = 0, off_bar = 0;
+  long long tiles = 0;
+};
+
+struct SoloKey {
+  int epoch, dev, bwd, N, n, L, dtype, residual, act;
+  long long B;
+  bool operator==(const SoloKey& o) const {
+    return epoch == o.epoch && dev == o.dev && bwd == o.bwd && N == o.N && n == o.n && L == o.L && dtype == o.dtype &&
+           residual == o.residual && act == o.act && B == o.B;
+  }
+};
+
+typedef cudaError_t (*SoloLaunchFn)(int, int, const SoloParams&, int, int, size_t, cudaStream_t, int*);
+
+static SoloLaunchFn solo_fn(int n, bool bwd) {
+  switch (n) {
+    case 8: return bwd ? launch_solo_bwd_n8 : launch_solo_fwd_n8;
+    case 16: return bwd ? launch_solo_bwd_n16 : launch_solo_fwd_n16;
+    default: return nullptr;
+  }
+}
+
+// Groups of 8 (where ncn_lanes.cuh does not take the row).  Measured against the shared-memory kernels, forward and backward,
+// 3 stages: fp32 2968 positions (371 blocks) 476 + 604 -> 322 + 610 us, 1048 (131) 191 + 256 -> 140 + 242, 720 (90) 303 + 530 ->
+// 265 + 450, 1200 (150) 250 + 449 -> 230 + 398, but 528 (66) 218 + 392 -> 230 + 401; bf16 2968 310 + 462 -> 222 + 490, 528
+// 138 + 274 -> 154 + 323, 1200 157 + 314 -> 154 + 327.
+static bool solo_pays_n8(bool bwd, int m, int dtype) {
+  if (dtype == DT_BF16) return m % 2 != 0 && !bwd;  // (stored states have the same order in either family)
+  return m % 2 != 0 || m >= 80;
+}
+
+// NCN_OK with pl filled, NCN_ERR_UNSUPPORTED when the kernels do not cover the arguments.  The kernels take whole rows, a
+// thread per group, one CTA at most.  Remembered per argument set.
+static int plan_solo(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, int L, int dtype, int flags, const DevInfo& dev, int act,
+                     SoloPlan& pl) {
+  if (!lanes_enabled() || (flags & F_RECOMPUTE) || solo_fn(n, bwd) == nullptr || !rows_shape_ok(N, E, n, C, dtype)) return NCN_ERR_UNSUPPORTED;
+  const int m = (int)(N / n);
+  if (N % n != 0 || m > kSoloThreads) return NCN_ERR_UNSUPPORTED;
+  if (n == 8 && !solo_pays_n8(bwd, m, dtype)) return NCN_ERR_UNSUPPORTED;
+  static std::mutex mu;
+  static std::vector<std::pair<SoloKey, std::pair<int, SoloPlan>>> cache;
+  const SoloKey key{g_plan_epoch.load(), dev.dev, bwd ? 1 : 0, (int)N, n, L, dtype, (flags & F_RESIDUAL) != 0, act, (long long)B};
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    for (auto& kv : cache)
+      if (kv.first == key) {
+        pl = kv.second.second;
+        return kv.second.first;
+      }
+  }
+  const int w = dtype == DT_BF16 ? 2 : 4;
+  // Rows per CTA: as many as make up 128 threads (small CTAs are small barrier domains), one more where that wastes fewer
+  // lanes of the last warp; no more than leave every SM a tile.
+  int R = m >= 128 ? 1 : 128 / m;
+  if (R < 4 && R * m % 32 != 0 && (R + 1) * m <= 256) {
+    auto used = [&](int rr) { return (double)(rr * m) / (((rr * m + 31) / 32) * 32); };
+    if (used(R + 1) > used(R) + 0.05) ++R;
+  }
+  if (R > 1 && B < (int64_t)R * dev.sms) R = B < dev.sms ? 1 : (int)(B / dev.sms);
+  SoloPlan p;
+  int rc = NCN_ERR_UNSUPPORTED;
+  const int warps = (R * m + 31) / 32;
+  uint64_t off = 0;
+  auto take = [&](uint64_t bytes) { uint64_t o = off; off = (off + bytes + 127) / 128 * 128; return (uint32_t)o; };
+  take((uint64_t)R * N * (bwd ? 16 : 8));
+  p.off_res = (flags & F_RESIDUAL) ? take((uint64_t)R * N * w) : 0;
+  p.off_red = take(bwd ? (uint64_t)2 * L * warps * 4 : 16);
+  p.off_w = take((uint64_t)16 * L);
+  p.off_bar = take(32);
+  if (off <= (uint64_t)dev.smem_optin) {
+    p.threads = warps * 32; p.R = R; p.smem = (size_t)off;
+    SoloParams dummy{};
+    cudaError_t e = solo_fn(n, bwd)(act, dtype, dummy, 0, p.threads, p.smem, nullptr, &p.occ);
+    if (e != cudaSuccess) return cuda_fail(e);
+    if (p.occ >= 1) {
+      p.tiles = (B + R - 1) / R;
+      long long grid = (long long)dev.sms * (p.occ > 32 ? 32 : p.occ);
+      p.grid = (int)(grid > p.tiles ? p.tiles : grid);
+      rc = NCN_OK;
+    }
+  }
+  pl = p;
+  std::lock_guard<std::mutex> lk(mu);
+  if (cache.size() >= 64) cache.erase(cache.begin());
+  cache.emplace_back(key, std::make_pair(rc, pl));
+  return rc;
+}
+
+static void fill_solo(SoloParams& p, const SoloPlan& pl, int64_t B, int64_t N, int n, int L, int first, double alpha, int flags) {
+  p.B = B; p.N = (int)N; p.m = (int)(N / n); p.L = L; p.l0 = first;
+  p.flags = flags & (F_RESIDUAL | F_TAPE);
+  p.alpha = (float)alpha;
+  p.oma = (float)(1.0 - alpha);
+  p.R = pl.R; p.tiles = pl.tiles;
+  p.off_res = pl.off_res; p.off_red = pl.off_red; p.off_w = pl.off_w; p.off_bar = pl.off_bar;
+}
+
 static void fill_lane(LaneParams& p, const LanePlan& pl) {
   p.R = pl.R; p.tpr = pl.tpr; p.thr = pl.thr; p.ragged = pl.ragged; p.ea_max = pl.ea_max; p.tiles = pl.tiles;
   p.off_work = pl.off_work; p.off_res = pl.off_res; p.off_ckpt = pl.off_ckpt; p.off_halo = pl.off_halo;
@@ -1017,16 +1120,21 @@ int ncn_net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, 
   Plan pl;
   if ((flags & F_TAPE) && (flags & F_RECOMPUTE)) return 0;
   const int n_ck = (flags & F_RECOMPUTE) ? 0 : ckpt_slots(L, ckpt_every, flags);
-  {
-    LanePlan lf, lb;
-    const int act = fused_act(ACT_TANH, dtype);
-    if (plan_lanes(false, B, N, E, n_cache, n_head, 0, L, dtype, flags, 0, dev, act, lf) == NCN_OK &&
-        plan_lanes(true, B, N, E, n_cache, n_head, 0, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK)
-      return 1;
-  }
-  if (plan_rows(false, B, (int)N, n_cache, L, dtype, flags, 0, false, dev, ACT_TANH, pl) != NCN_OK) return 0;
-  if (plan_rows(true, B, (int)N, n_cache, L, dtype, flags, n_ck, false, dev, ACT_TANH, pl) != NCN_OK) return 0;
-  return 1;
+  if (plan_rows(false, B, (int)N, n_cache, L, dtype, flags, 0, false, dev, ACT_TANH, pl) == NCN_OK &&
+      plan_rows(true, B, (int)N, n_cache, L, dtype, flags, n_ck, false, dev, ACT_TANH, pl) == NCN_OK)
+    return 1;
+  // Rows that only the kernels below take (8192 fp32 positions): where the walk back would be longer than kSegment steps
+  // between two stored states, stage by stage (from each stage's own output) is the more accurate way.
+  const int walk = n_cache * (ckpt_every > 0 && ckpt_every < L ? ckpt_every : L);
+  if (dtype == DT_F32 && walk > kSegment) return 0;
+  const int act = fused_act(ACT_TANH, dtype);
+  LanePlan lf, lb;
+  if (plan_lanes(false, B, N, E, n_cache, n_head, 0, L, dtype, flags, 0, dev, act, lf) == NCN_OK &&
+      plan_lanes(true, B, N, E, n_cache, n_head, 0, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK)
+    return 1;
+  SoloPlan sf, sb;  // (groups of 8: all rows that fit these fit the shared-memory kernels)
+  return plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sf) == NCN_OK &&
+         plan_solo(true, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sb) == NCN_OK;
 }
 
 int ncn_gather_weights(const float* const* weights, int L, int64_t cols, float* out, void* stream) {
@@ -1096,6 +1204,21 @@ int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya
       return e == cudaSuccess ? NCN_OK : cuda_fail(e);
     }
   }
+  {
+    SoloPlan sp;
+    if (plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sp) == NCN_OK) {
+      SoloParams q{};
+      q.in[0] = x; q.in[1] = xa;
+      q.out[0] = y; q.out[1] = ya;
+      q.ckpt = ck_used;
+      q.ckpt_every = ckpt_every;
+      q.W = W;
+      q.status = dev.status;
+      fill_solo(q, sp, B, N, n_cache, L, first_module, alpha, flags);
+      cudaError_t e = solo_fn(n_cache, false)(act, dtype, q, sp.grid, sp.threads, sp.smem, (cudaStream_t)stream, nullptr);
+      return e == cudaSuccess ? NCN_OK : cuda_fail(e);
+    }
+  }
   Plan pl;
   if ((rc = plan_rows(false, B, (int)N, n_cache, L, dtype, flags, 0, false, dev, act, pl)) != NCN_OK) return rc;
   RowsParams p{};
@@ -1141,6 +1264,17 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
   const int act = fused_act(map_act(activation), dtype);
   const bool use_ck = ckpt && !(flags & F_RECOMPUTE) && ckpt_slots(L, ckpt_every, flags) > 0;
   const int n_ck = use_ck ? ckpt_slots(L, ckpt_every, flags) : 0;
+  // One row of 2L partial sums per CTA.  The fixed array of ncn_net_bwd_noalloc takes what the shared-memory kernels need
+  // for the same arguments: kernels with more CTAs launch fewer where they would not fit.
+  auto fit_grid = [&](int& grid) {
+    if ((size_t)grid * 2 * (size_t)L <= capacity_floats) return (int)NCN_OK;
+    Plan pr;
+    if (plan_rows(true, B, (int)N, n_cache, L, dtype, flags, n_ck, x_rec != nullptr, dev, act, pr) == NCN_OK &&
+        (size_t)pr.grid * 2 * (size_t)L > capacity_floats)
+      return short_err;
+    grid = (int)(capacity_floats / (2 * (size_t)L));
+    return grid >= 1 ? (int)NCN_OK : short_err;
+  };
   {
     // register-resident family (with stored states: only where the forward is of this family too)
     LanePlan lp, lf;
@@ -1148,7 +1282,11 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
     if (lanes && n_ck > 0)
       lanes = plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, dev, act, lf) == NCN_OK;
     if (lanes) {
-      if ((size_t)lp.grid * 2 * (size_t)L > capacity_floats) return short_err;
+      if (lp.ragged || lp.tpr > kLaneThreads) {
+        if ((rc = fit_grid(lp.grid)) != NCN_OK) return rc;
+      } else if ((size_t)lp.grid * 2 * (size_t)L > capacity_floats) {
+        return short_err;
+      }
       LaneParams q{};
       q.in[0] = s0; q.in[1] = s1; q.in[2] = dy; q.in[3] = dya;
       q.out[0] = dx; q.out[1] = dxa; q.out[2] = x_rec; q.out[3] = xa_rec;
@@ -1165,6 +1303,25 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
       cudaError_t e = lane_fn(n_cache, true)(act, dtype, q, lp.grid, lp.threads, lp.smem, (cudaStream_t)stream, nullptr);
       if (e != cudaSuccess) return cuda_fail(e);
       return reduce_dw(partials, dW, lp.grid, 2 * L, dw_accumulate, (cudaStream_t)stream);
+    }
+  }
+  {
+    SoloPlan sp;
+    if (plan_solo(true, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sp) == NCN_OK) {
+      if ((rc = fit_grid(sp.grid)) != NCN_OK) return rc;
+      SoloParams q{};
+      q.in[0] = s0; q.in[1] = s1; q.in[2] = dy; q.in[3] = dya;
+      q.out[0] = dx; q.out[1] = dxa; q.out[2] = x_rec; q.out[3] = xa_rec;
+      q.ckpt = use_ck ? const_cast<float*>(ckpt) : nullptr;
+      q.ckpt_every = ckpt_every;
+      q.n_ckpt = n_ck;
+      q.W = W;
+      q.partials = partials;
+      q.status = dev.status;
+      fill_solo(q, sp, B, N, n_cache, L, first_module, alpha, flags);
+      cudaError_t e = solo_fn(n_cache, true)(act, dtype, q, sp.grid, sp.threads, sp.smem, (cudaStream_t)stream, nullptr);
+      if (e != cudaSuccess) return cuda_fail(e);
+      return reduce_dw(partials, dW, sp.grid, 2 * L, dw_accumulate, (cudaStream_t)stream);
     }
   }
   Plan pl;

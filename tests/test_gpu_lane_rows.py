@@ -1,4 +1,5 @@
-"""Register-resident row kernels on rows that do not fill their warps, and on rows of 8192 positions: where a warp's
+"""Register-resident row kernels on rows that do not fill their warps, on rows of 8192 positions, and with one group per
+thread: where a warp's
 share ends inside a thread's blocks, inside a warp and just behind one, halos as long as a warp's share, shifts through
 the tile buffer, several rows per CTA, a last tile that is not full.  Tolerances are those of test_gpu_sweep.py: 1e-5 (fp32) of
 the largest value, 2e-5 for the gradients of a walk back over more than 16 steps, 2e-2 (bf16)."""
@@ -69,8 +70,43 @@ def test_modes_and_first_stages(ncn, n, N, B, act, mode, first):
         assert O.rel_err(a, b) < 1e-5, name
 
 
-def test_residual_layers_on_such_rows(ncn):
-    n, N, B, layers, L = 8, 1040, 9, 3, 3
+@pytest.mark.parametrize("n,N", [(16, 16), (16, 48), (16, 240), (16, 512), (16, 528), (16, 1840), (16, 2048), (16, 2080), (16, 8176),
+                                 (16, 8192), (8, 8), (8, 1048), (8, 2968), (8, 4088)])  # 1, 3, 15, 32, 33, 115 ... 512 blocks
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_one_group_per_thread(ncn, n, N, dtype):
+    L = 4 if n == 16 else 5  # strides 0, 1, 2, 4 (8) mod m: rows of a few blocks wrap
+    x, xa, ws, dy, dya = _data(11, N, n, L, dtype, N)
+    ry, rya, rdx, rdxa, rdW = O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, "tanh", n, 1)
+    got = _step(ncn, x, xa, ws, dy, dya, "tanh", n, "auto", dtype)
+    for name, a, b in zip(("y", "ya", "dx", "dxa", "dW"), got, (ry, rya, rdx, rdxa, torch.stack(list(rdW)))):
+        assert O.rel_err(a, b) < (1e-5 if dtype == torch.float32 else 2e-2), name
+
+
+@pytest.mark.parametrize("n,N,B,act,mode,first,L", [
+    (16, 1840, 1, "linear", "checkpoint", 0, 3), (16, 240, 700, "sigmoid", "tape", 0, 2), (16, 2048, 3, "relu", "checkpoint", 2, 2),
+    (16, 1040, 5, "tanh", "invert", 1, 1), (16, 1040, 5, "tanh", "invert", 0, 2), (8, 1048, 5, "sigmoid", "checkpoint", 1, 3),
+])
+def test_one_group_per_thread_modes(ncn, n, N, B, act, mode, first, L):
+    x, xa, ws, dy, dya = _data(B, N, n, L, torch.float32, 5 * N + B)
+    ry, rya, rdx, rdxa, rdW = O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, act, n, 1, first_module=first)
+    got = _step(ncn, x, xa, ws, dy, dya, act, n, mode, torch.float32, first)
+    tol = 2e-5 if mode == "invert" and n * L > 16 else 1e-5
+    for name, a, b in zip(("y", "ya", "dx", "dxa", "dW"), got, (ry, rya, rdx, rdxa, torch.stack(list(rdW)))):
+        assert O.rel_err(a, b) < tol, name
+
+
+def test_long_walks_back_stay_stage_by_stage(ncn):
+    """8192 fp32 positions: fused where stored states keep a walk back to 16 steps, else a kernel per stage."""
+    x = torch.empty(2, 8192, 1, device="cuda")
+    for n in (2, 4, 8, 16):
+        assert ncn.ops.net_supported(x, n, 1, 4, 0, 16 // n)
+        assert not ncn.ops.net_supported(x, n, 1, 16 // n + 1, 0, 0)
+        assert ncn.ops.net_supported(x, n, 1, 16 // n, 0, 0)
+
+
+@pytest.mark.parametrize("n,N", [(8, 1040), (16, 1840)])
+def test_residual_layers_on_such_rows(ncn, n, N):
+    B, layers, L = 9, 3, 3 if n == 8 else 2
     stack = ncn.NCNResidualStack(layers, 0.9, "tanh", n, 1, L, 1).cuda()
     W = torch.randn(layers, L, 2, generator=torch.Generator().manual_seed(5)) * n ** -0.5
     with torch.no_grad():
@@ -84,13 +120,14 @@ def test_residual_layers_on_such_rows(ncn):
         assert O.rel_err(a.detach().cpu(), b) < 1e-5
 
 
-def test_the_weight_gradient_is_bitwise_repeatable(ncn):
-    x, xa, ws, dy, dya = _data(70, 3000, 4, 5, torch.float32, 11)
-    a, b = (_step(ncn, x, xa, ws, dy, dya, "tanh", 4, "auto", torch.float32) for _ in range(2))
+@pytest.mark.parametrize("n,N", [(4, 3000), (16, 1840)])
+def test_the_weight_gradient_is_bitwise_repeatable(ncn, n, N):
+    x, xa, ws, dy, dya = _data(70, N, n, 4, torch.float32, 11)
+    a, b = (_step(ncn, x, xa, ws, dy, dya, "tanh", n, "auto", torch.float32) for _ in range(2))
     assert all(torch.equal(p, q) for p, q in zip(a, b))
 
 
-@pytest.mark.parametrize("n,N", [(4, 1024), (4, 1048), (8, 1024), (8, 1040), (2, 1048)])
+@pytest.mark.parametrize("n,N", [(4, 1024), (4, 1048), (8, 1024), (8, 1040), (8, 1048), (2, 1048), (16, 1840)])
 def test_a_nan_reaches_the_groups_that_read_it_and_no_others(ncn, n, N):
     L = 3
     x, xa, ws, dy, dya = _data(3, N, n, L, torch.float32, 21)
