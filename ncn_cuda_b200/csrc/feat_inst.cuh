@@ -36,6 +36,9 @@ static cudaError_t launch_one(const FeatParamsX& p, int grid, int threads, cudaS
   if constexpr (SEVERAL && !BF16) {
     if (ctx) return go(NCN_KERNEL<NCN_NC, LD, KF, W, ACT, T, FM_MASK>, p);
   }
+  if constexpr (!SEVERAL && !BF16) {
+    if (ctx && p.even) return go(NCN_KERNEL<NCN_NC, LD, KF, W, ACT, T, FM_CTX>, p);
+  }
   if constexpr (OWN_PLAIN) {
     const FeatParams& plain = p;
     if (!ctx && !stored) return go(NCN_KERNEL<NCN_NC, LD, KF, W, ACT, T, FM_PLAIN>, plain);

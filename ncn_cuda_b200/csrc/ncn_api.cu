@@ -926,6 +926,7 @@ static int launch_feat(bool bwd, const void* const* in, void* const* out, const 
   p.alpha = (float)alpha;
   p.oma = (float)(1.0 - alpha);
   const long long want_teams = p.units * C;
+  p.even = p.ctxlen != nullptr && feat_ctx_even(B, want_teams, dev.sms);
   const int team = feat_team(rows, bwd, want_teams, dev.sms);
   // few groups (the reference's own bench has 128): smaller CTAs, so that the teams spread over all SMs
   int tpc = kFeatWarps / team;
@@ -942,7 +943,8 @@ static int launch_feat(bool bwd, const void* const* in, void* const* out, const 
   };
   static std::mutex mu;
   static std::vector<Seen> seen;
-  Seen key{fn, d, team, act, dtype, p.saved, p.mid != nullptr, p.ctxlen != nullptr, threads, dev.dev, -1};
+  const int ctx = p.ctxlen == nullptr ? 0 : p.even ? 1 : 2;
+  Seen key{fn, d, team, act, dtype, p.saved, p.mid != nullptr, ctx, threads, dev.dev, -1};
   {
     std::lock_guard<std::mutex> lk(mu);
     for (const Seen& q : seen)

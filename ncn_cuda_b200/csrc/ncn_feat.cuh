@@ -43,6 +43,7 @@ struct FeatParams {
 // What the kernels beyond the plain call take as well.
 struct FeatParamsX : FeatParams {
   const int* ctxlen;  // [B] context length per batch row, or null
+  int even;           // with ctxlen: the groups that take steps are dealt out evenly (FM_CTX)
   const void* xin[2]; // bwd with the stage input saved: x, xa
   float* mid;         // fp32 states after every 16th step: state k, stream s at mid + (2k + s) * bne, in the
                       // element order of the activations (fwd: written if not null; bwd with saved == 3: read)
@@ -57,7 +58,8 @@ enum FeatMode : int {
   FM_PLAIN,   // neither
   FM_STORED,  // stored states
   FM_REPLAY,  // backward: states replayed from the saved stage input
-  FM_MASK     // context lengths, groups with different numbers of steps side by side in a warp
+  FM_MASK,    // context lengths, groups with different numbers of steps side by side in a warp
+  FM_CTX      // context lengths, one group per team at a time, the groups that take steps dealt out evenly (FeatUnits)
 };
 template <int MODE>
 using FeatArgs = std::conditional_t<MODE == FM_PLAIN, FeatParams, FeatParamsX>;
@@ -123,17 +125,17 @@ constexpr bool feat_bwd_own(int mode, int n, int p, int w, int lanes, bool bf16)
 // Groups of 2 and 4 save next to nothing by it, and the multiplications back to true scale cost them 10 per cent in accuracy.
 constexpr bool feat_fwd_scaled(int mode, int n, int p, int w) {
   if (n <= 4) return false;
-  return mode == FM_ANY || mode == FM_MASK || p > 1 || w > 1 || feat_unrolled(n, p, w);
+  return mode == FM_ANY || mode == FM_MASK || mode == FM_CTX || p > 1 || w > 1 || feat_unrolled(n, p, w);
 }
 constexpr bool feat_bwd_scaled(int mode, int n, int p, int w, int lanes, int act) {
   if (n <= 4) return false;
   const bool exact = act == ACT_TANH || act == ACT_SIGMOID;
-  return !(exact && p >= 4 && w == 1 && mode != FM_ANY) || (mode == FM_PLAIN && lanes <= 4);
+  return !(exact && p >= 4 && w == 1 && mode != FM_ANY && mode != FM_CTX) || (mode == FM_PLAIN && lanes <= 4);
 }
 // Reciprocals of tanh / sigmoid that share one special-function reciprocal in the backward (act_r_all, ncn_common.cuh; 0 =
 // one each; the forward takes four): context lengths, four rows (64 x 256 x 128): two 85 us, single 86.5; the kernels of
 // their own 1040 -> 1030 with single ones (groups of 32), 1024 x 512 x 256, groups of 16 (two rows): 2346 -> 2279.
-constexpr int feat_bwd_batch(int mode, int p, int w) { return p >= 4 && (w > 1 || mode == FM_ANY) ? 2 : 0; }
+constexpr int feat_bwd_batch(int mode, int p, int w) { return p >= 4 && (w > 1 || mode == FM_ANY || mode == FM_CTX) ? 2 : 0; }
 constexpr int ilog2(int v) { return v <= 1 ? 0 : 1 + ilog2(v >> 1); }
 
 // m^k and m^-k: x = m^k X in the forward, x = m^-k X in the reverse sweep (k steps done), so that the
@@ -157,6 +159,64 @@ constexpr FeatPowers feat_powers() {
   return t;
 }
 static __constant__ FeatPowers kPow = feat_powers();
+
+// Which group of which row a team's unit is.
+template <bool EVEN>
+struct FeatUnits {  // in order of rows and groups
+  __device__ __forceinline__ void unit(long long u, int mg, long long& b, int& g) const {
+    b = u / mg;
+    g = (int)(u - b * mg);
+  }
+};
+// FM_CTX.  A row's groups take steps up to its length and none beyond, so by row and group half of a padded batch's units cost
+// nothing, and how many of the others a team gets is luck: of the 2048 groups of 64 x 256 x 128 (32 positions each) some of
+// 1184 warps took two and many none (forward 42 us, backward 80 a stage; so: 34 and 48).  Here the units count the groups
+// that take steps first, in row order, then the others: no team gets two of the former before all have one.  The counts come from a
+// scan of the lengths in every CTA (feat_ctx_even says where it pays).
+template <>
+struct FeatUnits<true> {
+  const int* pre;  // [B + 1]: groups that take steps in the rows before
+  int rows, m, total;
+  __device__ __forceinline__ void init(const int* ctxlen, int B, int m_, int n, int* pre_, int* warp_sum) {
+    pre = pre_;
+    rows = B;
+    m = m_;
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
+    const int per = (B + nthr - 1) / nthr, b0 = min(B, tid * per), b1 = min(B, b0 + per);
+    auto groups = [&](int b) { return (int)min((long long)m_, max(0LL, ((long long)ctxlen[b] + n - 1) / n)); };
+    int sum = 0;
+    for (int b = b0; b < b1; ++b) sum += pre_[b] = groups(b);
+    int inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += v;
+    }
+    if (lane == 31) warp_sum[tid >> 5] = inc;
+    __syncthreads();
+    int at = inc - sum;
+    for (int w = 0; w < (tid >> 5); ++w) at += warp_sum[w];
+    for (int b = b0; b < b1; ++b) {
+      const int own = pre_[b];
+      pre_[b] = at;
+      at += own;
+    }
+    if (tid == nthr - 1) pre_[B] = at;
+    __syncthreads();
+    total = pre_[B];
+  }
+  __device__ __forceinline__ void unit(long long u, int, long long& b, int& g) const {
+    const bool beyond = (int)u >= total;  // counts groups that take no steps: i m - pre[i] of them in the rows before i
+    const int v = beyond ? (int)u - total : (int)u;
+    int lo = 0, hi = rows;  // the last row that no more than v come before
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if ((beyond ? mid * m - pre[mid] : pre[mid]) <= v) lo = mid; else hi = mid;
+    }
+    b = lo;
+    g = beyond ? pre[lo + 1] - pre[lo] + v - (lo * m - pre[lo]) : v - pre[lo];
+  }
+};
 
 __device__ __forceinline__ float2 shfl2(float2 v, int src) {
   return make_float2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
@@ -394,7 +454,7 @@ template <int NC, int LD, int KF, int W, int ACT, typename T, int MODE>
 __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF, W>::P>::fwd_blocks) feat_fwd_kernel(const FeatArgs<MODE> p) {
   using G = FeatGeom<NC, LD, KF, W>;
   constexpr int P = G::P, KP = G::KP, SEG = G::SEG;
-  constexpr bool MASK = MODE == FM_MASK, CTX = MASK || (MODE == FM_ANY && G::GPW == 1);
+  constexpr bool MASK = MODE == FM_MASK, EVEN = MODE == FM_CTX, CTX = MASK || EVEN || (MODE == FM_ANY && G::GPW == 1);
   constexpr bool MID = NC >= 16 && (MODE == FM_ANY || MODE == FM_STORED);
   constexpr bool SC = feat_fwd_scaled(MODE, NC, P, W);
   __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
@@ -420,9 +480,14 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
   for (int r = 0; r < P; ++r) shift[r] = (int)((long long)th.pos(r) * p.stride % p.m);
   int par = 0;
 
+  __shared__ int rows_before[EVEN ? kFeatCtxRows + 1 : 1], warp_sum[kFeatWarps];
+  FeatUnits<EVEN> units;
+  if constexpr (EVEN) units.init(p.ctxlen, (int)p.B, p.m, NC, rows_before, warp_sum);
   for (long long u = th.first; u < p.units; u += th.step) {
-    const long long b = u / p.mg;
-    const int g = (int)(u - b * p.mg) * G::GPW + th.gw;
+    long long b;
+    int g;
+    units.unit(u, p.mg, b, g);
+    g = g * G::GPW + th.gw;
     const bool valid = G::GPW == 1 || g < p.m;
     float2 X[P][KP], A[P][KP];
     long long off[P];
@@ -532,7 +597,8 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
   using G = FeatGeom<NC, LD, KF, W>;
   using F = ActForm<ACT>;
   constexpr int P = G::P, SEG = G::SEG, KP = G::KP, D = G::D;
-  constexpr bool REPLAY = MODE == FM_REPLAY, MASK = MODE == FM_MASK, CTX = MASK || (MODE == FM_ANY && G::GPW == 1);
+  constexpr bool REPLAY = MODE == FM_REPLAY, MASK = MODE == FM_MASK, EVEN = MODE == FM_CTX,
+                 CTX = MASK || EVEN || (MODE == FM_ANY && G::GPW == 1);
   constexpr bool STORED = NC >= 16 && (MODE == FM_ANY || MODE == FM_STORED);
   constexpr bool SC = feat_bwd_scaled(MODE, NC, P, W, LD, ACT);
   // (bf16 with one row per lane comes out slower without the test that is always true: 2048 x 256 x 128, groups of 8 618 ->
@@ -588,9 +654,14 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
   for (int q = 0; q < KP; ++q) dwi[q] = dwj[q] = f2(0.0f);
   int par = 0;
 
+  __shared__ int rows_before[EVEN ? kFeatCtxRows + 1 : 1], warp_sum[kFeatWarps];
+  FeatUnits<EVEN> units;
+  if constexpr (EVEN) units.init(p.ctxlen, (int)p.B, p.m, NC, rows_before, warp_sum);
   for (long long u = th.first; u < p.units; u += th.step) {
-    const long long b = u / p.mg;
-    int g = (int)(u - b * p.mg) * G::GPW + th.gw;
+    long long b;
+    int g;
+    units.unit(u, p.mg, b, g);
+    g = g * G::GPW + th.gw;
     const bool valid = G::GPW == 1 || g < p.m;
     float2 X[P][KP], A[P][KP], H[P][KP], Gv[P][KP];
     auto offsets = [&](long long (&off)[P]) {

@@ -10,6 +10,13 @@ struct FeatParamsX;
 
 constexpr int kFeatWarps = 4;  // warps per CTA
 
+// Whether the groups of a padded batch are dealt out evenly (FeatUnits, ncn_feat.cuh).  Up to eight warps per SM have a group
+// each, and the scan of the lengths only costs (32 x 256 x 128, 1024 groups: forward 24.7 -> 26.3 us); more than 1024 rows have
+// enough groups per team to even out by themselves.  Between: 64 x 256 x 128 42 + 80 -> 34 + 48 us a stage, 128 rows 65 + 140 ->
+// 56 + 103, 300 x 128 x 128, groups of 16 39 + 78 -> 32 + 62, 1000 x 96 x 64 87 + 162 -> 75 + 138.
+constexpr int kFeatCtxRows = 1024;
+inline bool feat_ctx_even(long long rows, long long groups, int sms) { return rows <= kFeatCtxRows && groups > 8LL * sms; }
+
 // team: warps per group (feat_team)
 #define NCN_DECL(n)                                                                                                   \
   cudaError_t launch_feat_fwd_n##n(int d, int team, int act, int dtype, const FeatParamsX& p, int grid, int threads,   \

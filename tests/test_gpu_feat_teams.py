@@ -206,3 +206,31 @@ def test_forward_error_over_32_steps_is_that_of_roundings(B, d, ctx, activation)
     y, ya = ncn.fused_ncn_cuda_ctxlen(*args, cl.cuda(), ALPHA, act, n, heads, 1) if ctx else ncn.fused_ncn_cuda_v2(*args, ALPHA, act, n, heads, 1)
     for got, want in ((y, Y), (ya, YA)):
         assert (got.double().cpu() - want).norm() / want.norm() < 3.5e-7
+
+
+@pytest.mark.parametrize("n,d,heads,m", [(32, 32, 2, 3), (16, 32, 1, 5), (16, 64, 1, 4), (32, 24, 1, 2)])
+def test_a_padded_batch_is_dealt_out_without_loss(n, d, heads, m):
+    """Up to 1024 rows the groups that take steps are shared out evenly among the teams; a longer batch goes row by row.
+    Rows are independent, so the same rows give the same values either way."""
+    import ncn_cuda_b200 as ncn
+
+    B, N, E = 1025, m * n, heads * d
+    g = torch.Generator().manual_seed(n + d)
+    x, xa, dy, dya = (torch.randn(B, N, E, generator=g).cuda() for _ in range(4))
+    W = torch.randn(2 * E, generator=g).cuda() * d**-0.5
+    ctx = torch.randint(-2, N + 3, (B,), generator=g, dtype=torch.int32)
+    ctx[:3] = 0
+    ctx[1021:1024] = torch.tensor([N, 0, 1], dtype=torch.int32)
+
+    def run(rows):
+        ys = ncn.ops.stage_fwd_ctx(x[rows], xa[rows], W, ctx[rows], ALPHA, 0, n, heads, 1)
+        return (*ys, *ncn.ops.stage_bwd_ctx(*ys, dy[rows], dya[rows], W, ctx[rows], ALPHA, 0, n, heads, 1))
+
+    whole = run(slice(0, B))
+    for rows in (slice(0, 1024), slice(1, 8), slice(1023, 1025), slice(0, 3)):  # (smaller teams sum in another order)
+        for k, (p, q) in enumerate(zip(run(rows)[:4], whole[:4])):
+            # 1e-5 forward; gradients over up to 32 rebuilt steps 5e-5, as for the walk from the output alone
+            assert (p - q[rows]).abs().max() <= (1e-5 if k < 2 else 5e-5) * q.abs().max()
+    parts = [run(slice(0, 512))[4], run(slice(512, 1025))[4]]
+    # the weight gradient is a sum over at most 1025 m groups in another order
+    assert ((parts[0] + parts[1]) - whole[4]).abs().max() <= 2e-5 * whole[4].abs().max()
