@@ -125,6 +125,22 @@ int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void*
                       int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation,
                       int dtype, void* stream);
 
+/* A stage's backward without the last step of its weight gradient, for a caller that walks back several stages: `workspace`
+ * is left holding *rows rows of 2E partial sums, which ncn_reduce_partials adds up for all stages by one launch (one
+ * per 16 of them) in the order the single calls use, so the results are theirs.  keep names the call this stands for
+ * and with it the arguments that are read; the others may be null.  No counterpart in the reference. */
+enum {
+  NCN_KEEP_OUTPUT = 0, /* ncn_stage_bwd */
+  NCN_KEEP_INPUT = 1,  /* ncn_stage_bwd_saved */
+  NCN_KEEP_MID = 2,    /* ncn_stage_bwd_mid */
+  NCN_KEEP_CTX = 3     /* ncn_stage_bwd_ctx */
+};
+int ncn_stage_bwd_partial(int keep, const void* x, const void* xa, const void* y, const void* ya, const void* mid, size_t mid_bytes,
+                          const int* ctxlen, const void* dy, const void* dya, const float* W, void* dx, void* dxa, void* workspace,
+                          size_t workspace_bytes, int* rows, int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int module_l,
+                          double alpha, int activation, int dtype, void* stream);
+int ncn_reduce_partials(const float* const* partials, const int* rows, float* const* dW, int L, int64_t cols, void* stream);
+
 /* All L stages (module_l = first_module .. first_module+L-1) in one kernel.  Replaces the stage
  * loops NCNNetCuda.forward / NCNNetTestCuda.forward (ncn_pytorch_wrapper_v2.py:114-117,132-144).
  * ckpt (may be null without NCN_TAPE): fp32 buffer of ncn_ckpt_bytes(...) bytes that receives the state
@@ -134,6 +150,14 @@ int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void*
 int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya, float* ckpt, int ckpt_every,
                 int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L, double alpha,
                 int activation, int dtype, int flags, void* stream);
+
+/* ncn_net_fwd with the L weight vectors as the caller holds them (device pointers in the host array `weights`, one per
+ * stage); they are also written to W, [L][2E] fp32, for ncn_net_bwd.  One launch fewer than ncn_gather_weights and
+ * ncn_net_fwd where L <= 32 and the kernel takes the pointers; results as those two calls.  No counterpart in the
+ * reference (its stages read their weights one by one). */
+int ncn_net_fwd_list(const void* x, const void* xa, const float* const* weights, float* W, void* y, void* ya, float* ckpt,
+                     int ckpt_every, int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L,
+                     double alpha, int activation, int dtype, int flags, void* stream);
 
 /* Backward of ncn_net_fwd in one kernel.  s0/s1 are the net OUTPUT (y, ya) — every stage input is
  * rebuilt by the reversible inverse, restarting at each stored checkpoint — or, with NCN_RECOMPUTE,

@@ -46,6 +46,16 @@ SIGNATURES = {
         c_int,
         [c_void_p] * 5 + [c_void_p, c_int] + [c_int64] * 3 + [c_int] * 4 + [c_double, c_int, c_int, c_int, c_void_p],
     ),
+    "ncn_net_fwd_list": (
+        c_int,
+        [c_void_p] * 7 + [c_int] + [c_int64] * 3 + [c_int] * 4 + [c_double, c_int, c_int, c_int, c_void_p],
+    ),
+    "ncn_stage_bwd_partial": (
+        c_int,
+        [c_int] + [c_void_p] * 5 + [c_size_t] + [c_void_p] * 7 + [c_size_t, c_void_p] + [c_int64] * 3 + [c_int] * 3
+        + [c_double, c_int, c_int, c_void_p],
+    ),
+    "ncn_reduce_partials": (c_int, [c_void_p] * 3 + [c_int, c_int64, c_void_p]),
     "ncn_net_bwd": (
         c_int,
         [c_void_p] * 10

@@ -786,7 +786,15 @@ static int check_common(int64_t B, int64_t N, int64_t E, int n, int C, int dtype
   return NCN_OK;
 }
 
+// Set while a stage's backward leaves its partial sums to a reduction of several stages (ncn_stage_bwd_partial): receives
+// their number of rows.
+static thread_local int* tl_partial_rows = nullptr;
+
 static int reduce_dw(const float* partials, float* dW, int rows, int cols, int accumulate, cudaStream_t st) {
+  if (tl_partial_rows != nullptr) {
+    *tl_partial_rows = rows;
+    return NCN_OK;
+  }
   const int warps = 4;
   dw_reduce_kernel<<<(cols + warps - 1) / warps, warps * 32, 0, st>>>(partials, dW, rows, cols, accumulate);
   cudaError_t e = cudaGetLastError();
@@ -1048,6 +1056,26 @@ __global__ void gather_weights_kernel(const GatherParams p) {
   }
 }
 
+// ---- the weight gradients of several stages out of their partial sums, by one launch for up to 16 of them
+constexpr int kReduceMax = 16;
+struct ReduceParams {
+  const float* partials[kReduceMax];
+  float* out[kReduceMax];
+  int rows[kReduceMax];
+  int cols;
+};
+__global__ void dw_reduce_stages_kernel(const __grid_constant__ ReduceParams p) {
+  const int lane = threadIdx.x & 31, l = blockIdx.y;
+  const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (col >= p.cols) return;
+  const float* const part = p.partials[l];
+  const int rows = p.rows[l];
+  float acc = 0.0f;  // (the order of dw_reduce_kernel)
+  for (int r = lane; r < rows; r += 32) acc += part[(long long)r * p.cols + col];
+  acc = warp_sum(acc);
+  if (lane == 0) p.out[l][col] = acc;
+}
+
 static size_t workspace_floats(const DevInfo& dev, int64_t E, int L) {
   return (size_t)dev.sms * 32 * 2 * (size_t)E * (size_t)(L < 1 ? 1 : L);
 }
@@ -1159,9 +1187,10 @@ int ncn_gather_weights(const float* const* weights, int L, int64_t cols, float* 
   return e == cudaSuccess ? NCN_OK : cuda_fail(e);
 }
 
-int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya, float* ckpt, int ckpt_every,
-                int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L, double alpha,
-                int activation, int dtype, int flags, void* stream) {
+// list: L weight vectors instead of W; they are gathered into W, by the kernel itself where it takes a list.
+static int net_fwd_impl(const void* x, const void* xa, const float* const* list, const float* W, void* y, void* ya, float* ckpt,
+                        int ckpt_every, int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L,
+                        double alpha, int activation, int dtype, int flags, void* stream) {
   int rc = check_common(B, N, E, n_cache, n_head, dtype);
   if (rc != NCN_OK) return rc;
   if (L < 1 || first_module < 0) return NCN_ERR_SHAPE;
@@ -1174,6 +1203,11 @@ int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
   const int act = fused_act(map_act(activation), dtype);
   float* ck_used = (ckpt && ckpt_slots(L, ckpt_every, flags) > 0) ? ckpt : nullptr;
+  auto fill_list = [&](WeightList& wl) {
+    for (int l = 0; l < L; ++l) wl.src[l] = list[l];
+    wl.out = const_cast<float*>(W);
+  };
+  auto gather = [&]() { return ncn_gather_weights(list, L, 2, const_cast<float*>(W), stream); };
   {
     // register-resident family; its stored states have their own order, so with states it is used
     // only where the backward of the same arguments is of this family too
@@ -1202,6 +1236,8 @@ int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya
       q.oma = (float)(1.0 - alpha);
       fill_lane(q, lp);
       q.test_short_wait = env_switches().test_short_wait ? 1 : 0;
+      if (list && L <= kWeightList && !lp.pipelined) fill_list(q.list);
+      else if (list && (rc = gather()) != NCN_OK) return rc;
       cudaError_t e = lane_fn(n_cache, false)(act, dtype, q, lp.grid, lp.threads, lp.smem, (cudaStream_t)stream, nullptr);
       return e == cudaSuccess ? NCN_OK : cuda_fail(e);
     }
@@ -1217,12 +1253,15 @@ int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya
       q.W = W;
       q.status = dev.status;
       fill_solo(q, sp, B, N, n_cache, L, first_module, alpha, flags);
+      if (list && L <= kWeightList) fill_list(q.list);
+      else if (list && (rc = gather()) != NCN_OK) return rc;
       cudaError_t e = solo_fn(n_cache, false)(act, dtype, q, sp.grid, sp.threads, sp.smem, (cudaStream_t)stream, nullptr);
       return e == cudaSuccess ? NCN_OK : cuda_fail(e);
     }
   }
   Plan pl;
   if ((rc = plan_rows(false, B, (int)N, n_cache, L, dtype, flags, 0, false, dev, act, pl)) != NCN_OK) return rc;
+  if (list && (rc = gather()) != NCN_OK) return rc;
   RowsParams p{};
   p.in[0] = x; p.in[1] = xa;
   p.out[0] = y; p.out[1] = ya;
@@ -1238,6 +1277,23 @@ int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya
   cudaError_t e = (pl.pair ? pair_fn(n_cache, false) : rows_fn(n_cache, false))(act, dtype, p, pl.grid, pl.threads, pl.smem,
                                                                                (cudaStream_t)stream, nullptr);
   return e == cudaSuccess ? NCN_OK : cuda_fail(e);
+}
+
+int ncn_net_fwd(const void* x, const void* xa, const float* W, void* y, void* ya, float* ckpt, int ckpt_every,
+                int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L, double alpha,
+                int activation, int dtype, int flags, void* stream) {
+  return net_fwd_impl(x, xa, nullptr, W, y, ya, ckpt, ckpt_every, B, N, E, n_cache, n_head, first_module, L, alpha, activation,
+                      dtype, flags, stream);
+}
+
+int ncn_net_fwd_list(const void* x, const void* xa, const float* const* weights, float* W, void* y, void* ya, float* ckpt,
+                     int ckpt_every, int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L,
+                     double alpha, int activation, int dtype, int flags, void* stream) {
+  if (!weights) return NCN_ERR_NULL;
+  for (int l = 0; l < L; ++l)
+    if (!weights[l]) return NCN_ERR_NULL;
+  return net_fwd_impl(x, xa, weights, W, y, ya, ckpt, ckpt_every, B, N, E, n_cache, n_head, first_module, L, alpha, activation,
+                      dtype, flags, stream);
 }
 
 // Backward of a net, shared by ncn_net_bwd and ncn_net_bwd_noalloc: `partials` is the scratch for the
@@ -1567,6 +1623,58 @@ int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void*
   }
   return stage_bwd_generic(y, ya, dy, dya, W, ctxlen, dx, dxa, x_rec, xa_rec, dW, static_cast<float*>(workspace), B, N, E,
                            n_cache, n_head, module_l, alpha, activation, dtype, dev, stream);
+}
+
+int ncn_stage_bwd_partial(int keep, const void* x, const void* xa, const void* y, const void* ya, const void* mid, size_t mid_bytes,
+                          const int* ctxlen, const void* dy, const void* dya, const float* W, void* dx, void* dxa, void* workspace,
+                          size_t workspace_bytes, int* rows, int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int module_l,
+                          double alpha, int activation, int dtype, void* stream) {
+  if (!rows || !workspace) return NCN_ERR_NULL;
+  float* const unused = static_cast<float*>(workspace);  // (the place of dW: nothing is written to it)
+  *rows = 0;
+  tl_partial_rows = rows;
+  int rc;
+  switch (keep) {
+    case NCN_KEEP_OUTPUT:
+      rc = ncn_stage_bwd(y, ya, dy, dya, W, dx, dxa, nullptr, nullptr, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                         module_l, alpha, activation, dtype, stream);
+      break;
+    case NCN_KEEP_INPUT:
+      rc = ncn_stage_bwd_saved(x, xa, y, ya, dy, dya, W, dx, dxa, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                               module_l, alpha, activation, dtype, stream);
+      break;
+    case NCN_KEEP_MID:
+      rc = ncn_stage_bwd_mid(y, ya, mid, mid_bytes, dy, dya, W, dx, dxa, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                             module_l, alpha, activation, dtype, stream);
+      break;
+    case NCN_KEEP_CTX:
+      rc = ncn_stage_bwd_ctx(y, ya, dy, dya, W, ctxlen, dx, dxa, nullptr, nullptr, unused, workspace, workspace_bytes, B, N, E,
+                             n_cache, n_head, module_l, alpha, activation, dtype, stream);
+      break;
+    default: rc = NCN_ERR_UNSUPPORTED;
+  }
+  tl_partial_rows = nullptr;
+  return rc;
+}
+
+int ncn_reduce_partials(const float* const* partials, const int* rows, float* const* dW, int L, int64_t cols, void* stream) {
+  if (!partials || !rows || !dW) return NCN_ERR_NULL;
+  if (L < 1 || cols < 1 || cols > (1 << 25)) return NCN_ERR_SHAPE;
+  for (int l0 = 0; l0 < L; l0 += kReduceMax) {
+    ReduceParams p{};
+    const int cnt = L - l0 < kReduceMax ? L - l0 : kReduceMax;
+    for (int l = 0; l < cnt; ++l) {
+      if (!partials[l0 + l] || !dW[l0 + l]) return NCN_ERR_NULL;
+      p.partials[l] = partials[l0 + l];
+      p.out[l] = dW[l0 + l];
+      p.rows[l] = rows[l0 + l];
+    }
+    p.cols = (int)cols;
+    const int warps = 4;
+    dw_reduce_stages_kernel<<<dim3((unsigned)((cols + warps - 1) / warps), (unsigned)cnt), warps * 32, 0, (cudaStream_t)stream>>>(p);
+  }
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? NCN_OK : cuda_fail(e);
 }
 
 }  // extern "C"

@@ -618,7 +618,7 @@ __device__ __forceinline__ void lane_st_native(T* chunk, const float2 (&Sv)[G / 
 
 // ------------------------------------------------------------------------------------------ forward
 template <int NG, int ACT, typename T, int MAXT, int MINB, bool RAG, bool NANX>
-__global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p) {
+__global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_constant__ LaneParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
   constexpr int G = lane_groups(NG);
@@ -644,7 +644,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const LaneParams p
     *abort_flag = 0;
     fence_mbar_init();
   }
-  fill_stage_table(recs, p.W, p.oma, p.l0, p.m, p.L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr);
+  fill_stage_table(recs, p.W, p.oma, p.l0, p.m, p.L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr, &p.list);
   __syncthreads();
 
   auto issue_load = [&](long long tl) {

@@ -9,6 +9,7 @@ struct LaneParams {
   void* out[4];        // fwd: y, ya, -, - ; bwd: dx, dxa, x_rec (or null), xa_rec (or null)
   float* ckpt;         // [K][B*N] (x, a) pairs in this family's order, or null
   const float* W;      // [L][2]
+  WeightList list;     // fwd: the weights one by one
   float* partials;     // bwd: [gridDim.x][L][2]
   int* status;         // device status word
   long long B;

@@ -96,12 +96,20 @@ __device__ __forceinline__ void group_addrs(uint32_t row_addr, int g, int s, int
 // Stage table: scaled weights, stride s = 0 for stage 0 else 2^(stage-1) mod m
 // (torch_ref/ncn_pytorch.py:38), and the checkpoint index (a state is kept after every
 // ckpt_every-th stage except the last; with F_TAPE the last stage's state takes the slot after those).
+// list: the weights are one vector per stage; the first CTA also writes them to list->out, [L][2], for the backward.
 __device__ __forceinline__ void fill_stage_table(StageRec* rec, const float* W, float oma, int l0, int m, int L,
-                                                 int ckpt_every, int flags, bool have_ckpt, int tid, int nthr) {
+                                                 int ckpt_every, int flags, bool have_ckpt, int tid, int nthr,
+                                                 const WeightList* list = nullptr) {
   for (int i = tid; i < L; i += nthr) {
     StageRec r;
-    r.owi = W[2 * i] * oma;
-    r.owj = W[2 * i + 1] * oma;
+    const float* w = list && list->out ? list->src[i] : W + 2 * i;
+    const float wi = w[0], wj = w[1];
+    if (list && list->out && blockIdx.x == 0) {
+      list->out[2 * i] = wi;
+      list->out[2 * i + 1] = wj;
+    }
+    r.owi = wi * oma;
+    r.owj = wj * oma;
     r.s = stage_stride(l0 + i, m);
     r.ck = (have_ckpt && ckpt_every > 0 && i != L - 1 && ((i + 1) % ckpt_every == 0)) ? (i + 1) / ckpt_every - 1 : -1;
     if (have_ckpt && (flags & F_TAPE) && i == L - 1) r.ck = ckpt_every > 0 ? (L - 1) / ckpt_every : 0;

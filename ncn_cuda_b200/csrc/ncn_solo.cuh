@@ -133,7 +133,7 @@ __device__ __forceinline__ void solo_set(float2 (&v)[NG / 2], int o, float x) {
 
 // ------------------------------------------------------------------------------------------ forward
 template <int NG, int ACT, typename T, int MAXT, int MINB>
-__global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const SoloParams p) {
+__global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const __grid_constant__ SoloParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
   using S = LaneStage<NG, ACT>;
@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const SoloParams p
     *abort_flag = 0;
     fence_mbar_init();
   }
-  fill_stage_table(recs, p.W, p.oma, p.l0, m, L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr);
+  fill_stage_table(recs, p.W, p.oma, p.l0, m, L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr, &p.list);
   __syncthreads();
 
   const int r = tid / m, g = tid - r * m;  // row of the tile, group

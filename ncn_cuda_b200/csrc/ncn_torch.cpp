@@ -7,7 +7,7 @@
 // Why native: at small batches the host is the bound.  A training step of a 1024 x 1024 net runs 59 us
 // of kernels; through Python autograd functions, ctypes and torch.stack / unbind it took 294 us.
 // A chain of stages keeps its inner activations in one node, so that the engine hands over once per
-// direction instead of once per stage, and the weights of a fused net are gathered by one small kernel
+// direction instead of once per stage, the weights of a fused net are gathered by its own kernel
 // and their gradients returned as views of one buffer (as torch.stack and its backward would).
 //
 // Saved tensors go through SavedVariable, so in-place changes, saved-tensor hooks and a second backward
@@ -204,22 +204,6 @@ struct FusedNode : public NcnNode {
   }
 };
 
-// All stages' weights in one buffer, by one launch for up to 32 of them.
-Tensor gather_weights(const variable_list& ws, int64_t E, const Tensor& x) {
-  const int64_t L = (int64_t)ws.size();
-  Tensor W = at::empty({L * 2 * E}, x.options().dtype(at::kFloat));
-  std::vector<Tensor> keep;
-  std::vector<const float*> ptr;
-  keep.reserve(L);
-  ptr.reserve(L);
-  for (const Tensor& w : ws) {
-    keep.push_back(plain_weights(w, 2 * E, x.device()));
-    ptr.push_back(keep.back().const_data_ptr<float>());
-  }
-  check_status("ncn_gather_weights", ncn_gather_weights(ptr.data(), (int)L, 2 * E, W.mutable_data_ptr<float>(), stream_of(x)));
-  return W;
-}
-
 std::tuple<Tensor, Tensor> fused_forward(const Tensor& x_in, const Tensor& xa_in, const variable_list& ws, bool gathered,
                                          FusedCfg c) {
   const bool grad = wants_grad(x_in, xa_in, ws);
@@ -235,7 +219,18 @@ std::tuple<Tensor, Tensor> fused_forward(const Tensor& x_in, const Tensor& xa_in
     const Tensor x = x_in.contiguous(), xa = xa_in.contiguous();
     const int64_t B = x.size(0), N = x.size(1), E = x.size(2);
     c.dt = dtype_code(x);
-    const Tensor W = gathered ? gather_weights(ws, E, x) : plain_weights(ws[0], (int64_t)c.layers * c.L * 2 * E, x.device());
+    const Tensor W = gathered ? at::empty({(int64_t)ws.size() * 2 * E}, x.options().dtype(at::kFloat))
+                              : plain_weights(ws[0], (int64_t)c.layers * c.L * 2 * E, x.device());
+    std::vector<Tensor> each;  // gathered: the weights one by one, which the kernel gathers into W
+    std::vector<const float*> list;
+    if (gathered) {
+      each.reserve(ws.size());
+      list.reserve(ws.size());
+      for (const Tensor& w : ws) {
+        each.push_back(plain_weights(w, 2 * E, x.device()));
+        list.push_back(each.back().const_data_ptr<float>());
+      }
+    }
     if (!grad) {  // nothing will be walked back: no states are stored
       c.every = 0;
       c.tape = c.recompute = false;
@@ -249,10 +244,15 @@ std::tuple<Tensor, Tensor> fused_forward(const Tensor& x_in, const Tensor& xa_in
       ya = at::empty_like(xa);
       Tensor ck;
       if (ck_bytes) ck = at::empty({(int64_t)(ck_bytes / 4)}, x.options().dtype(at::kFloat));
-      check_status("ncn_net_fwd",
-                   ncn_net_fwd(in.data_ptr(), ina.data_ptr(), W.const_data_ptr<float>() + (int64_t)k * c.L * 2 * E, y.data_ptr(),
-                               ya.data_ptr(), ck.defined() ? ck.mutable_data_ptr<float>() : nullptr, c.every, B, N, E, c.n, c.C,
-                               c.first, c.L, c.alpha, c.act, c.dt, flags, st));
+      float* const ckp = ck.defined() ? ck.mutable_data_ptr<float>() : nullptr;
+      if (gathered)
+        check_status("ncn_net_fwd",
+                     ncn_net_fwd_list(in.data_ptr(), ina.data_ptr(), list.data(), W.mutable_data_ptr<float>(), y.data_ptr(),
+                                      ya.data_ptr(), ckp, c.every, B, N, E, c.n, c.C, c.first, c.L, c.alpha, c.act, c.dt, flags, st));
+      else
+        check_status("ncn_net_fwd",
+                     ncn_net_fwd(in.data_ptr(), ina.data_ptr(), W.const_data_ptr<float>() + (int64_t)k * c.L * 2 * E, y.data_ptr(),
+                                 ya.data_ptr(), ckp, c.every, B, N, E, c.n, c.C, c.first, c.L, c.alpha, c.act, c.dt, flags, st));
       if (grad) {
         if (c.recompute) {
           node->s0.emplace_back(k == 0 && x.is_same(x_in) ? x_in : in, false);
@@ -313,8 +313,15 @@ struct ChainNode : public NcnNode {
     incoming(g, dy, dya);
     const c10::cuda::OptionalCUDAGuard guard(dy.device());
     const int64_t B = shape_[0], N = shape_[1], E = shape_[2];
-    const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, 1, c.dt);
-    const Tensor ws = at::empty({(int64_t)ws_bytes}, dy.options().dtype(at::kByte));
+    // The stages leave their partial sums side by side in the workspace, and one launch adds up those of all (of as many as
+    // fit): a call asks for ws_bytes and uses a fraction of them.
+    const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, 1, c.dt), room = c.L > 1 ? 2 * ws_bytes : ws_bytes;
+    const Tensor ws = at::empty({(int64_t)room}, dy.options().dtype(at::kByte));
+    char* const ws_base = static_cast<char*>(ws.data_ptr());
+    size_t used = 0;
+    std::vector<const float*> partial;
+    std::vector<int> partial_rows;
+    std::vector<float*> partial_out;
     std::vector<Tensor> dW(c.L);  // a tensor of its own per stage: a weight's .grad holds no other's memory
     const size_t mid_bytes = c.keep == KEEP_MID ? ncn_stage_mid_bytes(B, N, E, c.n, c.dt) : 0;
     const Tensor cl = has_ctx ? ctxlen.unpack() : Tensor();
@@ -329,38 +336,47 @@ struct ChainNode : public NcnNode {
     int last = 0;
     if (!inputs)
       while (last < c.L - 1 && !task_should_compute_output(2 + last)) ++last;
+    auto reduce = [&]() {
+      if (partial.empty()) return;
+      check_status("ncn_reduce_partials", ncn_reduce_partials(partial.data(), partial_rows.data(), partial_out.data(),
+                                                              (int)partial.size(), 2 * E, st));
+      partial.clear();
+      partial_rows.clear();
+      partial_out.clear();
+      used = 0;
+    };
     for (int l = c.L - 1; l >= last; --l) {
       const Tensor w = plain_weights(W[l].unpack(), 2 * E, dy.device());
       const Tensor yl = out_of(y, l), yal = out_of(ya, l);
       Tensor dx = at::empty(shape_, options_), dxa = at::empty(shape_, options_);
       dW[l] = at::empty(wshape_[l], dy.options().dtype(at::kFloat));
-      float* const dwl = dW[l].mutable_data_ptr<float>();
-      const float* const wp = w.const_data_ptr<float>();
-      const int module_l = c.first + l;
+      Tensor xc, xac, m;
+      int keep = NCN_KEEP_OUTPUT;
+      const char* call = "ncn_stage_bwd";
       if (has_ctx) {
-        check_status("ncn_stage_bwd_ctx",
-                     ncn_stage_bwd_ctx(yl.data_ptr(), yal.data_ptr(), dy.data_ptr(), dya.data_ptr(), wp, cl.const_data_ptr<int>(),
-                                       dx.data_ptr(), dxa.data_ptr(), nullptr, nullptr, dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n,
-                                       c.C, module_l, c.alpha, c.act, c.dt, st));
+        keep = NCN_KEEP_CTX;
+        call = "ncn_stage_bwd_ctx";
       } else if (c.keep == KEEP_INPUT) {
-        const Tensor xl = l == 0 ? x0.unpack() : y[l - 1].unpack(), xal = l == 0 ? xa0.unpack() : ya[l - 1].unpack();
-        const Tensor xc = xl.contiguous(), xac = xal.contiguous();
-        check_status("ncn_stage_bwd_saved",
-                     ncn_stage_bwd_saved(xc.data_ptr(), xac.data_ptr(), yl.data_ptr(), yal.data_ptr(), dy.data_ptr(), dya.data_ptr(),
-                                         wp, dx.data_ptr(), dxa.data_ptr(), dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n, c.C,
-                                         module_l, c.alpha, c.act, c.dt, st));
+        keep = NCN_KEEP_INPUT;
+        call = "ncn_stage_bwd_saved";
+        xc = (l == 0 ? x0.unpack() : y[l - 1].unpack()).contiguous();
+        xac = (l == 0 ? xa0.unpack() : ya[l - 1].unpack()).contiguous();
       } else if (mid_bytes) {
-        const Tensor m = mid[l].unpack();
-        check_status("ncn_stage_bwd_mid",
-                     ncn_stage_bwd_mid(yl.data_ptr(), yal.data_ptr(), m.data_ptr(), mid_bytes, dy.data_ptr(), dya.data_ptr(), wp,
-                                       dx.data_ptr(), dxa.data_ptr(), dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n, c.C, module_l,
-                                       c.alpha, c.act, c.dt, st));
-      } else {
-        check_status("ncn_stage_bwd",
-                     ncn_stage_bwd(yl.data_ptr(), yal.data_ptr(), dy.data_ptr(), dya.data_ptr(), wp, dx.data_ptr(), dxa.data_ptr(),
-                                   nullptr, nullptr, dwl, ws.data_ptr(), ws_bytes, B, N, E, c.n, c.C, module_l, c.alpha, c.act,
-                                   c.dt, st));
+        keep = NCN_KEEP_MID;
+        call = "ncn_stage_bwd_mid";
+        m = mid[l].unpack();
       }
+      auto ptr = [](const Tensor& t) -> const void* { return t.defined() ? t.const_data_ptr() : nullptr; };
+      if (used + ws_bytes > room) reduce();
+      int rows = 0;
+      check_status(call, ncn_stage_bwd_partial(keep, ptr(xc), ptr(xac), yl.const_data_ptr(), yal.const_data_ptr(), ptr(m), mid_bytes,
+                                               has_ctx ? cl.const_data_ptr<int>() : nullptr, dy.const_data_ptr(), dya.const_data_ptr(),
+                                               w.const_data_ptr<float>(), dx.data_ptr(), dxa.data_ptr(), ws_base + used, ws_bytes,
+                                               &rows, B, N, E, c.n, c.C, c.first + l, c.alpha, c.act, c.dt, st));
+      partial.push_back(reinterpret_cast<const float*>(ws_base + used));
+      partial_rows.push_back(rows);
+      partial_out.push_back(dW[l].mutable_data_ptr<float>());
+      used += ((size_t)rows * 2 * E * sizeof(float) + 255) / 256 * 256;
       dy = std::move(dx);
       dya = std::move(dxa);
       if (release) {
@@ -368,6 +384,7 @@ struct ChainNode : public NcnNode {
           if (!v->empty()) (*v)[l].reset_data();
       }
     }
+    reduce();
     variable_list out(2 + wshape_.size());
     if (inputs) {
       out[0] = std::move(dy);
