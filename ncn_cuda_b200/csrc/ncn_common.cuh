@@ -422,31 +422,31 @@ __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG
 }
 
 // forward offsets after k steps: C_k = sum_{i=1..k} c f0 / m^i ; D_k = sum_{i=1..k} c C_i
-constexpr double fwd_C(int k, double f0, double md = kMd, double cd = kCd) {
+constexpr double fwd_C(int k, double f0) {
   double C = 0.0;
-  for (int i = 1; i <= k; ++i) C += cd * f0 / cpow(md, i);
+  for (int i = 1; i <= k; ++i) C += kCd * f0 / cpow(kMd, i);
   return C;
 }
-constexpr double fwd_D(int k, double f0, double md = kMd, double cd = kCd) {
+constexpr double fwd_D(int k, double f0) {
   double C = 0.0, D = 0.0;
   for (int i = 1; i <= k; ++i) {
-    C += cd * f0 / cpow(md, i);
-    D += cd * C;
+    C += kCd * f0 / cpow(kMd, i);
+    D += kCd * C;
   }
   return D;
 }
 // reverse offsets after k inverse steps: x = m^-k (X + DX_k), a = m^-k (A + CA_k)
 //   CA_{k+1} = CA_k - c f0 m^k ;  DX_{k+1} = DX_k - c CA_k
-constexpr double bwd_CA(int k, double f0, double md = kMd, double cd = kCd) {
+constexpr double bwd_CA(int k, double f0) {
   double CA = 0.0;
-  for (int i = 0; i < k; ++i) CA -= cd * f0 * cpow(md, i);
+  for (int i = 0; i < k; ++i) CA -= kCd * f0 * cpow(kMd, i);
   return CA;
 }
-constexpr double bwd_DX(int k, double f0, double md = kMd, double cd = kCd) {
+constexpr double bwd_DX(int k, double f0) {
   double CA = 0.0, DX = 0.0;
   for (int i = 0; i < k; ++i) {
-    DX -= cd * CA;
-    CA -= cd * f0 * cpow(md, i);
+    DX -= kCd * CA;
+    CA -= kCd * f0 * cpow(kMd, i);
   }
   return DX;
 }

@@ -71,41 +71,22 @@ struct LaneBatch {
 };
 
 // ------------------------------------------------------------------ step math (scaled variables of ncn_common.cuh)
-// The powers of groups of 2 and 4 are those of 0.9 itself: its fp32 value is 2.6e-8 off, the same way in every step, which
-// after 20 steps is more than all roundings together (4096 positions, groups of 4, 6 stages, against fp64: y 6.7e-7 -> 2.2e-7, dx
-// 6.8e-7 -> 2.8e-7).  c is the fp32 value that the steps multiply by (kC): offsets made of another c would not cancel in the
-// inverse.  Groups of 8 keep the powers of the fp32 value: with them the roundings of the constants happen to cancel over long
-// walks back (40 steps from the output: dW within 4e-5 of its size, with those of 0.9 within 1.8e-4).
-template <int NG>
-constexpr double lane_m() { return NG == 8 ? kMd : 0.9; }
-constexpr double kLaneC = kCd;
-template <int NG>
-constexpr double lane_bwd_DX(int k, double f0) { return bwd_DX(k, f0, lane_m<NG>(), kLaneC); }
-
-// The constants of a forward stage as the steps use them, rounded to fp32, and those that undo it.  Groups of 2 and 4: the
-// latter are made of the former and not of the powers, or two independent roundings of m^n would leave a factor that every
-// earlier stage multiplies (32 steps back, groups of 4: dx 2.9e-6 -> 2.6e-6 of its size).
+// The constants of a forward stage and those that undo it.
 template <int NG, int ACT>
 struct LaneStage {
   using F = ActForm<ACT>;
-  static constexpr double m = lane_m<NG>();
-  static constexpr double mN = (double)(float)cpow(m, NG);
-  static constexpr double mNC = (double)(float)(cpow(m, NG) * fwd_C(NG, F::f0, m, kLaneC));
-  static constexpr double mND = (double)(float)(cpow(m, NG) * fwd_D(NG, F::f0, m, kLaneC));
-  static constexpr double cA(int J) { return (double)(float)(kLaneC * F::f1 / cpow(m, J + 1)); }
-  static constexpr bool own = NG != 8;
-  static constexpr double imN = own ? 1.0 / mN : 1.0 / cpow(m, NG);
-  static constexpr double imNDX = own ? (NG * (double)kC * mNC - mND) / mN : bwd_DX(NG, F::f0, m, kLaneC) / cpow(m, NG);
-  static constexpr double imNCA = own ? -mNC / mN : bwd_CA(NG, F::f0, m, kLaneC) / cpow(m, NG);
-  static constexpr double cAr(int J) { return own ? -mN * cA(J) : -kLaneC * F::f1 * cpow(m, NG - 1 - J); }
+  static constexpr double mN = cpow(kMd, NG), mNC = mN * fwd_C(NG, F::f0), mND = mN * fwd_D(NG, F::f0);
+  static constexpr double imN = 1.0 / mN, imNDX = bwd_DX(NG, F::f0) / mN, imNCA = bwd_CA(NG, F::f0) / mN;
+  static constexpr double cA(int J) { return kCd * F::f1 / cpow(kMd, J + 1); }
+  static constexpr double cAr(int J) { return -kCd * F::f1 * cpow(kMd, NG - 1 - J); }
 };
 
 template <int NG, int ACT, int J, bool NANX>
 struct LFwdSteps {
   static __device__ __forceinline__ void run(float2 (&X)[NG], float2 (&A)[NG], const PairW& w) {
     using F = ActForm<ACT>;
-    constexpr float mk = (float)cpow(lane_m<NG>(), J);
-    constexpr float mkDk = (float)(cpow(lane_m<NG>(), J) * fwd_D(J, F::f0, lane_m<NG>(), kLaneC));
+    constexpr float mk = (float)cpow(kMd, J);
+    constexpr float mkDk = (float)(cpow(kMd, J) * fwd_D(J, F::f0));
     constexpr float cA = (float)LaneStage<NG, ACT>::cA(J);
     float2 xj, P, Q;
     if constexpr (J == 0) {
@@ -174,15 +155,15 @@ struct LBwdSteps {
                                              const PairWB& w, float2& dwi, float2& dwj) {
     using F = ActForm<ACT>;
     constexpr int k = NG - 1 - J;
-    constexpr double mkd = cpow(lane_m<NG>(), k);
-    constexpr float imk1 = (float)(1.0 / cpow(lane_m<NG>(), k + 1));
-    constexpr float DX1 = (float)lane_bwd_DX<NG>(k + 1, F::f0);
-    constexpr float imk1DX1 = (float)(lane_bwd_DX<NG>(k + 1, F::f0) / cpow(lane_m<NG>(), k + 1));
+    constexpr double mkd = cpow(kMd, k);
+    constexpr float imk1 = (float)(1.0 / cpow(kMd, k + 1));
+    constexpr float DX1 = (float)bwd_DX(k + 1, F::f0);
+    constexpr float imk1DX1 = (float)(bwd_DX(k + 1, F::f0) / cpow(kMd, k + 1));
     constexpr float cAr = (float)LaneStage<NG, ACT>::cAr(J);
-    constexpr float sTimk1 = (float)(F::sT / cpow(lane_m<NG>(), k + 1));
-    constexpr float cdsm = (float)(kLaneC * F::ds / lane_m<NG>());
-    constexpr float K1 = (float)(kLaneC * F::ds / lane_m<NG>() / cpow(lane_m<NG>(), k + 1));  // c ds / m^(k+2)
-    constexpr float twomk1 = (float)(2.0 * cpow(lane_m<NG>(), k + 1));
+    constexpr float sTimk1 = (float)(F::sT / cpow(kMd, k + 1));
+    constexpr float cdsm = (float)(kCd * F::ds / kMd);
+    constexpr float K1 = (float)(kCd * F::ds / kMd / cpow(kMd, k + 1));  // c ds / m^(k+2)
+    constexpr float twomk1 = (float)(2.0 * cpow(kMd, k + 1));
     constexpr float mk = (float)mkd;
 #pragma unroll
     for (int i = 0; i < NG; ++i) X[i] = ffma2(f2(-kC), A[i], X[i]);
@@ -238,7 +219,7 @@ __device__ __forceinline__ void lane_backward(float2 (&X)[NG], float2 (&A)[NG], 
   LBwdSteps<NG, ACT, NG - 1>::run(X, A, H, G, w, dwi, dwj);
   using S = LaneStage<NG, ACT>;
   constexpr float imN = (float)S::imN, imNDX = (float)S::imNDX, imNCA = (float)S::imNCA;
-  constexpr float mN = (float)cpow(lane_m<NG>(), NG);
+  constexpr float mN = (float)cpow(kMd, NG);
 #pragma unroll
   for (int i = 0; i < NG; ++i) {
     if constexpr (imNDX != 0.0f) X[i] = ffma2(X[i], f2(imN), f2(imNDX)); else X[i] = fmul2(X[i], f2(imN));
@@ -247,13 +228,13 @@ __device__ __forceinline__ void lane_backward(float2 (&X)[NG], float2 (&A)[NG], 
     G[i] = fmul2(G[i], f2(mN));
   }
 }
-template <int NG, int ACT>
+template <int ACT>
 __device__ __forceinline__ float lane_dw_scale_i(float oma) {  // (1-alpha) c ds / m
-  return oma * (float)(kLaneC * ActForm<ACT>::ds / lane_m<NG>());
+  return oma * (float)(kCd * ActForm<ACT>::ds / kMd);
 }
 template <int ACT>
 __device__ __forceinline__ float lane_dw_scale_j(float oma) {  // (1-alpha) c ds
-  return oma * (float)(kLaneC * ActForm<ACT>::ds);
+  return oma * (float)(kCd * ActForm<ACT>::ds);
 }
 
 // ------------------------------------------------------------------ exchanges
@@ -845,7 +826,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
   PairWB w;
   w.alpha = f2(p.alpha);
   w.oma = f2(p.oma);
-  const float dsi = lane_dw_scale_i<NG, ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
+  const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
   for (long long tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {

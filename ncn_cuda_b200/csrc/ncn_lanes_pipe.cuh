@@ -430,7 +430,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
   PairWB w;
   w.alpha = f2(p.alpha);
   w.oma = f2(p.oma);
-  const float dsi = lane_dw_scale_i<NG, ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
+  const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
   for (long long tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {

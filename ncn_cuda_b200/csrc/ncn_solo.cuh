@@ -31,7 +31,7 @@ struct SoloFwd {
   static __device__ __forceinline__ void run(float2 (&X)[NG / 2], float2 (&A)[NG / 2], float owi, float owj, float alpha) {
     using F = ActForm<ACT>;
     using S = LaneStage<NG, ACT>;
-    constexpr float mk = (float)cpow(S::m, J), mkDk = (float)(cpow(S::m, J) * fwd_D(J, F::f0, S::m, kLaneC));
+    constexpr float mk = (float)cpow(kMd, J), mkDk = (float)(cpow(kMd, J) * fwd_D(J, F::f0));
     constexpr float cA = (float)S::cA(J);
     const float XJ = (J & 1) ? X[J / 2].y : X[J / 2].x;
     const float xj = J == 0 ? XJ : fmaf(XJ, mk, mkDk);
@@ -64,11 +64,11 @@ struct SoloBwd {
     using F = ActForm<ACT>;
     using S = LaneStage<NG, ACT>;
     constexpr int k = NG - 1 - J;
-    constexpr double mkd = cpow(S::m, k), DX = bwd_DX(k + 1, F::f0, S::m, kLaneC);
-    constexpr float imk1 = (float)(1.0 / cpow(S::m, k + 1)), DX1 = (float)DX, imk1DX1 = (float)(DX / cpow(S::m, k + 1));
+    constexpr double mkd = cpow(kMd, k), DX = bwd_DX(k + 1, F::f0);
+    constexpr float imk1 = (float)(1.0 / cpow(kMd, k + 1)), DX1 = (float)DX, imk1DX1 = (float)(DX / cpow(kMd, k + 1));
     constexpr float cAr = (float)S::cAr(J);
-    constexpr float sTimk1 = (float)(F::sT / cpow(S::m, k + 1)), cdsm = (float)(kLaneC * F::ds / S::m);
-    constexpr float K1 = (float)(kLaneC * F::ds / S::m / cpow(S::m, k + 1)), K2 = (float)(2.0 * kLaneC * F::ds / S::m);
+    constexpr float sTimk1 = (float)(F::sT / cpow(kMd, k + 1)), cdsm = (float)(kCd * F::ds / kMd);
+    constexpr float K1 = (float)(kCd * F::ds / kMd / cpow(kMd, k + 1)), K2 = (float)(2.0 * kCd * F::ds / kMd);
 #pragma unroll
     for (int i = 0; i < NG / 2; ++i) X[i] = __ffma2_rn(f2(-kC), A[i], X[i]);
     const float XJ = (J & 1) ? X[J / 2].y : X[J / 2].x;
@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
   const int base = r * N;
   const uint32_t row = smem_u32(smem) + 16u * (uint32_t)base;
   constexpr float sT = (float)F::sT;
-  const float dsi = lane_dw_scale_i<NG, ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
+  const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
   for (long long tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
