@@ -4,12 +4,12 @@
 
 namespace ncn {
 
-template <int ACT, typename T, bool RAG, bool NANX>
+template <int ACT, typename T, bool RAG>
 static cudaError_t launch_form(const LaneParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
 #ifdef NCN_BWD
   auto k = lane_bwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads, RAG>;
 #else
-  auto k = lane_fwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneFwdBlocks * kLaneThreads / kLaneMaxThreads, RAG, NANX>;
+  auto k = lane_fwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneFwdBlocks * kLaneThreads / kLaneMaxThreads, RAG>;
 #endif
   static SmemGrant granted;
   cudaError_t e = grant_smem(granted, k, smem);
@@ -46,11 +46,7 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
   }
 #endif
 #endif
-  if (p.ragged) return launch_form<ACT, T, true, true>(p, grid, threads, smem, st, occ);
-#ifndef NCN_BWD
-  if (p.tpr > kLaneThreads) return launch_form<ACT, T, false, true>(p, grid, threads, smem, st, occ);
-#endif
-  return launch_form<ACT, T, false, false>(p, grid, threads, smem, st, occ);
+  return p.ragged ? launch_form<ACT, T, true>(p, grid, threads, smem, st, occ) : launch_form<ACT, T, false>(p, grid, threads, smem, st, occ);
 }
 
 template <typename T>

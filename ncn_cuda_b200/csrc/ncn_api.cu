@@ -475,7 +475,7 @@ static bool lane_shape_ok(int64_t N, int64_t E, int n, int C, int l0, int L, int
   sh->ragged = (m & (m - 1)) != 0 || m != sh->tpr * G;
   sh->min_blocks = 32 * G;
   if (sh->ragged) {
-    // a single stage stays where a NaN in xa alone reaches no other position of its group
+    // (a single stage, with one boundary on each side, was not measured here)
     if (L < 2 || !lane_ragged_pays(n, sh->thr, sh->tpr)) return false;
     for (int w = 0; w < wpr; ++w) {  // as LaneShare (ncn_lanes.cuh) deals them
       const int end = G * ((w + 1) * sh->thr / wpr), vb = (end < m ? end : m) - G * (w * sh->thr / wpr);
@@ -491,9 +491,9 @@ static bool lane_shape_ok(int64_t N, int64_t E, int n, int C, int l0, int L, int
 }
 
 // Lay one CTA out.  ea: shifts of up to 2^ea blocks go by shuffles + halo, longer ones through the
-// tile buffer (which must then hold fp32 values).
+// tile buffer (which must then hold fp32 values).  terms: the buffer also takes one row in fp32 (ncn_terms.cuh).
 static bool lane_layout(bool bwd, int N, int n, int L, int dtype, int flags, int n_ck, int R, int tpr, int ea, int e_need,
-                        uint32_t limit, LanePlan& pl) {
+                        bool terms, uint32_t limit, LanePlan& pl) {
   const int w = dtype == DT_BF16 ? 2 : 4;
   const int NS = bwd ? 4 : 2;
   const bool residual = (flags & F_RESIDUAL) != 0;
@@ -503,7 +503,8 @@ static bool lane_layout(bool bwd, int N, int n, int L, int dtype, int flags, int
   const int warps = threads / 32;
   uint64_t off = 0;
   auto take = [&](uint64_t bytes) { uint64_t o = off; off = (off + bytes + 127) / 128 * 128; return (uint32_t)o; };
-  pl.off_work = take(NS * RN * (long_shifts ? 4 : w));
+  const uint64_t work = NS * RN * (long_shifts ? 4 : w);
+  pl.off_work = take(terms && work < (uint64_t)8 * N ? (uint64_t)8 * N : work);
   pl.off_res = residual ? take(RN * w) : pl.off_work;
   pl.off_ckpt = take(n_ck ? (uint64_t)n_ck * RN * 8 : 16);
   pl.halo_warp_bytes = ea >= 0 ? (uint32_t)(NS * lane_halo_floats(n, ea) * 4) : 0;
@@ -601,6 +602,7 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   int ea_lo = shape.ragged ? 0 : lane_ilog2(G) - 1;
   while (shape.ragged && ea_hi > 0 && ((n - 1) << ea_hi) > shape.min_blocks) --ea_hi;
   if (ea_lo > ea_hi) ea_lo = ea_hi;
+  const bool terms = !bwd && (act == ACT_TANH || act == ACT_SIGMOID);
   int rc = NCN_ERR_UNSUPPORTED;
   LanePlan best;
   bool have_pipe = false;
@@ -622,7 +624,8 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   }
   for (int ea = ea_hi; !have_pipe && ea >= ea_lo; --ea) {
     LanePlan trial;
-    if (!lane_layout(bwd, (int)N, n, L, dtype, flags, n_ck, R, tpr, ea, e_need, (uint32_t)dev.smem_optin, trial)) continue;
+    if (!lane_layout(bwd, (int)N, n, L, dtype, flags, n_ck, R, tpr, ea, e_need, terms, (uint32_t)dev.smem_optin, trial))
+      continue;
     int occ = 0;
     LaneParams dummy{};
     dummy.ragged = shape.ragged ? 1 : 0;
@@ -747,7 +750,7 @@ static int plan_solo(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, in
 
 static void fill_solo(SoloParams& p, const SoloPlan& pl, int64_t B, int64_t N, int n, int L, int first, double alpha, int flags) {
   p.B = B; p.N = (int)N; p.m = (int)(N / n); p.L = L; p.l0 = first;
-  p.flags = flags & (F_RESIDUAL | F_TAPE);
+  p.flags = flags & (F_RESIDUAL | F_TAPE | F_OVERLAP);
   p.alpha = (float)alpha;
   p.oma = (float)(1.0 - alpha);
   p.R = pl.R; p.tiles = pl.tiles;
@@ -1203,6 +1206,12 @@ static int net_fwd_impl(const void* x, const void* xa, const float* const* list,
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
   const int act = fused_act(map_act(activation), dtype);
   float* ck_used = (ckpt && ckpt_slots(L, ckpt_every, flags) > 0) ? ckpt : nullptr;
+  const size_t bytes = (size_t)B * (size_t)N * (dtype == DT_BF16 ? 2 : 4);
+  auto over = [&](const void* p, const void* q) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+    return a < b ? b - a < bytes : a - b < bytes;
+  };
+  const int overlap = over(y, x) || over(y, xa) || over(ya, x) || over(ya, xa) ? F_OVERLAP : 0;
   auto fill_list = [&](WeightList& wl) {
     for (int l = 0; l < L; ++l) wl.src[l] = list[l];
     wl.out = const_cast<float*>(W);
@@ -1231,7 +1240,7 @@ static int net_fwd_impl(const void* x, const void* xa, const float* const* list,
       q.W = W;
       q.status = dev.status;
       q.B = B; q.N = (int)N; q.m = (int)(N / n_cache); q.L = L; q.l0 = first_module;
-      q.flags = flags & (F_RESIDUAL | F_TAPE);
+      q.flags = (flags & (F_RESIDUAL | F_TAPE)) | overlap;
       q.alpha = (float)alpha;
       q.oma = (float)(1.0 - alpha);
       fill_lane(q, lp);
@@ -1252,7 +1261,7 @@ static int net_fwd_impl(const void* x, const void* xa, const float* const* list,
       q.ckpt_every = ckpt_every;
       q.W = W;
       q.status = dev.status;
-      fill_solo(q, sp, B, N, n_cache, L, first_module, alpha, flags);
+      fill_solo(q, sp, B, N, n_cache, L, first_module, alpha, flags | overlap);
       if (list && L <= kWeightList) fill_list(q.list);
       else if (list && (rc = gather()) != NCN_OK) return rc;
       cudaError_t e = solo_fn(n_cache, false)(act, dtype, q, sp.grid, sp.threads, sp.smem, (cudaStream_t)stream, nullptr);

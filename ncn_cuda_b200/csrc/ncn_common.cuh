@@ -49,6 +49,7 @@ enum : int {
   F_RECOMPUTE = 2,  // backward: inputs are the net INPUT; replay the forward, then walk back
   F_RED_THREAD = 4, // backward (set by the launch plan): dW partial slots per thread instead of per warp
   F_TAPE = 8,       // the state after the LAST stage is checkpointed too (fp32); the backward starts from it
+  F_OVERLAP = 16,   // forward (set by the call): a result lies over an input
 };
 
 // error codes stored in the device status word by a kernel that gave up a wait
@@ -368,17 +369,17 @@ struct ActForm<ACT_LINEAR> {
 // (4: 1.25, 2: 1.5, 1: 2 special-function instructions per position and step; the smaller the batch
 // the fewer multiplies on the FMA pipe).
 // The exponent is capped at 30: beyond it r < 1e-9 (tanh = 1 to the last bit) and the product of four d stays a normal
-// fp32 number, as does its reciprocal.  A NaN reaches all values that share its reciprocal, where these would see it all
-// the same: the features of one position through their dot product, the positions of a group in the reverse sweep, which
-// the NaN joins when its position is x_j.  Without KEEP_NAN the cap drops it (r = 2^-30) and the caller sees to it.
-template <int ACT, int NG, int BATCH, bool KEEP_NAN = true>
+// fp32 number, as does its reciprocal.  A NaN reaches all values that share its reciprocal.  These would see it all the same
+// where they are the features of one position, through their dot product, and in the reverse sweep, where the sums for gx_j
+// bring a NaN in any x of a group to all of its cotangents.  They would not in the forward steps of a group's positions: a row
+// with a NaN is taken again there (ncn_terms.cuh).
+template <int ACT, int NG, int BATCH>
 __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG]) {
   if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {
     float2 d[NG];
 #pragma unroll
     for (int i = 0; i < NG; ++i) {
-      const float2 e = KEEP_NAN ? make_float2(min_nan(ts[i].x, 30.0f), min_nan(ts[i].y, 30.0f))
-                                : make_float2(fminf(ts[i].x, 30.0f), fminf(ts[i].y, 30.0f));
+      const float2 e = make_float2(min_nan(ts[i].x, 30.0f), min_nan(ts[i].y, 30.0f));
       d[i] = __fadd2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), f2(1.0f));
     }
     if constexpr (BATCH == 1) {

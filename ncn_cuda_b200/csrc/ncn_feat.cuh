@@ -316,7 +316,7 @@ struct FeatThread {
 template <int ACT, int KP, int BATCH>
 __device__ __forceinline__ void feat_act(const float2 (&ts)[KP], float2 (&rr)[KP]) {
   if constexpr (KP >= 2 && BATCH > 1) {
-    act_r_all<ACT, KP, BATCH, /*KEEP_NAN=*/true>(ts, rr);
+    act_r_all<ACT, KP, BATCH>(ts, rr);
   } else {
 #pragma unroll
     for (int q = 0; q < KP; ++q) rr[q] = ActForm<ACT>::r(ts[q]);

@@ -28,6 +28,7 @@
 #pragma once
 #include "ncn_pairs.cuh"
 #include "ncn_lanes_launch.h"
+#include "ncn_terms.cuh"
 
 namespace ncn {
 
@@ -81,7 +82,7 @@ struct LaneStage {
   static constexpr double cAr(int J) { return -kCd * F::f1 * cpow(kMd, NG - 1 - J); }
 };
 
-template <int NG, int ACT, int J, bool NANX>
+template <int NG, int ACT, int J>
 struct LFwdSteps {
   static __device__ __forceinline__ void run(float2 (&X)[NG], float2 (&A)[NG], const PairW& w) {
     using F = ActForm<ACT>;
@@ -103,41 +104,24 @@ struct LFwdSteps {
     float2 ts[NG], r[NG];
 #pragma unroll
     for (int i = 0; i < NG; ++i) ts[i] = ffma2(X[i], P, Q);
-    act_r_all<ACT, NG, LaneBatch<NG>::fwd, /*KEEP_NAN=*/!NANX>(ts, r);
-    // A NaN that is x_j reaches every position of the group through the constant; one elsewhere stays in its own x, and
-    // joins its a when the results are stored (lane_keep_nan).  |x_j| is never less than a negative constant.
-    float2 c = f2(cA);
-    if constexpr (NANX && ACT == ACT_TANH) c = make_float2(min_nan(cA, fabsf(xj.x)), min_nan(cA, fabsf(xj.y)));
-    if constexpr (NANX && ACT == ACT_SIGMOID) c = make_float2(-min_nan(-cA, fabsf(xj.x)), -min_nan(-cA, fabsf(xj.y)));
+    act_r_all<ACT, NG, LaneBatch<NG>::fwd>(ts, r);
 #pragma unroll
     for (int i = 0; i < NG; ++i) {
-      A[i] = ffma2(r[i], c, A[i]);
+      A[i] = ffma2(r[i], f2(cA), A[i]);
       X[i] = ffma2(A[i], f2(kC), X[i]);
     }
-    LFwdSteps<NG, ACT, J + 1, NANX>::run(X, A, w);
+    LFwdSteps<NG, ACT, J + 1>::run(X, A, w);
   }
 };
-template <int NG, int ACT, bool NANX>
-struct LFwdSteps<NG, ACT, NG, NANX> {
+template <int NG, int ACT>
+struct LFwdSteps<NG, ACT, NG> {
   static __device__ __forceinline__ void run(float2 (&)[NG], float2 (&)[NG], const PairW&) {}
 };
 
-// a is NaN where x is (tanh and sigmoid drop it on the way).
 template <int NG, int ACT>
-__device__ __forceinline__ void lane_keep_nan(const float2 (&X)[NG], float2 (&A)[NG]) {
-  if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {
-#pragma unroll
-    for (int i = 0; i < NG; ++i) {
-      if (X[i].x != X[i].x) A[i].x = X[i].x;
-      if (X[i].y != X[i].y) A[i].y = X[i].y;
-    }
-  }
-}
-
-template <int NG, int ACT, bool NANX = false>
 __device__ __forceinline__ void lane_forward(float2 (&X)[NG], float2 (&A)[NG], const PairW& w) {
   using F = ActForm<ACT>;
-  LFwdSteps<NG, ACT, 0, NANX>::run(X, A, w);
+  LFwdSteps<NG, ACT, 0>::run(X, A, w);
   constexpr float mN = (float)LaneStage<NG, ACT>::mN, mNC = (float)LaneStage<NG, ACT>::mNC, mND = (float)LaneStage<NG, ACT>::mND;
 #pragma unroll
   for (int i = 0; i < NG; ++i) {
@@ -598,7 +582,7 @@ __device__ __forceinline__ void lane_st_native(T* chunk, const float2 (&Sv)[G / 
 }
 
 // ------------------------------------------------------------------------------------------ forward
-template <int NG, int ACT, typename T, int MAXT, int MINB, bool RAG, bool NANX>
+template <int NG, int ACT, typename T, int MAXT, int MINB, bool RAG>
 __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_constant__ LaneParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
@@ -612,6 +596,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_const
   StageRec* recs = reinterpret_cast<StageRec*>(smem + p.off_w);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + p.off_bar);
   int* abort_flag = reinterpret_cast<int*>(bar + 2);
+  int* wild = abort_flag + 1;  // a row did not come out finite (ncn_terms.cuh)
   const T* gx_in = static_cast<const T*>(p.in[0]);
   const T* ga_in = static_cast<const T*>(p.in[1]);
   T* gy_out = static_cast<T*>(p.out[0]);
@@ -623,6 +608,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_const
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     *abort_flag = 0;
+    *wild = 0;
     fence_mbar_init();
   }
   fill_stage_table(recs, p.W, p.oma, p.l0, p.m, p.L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr, &p.list);
@@ -703,7 +689,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_const
       w.owi = f2(rec.owi * sT);
       w.owj = f2(rec.owj * sT);
 #pragma unroll
-      for (int pp = 0; pp < G / 2; ++pp) lane_forward<NG, ACT, NANX>(V[0][pp], V[1][pp], w);
+      for (int pp = 0; pp < G / 2; ++pp) lane_forward<NG, ACT>(V[0][pp], V[1][pp], w);
       if (rec.ck >= 0 && active) {
         // order of a stored state: [stream][offset][pair of groups], a pair = groups 2q, 2q+1 of the stage
         float2* ck = ckpt + (long long)rec.ck * BN + (row0 + r) * N + (sh.blk >> 1);
@@ -726,9 +712,14 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_const
           }
       }
     }
-    if constexpr (NANX) {
+    if constexpr (act_shares<ACT>()) {  // (before the exchange: its shuffles and the look overlap)
+      float2 q = f2(0.0f);
 #pragma unroll
-      for (int pp = 0; pp < G / 2; ++pp) lane_keep_nan<NG, ACT>(V[0][pp], V[1][pp]);
+      for (int pp = 0; pp < G / 2; ++pp)
+#pragma unroll
+        for (int o = 0; o < NG; ++o)
+          if (sh.pair(pp)) q = ffma2(V[0][pp][o], V[0][pp][o], q);
+      if (active && !finite(q)) *wild = 1;
     }
     lane_exchange<NG, G, 2, RAG>(V, -s_cur, p.ea_max, halo, lane, xrow, sh, m);  // back to stride 0 = native order
     if (active) {
@@ -752,6 +743,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_const
       bulk_commit();
     }
   }
+  if constexpr (act_shares<ACT>()) wild_rows_by_terms<NG, ACT, T, /*PAIRS=*/true>(p, wild, abort_flag, recs, reinterpret_cast<float*>(win));
   if (tid == 0) {
     bulk_wait_all0();
     if (*abort_flag) atomicExch(p.status, DEV_WAIT_TIMEOUT);

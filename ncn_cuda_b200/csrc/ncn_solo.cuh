@@ -36,17 +36,16 @@ struct SoloFwd {
     const float XJ = (J & 1) ? X[J / 2].y : X[J / 2].x;
     const float xj = J == 0 ? XJ : fmaf(XJ, mk, mkDk);
     const float pp = fmaf(owi, xj, alpha);  // sT (alpha + (1-alpha) wi xj)
-    const float2 P = f2(pp * mk), Q = f2(fmaf(pp, mkDk, (owj * xj) * xj));
+    float q = (owj * xj) * xj;
+    if constexpr (mkDk != 0.0f) q = fmaf(pp, mkDk, q);  // (no product by zero: pp may be infinite)
+    const float2 P = f2(pp * mk), Q = f2(q);
     float2 ts[NG / 2], r[NG / 2];
 #pragma unroll
     for (int i = 0; i < NG / 2; ++i) ts[i] = __ffma2_rn(X[i], P, Q);
-    act_r_all<ACT, NG / 2, 4, /*KEEP_NAN=*/false>(ts, r);
-    float c = cA;  // a NaN that is x_j reaches the whole group through the constant (as in LFwdSteps)
-    if constexpr (ACT == ACT_TANH) c = min_nan(cA, fabsf(xj));
-    if constexpr (ACT == ACT_SIGMOID) c = -min_nan(-cA, fabsf(xj));
+    act_r_all<ACT, NG / 2, 4>(ts, r);
 #pragma unroll
     for (int i = 0; i < NG / 2; ++i) {
-      A[i] = __ffma2_rn(r[i], f2(c), A[i]);
+      A[i] = __ffma2_rn(r[i], f2(cA), A[i]);
       X[i] = __ffma2_rn(A[i], f2(kC), X[i]);
     }
     SoloFwd<NG, ACT, J + 1>::run(X, A, owi, owj, alpha);
@@ -145,6 +144,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const __grid_const
   StageRec* recs = reinterpret_cast<StageRec*>(smem + p.off_w);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + p.off_bar);
   int* abort_flag = reinterpret_cast<int*>(bar + 2);
+  int* wild = abort_flag + 1;  // a row did not come out finite (ncn_terms.cuh)
   const T* gx_in = static_cast<const T*>(p.in[0]);
   const T* ga_in = static_cast<const T*>(p.in[1]);
   T* gy_out = static_cast<T*>(p.out[0]);
@@ -156,6 +156,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const __grid_const
   if (tid == 0) {
     mbar_init(&bar[0], 1);
     *abort_flag = 0;
+    *wild = 0;
     fence_mbar_init();
   }
   fill_stage_table(recs, p.W, p.oma, p.l0, m, L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr, &p.list);
@@ -238,7 +239,12 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const __grid_const
         for (int o = 0; o < NG; ++o) ck[o * m] = make_float2(solo_get<NG>(X, o), solo_get<NG>(A, o));
       }
     }
-    lane_keep_nan<NG / 2, ACT>(X, A);
+    if constexpr (act_shares<ACT>()) {
+      float2 q = f2(0.0f);
+#pragma unroll
+      for (int i = 0; i < NG / 2; ++i) q = __ffma2_rn(X[i], X[i], q);
+      if (active && !finite(q)) *wild = 1;
+    }
     exchange(0);
     __syncthreads();  // every slot has been read; the buffer may take the native results
     if (active) {
@@ -259,6 +265,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const __grid_const
       bulk_commit();
     }
   }
+  if constexpr (act_shares<ACT>()) wild_rows_by_terms<NG, ACT, T, /*PAIRS=*/false>(p, wild, abort_flag, recs, reinterpret_cast<float*>(win));
   if (tid == 0) {
     bulk_wait_all0();
     if (*abort_flag) atomicExch(p.status, DEV_WAIT_TIMEOUT);
