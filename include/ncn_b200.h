@@ -191,10 +191,16 @@ int ncn_net_bwd_noalloc(const void* s0, const void* s1, const void* dy, const vo
                         int activation, int dtype, int flags, int dw_accumulate, void* stream);
 
 /* 1 if ncn_net_fwd / ncn_net_bwd (without x_rec / xa_rec, whose staging needs more shared memory and
- * may still return NCN_ERR_SMEM for the longest rows) cover these arguments on the current device,
- * else 0.  flags and ckpt_every as they will be passed to the net calls. */
+ * may still return NCN_ERR_SMEM for the longest rows) cover these arguments on the current device with any
+ * first_module, else 0.  flags and ckpt_every as they will be passed to the net calls.
+ * ncn_net_supported_from: with this first_module (0 if it is negative).  It also says 1 for rows of 8192 fp32 positions in groups of
+ * 2, 4 and 8, which the calls cover as long as the strides of the stages do not wrap, 2^(first_module + L - 2) < N / n_cache.
+ * Both say 0 for fp32 rows of that length where more than 16 steps lie between two stored states: the net calls
+ * cover them, the per-stage calls are the more accurate way. */
 int ncn_net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int L, int dtype, int flags,
                       int ckpt_every);
+int ncn_net_supported_from(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L, int dtype, int flags,
+                           int ckpt_every);
 
 /* Workspace (bytes) that ncn_stage_bwd (L = 1) or ncn_net_bwd needs for these arguments. */
 size_t ncn_bwd_workspace_bytes(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int L, int dtype);

@@ -69,6 +69,7 @@ SIGNATURES = {
         [c_void_p] * 10 + [c_void_p, c_int] + [c_int64] * 3 + [c_int] * 4 + [c_double, c_int, c_int, c_int, c_int, c_void_p],
     ),
     "ncn_net_supported": (c_int, [c_int64] * 3 + [c_int] * 6),
+    "ncn_net_supported_from": (c_int, [c_int64] * 3 + [c_int] * 7),
     "ncn_bwd_workspace_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 4),
     "ncn_ckpt_bytes": (c_size_t, [c_int64] * 3 + [c_int] * 3),
     "ncn_gather_weights": (c_int, [c_void_p, c_int, c_int64, c_void_p, c_void_p]),

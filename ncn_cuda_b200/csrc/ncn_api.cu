@@ -1144,8 +1144,8 @@ size_t ncn_ckpt_bytes(int64_t B, int64_t N, int64_t E, int L, int ckpt_every, in
   return (size_t)ckpt_slots(L, ckpt_every, flags) * 2 * (size_t)B * (size_t)N * (size_t)E * sizeof(float);
 }
 
-int ncn_net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int L, int dtype, int flags,
-                      int ckpt_every) {
+// first: the first stage, or -1 for any.
+static int net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first, int L, int dtype, int flags, int ckpt_every) {
   if (check_common(B, N, E, n_cache, n_head, dtype) != NCN_OK || L < 1) return 0;
   if (!rows_shape_ok(N, E, n_cache, n_head, dtype)) return 0;
   DevInfo dev;
@@ -1161,13 +1161,22 @@ int ncn_net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, 
   const int walk = n_cache * (ckpt_every > 0 && ckpt_every < L ? ckpt_every : L);
   if (dtype == DT_F32 && walk > kSegment) return 0;
   const int act = fused_act(ACT_TANH, dtype);
-  LanePlan lf, lb;
-  if (plan_lanes(false, B, N, E, n_cache, n_head, 0, L, dtype, flags, 0, dev, act, lf) == NCN_OK &&
-      plan_lanes(true, B, N, E, n_cache, n_head, 0, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK)
+  LanePlan lf, lb;  // (only while the strides of the stages do not wrap)
+  if (first >= 0 && plan_lanes(false, B, N, E, n_cache, n_head, first, L, dtype, flags, 0, dev, act, lf) == NCN_OK &&
+      plan_lanes(true, B, N, E, n_cache, n_head, first, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK)
     return 1;
   SoloPlan sf, sb;  // (groups of 8: all rows that fit these fit the shared-memory kernels)
   return plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sf) == NCN_OK &&
          plan_solo(true, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sb) == NCN_OK;
+}
+
+int ncn_net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int L, int dtype, int flags, int ckpt_every) {
+  return net_supported(B, N, E, n_cache, n_head, -1, L, dtype, flags, ckpt_every);
+}
+
+int ncn_net_supported_from(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int first_module, int L, int dtype, int flags,
+                           int ckpt_every) {
+  return first_module < 0 ? 0 : net_supported(B, N, E, n_cache, n_head, first_module, L, dtype, flags, ckpt_every);
 }
 
 int ncn_gather_weights(const float* const* weights, int L, int64_t cols, float* out, void* stream) {

@@ -543,7 +543,7 @@ Result py_net_list(const Tensor& x, const Tensor& xa, const variable_list& ws, d
   if (act != 3) {  // leaky-relu has per-stage kernels only
     const c10::cuda::OptionalCUDAGuard guard(x.device());
     const int flags = (recompute ? NCN_RECOMPUTE : 0) | (tape ? NCN_TAPE : 0);
-    fused = ncn_net_supported(x.size(0), x.size(1), x.size(2), n, C, L, dtype_code(x), flags, every) != 0;
+    fused = ncn_net_supported_from(x.size(0), x.size(1), x.size(2), n, C, 0, L, dtype_code(x), flags, every) != 0;
   }
   if (fused) return fused_forward(x, xa, ws, true, FusedCfg{alpha, act, n, C, 0, L, 1, every, 0, recompute, false, tape});
   return chain_forward(x, xa, ws, Tensor(), ChainCfg{alpha, act, n, C, 0, L, keep, 0});

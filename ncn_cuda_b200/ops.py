@@ -82,11 +82,12 @@ def _workspace(lib, device, B, N, E, n_cache, n_head, L, dt) -> torch.Tensor:
     return ws
 
 
-def net_supported(x: torch.Tensor, n_cache: int, n_head: int, L: int, flags: int = 0, ckpt_every: int = 0) -> bool:
+def net_supported(x: torch.Tensor, n_cache: int, n_head: int, L: int, flags: int = 0, ckpt_every: int = 0,
+                  first_module: int = 0) -> bool:
     lib = _lib.load()
     B, N, E = x.shape
     with _on(x.device):
-        return bool(lib.ncn_net_supported(B, N, E, n_cache, n_head, L, _dtype_code(x), flags, ckpt_every))
+        return bool(lib.ncn_net_supported_from(B, N, E, n_cache, n_head, first_module, L, _dtype_code(x), flags, ckpt_every))
 
 
 def stage_fwd(x, xa, W, alpha, activation, n_cache, n_head, module_l) -> Tuple[torch.Tensor, torch.Tensor]:

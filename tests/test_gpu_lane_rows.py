@@ -104,6 +104,28 @@ def test_long_walks_back_stay_stage_by_stage(ncn):
         assert ncn.ops.net_supported(x, n, 1, 16 // n, 0, 0)
 
 
+@pytest.mark.parametrize("n,N", [(2, 8192), (4, 8192), (8, 8192), (16, 8192), (4, 3000), (2, 1024)])
+def test_what_is_called_covered_is(ncn, n, N):
+    """Stage strides that wrap (2^(stage - 1) >= N / n) leave the register-resident kernels; whole rows of 8192 fp32 positions
+    have no others in groups of 2, 4 and 8."""
+    from ncn_cuda_b200 import _lib
+
+    lib = _lib.load()
+    x = torch.randn(2, N, 1, device="cuda")
+    W = torch.randn(2, 2, device="cuda") * n**-0.5
+    every = 1 if n == 16 else 0
+    for first in (0, 1, 9, 13):
+        covered = ncn.ops.net_supported(x, n, 1, 2, 0, every, first_module=first)
+        wraps = first > 0 and 2**first >= N // n
+        assert covered == (not (wraps and N == 8192 and n < 16))
+        if lib.ncn_net_supported(2, N, 1, n, 1, 2, 0, 0, every):
+            assert covered
+        if covered:
+            y, ya, ck = ncn.ops.net_fwd(x, x, W, 0.9, 0, n, 1, first, every)
+            ncn.ops.net_bwd(y, ya, x, x, W, 0.9, 0, n, 1, first, ckpt=ck, ckpt_every=every)
+    assert lib.ncn_net_supported(2, N, 1, n, 1, 2, 0, 0, every) == (not (N == 8192 and n < 16))
+
+
 @pytest.mark.parametrize("n,N", [(8, 1040), (16, 1840)])
 def test_residual_layers_on_such_rows(ncn, n, N):
     B, layers, L = 9, 3, 3 if n == 8 else 2
