@@ -789,13 +789,11 @@ static int check_common(int64_t B, int64_t N, int64_t E, int n, int C, int dtype
   return NCN_OK;
 }
 
-// Set while a stage's backward leaves its partial sums to a reduction of several stages (ncn_stage_bwd_partial): receives
-// their number of rows.
-static thread_local int* tl_partial_rows = nullptr;
-
-static int reduce_dw(const float* partials, float* dW, int rows, int cols, int accumulate, cudaStream_t st) {
-  if (tl_partial_rows != nullptr) {
-    *tl_partial_rows = rows;
+// left: not null where a stage's backward leaves its partial sums to a reduction of several stages (ncn_stage_bwd_partial);
+// receives their number of rows.
+static int reduce_dw(const float* partials, float* dW, int rows, int cols, int accumulate, cudaStream_t st, int* left) {
+  if (left != nullptr) {
+    *left = rows;
     return NCN_OK;
   }
   const int warps = 4;
@@ -907,7 +905,8 @@ struct FeatExtra {
 // back to the shared-memory kernels); anything else is an error.
 static int launch_feat(bool bwd, const void* const* in, void* const* out, const float* W, float* partials, int64_t B,
                        int64_t N, int64_t E, int n, int C, int module_l, double alpha, int activation, int dtype,
-                       const DevInfo& dev, cudaStream_t st, int* grid_out, const FeatExtra& ex = FeatExtra()) {
+                       const DevInfo& dev, cudaStream_t st, int* grid_out, const FeatExtra& ex = FeatExtra(),
+                       long long max_rows = 1LL << 40) {
   const int d = (int)(E / C);
   const int lanes = feat_lanes(d), rows = feat_rows(n, lanes);
   const FeatLaunchFn fn = feat_fn(n, bwd);
@@ -979,6 +978,7 @@ static int launch_feat(bool bwd, const void* const* in, void* const* out, const 
   const long long q = C / gcd_ll(C, tpc);
   grid = (grid + q - 1) / q * q;
   if (grid > (long long)dev.sms * 32) return NCN_ERR_UNSUPPORTED;  // more heads than the workspace covers
+  if (grid > max_rows) return NCN_ERR_WORKSPACE;
   e = fn(d, team, act, dtype, p, (int)grid, threads, st, nullptr);
   if (e != cudaSuccess) return cuda_fail(e);
   if (grid_out) *grid_out = (int)grid;
@@ -1017,7 +1017,7 @@ static int stage_bwd_generic(const void* y, const void* ya, const void* dy, cons
                              int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha,
                              int activation, int dtype, const DevInfo& dev, void* stream, const void* x_saved = nullptr,
                              const void* xa_saved = nullptr, int replay_all = 0, const float* mid = nullptr,
-                             int mid_end = 0) {
+                             int mid_end = 0, int* left = nullptr, long long max_rows = 1LL << 40) {
   StageParams p{};
   fill_stage(p, B, N, E, n_cache, n_head, module_l, alpha);
   p.xin[0] = x_saved; p.xin[1] = xa_saved;
@@ -1033,16 +1033,18 @@ static int stage_bwd_generic(const void* y, const void* ya, const void* dy, cons
   const int act = map_act(activation);
   if (dtype == DT_BF16) {
     if ((rc = plan_generic(stage_bwd_kernel<__nv_bfloat16>, true, p.groups, p.n, p.d, p.E, dev, g)) != NCN_OK) return rc;
+    if (g.grid > max_rows) return NCN_ERR_WORKSPACE;
     p.warps = g.warps; p.warp_floats = g.warp_floats;
     stage_bwd_kernel<__nv_bfloat16><<<g.grid, g.warps * 32, g.smem, (cudaStream_t)stream>>>(p, act);
   } else {
     if ((rc = plan_generic(stage_bwd_kernel<float>, true, p.groups, p.n, p.d, p.E, dev, g)) != NCN_OK) return rc;
+    if (g.grid > max_rows) return NCN_ERR_WORKSPACE;
     p.warps = g.warps; p.warp_floats = g.warp_floats;
     stage_bwd_kernel<float><<<g.grid, g.warps * 32, g.smem, (cudaStream_t)stream>>>(p, act);
   }
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e);
-  return reduce_dw(p.partials, dW, g.grid, 2 * (int)E, 0, (cudaStream_t)stream);
+  return reduce_dw(p.partials, dW, g.grid, 2 * (int)E, 0, (cudaStream_t)stream, left);
 }
 
 // ---- one [L][cols] buffer out of L weight vectors: the pointers travel in the parameter block, 32 to a launch
@@ -1321,7 +1323,7 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
                         float* partials, size_t capacity_floats, bool full_workspace, int short_err, int64_t B,
                         int64_t N, int64_t E,
                         int n_cache, int n_head, int first_module, int L, double alpha, int activation, int dtype,
-                        int flags, int dw_accumulate, void* stream) {
+                        int flags, int dw_accumulate, void* stream, int* left = nullptr) {
   int rc = check_common(B, N, E, n_cache, n_head, dtype);
   if (rc != NCN_OK) return rc;
   if (L < 1 || first_module < 0) return NCN_ERR_SHAPE;
@@ -1344,6 +1346,7 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
   // for the same arguments: kernels with more CTAs launch fewer where they would not fit.
   auto fit_grid = [&](int& grid) {
     if ((size_t)grid * 2 * (size_t)L <= capacity_floats) return (int)NCN_OK;
+    if (left != nullptr) return short_err;  // (the sums of several stages are in the order of the single calls)
     Plan pr;
     if (plan_rows(true, B, (int)N, n_cache, L, dtype, flags, n_ck, x_rec != nullptr, dev, act, pr) == NCN_OK &&
         (size_t)pr.grid * 2 * (size_t)L > capacity_floats)
@@ -1378,7 +1381,7 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
       fill_lane(q, lp);
       cudaError_t e = lane_fn(n_cache, true)(act, dtype, q, lp.grid, lp.threads, lp.smem, (cudaStream_t)stream, nullptr);
       if (e != cudaSuccess) return cuda_fail(e);
-      return reduce_dw(partials, dW, lp.grid, 2 * L, dw_accumulate, (cudaStream_t)stream);
+      return reduce_dw(partials, dW, lp.grid, 2 * L, dw_accumulate, (cudaStream_t)stream, left);
     }
   }
   {
@@ -1397,7 +1400,7 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
       fill_solo(q, sp, B, N, n_cache, L, first_module, alpha, flags);
       cudaError_t e = solo_fn(n_cache, true)(act, dtype, q, sp.grid, sp.threads, sp.smem, (cudaStream_t)stream, nullptr);
       if (e != cudaSuccess) return cuda_fail(e);
-      return reduce_dw(partials, dW, sp.grid, 2 * L, dw_accumulate, (cudaStream_t)stream);
+      return reduce_dw(partials, dW, sp.grid, 2 * L, dw_accumulate, (cudaStream_t)stream, left);
     }
   }
   Plan pl;
@@ -1421,7 +1424,7 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
   cudaError_t e = (pl.pair ? pair_fn(n_cache, true) : rows_fn(n_cache, true))(act, dtype, p, pl.grid, pl.threads, pl.smem,
                                                                              (cudaStream_t)stream, nullptr);
   if (e != cudaSuccess) return cuda_fail(e);
-  return reduce_dw(p.partials, dW, pl.grid, 2 * L, dw_accumulate, (cudaStream_t)stream);
+  return reduce_dw(p.partials, dW, pl.grid, 2 * L, dw_accumulate, (cudaStream_t)stream, left);
 }
 
 int ncn_net_bwd(const void* s0, const void* s1, const void* dy, const void* dya, const float* W, void* dx, void* dxa,
@@ -1457,10 +1460,10 @@ int ncn_stage_fwd(const void* x, const void* xa, const float* W, void* y, void* 
                            stream);
 }
 
-int ncn_stage_bwd(const void* y, const void* ya, const void* dy, const void* dya, const float* W, void* dx, void* dxa,
+static int stage_bwd_impl(const void* y, const void* ya, const void* dy, const void* dya, const float* W, void* dx, void* dxa,
                   void* x_rec, void* xa_rec, float* dW, void* workspace, size_t workspace_bytes, int64_t B, int64_t N,
                   int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation, int dtype,
-                  void* stream) {
+                  void* stream, int* left) {
   int rc = check_common(B, N, E, n_cache, n_head, dtype);
   if (rc != NCN_OK) return rc;
   if (module_l < 0) return NCN_ERR_SHAPE;
@@ -1468,11 +1471,13 @@ int ncn_stage_bwd(const void* y, const void* ya, const void* dy, const void* dya
   if ((x_rec == nullptr) != (xa_rec == nullptr)) return NCN_ERR_NULL;
   DevInfo dev;
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
-  if (!workspace || workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float)) return NCN_ERR_WORKSPACE;
+  if (!workspace || (!left && workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float))) return NCN_ERR_WORKSPACE;
+  const long long max_rows = (long long)(workspace_bytes / (2 * (size_t)E * sizeof(float)));
   if (rows_shape_ok(N, E, n_cache, n_head, dtype) && aligned16(y) && aligned16(ya) && aligned16(dy) && aligned16(dya) &&
       aligned16(dx) && aligned16(dxa) && (!x_rec || (aligned16(x_rec) && aligned16(xa_rec)))) {
-    rc = ncn_net_bwd(y, ya, dy, dya, W, dx, dxa, x_rec, xa_rec, dW, nullptr, 0, workspace, workspace_bytes, B, N, E,
-                     n_cache, n_head, module_l, 1, alpha, activation, dtype, 0, 0, stream);
+    rc = net_bwd_impl(y, ya, dy, dya, W, dx, dxa, x_rec, xa_rec, dW, nullptr, 0, static_cast<float*>(workspace),
+                      workspace_bytes / sizeof(float), !left, NCN_ERR_WORKSPACE, B, N, E, n_cache, n_head, module_l, 1, alpha, activation,
+                      dtype, 0, 0, stream, left);
     if (rc != NCN_ERR_SMEM && rc != NCN_ERR_UNSUPPORTED) return rc;
   }
   {
@@ -1480,18 +1485,27 @@ int ncn_stage_bwd(const void* y, const void* ya, const void* dy, const void* dya
     void* fout[4] = {dx, dxa, x_rec, xa_rec};
     int fgrid = 0;
     rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
-                     activation, dtype, dev, (cudaStream_t)stream, &fgrid);
-    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream);
+                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, FeatExtra(), max_rows);
+    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream, left);
     if (rc != NCN_ERR_UNSUPPORTED) return rc;
   }
   return stage_bwd_generic(y, ya, dy, dya, W, nullptr, dx, dxa, x_rec, xa_rec, dW, static_cast<float*>(workspace), B, N, E,
-                           n_cache, n_head, module_l, alpha, activation, dtype, dev, stream);
+                           n_cache, n_head, module_l, alpha, activation, dtype, dev, stream, nullptr, nullptr, 0, nullptr, 0,
+                           left, max_rows);
 }
 
-int ncn_stage_bwd_saved(const void* x, const void* xa, const void* y, const void* ya, const void* dy, const void* dya,
+int ncn_stage_bwd(const void* y, const void* ya, const void* dy, const void* dya, const float* W, void* dx, void* dxa,
+                  void* x_rec, void* xa_rec, float* dW, void* workspace, size_t workspace_bytes, int64_t B, int64_t N,
+                  int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation, int dtype,
+                  void* stream) {
+  return stage_bwd_impl(y, ya, dy, dya, W, dx, dxa, x_rec, xa_rec, dW, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                        module_l, alpha, activation, dtype, stream, nullptr);
+}
+
+static int stage_bwd_saved_impl(const void* x, const void* xa, const void* y, const void* ya, const void* dy, const void* dya,
                         const float* W, void* dx, void* dxa, float* dW, void* workspace, size_t workspace_bytes, int64_t B,
                         int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation,
-                        int dtype, void* stream) {
+                        int dtype, void* stream, int* left) {
   int rc = check_common(B, N, E, n_cache, n_head, dtype);
   if (rc != NCN_OK) return rc;
   if (module_l < 0) return NCN_ERR_SHAPE;
@@ -1500,11 +1514,12 @@ int ncn_stage_bwd_saved(const void* x, const void* xa, const void* y, const void
   const int replay_all = dtype == DT_BF16 ? 1 : 0;
   if (!replay_all && (!y || !ya)) return NCN_ERR_NULL;
   if (!replay_all && n_cache <= kSegment)  // the chain from the output is short enough: the input is not needed
-    return ncn_stage_bwd(y, ya, dy, dya, W, dx, dxa, nullptr, nullptr, dW, workspace, workspace_bytes, B, N, E, n_cache,
-                         n_head, module_l, alpha, activation, dtype, stream);
+    return stage_bwd_impl(y, ya, dy, dya, W, dx, dxa, nullptr, nullptr, dW, workspace, workspace_bytes, B, N, E, n_cache,
+                         n_head, module_l, alpha, activation, dtype, stream, left);
   DevInfo dev;
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
-  if (!workspace || workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float)) return NCN_ERR_WORKSPACE;
+  if (!workspace || (!left && workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float))) return NCN_ERR_WORKSPACE;
+  const long long max_rows = (long long)(workspace_bytes / (2 * (size_t)E * sizeof(float)));
   {
     const void* fin[4] = {replay_all ? nullptr : y, replay_all ? nullptr : ya, dy, dya};
     void* fout[4] = {dx, dxa, nullptr, nullptr};
@@ -1513,12 +1528,21 @@ int ncn_stage_bwd_saved(const void* x, const void* xa, const void* y, const void
     ex.saved = 1;
     int fgrid = 0;
     rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
-                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex);
-    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream);
+                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex, max_rows);
+    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream, left);
     if (rc != NCN_ERR_UNSUPPORTED) return rc;
   }
   return stage_bwd_generic(y, ya, dy, dya, W, nullptr, dx, dxa, nullptr, nullptr, dW, static_cast<float*>(workspace), B, N,
-                           E, n_cache, n_head, module_l, alpha, activation, dtype, dev, stream, x, xa, replay_all);
+                           E, n_cache, n_head, module_l, alpha, activation, dtype, dev, stream, x, xa, replay_all, nullptr, 0,
+                           left, max_rows);
+}
+
+int ncn_stage_bwd_saved(const void* x, const void* xa, const void* y, const void* ya, const void* dy, const void* dya,
+                        const float* W, void* dx, void* dxa, float* dW, void* workspace, size_t workspace_bytes, int64_t B,
+                        int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation,
+                        int dtype, void* stream) {
+  return stage_bwd_saved_impl(x, xa, y, ya, dy, dya, W, dx, dxa, dW, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                              module_l, alpha, activation, dtype, stream, nullptr);
 }
 
 // states the per-stage forward stores for ncn_stage_bwd_mid: one after every 16th step short of the last, and with
@@ -1558,25 +1582,26 @@ int ncn_stage_fwd_mid(const void* x, const void* xa, const float* W, void* y, vo
                            stream, static_cast<float*>(mid), mid_end);
 }
 
-int ncn_stage_bwd_mid(const void* y, const void* ya, const void* mid, size_t mid_bytes, const void* dy, const void* dya,
+static int stage_bwd_mid_impl(const void* y, const void* ya, const void* mid, size_t mid_bytes, const void* dy, const void* dya,
                       const float* W, void* dx, void* dxa, float* dW, void* workspace, size_t workspace_bytes, int64_t B,
                       int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation,
-                      int dtype, void* stream) {
+                      int dtype, void* stream, int* left) {
   int rc = check_common(B, N, E, n_cache, n_head, dtype);
   if (rc != NCN_OK) return rc;
   if (module_l < 0) return NCN_ERR_SHAPE;
   if (!dy || !dya || !W || !dx || !dxa || !dW) return NCN_ERR_NULL;
   const size_t need = ncn_stage_mid_bytes(B, N, E, n_cache, dtype);
   if (need == 0)
-    return ncn_stage_bwd(y, ya, dy, dya, W, dx, dxa, nullptr, nullptr, dW, workspace, workspace_bytes, B, N, E, n_cache,
-                         n_head, module_l, alpha, activation, dtype, stream);
+    return stage_bwd_impl(y, ya, dy, dya, W, dx, dxa, nullptr, nullptr, dW, workspace, workspace_bytes, B, N, E, n_cache,
+                         n_head, module_l, alpha, activation, dtype, stream, left);
   if (!mid) return NCN_ERR_NULL;
   if (mid_bytes < need) return NCN_ERR_WORKSPACE;
   const int mid_end = dtype == DT_BF16 ? 1 : 0;
   if (!mid_end && (!y || !ya)) return NCN_ERR_NULL;
   DevInfo dev;
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
-  if (!workspace || workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float)) return NCN_ERR_WORKSPACE;
+  if (!workspace || (!left && workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float))) return NCN_ERR_WORKSPACE;
+  const long long max_rows = (long long)(workspace_bytes / (2 * (size_t)E * sizeof(float)));
   {
     const void* fin[4] = {mid_end ? nullptr : y, mid_end ? nullptr : ya, dy, dya};
     void* fout[4] = {dx, dxa, nullptr, nullptr};
@@ -1585,13 +1610,21 @@ int ncn_stage_bwd_mid(const void* y, const void* ya, const void* mid, size_t mid
     ex.mid = const_cast<float*>(static_cast<const float*>(mid)); ex.mid_end = mid_end;
     int fgrid = 0;
     rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
-                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex);
-    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream);
+                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex, max_rows);
+    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream, left);
     if (rc != NCN_ERR_UNSUPPORTED) return rc;
   }
   return stage_bwd_generic(y, ya, dy, dya, W, nullptr, dx, dxa, nullptr, nullptr, dW, static_cast<float*>(workspace), B, N,
                            E, n_cache, n_head, module_l, alpha, activation, dtype, dev, stream, nullptr, nullptr, 0,
-                           static_cast<const float*>(mid), mid_end);
+                           static_cast<const float*>(mid), mid_end, left, max_rows);
+}
+
+int ncn_stage_bwd_mid(const void* y, const void* ya, const void* mid, size_t mid_bytes, const void* dy, const void* dya,
+                      const float* W, void* dx, void* dxa, float* dW, void* workspace, size_t workspace_bytes, int64_t B,
+                      int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation,
+                      int dtype, void* stream) {
+  return stage_bwd_mid_impl(y, ya, mid, mid_bytes, dy, dya, W, dx, dxa, dW, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                            module_l, alpha, activation, dtype, stream, nullptr);
 }
 
 int ncn_stage_fwd_ctx(const void* x, const void* xa, const float* W, const int* ctxlen, void* y, void* ya, int64_t B,
@@ -1616,10 +1649,10 @@ int ncn_stage_fwd_ctx(const void* x, const void* xa, const float* W, const int* 
                            stream);
 }
 
-int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void* dya, const float* W, const int* ctxlen,
+static int stage_bwd_ctx_impl(const void* y, const void* ya, const void* dy, const void* dya, const float* W, const int* ctxlen,
                       void* dx, void* dxa, void* x_rec, void* xa_rec, float* dW, void* workspace, size_t workspace_bytes,
                       int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation,
-                      int dtype, void* stream) {
+                      int dtype, void* stream, int* left) {
   int rc = check_common(B, N, E, n_cache, n_head, dtype);
   if (rc != NCN_OK) return rc;
   if (module_l < 0) return NCN_ERR_SHAPE;
@@ -1627,7 +1660,8 @@ int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void*
   if ((x_rec == nullptr) != (xa_rec == nullptr)) return NCN_ERR_NULL;
   DevInfo dev;
   if ((rc = get_dev(dev)) != NCN_OK) return rc;
-  if (!workspace || workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float)) return NCN_ERR_WORKSPACE;
+  if (!workspace || (!left && workspace_bytes < workspace_floats(dev, E, 1) * sizeof(float))) return NCN_ERR_WORKSPACE;
+  const long long max_rows = (long long)(workspace_bytes / (2 * (size_t)E * sizeof(float)));
   {
     const void* fin[4] = {y, ya, dy, dya};
     void* fout[4] = {dx, dxa, x_rec, xa_rec};
@@ -1635,12 +1669,21 @@ int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void*
     ex.ctxlen = ctxlen;
     int fgrid = 0;
     rc = launch_feat(true, fin, fout, W, static_cast<float*>(workspace), B, N, E, n_cache, n_head, module_l, alpha,
-                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex);
-    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream);
+                     activation, dtype, dev, (cudaStream_t)stream, &fgrid, ex, max_rows);
+    if (rc == NCN_OK) return reduce_dw(static_cast<float*>(workspace), dW, fgrid, 2 * (int)E, 0, (cudaStream_t)stream, left);
     if (rc != NCN_ERR_UNSUPPORTED) return rc;
   }
   return stage_bwd_generic(y, ya, dy, dya, W, ctxlen, dx, dxa, x_rec, xa_rec, dW, static_cast<float*>(workspace), B, N, E,
-                           n_cache, n_head, module_l, alpha, activation, dtype, dev, stream);
+                           n_cache, n_head, module_l, alpha, activation, dtype, dev, stream, nullptr, nullptr, 0, nullptr, 0,
+                           left, max_rows);
+}
+
+int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void* dya, const float* W, const int* ctxlen,
+                      void* dx, void* dxa, void* x_rec, void* xa_rec, float* dW, void* workspace, size_t workspace_bytes,
+                      int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int module_l, double alpha, int activation,
+                      int dtype, void* stream) {
+  return stage_bwd_ctx_impl(y, ya, dy, dya, W, ctxlen, dx, dxa, x_rec, xa_rec, dW, workspace, workspace_bytes, B, N, E, n_cache,
+                            n_head, module_l, alpha, activation, dtype, stream, nullptr);
 }
 
 int ncn_stage_bwd_partial(int keep, const void* x, const void* xa, const void* y, const void* ya, const void* mid, size_t mid_bytes,
@@ -1650,29 +1693,21 @@ int ncn_stage_bwd_partial(int keep, const void* x, const void* xa, const void* y
   if (!rows || !workspace) return NCN_ERR_NULL;
   float* const unused = static_cast<float*>(workspace);  // (the place of dW: nothing is written to it)
   *rows = 0;
-  tl_partial_rows = rows;
-  int rc;
   switch (keep) {
     case NCN_KEEP_OUTPUT:
-      rc = ncn_stage_bwd(y, ya, dy, dya, W, dx, dxa, nullptr, nullptr, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
-                         module_l, alpha, activation, dtype, stream);
-      break;
+      return stage_bwd_impl(y, ya, dy, dya, W, dx, dxa, nullptr, nullptr, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                         module_l, alpha, activation, dtype, stream, rows);
     case NCN_KEEP_INPUT:
-      rc = ncn_stage_bwd_saved(x, xa, y, ya, dy, dya, W, dx, dxa, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
-                               module_l, alpha, activation, dtype, stream);
-      break;
+      return stage_bwd_saved_impl(x, xa, y, ya, dy, dya, W, dx, dxa, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                               module_l, alpha, activation, dtype, stream, rows);
     case NCN_KEEP_MID:
-      rc = ncn_stage_bwd_mid(y, ya, mid, mid_bytes, dy, dya, W, dx, dxa, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
-                             module_l, alpha, activation, dtype, stream);
-      break;
+      return stage_bwd_mid_impl(y, ya, mid, mid_bytes, dy, dya, W, dx, dxa, unused, workspace, workspace_bytes, B, N, E, n_cache, n_head,
+                             module_l, alpha, activation, dtype, stream, rows);
     case NCN_KEEP_CTX:
-      rc = ncn_stage_bwd_ctx(y, ya, dy, dya, W, ctxlen, dx, dxa, nullptr, nullptr, unused, workspace, workspace_bytes, B, N, E,
-                             n_cache, n_head, module_l, alpha, activation, dtype, stream);
-      break;
-    default: rc = NCN_ERR_UNSUPPORTED;
+      return stage_bwd_ctx_impl(y, ya, dy, dya, W, ctxlen, dx, dxa, nullptr, nullptr, unused, workspace, workspace_bytes, B, N, E,
+                             n_cache, n_head, module_l, alpha, activation, dtype, stream, rows);
+    default: return NCN_ERR_UNSUPPORTED;
   }
-  tl_partial_rows = nullptr;
-  return rc;
 }
 
 int ncn_reduce_partials(const float* const* partials, const int* rows, float* const* dW, int L, int64_t cols, void* stream) {
