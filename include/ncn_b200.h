@@ -127,7 +127,8 @@ int ncn_stage_bwd_ctx(const void* y, const void* ya, const void* dy, const void*
 
 /* A stage's backward without the last step of its weight gradient, for a caller that walks back several stages: `workspace`
  * is left holding *rows rows of 2E partial sums, which ncn_reduce_partials adds up for all stages by one launch (one
- * per 16 of them) in the order the single calls use, so the results are theirs.  keep names the call this stands for
+ * per 16 of them) in the order the single calls use, so the results are theirs.  workspace_bytes: room for these rows
+ * (ncn_bwd_workspace_bytes always is); where it is less, NCN_ERR_WORKSPACE and nothing is launched.  keep names the call this stands for
  * and with it the arguments that are read; the others may be null.  No counterpart in the reference. */
 enum {
   NCN_KEEP_OUTPUT = 0, /* ncn_stage_bwd */

@@ -314,9 +314,9 @@ struct ChainNode : public NcnNode {
     const c10::cuda::OptionalCUDAGuard guard(dy.device());
     const int64_t B = shape_[0], N = shape_[1], E = shape_[2];
     // The stages leave their partial sums side by side in the workspace, and one launch adds up those of all (of as many as
-    // fit): a call asks for ws_bytes and uses a fraction of them.
-    const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, 1, c.dt), room = c.L > 1 ? 2 * ws_bytes : ws_bytes;
-    const Tensor ws = at::empty({(int64_t)room}, dy.options().dtype(at::kByte));
+    // fit: a stage uses a fraction of the ws_bytes that always suffice).
+    const size_t ws_bytes = ncn_bwd_workspace_bytes(B, N, E, c.n, c.C, 1, c.dt);
+    const Tensor ws = at::empty({(int64_t)ws_bytes}, dy.options().dtype(at::kByte));
     char* const ws_base = static_cast<char*>(ws.data_ptr());
     size_t used = 0;
     std::vector<const float*> partial;
@@ -367,12 +367,19 @@ struct ChainNode : public NcnNode {
         m = mid[l].unpack();
       }
       auto ptr = [](const Tensor& t) -> const void* { return t.defined() ? t.const_data_ptr() : nullptr; };
-      if (used + ws_bytes > room) reduce();
       int rows = 0;
-      check_status(call, ncn_stage_bwd_partial(keep, ptr(xc), ptr(xac), yl.const_data_ptr(), yal.const_data_ptr(), ptr(m), mid_bytes,
-                                               has_ctx ? cl.const_data_ptr<int>() : nullptr, dy.const_data_ptr(), dya.const_data_ptr(),
-                                               w.const_data_ptr<float>(), dx.data_ptr(), dxa.data_ptr(), ws_base + used, ws_bytes,
-                                               &rows, B, N, E, c.n, c.C, c.first + l, c.alpha, c.act, c.dt, st));
+      auto walk = [&]() {
+        return ncn_stage_bwd_partial(keep, ptr(xc), ptr(xac), yl.const_data_ptr(), yal.const_data_ptr(), ptr(m), mid_bytes,
+                                     has_ctx ? cl.const_data_ptr<int>() : nullptr, dy.const_data_ptr(), dya.const_data_ptr(),
+                                     w.const_data_ptr<float>(), dx.data_ptr(), dxa.data_ptr(), ws_base + used, ws_bytes - used, &rows,
+                                     B, N, E, c.n, c.C, c.first + l, c.alpha, c.act, c.dt, st);
+      };
+      int rc = used < ws_bytes ? walk() : NCN_ERR_WORKSPACE;
+      if (rc == NCN_ERR_WORKSPACE && used > 0) {  // (nothing has been launched)
+        reduce();
+        rc = walk();
+      }
+      check_status(call, rc);
       partial.push_back(reinterpret_cast<const float*>(ws_base + used));
       partial_rows.push_back(rows);
       partial_out.push_back(dW[l].mutable_data_ptr<float>());
