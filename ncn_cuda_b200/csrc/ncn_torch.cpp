@@ -336,6 +336,12 @@ struct ChainNode : public NcnNode {
     int last = 0;
     if (!inputs)
       while (last < c.L - 1 && !task_should_compute_output(2 + last)) ++last;
+    const bool several = last < c.L - 1;  // a single stage sums its own: no launch would be saved
+    if (several) {
+      partial.reserve(c.L - last);
+      partial_rows.reserve(c.L - last);
+      partial_out.reserve(c.L - last);
+    }
     auto reduce = [&]() {
       if (partial.empty()) return;
       check_status("ncn_reduce_partials", ncn_reduce_partials(partial.data(), partial_rows.data(), partial_out.data(),
@@ -367,23 +373,49 @@ struct ChainNode : public NcnNode {
         m = mid[l].unpack();
       }
       auto ptr = [](const Tensor& t) -> const void* { return t.defined() ? t.const_data_ptr() : nullptr; };
-      int rows = 0;
-      auto walk = [&]() {
-        return ncn_stage_bwd_partial(keep, ptr(xc), ptr(xac), yl.const_data_ptr(), yal.const_data_ptr(), ptr(m), mid_bytes,
-                                     has_ctx ? cl.const_data_ptr<int>() : nullptr, dy.const_data_ptr(), dya.const_data_ptr(),
-                                     w.const_data_ptr<float>(), dx.data_ptr(), dxa.data_ptr(), ws_base + used, ws_bytes - used, &rows,
-                                     B, N, E, c.n, c.C, c.first + l, c.alpha, c.act, c.dt, st);
-      };
-      int rc = used < ws_bytes ? walk() : NCN_ERR_WORKSPACE;
-      if (rc == NCN_ERR_WORKSPACE && used > 0) {  // (nothing has been launched)
-        reduce();
-        rc = walk();
+      const void *yp = yl.const_data_ptr(), *yap = yal.const_data_ptr(), *dyp = dy.const_data_ptr(), *dyap = dya.const_data_ptr();
+      const int* const clp = has_ctx ? cl.const_data_ptr<int>() : nullptr;
+      const float* const wp = w.const_data_ptr<float>();
+      float* const dwp = dW[l].mutable_data_ptr<float>();
+      void *dxp = dx.data_ptr(), *dxap = dxa.data_ptr();
+      const int module_l = c.first + l;
+      int rc, rows = 0;
+      if (!several) {
+        switch (keep) {
+          case NCN_KEEP_CTX:
+            rc = ncn_stage_bwd_ctx(yp, yap, dyp, dyap, wp, clp, dxp, dxap, nullptr, nullptr, dwp, ws_base, ws_bytes, B, N, E, c.n, c.C,
+                                   module_l, c.alpha, c.act, c.dt, st);
+            break;
+          case NCN_KEEP_INPUT:
+            rc = ncn_stage_bwd_saved(ptr(xc), ptr(xac), yp, yap, dyp, dyap, wp, dxp, dxap, dwp, ws_base, ws_bytes, B, N, E, c.n, c.C,
+                                     module_l, c.alpha, c.act, c.dt, st);
+            break;
+          case NCN_KEEP_MID:
+            rc = ncn_stage_bwd_mid(yp, yap, ptr(m), mid_bytes, dyp, dyap, wp, dxp, dxap, dwp, ws_base, ws_bytes, B, N, E, c.n, c.C,
+                                   module_l, c.alpha, c.act, c.dt, st);
+            break;
+          default:
+            rc = ncn_stage_bwd(yp, yap, dyp, dyap, wp, dxp, dxap, nullptr, nullptr, dwp, ws_base, ws_bytes, B, N, E, c.n, c.C, module_l,
+                               c.alpha, c.act, c.dt, st);
+        }
+      } else {
+        auto walk = [&]() {
+          return ncn_stage_bwd_partial(keep, ptr(xc), ptr(xac), yp, yap, ptr(m), mid_bytes, clp, dyp, dyap, wp, dxp, dxap, ws_base + used,
+                                       ws_bytes - used, &rows, B, N, E, c.n, c.C, module_l, c.alpha, c.act, c.dt, st);
+        };
+        rc = used < ws_bytes ? walk() : NCN_ERR_WORKSPACE;
+        if (rc == NCN_ERR_WORKSPACE && used > 0) {  // (nothing has been launched)
+          reduce();
+          rc = walk();
+        }
       }
       check_status(call, rc);
-      partial.push_back(reinterpret_cast<const float*>(ws_base + used));
-      partial_rows.push_back(rows);
-      partial_out.push_back(dW[l].mutable_data_ptr<float>());
-      used += ((size_t)rows * 2 * E * sizeof(float) + 255) / 256 * 256;
+      if (several) {
+        partial.push_back(reinterpret_cast<const float*>(ws_base + used));
+        partial_rows.push_back(rows);
+        partial_out.push_back(dwp);
+        used += ((size_t)rows * 2 * E * sizeof(float) + 255) / 256 * 256;
+      }
       dy = std::move(dx);
       dya = std::move(dxa);
       if (release) {
