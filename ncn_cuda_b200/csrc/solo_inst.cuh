@@ -41,7 +41,11 @@ static cudaError_t launch_act(int act, const SoloParams& p, int grid, int thread
 #endif
 
 cudaError_t NCN_FN(int act, int dtype, const SoloParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
+#if defined(NCN_BWD) && NCN_NG == 8
+  if (dtype == DT_BF16) return cudaErrorNotSupported;  // the shared-memory kernels are faster there (solo_pays_n8)
+#else
   if (dtype == DT_BF16) return launch_act<__nv_bfloat16>(act, p, grid, threads, smem, st, occ);
+#endif
   return launch_act<float>(act, p, grid, threads, smem, st, occ);
 }
 
