@@ -5,6 +5,8 @@ import torch
 
 from oracle import ncn_oracle as O
 
+from .kernels_util import kernels_of, launched
+
 pytestmark = pytest.mark.gpu
 
 ALPHA = 0.9
@@ -102,6 +104,36 @@ def test_context_lengths(B, N, heads, d, n):
     grads = torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda()))
     # the walk back from the output: rounding grows by 1 / 0.9 per step, 29-fold over 32 steps
     _check((y, ya, *grads), want, 1e-5 if n <= 16 else 3e-5)
+
+
+@pytest.mark.parametrize("activation", ["tanh", "linear", "relu", "sigmoid", "leaky-relu"])
+@pytest.mark.parametrize("B,N,heads,d,n", [(160, 96, 4, 32, 32), (320, 80, 1, 64, 16), (700, 32, 2, 32, 16)])
+def test_context_lengths_dealt_out_evenly(B, N, heads, d, n, activation):
+    """More than eight groups per SM: kernels of their own (the last template argument), in every activation."""
+    import ncn_cuda_b200 as ncn
+
+    x, xa, W, dy, dya = _case(B, N, heads, d, seed=4)
+    ctx = torch.randint(0, N + 3, (B,), generator=torch.Generator().manual_seed(5), dtype=torch.int32)
+    want = _oracle(lambda a, b, w: O.stage_forward_ctxlen(a, b, w, ctx, ALPHA, activation, n, heads, 1), x, xa, W, dy, dya)
+    leaves = [t.cuda().requires_grad_(True) for t in (x, xa, W)]
+
+    def step():
+        y, ya = ncn.fused_ncn_cuda_ctxlen(*leaves, ctx.cuda(), ALPHA, ncn.ops.ACTIVATION_CODES[activation], n, heads, 1)
+        return (y, ya, *torch.autograd.grad((y, ya), leaves, (dy.cuda(), dya.cuda())))
+
+    got, names = kernels_of(step)
+    assert launched(names, r"feat_fwd_kernel<.*5>") and launched(names, r"feat_bwd_kernel<.*5>"), names
+    _check(got[:2], want[:2], 1e-5)
+    if "relu" in activation:
+        # the derivative jumps at 0: a pre-activation of order 1 carries 1e-7 of rounding, 1 / 0.9^n times that at the end of a walk back, so a
+        # share of `flips` of them (0.4: the density at 0) has the other sign; each changes its element's gradient by up to a tenth
+        # and a term of dW, (1 - alpha) c x_j x_i gT, by up to 1e-2
+        flips = 2 * 0.4 * 1e-7 / 0.9**n
+        for a, b in zip(got[2:4], want[2:4]):
+            assert (a.double().cpu() - b).norm() / b.norm() < 1e-5 + 0.1 * (n * flips) ** 0.5
+        assert (got[4].double().cpu() - want[4]).norm() < 1e-5 * want[4].norm() + 1e-2 * (x.numel() * n * flips) ** 0.5
+    else:
+        _check(got[2:], want[2:], 1e-5 if n <= 16 else 3e-5)
 
 
 @pytest.mark.parametrize("n,d", [(4, 8), (16, 24)])

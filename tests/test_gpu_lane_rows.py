@@ -1,12 +1,14 @@
-"""Register-resident row kernels on rows that do not fill their warps, on rows of 8192 positions, and with one group per
-thread: where a warp's
-share ends inside a thread's blocks, inside a warp and just behind one, halos as long as a warp's share, shifts through
-the tile buffer, several rows per CTA, a last tile that is not full.  Tolerances are those of test_gpu_sweep.py: 1e-5 (fp32) of
+"""Row kernels around the line between the register-resident ones (rows that do not fill their warps, rows of 8192 positions, one
+group per thread) and the shared-memory ones: where a warp's share ends inside a thread's blocks, inside a warp and just behind one,
+halos as long as a warp's share, shifts through the tile buffer, several rows per CTA, several tiles per CTA, a last tile that is not
+full.  The short rows of SHAPES lie on the other side of the line; the tests that name a family ask which kernels ran.  Tolerances are those of test_gpu_sweep.py: 1e-5 (fp32) of
 the largest value, 2e-5 for the gradients of a walk back over more than 16 steps, 2e-2 (bf16)."""
 import pytest
 import torch
 
 from oracle import ncn_oracle as O
+
+from .kernels_util import kernels_of, launched
 
 pytestmark = pytest.mark.gpu
 
@@ -33,6 +35,21 @@ def _step(ncn, x, xa, ws, dy, dya, act, n, mode, dtype, first=0):
     torch.autograd.backward([y, ya], [dy.cuda().to(dtype), dya.cuda().to(dtype)])
     ncn.ops.device_status()
     return [t.float().cpu() for t in (y.detach(), ya.detach(), xd.grad, xad.grad, W.grad)]
+
+
+def _against_oracle(got, x, xa, ws, dy, dya, act, n, first):
+    ry, rya, rdx, rdxa, rdW = O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, act, n, 1, first_module=first)
+    for name, a, b in zip(("y", "ya", "dx", "dxa"), got, (ry, rya, rdx, rdxa)):
+        if act == "relu" and name[0] == "d":
+            # the derivative jumps at 0: a pre-activation of order 1 carries 2e-7 of rounding, five times that at the end of a walk back
+            # over 16 steps, so 16 * 1e-6 * 0.4 (the density at 0) of the elements have one of the other sign, and each changes its
+            # element's gradient by up to a tenth: 0.1 * sqrt(6e-6) = 2.5e-4 of the 2-norm
+            assert (a - b).norm() / b.norm() < 3e-4, name
+        else:
+            assert O.rel_err(a, b) < 1e-5, name
+    # the weight gradient sums B N terms that largely cancel, the oracle's in fp32 as well: 1e-5 of the terms' size per sqrt(count)
+    got_w, want_w = got[4], torch.stack(list(rdW))
+    assert (got_w - want_w).abs().max() < 1e-4 * max(1.0, want_w.abs().max().item(), (x.numel() ** 0.5)), "dW"
 
 
 # (n, N): blocks per row m = N / n in the comment
@@ -68,6 +85,33 @@ def test_modes_and_first_stages(ncn, n, N, B, act, mode, first):
     got = _step(ncn, x, xa, ws, dy, dya, act, n, mode, torch.float32, first)
     for name, a, b in zip(("y", "ya", "dx", "dxa", "dW"), got, (ry, rya, rdx, rdxa, torch.stack(list(rdW)))):
         assert O.rel_err(a, b) < 1e-5, name
+
+
+# Ragged rows in every mode and activation, with more tiles than CTAs (2 to 5 CTAs per SM); (2, 1044) and (8, 1008) have several rows
+# to a tile and a last tile that is not full.
+@pytest.mark.parametrize("n,N,B,act,mode,first", [
+    (4, 3000, 800, "linear", "checkpoint", 0), (4, 4112, 700, "sigmoid", "tape", 0), (8, 3008, 800, "relu", "invert", 1),
+    (2, 1044, 3001, "sigmoid", "checkpoint", 0), (2, 1044, 3001, "tanh", "tape", 2), (8, 1008, 3003, "tanh", "checkpoint", 0),
+    (8, 1008, 3003, "linear", "tape", 0), (4, 3000, 800, "tanh", "invert", 0),
+])
+def test_ragged_rows_in_many_tiles(ncn, n, N, B, act, mode, first):
+    L = {2: 5, 4: 3, 8: 2}[n]
+    x, xa, ws, dy, dya = _data(B, N, n, L, torch.float32, N + B)
+    got, names = kernels_of(lambda: _step(ncn, x, xa, ws, dy, dya, act, n, mode, torch.float32, first))
+    assert launched(names, rf"lane_fwd_kernel<{n}, .*true>") and launched(names, rf"lane_bwd_kernel<{n}, .*true>"), names
+    _against_oracle(got, x, xa, ws, dy, dya, act, n, first)
+
+
+@pytest.mark.parametrize("n,N,B,act,mode", [
+    (16, 240, 5003, "tanh", "checkpoint"), (16, 1840, 700, "sigmoid", "tape"), (8, 1048, 2001, "linear", "checkpoint"),
+    (8, 1048, 2001, "tanh", "tape"), (16, 2048, 600, "relu", "checkpoint"),
+])
+def test_one_group_per_thread_in_many_tiles(ncn, n, N, B, act, mode):
+    L = 2
+    x, xa, ws, dy, dya = _data(B, N, n, L, torch.float32, N + B)
+    got, names = kernels_of(lambda: _step(ncn, x, xa, ws, dy, dya, act, n, mode, torch.float32))
+    assert launched(names, rf"solo_fwd_kernel<{n},") and launched(names, rf"solo_bwd_kernel<{n},"), names
+    _against_oracle(got, x, xa, ws, dy, dya, act, n, 0)
 
 
 @pytest.mark.parametrize("n,N", [(16, 16), (16, 48), (16, 240), (16, 512), (16, 528), (16, 1840), (16, 2048), (16, 2080), (16, 8176),
