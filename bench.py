@@ -234,8 +234,10 @@ def kernel_names(wl, mode):
     if wl.get("E", 1) > 1:
         return "feat_fwd_kernel (ncn_feat.cuh)", "feat_bwd_kernel (ncn_feat.cuh)"
     n = wl["n"]
-    if n == 16 or mode == "recompute":
+    if mode == "recompute":
         return "pair_fwd_dual_kernel (ncn_pairs.cuh)", "rows_bwd_kernel / pair_bwd_wide_kernel"
+    if n == 16:
+        return "solo_fwd_kernel (ncn_solo.cuh)", "solo_bwd_kernel (ncn_solo.cuh)"
     if n == 4 and wl["L"] <= 6:
         return "lane_fwd_kernel (ncn_lanes.cuh)", "lanep_bwd_kernel (ncn_lanes_pipe.cuh)"
     return "lane_fwd_kernel (ncn_lanes.cuh)", "lane_bwd_kernel (ncn_lanes.cuh)"
