@@ -366,13 +366,12 @@ struct ActForm<ACT_LINEAR> {
 // r = 1 / (1 + 2^ts) for all N values of an array at once (the positions of a group, or the features of a
 // position).
 // BATCH: reciprocals taken from one special-function reciprocal of the product of BATCH values
-// (4: 1.25, 2: 1.5, 1: 2 special-function instructions per position and step; the smaller the batch
-// the fewer multiplies on the FMA pipe).
+// (4: 1.25, 2: 1.5 special-function instructions per position and step, one each 2; the smaller the batch
+// the fewer multiplies on the FMA pipe, and one each, ActForm::r, needs no cap).
 // The exponent is capped at 30: beyond it r < 1e-9 (tanh = 1 to the last bit) and the product of four d stays a normal
 // fp32 number, as does its reciprocal.  A NaN reaches all values that share its reciprocal.  These would see it all the same
-// where they are the features of one position, through their dot product, and in the reverse sweep, where the sums for gx_j
-// bring a NaN in any x of a group to all of its cotangents.  They would not in the forward steps of a group's positions: a row
-// with a NaN is taken again there (ncn_terms.cuh).
+// where they are the features of one position, through their dot product.  They would not in the forward steps of a group's
+// positions: a row with a NaN is taken again there (ncn_terms.cuh).
 template <int ACT, int NG, int BATCH>
 __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG]) {
   if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {
@@ -382,10 +381,7 @@ __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG
       const float2 e = make_float2(min_nan(ts[i].x, 30.0f), min_nan(ts[i].y, 30.0f));
       d[i] = __fadd2_rn(make_float2(ex2_approx(e.x), ex2_approx(e.y)), f2(1.0f));
     }
-    if constexpr (BATCH == 1) {
-#pragma unroll
-      for (int i = 0; i < NG; ++i) r[i] = make_float2(rcp_approx(d[i].x), rcp_approx(d[i].y));
-    } else if constexpr (NG == 3) {  // one reciprocal of the product of all three
+    if constexpr (NG == 3) {  // one reciprocal of the product of all three
       const float2 P01 = __fmul2_rn(d[0], d[1]);
       const float2 PP = __fmul2_rn(P01, d[2]);
       const float2 R = make_float2(rcp_approx(PP.x), rcp_approx(PP.y));
