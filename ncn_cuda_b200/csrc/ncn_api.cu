@@ -659,16 +659,17 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
 struct SoloPlan {
   int threads = 0, R = 0, grid = 0, occ = 0;
   size_t smem = 0;
-  uint32_t off_res = 0, off_red = 0, off_w = 0, off_bar = 0;
+  uint32_t off_res = 0, off_red = 0, off_w = 0, off_bar = 0, off_land = 0;
+  int ahead = SOLO_AHEAD_NONE;
   long long tiles = 0;
 };
 
 struct SoloKey {
-  int epoch, dev, bwd, N, n, L, dtype, residual, act;
+  int epoch, dev, bwd, N, n, L, dtype, residual, tape, rec, act;
   long long B;
   bool operator==(const SoloKey& o) const {
     return epoch == o.epoch && dev == o.dev && bwd == o.bwd && N == o.N && n == o.n && L == o.L && dtype == o.dtype &&
-           residual == o.residual && act == o.act && B == o.B;
+           residual == o.residual && tape == o.tape && rec == o.rec && act == o.act && B == o.B;
   }
 };
 
@@ -693,7 +694,7 @@ static bool solo_pays_n8(bool bwd, int m, int dtype) {
 
 // NCN_OK with pl filled, NCN_ERR_UNSUPPORTED when the kernels do not cover the arguments.  The kernels take whole rows, a
 // thread per group, one CTA at most.  Remembered per argument set.
-static int plan_solo(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, int L, int dtype, int flags, const DevInfo& dev, int act,
+static int plan_solo(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, int L, int dtype, int flags, bool rec, const DevInfo& dev, int act,
                      SoloPlan& pl) {
   if (!lanes_enabled() || (flags & F_RECOMPUTE) || solo_fn(n, bwd) == nullptr || !rows_shape_ok(N, E, n, C, dtype)) return NCN_ERR_UNSUPPORTED;
   const int m = (int)(N / n);
@@ -701,7 +702,8 @@ static int plan_solo(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, in
   if (n == 8 && !solo_pays_n8(bwd, m, dtype)) return NCN_ERR_UNSUPPORTED;
   static std::mutex mu;
   static std::vector<std::pair<SoloKey, std::pair<int, SoloPlan>>> cache;
-  const SoloKey key{g_plan_epoch.load(), dev.dev, bwd ? 1 : 0, (int)N, n, L, dtype, (flags & F_RESIDUAL) != 0, act, (long long)B};
+  const bool tape = bwd && (flags & F_TAPE) != 0;
+  const SoloKey key{g_plan_epoch.load(), dev.dev, bwd ? 1 : 0, (int)N, n, L, dtype, (flags & F_RESIDUAL) != 0, tape, rec, act, (long long)B};
   {
     std::lock_guard<std::mutex> lk(mu);
     for (auto& kv : cache)
@@ -731,9 +733,28 @@ static int plan_solo(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, in
   p.off_bar = take(32);
   if (off <= (uint64_t)dev.smem_optin) {
     p.threads = warps * 32; p.R = R; p.smem = (size_t)off;
-    SoloParams dummy{};
-    cudaError_t e = solo_fn(n, bwd)(act, dtype, dummy, 0, p.threads, p.smem, nullptr, &p.occ);
+    auto occupancy = [&](size_t smem, int ahead, int& occ) {
+      SoloParams dummy{};
+      dummy.ahead = ahead;
+      return solo_fn(n, bwd)(act, dtype, dummy, 0, p.threads, smem, nullptr, &occ);
+    };
+    cudaError_t e = occupancy(p.smem, SOLO_AHEAD_NONE, p.occ);
     if (e != cudaSuccess) return cuda_fail(e);
+    // Backward: the inputs a tile ahead, where their buffer costs no CTA.  Without -> with, us: 16384 x 8192 bf16, groups of 16, 4
+    // stages 4046 -> 3929; 8192 x 8192 fp32 with the end state stored 2158 -> 2048; 25000 x 2048 1650 -> 1562; 50000 x 2048 bf16
+    // 2963 -> 2934, 16384 x 4096 bf16 1932 -> 1925; 10000 x 2968 fp32, groups of 8, 3 stages 680 -> 613.  Where it does cost one (fp32
+    // from the output, 2048 and 4096 positions) the other CTAs cover the loads.
+    if (bwd && !rec && !(flags & F_RESIDUAL)) {
+      const size_t more = ((size_t)(tape ? 2 : 4) * R * N * w + 127) / 128 * 128;
+      const int ahead = tape ? SOLO_AHEAD_TAPE : SOLO_AHEAD_OUTPUT;
+      int occ = 0;
+      if (p.smem + more <= (size_t)dev.smem_optin && (e = occupancy(p.smem + more, ahead, occ)) != cudaSuccess) return cuda_fail(e);
+      if (occ >= 1 && occ >= p.occ) {
+        p.off_land = (uint32_t)p.smem;
+        p.ahead = ahead;
+        p.smem += more;
+      }
+    }
     if (p.occ >= 1) {
       p.tiles = (B + R - 1) / R;
       long long grid = (long long)dev.sms * (p.occ > 32 ? 32 : p.occ);
@@ -755,6 +776,7 @@ static void fill_solo(SoloParams& p, const SoloPlan& pl, int64_t B, int64_t N, i
   p.oma = (float)(1.0 - alpha);
   p.R = pl.R; p.tiles = pl.tiles;
   p.off_res = pl.off_res; p.off_red = pl.off_red; p.off_w = pl.off_w; p.off_bar = pl.off_bar;
+  p.off_land = pl.off_land; p.ahead = pl.ahead;
 }
 
 static void fill_lane(LaneParams& p, const LanePlan& pl) {
@@ -1168,8 +1190,8 @@ static int net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_hea
       plan_lanes(true, B, N, E, n_cache, n_head, first, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK)
     return 1;
   SoloPlan sf, sb;  // (groups of 8: all rows that fit these fit the shared-memory kernels)
-  return plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sf) == NCN_OK &&
-         plan_solo(true, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sb) == NCN_OK;
+  return plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, false, dev, act, sf) == NCN_OK &&
+         plan_solo(true, B, N, E, n_cache, n_head, L, dtype, flags, false, dev, act, sb) == NCN_OK;
 }
 
 int ncn_net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_head, int L, int dtype, int flags, int ckpt_every) {
@@ -1264,7 +1286,7 @@ static int net_fwd_impl(const void* x, const void* xa, const float* const* list,
   }
   {
     SoloPlan sp;
-    if (plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sp) == NCN_OK) {
+    if (plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, false, dev, act, sp) == NCN_OK) {
       SoloParams q{};
       q.in[0] = x; q.in[1] = xa;
       q.out[0] = y; q.out[1] = ya;
@@ -1386,7 +1408,7 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
   }
   {
     SoloPlan sp;
-    if (plan_solo(true, B, N, E, n_cache, n_head, L, dtype, flags, dev, act, sp) == NCN_OK) {
+    if (plan_solo(true, B, N, E, n_cache, n_head, L, dtype, flags, x_rec != nullptr, dev, act, sp) == NCN_OK) {
       if ((rc = fit_grid(sp.grid)) != NCN_OK) return rc;
       SoloParams q{};
       q.in[0] = s0; q.in[1] = s1; q.in[2] = dy; q.in[3] = dya;

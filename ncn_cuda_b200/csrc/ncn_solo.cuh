@@ -16,8 +16,8 @@
 // Any number of blocks up to 512 per row, any stride; R rows side by side in a CTA.
 //
 // Measured on a B200 (forward + backward, before = ncn_pairs.cuh forward and ncn_rows.cuh backward): 25000 x 2048 fp32, groups of
-// 16, 3 stages 1447 + 1947 -> 945 + 1650 us; 65536 x 8192 bf16, 4 stages 9.93 + 16.2 -> 9.23 + 16.2 ms.  Cycles per
-// warp, position and step: fp32 13.9 + 24.1, arithmetic alone 11.5 + 19.2; bf16 10.0 + 17.5, alone 8.3 + 12.6 (rows of 8192: one
+// 16, 3 stages 1447 + 1947 -> 945 + 1604 us; 65536 x 8192 bf16, 4 stages 9.93 + 16.2 -> 9.23 + 15.6 ms.  Cycles per
+// warp, position and step: fp32 13.9 + 23.4, arithmetic alone 11.5 + 19.2; bf16 10.0 + 16.9, alone 8.3 + 12.6 (rows of 8192: one
 // CTA of 512 threads per SM, whose boundaries nothing overlaps).
 #pragma once
 #include "ncn_lanes.cuh"
@@ -293,7 +293,11 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const __grid_const
 
 // ------------------------------------------------------------------------------------------ backward
 // From the net output (reversible inverse), from stored states (checkpoints, F_TAPE), F_RESIDUAL; no forward replay.
-template <int NG, int ACT, typename T, int MAXT, int MINB>
+//
+// AHEAD (not with F_RESIDUAL, nor where the rebuilt input is asked for): the streams of the next tile are copied to a buffer of their
+// own while this one is worked on, and with F_TAPE the state it starts from is read into x and a as soon as they are done with.  (A
+// kernel of its own: the choice at run time costs the plain one 5 to 10 per cent, in registers.)
+template <int NG, int ACT, typename T, int MAXT, int MINB, int AHEAD>
 __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
@@ -311,9 +315,10 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
   const T* g_in[4] = {static_cast<const T*>(p.in[0]), static_cast<const T*>(p.in[1]), static_cast<const T*>(p.in[2]),
                       static_cast<const T*>(p.in[3])};
   const float2* ckpt = reinterpret_cast<const float2*>(p.ckpt);
-  const bool want_rec = p.out[2] != nullptr;
-  const bool residual = (p.flags & F_RESIDUAL) != 0;
-  const bool tape = (p.flags & F_TAPE) != 0;  // the last stage's output state comes from its checkpoint
+  const bool want_rec = !AHEAD && p.out[2] != nullptr;
+  const bool residual = !AHEAD && (p.flags & F_RESIDUAL) != 0;
+  // the last stage's output state comes from its checkpoint
+  const bool tape = AHEAD ? AHEAD == SOLO_AHEAD_TAPE : (p.flags & F_TAPE) != 0;
   const long long BN = p.B * (long long)N;
 
   if (tid == 0) {
@@ -332,11 +337,36 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
   const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
+  constexpr int Q0 = AHEAD == SOLO_AHEAD_TAPE ? 2 : 0;  // AHEAD: the first stream that is read, at land
+  T* const land = reinterpret_cast<T*>(smem + p.off_land);
+  auto copy_ahead = [&](long long tl) {
+    const uint32_t nbytes = (uint32_t)(min((long long)R, p.B - tl * R) * N * sizeof(T));
+    mbar_expect_tx(&bar[0], (4 - Q0) * nbytes);
+#pragma unroll
+    for (int q = Q0; q < 4; ++q) bulk_g2s(land + (q - Q0) * RN, g_in[q] + tl * R * N, nbytes, &bar[0]);
+  };
+  float2 X[NG / 2], A[NG / 2];
+  auto load_state = [&](long long tl, int ck) {
+    const float2* c = ckpt + (long long)ck * BN + (tl * R + r) * N + g;
+#pragma unroll
+    for (int o = 0; o < NG; ++o) {
+      const float2 v = __ldg(c + o * m);
+      solo_set<NG>(X, o, v.x);
+      solo_set<NG>(A, o, v.y);
+    }
+  };
+  if (AHEAD) {
+    if (tid == 0) copy_ahead(blockIdx.x);  // (there is a tile for every CTA)
+#pragma unroll
+    for (int i = 0; i < NG / 2; ++i) X[i] = A[i] = f2(0.0f);
+    if (AHEAD == SOLO_AHEAD_TAPE && r < min((long long)R, p.B - (long long)blockIdx.x * R)) load_state(blockIdx.x, recs[L - 1].ck);
+  }
+
   for (long long tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
     const long long row0 = tile * R;
     const int rows = (int)min((long long)R, p.B - row0);
     const uint32_t bytes = (uint32_t)(rows * N * sizeof(T));
-    if (tid == 0) {
+    if (!AHEAD && tid == 0) {
       bulk_wait_read0();  // the previous tile's stores have left the buffer
       mbar_expect_tx(&bar[0], (tape ? 2 : 4) * bytes + (residual ? bytes : 0));
 #pragma unroll
@@ -350,11 +380,14 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
     if (*abort_flag) break;
     const bool active = r < rows;
 
-    float2 X[NG / 2], A[NG / 2], H[NG / 2], G[NG / 2];
+    float2 H[NG / 2], G[NG / 2];
 #pragma unroll
-    for (int i = 0; i < NG / 2; ++i) X[i] = A[i] = H[i] = G[i] = f2(0.0f);
+    for (int i = 0; i < NG / 2; ++i) {
+      H[i] = G[i] = f2(0.0f);
+      if (AHEAD != SOLO_AHEAD_TAPE) X[i] = A[i] = f2(0.0f);
+    }
     if (active) {
-      const T* c = win + base + g * NG;
+      const T* c = (AHEAD ? land - Q0 * RN : win) + base + g * NG;
       if (!tape) {
         solo_ld<NG, T>(c, X, g);
         solo_ld<NG, T>(c + RN, A, g);
@@ -362,13 +395,15 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
       solo_ld<NG, T>(c + 2 * RN, H, g);
       solo_ld<NG, T>(c + 3 * RN, G, g);
     }
+    if (AHEAD && tid == 0) bulk_wait_read0();  // the previous tile's stores have left the buffer
     __syncthreads();  // native inputs are in registers; the buffer may take slots
+    if (AHEAD && tid == 0 && tile + gridDim.x < p.tiles) copy_ahead(tile + gridDim.x);
     if (tid == 0 && tile + gridDim.x < p.tiles) {  // next tile towards L2 while this one is worked on
       const long long nrow0 = (tile + gridDim.x) * R;
       const int nrows = (int)min((long long)R, p.B - nrow0);
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (q >= 2 || !tape) l2_prefetch(g_in[q] + nrow0 * N, (uint32_t)(nrows * N * sizeof(T)));
+        if (!AHEAD && (q >= 2 || !tape)) l2_prefetch(g_in[q] + nrow0 * N, (uint32_t)(nrows * N * sizeof(T)));
       for (int k = 0; k < p.n_ckpt; ++k) l2_prefetch(ckpt + (long long)k * BN + nrow0 * N, (uint32_t)(nrows * N * sizeof(float2)));
     }
     int s_cur = 0;
@@ -405,15 +440,8 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
     for (int l = L - 1; l >= 0; --l) {
       const StageRec rec = recs[l];
       exchange(rec.s, rec.ck < 0);
-      if (rec.ck >= 0 && active) {  // a state saved after stage l replaces the rebuilt one
-        const float2* c = ckpt + (long long)rec.ck * BN + (row0 + r) * N + g;
-#pragma unroll
-        for (int o = 0; o < NG; ++o) {
-          const float2 v = __ldg(c + o * m);
-          solo_set<NG>(X, o, v.x);
-          solo_set<NG>(A, o, v.y);
-        }
-      }
+      // a state saved after stage l replaces the rebuilt one
+      if (rec.ck >= 0 && active && (AHEAD != SOLO_AHEAD_TAPE || l < L - 1)) load_state(tile, rec.ck);
       float dwi = 0.0f, dwj = 0.0f;
       SoloBwd<NG, ACT, NG - 1>::run(X, A, H, G, rec.owi, p.alpha, rec.owj * 2.0f * kph, rec.owj * sT, dwi, dwj);
 #pragma unroll
@@ -435,6 +463,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
         if ((lane & 15) == 0) red[(l * nwarp + warp) * 2 + (hi ? 1 : 0)] += keep;
       }
     }
+    if (AHEAD == SOLO_AHEAD_TAPE && r < min((long long)R, p.B - (tile + gridDim.x) * R)) load_state(tile + gridDim.x, recs[L - 1].ck);
     exchange(0, want_rec);
     __syncthreads();  // every slot has been read; the buffer may take the native results
     if (active) {

@@ -17,7 +17,12 @@ struct SoloParams {
   int N, m, R, L, l0, ckpt_every, n_ckpt, flags;
   float alpha, oma;
   uint32_t off_res, off_red, off_w, off_bar;  // byte offsets into dynamic shared memory; the tile buffer is at 0
+  uint32_t off_land;   // bwd: buffer of the streams that are copied a tile ahead
+  int ahead;           // bwd: SoloAhead
 };
+
+// Backward: what is fetched a tile ahead (solo_bwd_kernel): nothing; all four streams; with F_TAPE dy, dya and the state.
+enum SoloAhead : int { SOLO_AHEAD_NONE = 0, SOLO_AHEAD_OUTPUT = 1, SOLO_AHEAD_TAPE = 2 };
 
 constexpr int kSoloThreads = 512;  // block size the kernels are compiled for: backward one such CTA per SM, forward two
 constexpr int kSoloFwdBlocks = 2, kSoloBwdBlocks = 1;

@@ -4,19 +4,28 @@
 
 namespace ncn {
 
-template <int ACT, typename T>
-static cudaError_t launch_one(const SoloParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
-#ifdef NCN_BWD
-  auto k = solo_bwd_kernel<NCN_NG, ACT, T, kSoloThreads, kSoloBwdBlocks>;
-#else
-  auto k = solo_fwd_kernel<NCN_NG, ACT, T, kSoloThreads, kSoloFwdBlocks>;
-#endif
-  static SmemGrant granted;
+template <typename K>
+static cudaError_t launch_kernel(K k, SmemGrant& granted, const SoloParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
   cudaError_t e = grant_smem(granted, k, smem);
   if (e != cudaSuccess) return e;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, smem);
   k<<<grid, threads, smem, st>>>(p);
   return cudaGetLastError();
+}
+
+template <int ACT, typename T>
+static cudaError_t launch_one(const SoloParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
+#ifdef NCN_BWD
+  static SmemGrant granted[3];
+#define NCN_GO(A) return launch_kernel(solo_bwd_kernel<NCN_NG, ACT, T, kSoloThreads, kSoloBwdBlocks, A>, granted[A], p, grid, threads, smem, st, occ)
+  if (p.ahead == SOLO_AHEAD_OUTPUT) NCN_GO(SOLO_AHEAD_OUTPUT);
+  if (p.ahead == SOLO_AHEAD_TAPE) NCN_GO(SOLO_AHEAD_TAPE);
+  NCN_GO(SOLO_AHEAD_NONE);
+#undef NCN_GO
+#else
+  static SmemGrant granted;
+  return launch_kernel(solo_fwd_kernel<NCN_NG, ACT, T, kSoloThreads, kSoloFwdBlocks>, granted, p, grid, threads, smem, st, occ);
+#endif
 }
 
 template <typename T>

@@ -126,6 +126,24 @@ def test_one_group_per_thread(ncn, n, N, dtype):
         assert O.rel_err(a, b) < (1e-5 if dtype == torch.float32 else 2e-2), name
 
 
+# What the backward fetches a tile ahead: with the end state stored (2) or from the output (1); one tile per CTA, many, several rows to
+# a tile and a last tile that is not full.  fp32 rows of 4096 positions from the output have no room for it (0).
+@pytest.mark.parametrize("n,N,B,act,mode,dtype,ahead", [
+    (16, 8192, 1, "tanh", "tape", torch.float32, 2), (16, 8192, 500, "tanh", "tape", torch.bfloat16, 2), (16, 240, 5003, "sigmoid", "tape", torch.float32, 2),
+    (16, 16, 9, "tanh", "tape", torch.bfloat16, 2), (8, 1048, 2001, "linear", "tape", torch.float32, 2), (8, 2968, 700, "tanh", "checkpoint", torch.float32, 1),
+    (16, 6000, 301, "relu", "checkpoint", torch.float32, 1), (16, 4096, 700, "tanh", "checkpoint", torch.float32, 0),
+])
+def test_one_group_per_thread_a_tile_ahead(ncn, n, N, B, act, mode, dtype, ahead):
+    x, xa, ws, dy, dya = _data(B, N, n, 2, dtype, N + B)
+    got, names = kernels_of(lambda: _step(ncn, x, xa, ws, dy, dya, act, n, mode, dtype))
+    assert launched(names, rf"solo_bwd_kernel<{n},.* {ahead}>"), names
+    if dtype == torch.float32:
+        _against_oracle(got, x, xa, ws, dy, dya, act, n, 0)
+    else:
+        for name, a, b in zip(("y", "ya", "dx", "dxa"), got, O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, act, n, 1)):
+            assert O.rel_err(a, b) < 2e-2, name
+
+
 @pytest.mark.parametrize("n,N,B,act,mode,first,L", [
     (16, 1840, 1, "linear", "checkpoint", 0, 3), (16, 240, 700, "sigmoid", "tape", 0, 2), (16, 2048, 3, "relu", "checkpoint", 2, 2),
     (16, 1040, 5, "tanh", "invert", 1, 1), (16, 1040, 5, "tanh", "invert", 0, 2), (8, 1048, 5, "sigmoid", "checkpoint", 1, 3),
