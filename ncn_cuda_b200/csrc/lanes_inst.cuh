@@ -4,10 +4,10 @@
 
 namespace ncn {
 
-template <int ACT, typename T, bool RAG>
+template <int ACT, typename T, bool RAG, int AHEAD = LANE_AHEAD_NONE>
 static cudaError_t launch_form(const LaneParams& p, int grid, int threads, size_t smem, cudaStream_t st, int* occ) {
 #ifdef NCN_BWD
-  auto k = lane_bwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads, RAG>;
+  auto k = lane_bwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads, AHEAD, RAG>;
 #else
   auto k = lane_fwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneFwdBlocks * kLaneThreads / kLaneMaxThreads, RAG>;
 #endif
@@ -45,6 +45,11 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
     return cudaGetLastError();
   }
 #endif
+#endif
+#ifdef NCN_BWD
+  if (p.ahead == LANE_AHEAD_OUTPUT) return launch_form<ACT, T, false, LANE_AHEAD_OUTPUT>(p, grid, threads, smem, st, occ);
+  if (p.ahead == LANE_AHEAD_TAPES) return launch_form<ACT, T, false, LANE_AHEAD_TAPES>(p, grid, threads, smem, st, occ);
+  if (p.ahead == LANE_AHEAD_TAPE) return launch_form<ACT, T, false, LANE_AHEAD_TAPE>(p, grid, threads, smem, st, occ);
 #endif
   return p.ragged ? launch_form<ACT, T, true>(p, grid, threads, smem, st, occ) : launch_form<ACT, T, false>(p, grid, threads, smem, st, occ);
 }

@@ -424,9 +424,9 @@ static bool lanes_enabled() { return !env_switches().lanes_off; }
 struct LanePlan {
   int threads = 0, R = 0, grid = 0, tpr = 0, thr = 0, ragged = 0, ea_max = 0, occ = 0;
   size_t smem = 0;
-  uint32_t off_work = 0, off_res = 0, off_ckpt = 0, off_halo = 0, off_red = 0, off_w = 0, off_bar = 0;
+  uint32_t off_work = 0, off_res = 0, off_ckpt = 0, off_halo = 0, off_red = 0, off_w = 0, off_bar = 0, off_land = 0;
   uint32_t halo_warp_bytes = 0, n_ckpt_slots = 0;
-  int pipelined = 0;
+  int pipelined = 0, ahead = LANE_AHEAD_NONE;
   long long tiles = 0;
 };
 
@@ -492,8 +492,10 @@ static bool lane_shape_ok(int64_t N, int64_t E, int n, int C, int l0, int L, int
 
 // Lay one CTA out.  ea: shifts of up to 2^ea blocks go by shuffles + halo, longer ones through the
 // tile buffer (which must then hold fp32 values).  terms: the buffer also takes one row in fp32 (ncn_terms.cuh).
+// ahead (backward): the tile buffer takes the two results, the next tile's streams have one of their own, and stored states go straight to
+// registers; alias: the halo lies in the tile buffer.
 static bool lane_layout(bool bwd, int N, int n, int L, int dtype, int flags, int n_ck, int R, int tpr, int ea, int e_need,
-                        bool terms, uint32_t limit, LanePlan& pl) {
+                        bool terms, int ahead, bool alias, uint32_t limit, LanePlan& pl) {
   const int w = dtype == DT_BF16 ? 2 : 4;
   const int NS = bwd ? 4 : 2;
   const bool residual = (flags & F_RESIDUAL) != 0;
@@ -503,19 +505,25 @@ static bool lane_layout(bool bwd, int N, int n, int L, int dtype, int flags, int
   const int warps = threads / 32;
   uint64_t off = 0;
   auto take = [&](uint64_t bytes) { uint64_t o = off; off = (off + bytes + 127) / 128 * 128; return (uint32_t)o; };
-  const uint64_t work = NS * RN * (long_shifts ? 4 : w);
-  pl.off_work = take(terms && work < (uint64_t)8 * N ? (uint64_t)8 * N : work);
-  pl.off_res = residual ? take(RN * w) : pl.off_work;
-  pl.off_ckpt = take(n_ck ? (uint64_t)n_ck * RN * 8 : 16);
+  if (ahead && long_shifts) return false;
   pl.halo_warp_bytes = ea >= 0 ? (uint32_t)(NS * lane_halo_floats(n, ea) * 4) : 0;
   pl.halo_warp_bytes = (pl.halo_warp_bytes + 15u) / 16u * 16u;
-  pl.off_halo = take((uint64_t)2 * warps * pl.halo_warp_bytes + 16);
+  const uint64_t halo = (uint64_t)2 * warps * pl.halo_warp_bytes + 16;
+  uint64_t work = (ahead ? 2 : NS) * RN * (long_shifts ? 4 : w);
+  if (terms && work < (uint64_t)8 * N) work = (uint64_t)8 * N;
+  if (alias && work < halo) work = halo;
+  pl.off_work = take(work);
+  pl.off_land = ahead ? take((ahead == LANE_AHEAD_OUTPUT ? 4 : 2) * RN * w) : pl.off_work;
+  pl.off_res = residual ? take(RN * w) : pl.off_work;
+  pl.off_ckpt = take(n_ck && !ahead ? (uint64_t)n_ck * RN * 8 : 16);
+  pl.off_halo = alias ? pl.off_work : take(halo);
   pl.off_red = take(bwd ? (uint64_t)2 * L * warps * 4 : 16);
   pl.off_w = take((uint64_t)16 * L);
   pl.off_bar = take(32);
   if (off > limit) return false;
   pl.threads = threads; pl.R = R; pl.tpr = tpr; pl.ea_max = ea; pl.smem = (size_t)off;
   pl.n_ckpt_slots = (uint32_t)n_ck;
+  pl.ahead = ahead;
   return true;
 }
 
@@ -552,18 +560,18 @@ static bool lanep_layout(bool bwd, int N, int L, int dtype, int flags, int n_ck,
 }
 
 struct LaneKey {
-  int epoch, dev, bwd, N, n, L, l0, dtype, flags, n_ck, act;
+  int epoch, dev, bwd, N, n, L, l0, dtype, flags, n_ck, rec, act;
   long long B;
   bool operator==(const LaneKey& o) const {
     return epoch == o.epoch && dev == o.dev && bwd == o.bwd && N == o.N && n == o.n && L == o.L && l0 == o.l0 && dtype == o.dtype &&
-           flags == o.flags && n_ck == o.n_ck && act == o.act && B == o.B;
+           flags == o.flags && n_ck == o.n_ck && rec == o.rec && act == o.act && B == o.B;
   }
 };
 
 // NCN_OK with pl filled, NCN_ERR_UNSUPPORTED when the family does not cover the arguments.
 // Plans are remembered per argument set: a plan costs a few occupancy queries.
 static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, int l0, int L, int dtype, int flags,
-                      int n_ck, const DevInfo& dev, int act, LanePlan& pl) {
+                      int n_ck, bool rec, const DevInfo& dev, int act, LanePlan& pl) {
   if (!lanes_enabled()) return NCN_ERR_UNSUPPORTED;
   if (flags & F_RECOMPUTE) return NCN_ERR_UNSUPPORTED;
   LaneShape shape{};
@@ -571,7 +579,7 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   const int e_need = shape.e_need;
   static std::mutex mu;
   static std::vector<std::pair<LaneKey, std::pair<int, LanePlan>>> cache;
-  const LaneKey key{g_plan_epoch.load(), dev.dev, bwd ? 1 : 0, (int)N, n, L, l0, dtype, flags & (F_RESIDUAL | F_TAPE), n_ck, act, (long long)B};
+  const LaneKey key{g_plan_epoch.load(), dev.dev, bwd ? 1 : 0, (int)N, n, L, l0, dtype, flags & (F_RESIDUAL | F_TAPE), n_ck, rec, act, (long long)B};
   {
     std::lock_guard<std::mutex> lk(mu);
     for (auto& kv : cache)
@@ -624,7 +632,7 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   }
   for (int ea = ea_hi; !have_pipe && ea >= ea_lo; --ea) {
     LanePlan trial;
-    if (!lane_layout(bwd, (int)N, n, L, dtype, flags, n_ck, R, tpr, ea, e_need, terms, (uint32_t)dev.smem_optin, trial))
+    if (!lane_layout(bwd, (int)N, n, L, dtype, flags, n_ck, R, tpr, ea, e_need, terms, LANE_AHEAD_NONE, false, (uint32_t)dev.smem_optin, trial))
       continue;
     int occ = 0;
     LaneParams dummy{};
@@ -637,6 +645,29 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
     trial.occ = occ;
     if (rc != NCN_OK || occ > best.occ) { best = trial; rc = NCN_OK; }
     if (occ >= want_occ) break;
+  }
+  // The inputs a tile ahead, where their buffer costs no CTA.  Backward, us, without -> with: bf16, end state stored: 65536 x 2048, groups
+  // of 8, 4 stages 2126 -> 2065; 32768 x 4096 2295 -> 2203; 16384 x 8192, 3 stages 1960 -> 1770; groups of 2, 6 stages 1699 -> 1505.
+  // fp32 from the output: 8192 x 8192, groups of 8, 3 stages 1305 -> 1214; 16384 x 4096, groups of 2, 8 stages 1139 -> 1085; groups of 8,
+  // 4 stages 1437 -> 1428.  fp32 with all states stored, which then need no shared memory: 16384 x 4096, groups of 8 1880 -> 1414.
+  // The pipelined kernel of groups of 4 stays ahead of it (32768 x 4096, 5 stages bf16 1738 against 1810, fp32 2140 against 2328) unless its
+  // stored states cost it a CTA (fp32, end state stored 2764 against 2195).
+  if (rc == NCN_OK && bwd && !rec && !shape.ragged && (!have_pipe || best.occ < want_occ)) {
+    const int enough = best.occ + (have_pipe ? 1 : 0);  // CTAs per SM that make it worth while
+    const int ahead = !(flags & F_TAPE) ? LANE_AHEAD_OUTPUT : n_ck > 1 ? LANE_AHEAD_TAPES : LANE_AHEAD_TAPE;
+    for (int alias = 0; alias < 2 && best.ahead == LANE_AHEAD_NONE; ++alias) {
+      LanePlan trial;
+      if (!lane_layout(bwd, (int)N, n, L, dtype, flags, n_ck, R, tpr, ea_hi, e_need, terms, ahead, alias != 0, (uint32_t)dev.smem_optin, trial))
+        continue;
+      int occ = 0;
+      LaneParams dummy{};
+      dummy.tpr = tpr;
+      dummy.ahead = ahead;
+      cudaError_t e = lane_fn(n, bwd)(act, dtype, dummy, 0, trial.threads, trial.smem, nullptr, &occ);
+      if (e != cudaSuccess) return cuda_fail(e);
+      trial.occ = occ > want_occ ? want_occ : occ;
+      if (trial.occ >= enough) best = trial;
+    }
   }
   if (rc == NCN_OK) {
     best.thr = shape.thr;
@@ -783,8 +814,9 @@ static void fill_lane(LaneParams& p, const LanePlan& pl) {
   p.R = pl.R; p.tpr = pl.tpr; p.thr = pl.thr; p.ragged = pl.ragged; p.ea_max = pl.ea_max; p.tiles = pl.tiles;
   p.off_work = pl.off_work; p.off_res = pl.off_res; p.off_ckpt = pl.off_ckpt; p.off_halo = pl.off_halo;
   p.off_red = pl.off_red; p.off_w = pl.off_w; p.off_bar = pl.off_bar;
+  p.off_land = pl.off_land;
   p.halo_warp_bytes = pl.halo_warp_bytes; p.n_ckpt_slots = pl.n_ckpt_slots;
-  p.pipelined = pl.pipelined;
+  p.pipelined = pl.pipelined; p.ahead = pl.ahead;
 }
 
 static void fill_offsets(RowsParams& p, const Plan& pl) {
@@ -1186,8 +1218,8 @@ static int net_supported(int64_t B, int64_t N, int64_t E, int n_cache, int n_hea
   if (dtype == DT_F32 && walk > kSegment) return 0;
   const int act = fused_act(ACT_TANH, dtype);
   LanePlan lf, lb;  // (only while the strides of the stages do not wrap)
-  if (first >= 0 && plan_lanes(false, B, N, E, n_cache, n_head, first, L, dtype, flags, 0, dev, act, lf) == NCN_OK &&
-      plan_lanes(true, B, N, E, n_cache, n_head, first, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK)
+  if (first >= 0 && plan_lanes(false, B, N, E, n_cache, n_head, first, L, dtype, flags, 0, false, dev, act, lf) == NCN_OK &&
+      plan_lanes(true, B, N, E, n_cache, n_head, first, L, dtype, flags, n_ck, false, dev, act, lb) == NCN_OK)
     return 1;
   SoloPlan sf, sb;  // (groups of 8: all rows that fit these fit the shared-memory kernels)
   return plan_solo(false, B, N, E, n_cache, n_head, L, dtype, flags, false, dev, act, sf) == NCN_OK &&
@@ -1255,9 +1287,9 @@ static int net_fwd_impl(const void* x, const void* xa, const float* const* list,
     // only where the backward of the same arguments is of this family too
     LanePlan lp, lb;
     const int n_ck = ck_used ? ckpt_slots(L, ckpt_every, flags) : 0;
-    bool lanes = plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, dev, act, lp) == NCN_OK;
+    bool lanes = plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, false, dev, act, lp) == NCN_OK;
     if (lanes && n_ck > 0)
-      lanes = plan_lanes(true, B, N, E, n_cache, n_head, first_module, L, dtype, flags, n_ck, dev, act, lb) == NCN_OK;
+      lanes = plan_lanes(true, B, N, E, n_cache, n_head, first_module, L, dtype, flags, n_ck, false, dev, act, lb) == NCN_OK;
     // With tanh.approx the pair forward is as fast on ragged rows of 2 and 8 (1008 x 16.6 K rows, n = 2: 142 us against 148; 3264,
     // n = 8: 152 against 157), where it fits.
     if (lanes && lp.ragged && n_ck == 0 && dtype == DT_BF16 && n_cache != 4) {
@@ -1379,9 +1411,9 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
   {
     // register-resident family (with stored states: only where the forward is of this family too)
     LanePlan lp, lf;
-    bool lanes = plan_lanes(true, B, N, E, n_cache, n_head, first_module, L, dtype, flags, n_ck, dev, act, lp) == NCN_OK;
+    bool lanes = plan_lanes(true, B, N, E, n_cache, n_head, first_module, L, dtype, flags, n_ck, x_rec != nullptr, dev, act, lp) == NCN_OK;
     if (lanes && n_ck > 0)
-      lanes = plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, dev, act, lf) == NCN_OK;
+      lanes = plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, false, dev, act, lf) == NCN_OK;
     if (lanes) {
       if (lp.ragged || lp.tpr > kLaneThreads) {
         if ((rc = fit_grid(lp.grid)) != NCN_OK) return rc;

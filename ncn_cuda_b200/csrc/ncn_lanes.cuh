@@ -246,8 +246,8 @@ __device__ __forceinline__ void cta_sync() { __syncthreads(); }
 // from higher threads) or - k (UP = true).  halo_pub / halo_nbr: this warp's and the source
 // neighbour's halo area of the current buffer (shared-window byte addresses).  RAG: the warp holds vb blocks, an even
 // number of at least (NG-1) 2^E, and its last lanes may hold none; the halo of a shift by k is exchanged by the blocks
-// c < k (UP: c >= vb - k) as in a full warp, with vb in the place of 32 G.
-template <int NG, int G, int NS, int E, bool UP, bool RAG>
+// c < k (UP: c >= vb - k) as in a full warp, with vb in the place of 32 G.  Streams S0 .. NS-1.
+template <int NG, int G, int NS, int E, bool UP, bool RAG, int S0>
 __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32_t halo_pub, uint32_t halo_nbr, int lane, int vb) {
   constexpr int D = 1 << E;
   constexpr int HS = lane_halo_floats(NG, E);  // floats per stream
@@ -258,10 +258,10 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
     // One pair per thread and shifts by k = o blocks.  The pair is published whole (for odd k one value more than
     // the neighbour reads); odd shifts swap the halves of a pair: x <- y of lane +- (k-1)/2, y <- x of lane +- (k+1)/2.
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
+    for (int s = S0; s < NS; ++s) {
 #pragma unroll
       for (int o = 1; o < NG; ++o) {
-        const uint32_t reg = halo_pub + 4u * (uint32_t)(s * HS + lane_halo_pair_base(o));
+        const uint32_t reg = halo_pub + 4u * (uint32_t)((s - S0) * HS + lane_halo_pair_base(o));
         if (!UP) {
           sts64_if(2 * lane < o, reg + 8u * (uint32_t)lane, V[s][0][o].x, V[s][0][o].y);
         } else {
@@ -272,10 +272,10 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
     }
     cta_sync();
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
+    for (int s = S0; s < NS; ++s) {
 #pragma unroll
       for (int o = 1; o < NG; ++o) {
-        const uint32_t reg = halo_nbr + 4u * (uint32_t)(s * HS + lane_halo_pair_base(o));
+        const uint32_t reg = halo_nbr + 4u * (uint32_t)((s - S0) * HS + lane_halo_pair_base(o));
         const float2 v = V[s][0][o];
         float2 n;
         if (o & 1) {
@@ -311,11 +311,11 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
   const int c0 = G * lane;
   // ---- publish what the neighbouring warp will want
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
+  for (int s = S0; s < NS; ++s) {
 #pragma unroll
     for (int o = 1; o < NG; ++o) {
       const int k = o * D;
-      const int base = s * HS + D * o * (o - 1) / 2;
+      const int base = (s - S0) * HS + D * o * (o - 1) / 2;
       if constexpr (E >= 1) {
 #pragma unroll
         for (int p = 0; p < G / 2; ++p) {
@@ -342,11 +342,11 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
   cta_sync();
   // ---- fetch
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
+  for (int s = S0; s < NS; ++s) {
 #pragma unroll
     for (int o = 1; o < NG; ++o) {
       const int k = o * D;
-      const int base = s * HS + D * o * (o - 1) / 2;
+      const int base = (s - S0) * HS + D * o * (o - 1) / 2;
       float nv[G];
 #pragma unroll
       for (int j = 0; j < G; ++j) {
@@ -402,11 +402,11 @@ __device__ __forceinline__ void exchange_shfl(float2 (&V)[NS][G / 2][NG], uint32
 // Shift by any multiple of G blocks (RAG: any even number) per offset through the tile buffer, viewed as fp32 arrays
 // [stream][offset][m] of the row (row_addr: shared-window byte address of the row's part of it).  blk: first block of the
 // thread, vg: how many of its G blocks exist.
-template <int NG, int G, int NS, bool RAG>
+template <int NG, int G, int NS, bool RAG, int S0>
 __device__ __forceinline__ void exchange_smem(float2 (&V)[NS][G / 2][NG], uint32_t row_addr, int blk, int vg, int m, int delta) {
   const int mmask = m - 1;
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
+  for (int s = S0; s < NS; ++s) {
 #pragma unroll
     for (int o = 1; o < NG; ++o) {
       const uint32_t arr = row_addr + 4u * (uint32_t)((s * NG + o) * m);
@@ -426,7 +426,7 @@ __device__ __forceinline__ void exchange_smem(float2 (&V)[NS][G / 2][NG], uint32
       src = (blk + o * delta) & mmask;  // multiple of G: the G values stay contiguous
     }
 #pragma unroll
-    for (int s = 0; s < NS; ++s) {
+    for (int s = S0; s < NS; ++s) {
       const uint32_t arr = row_addr + 4u * (uint32_t)((s * NG + o) * m);
 #pragma unroll
       for (int p = 0; p < G / 2; ++p) {
@@ -470,8 +470,8 @@ struct LaneShare {
   __device__ __forceinline__ bool pair(int p) const { return !RAG || 2 * p < vg; }
 };
 
-// delta = s_new - s_old (0, or +-2^e).  Shuffle exchange up to 2^ea_max, tile buffer beyond.
-template <int NG, int G, int NS, bool RAG>
+// delta = s_new - s_old (0, or +-2^e).  Shuffle exchange up to 2^ea_max, tile buffer beyond.  Streams S0 .. NS-1.
+template <int NG, int G, int NS, bool RAG, int S0 = 0>
 __device__ __forceinline__ void lane_exchange(float2 (&V)[NS][G / 2][NG], int delta, int ea_max, LaneHalo& h, int lane,
                                               uint32_t row_addr, const LaneShare<G, RAG>& sh, int m) {
   if (delta == 0) return;
@@ -479,7 +479,7 @@ __device__ __forceinline__ void lane_exchange(float2 (&V)[NS][G / 2][NG], int de
   const int ad = up ? -delta : delta;
   const int e = 31 - __clz(ad);
   if (e > ea_max) {
-    exchange_smem<NG, G, NS, RAG>(V, row_addr, sh.blk, sh.vg, m, delta);
+    exchange_smem<NG, G, NS, RAG, S0>(V, row_addr, sh.blk, sh.vg, m, delta);
     return;
   }
   const uint32_t bufa = h.base + (uint32_t)h.parity * h.buf_bytes;
@@ -490,8 +490,8 @@ __device__ __forceinline__ void lane_exchange(float2 (&V)[NS][G / 2][NG], int de
   // one dense switch over (e, direction): a jump table instead of a chain of compares, each of which would be a
   // possibly divergent branch with its own reconvergence point
 #define NCN_LANE_CASE(EE)                                                                                   \
-  case 2 * EE: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, false, RAG>(V, pub, nbr, lane, sh.vb); break; \
-  case 2 * EE + 1: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, true, RAG>(V, pub, nbr, lane, sh.vb); break;
+  case 2 * EE: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, false, RAG, S0>(V, pub, nbr, lane, sh.vb); break; \
+  case 2 * EE + 1: if constexpr (CAP >= EE) exchange_shfl<NG, G, NS, EE, true, RAG, S0>(V, pub, nbr, lane, sh.vb); break;
   switch (2 * e + (up ? 1 : 0)) {
     NCN_LANE_CASE(0)
     NCN_LANE_CASE(1)
@@ -761,7 +761,11 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_fwd_kernel(const __grid_const
 // ------------------------------------------------------------------------------------------ backward
 // From the net output (reversible inverse), from stored states (checkpoints, F_TAPE), F_RESIDUAL; no
 // forward replay.
-template <int NG, int ACT, typename T, int MAXT, int MINB, bool RAG>
+//
+// AHEAD (shuffled shifts only, and not where the rebuilt input is asked for): what is read of the next tile (with F_TAPE dy and dya,
+// else y and ya too) is copied to a buffer of its own while this one is worked on.  Stored states go from global memory to x and a as soon
+// as these are done with, the last stage's before the tile starts, and the shift that follows moves the cotangents alone.
+template <int NG, int ACT, typename T, int MAXT, int MINB, int AHEAD, bool RAG>
 __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
@@ -780,14 +784,19 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
   const T* g_in[4] = {static_cast<const T*>(p.in[0]), static_cast<const T*>(p.in[1]), static_cast<const T*>(p.in[2]),
                       static_cast<const T*>(p.in[3])};
   const float2* ckpt = reinterpret_cast<const float2*>(p.ckpt);
-  const bool want_rec = p.out[2] != nullptr;
+  const bool want_rec = !AHEAD && p.out[2] != nullptr;
   const bool residual = (p.flags & F_RESIDUAL) != 0;
-  const bool tape = (p.flags & F_TAPE) != 0;  // the last stage's output state comes from its checkpoint
+  // the last stage's output state comes from its checkpoint
+  constexpr bool ENDS = AHEAD == LANE_AHEAD_TAPE || AHEAD == LANE_AHEAD_TAPES, INNER = AHEAD == LANE_AHEAD_OUTPUT || AHEAD == LANE_AHEAD_TAPES;
+  const bool tape = AHEAD ? ENDS : (p.flags & F_TAPE) != 0;
   const long long BN = p.B * (long long)N;
   const uint32_t n_ck = p.n_ckpt_slots;
+  constexpr int Q0 = ENDS ? 2 : 0;      // AHEAD: native streams q >= Q0 at land + (q - Q0)*RN
+  T* const land = reinterpret_cast<T*>(smem + p.off_land);
 
   if (tid == 0) {
     mbar_init(&bar[0], 1);
+    if (AHEAD) mbar_init(&bar[1], 1);  // F_RESIDUAL: dy of the tile once more, for its end
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -827,8 +836,43 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
   const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
+  auto rows_of = [&](long long tl) { return (int)min((long long)R, p.B - tl * R); };
+  auto copy_ahead = [&](long long tl) {
+    const uint32_t bytes = (uint32_t)(rows_of(tl) * N * sizeof(T));
+    mbar_expect_tx(&bar[0], (4 - Q0) * bytes);
+#pragma unroll
+    for (int q = Q0; q < 4; ++q) bulk_g2s(land + (q - Q0) * RN, g_in[q] + tl * R * N, bytes, &bar[0]);
+  };
+  float2 V[4][G / 2][NG];  // x, xa, gx, ga
+  auto load_state = [&](long long tl, int ck) {
+    const float2* c = ckpt + (long long)ck * BN + (tl * R + r) * N + (sh.blk >> 1);
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int o = 0; o < NG; ++o)
+#pragma unroll
+        for (int pp = 0; pp < G / 2; ++pp)
+          if (sh.pair(pp)) V[s][pp][o] = __ldg(c + (s * NG + o) * (m >> 1) + pp);
+  };
+  if constexpr (AHEAD) {
+    if (tid == 0) copy_ahead(blockIdx.x);  // (there is a tile for every CTA)
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int pp = 0; pp < G / 2; ++pp)
+#pragma unroll
+        for (int o = 0; o < NG; ++o) V[s][pp][o] = f2(0.0f);
+    if (ENDS && r < rows_of(blockIdx.x)) load_state(blockIdx.x, recs[L - 1].ck);
+  }
+
   for (long long tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
-    if (tid == 0) {
+    if constexpr (AHEAD) {
+      if (tid == 0 && residual) {
+        const uint32_t bytes = (uint32_t)(rows_of(tile) * N * sizeof(T));
+        mbar_expect_tx(&bar[1], bytes);
+        bulk_g2s(sdy, g_in[2] + tile * R * N, bytes, &bar[1]);
+      }
+    } else if (tid == 0) {
       bulk_wait_read0();  // the previous tile's stores have left the buffer
       issue_load(tile);
     }
@@ -841,41 +885,48 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
     const int rows = (int)min((long long)R, p.B - row0);
     const bool on_row = r < rows, active = on_row && sh.any();
 
-    float2 V[4][G / 2][NG];  // x, xa, gx, ga
 #pragma unroll
-    for (int s = 0; s < 4; ++s)
+    for (int s = Q0; s < 4; ++s)
 #pragma unroll
       for (int pp = 0; pp < G / 2; ++pp)
 #pragma unroll
         for (int o = 0; o < NG; ++o) V[s][pp][o] = f2(0.0f);
     if (active) {
+      const T* c = AHEAD ? land - Q0 * RN : win;
       if (!tape) {
-        lane_ld_native<NG, G, T>(win + chunk, V[0], t);
-        lane_ld_native<NG, G, T>(win + RN + chunk, V[1], t);
+        lane_ld_native<NG, G, T>(c + chunk, V[0], t);
+        lane_ld_native<NG, G, T>(c + RN + chunk, V[1], t);
       }
-      lane_ld_native<NG, G, T>(win + 2 * RN + chunk, V[2], t);
-      lane_ld_native<NG, G, T>(win + 3 * RN + chunk, V[3], t);
+      lane_ld_native<NG, G, T>(c + 2 * RN + chunk, V[2], t);
+      lane_ld_native<NG, G, T>(c + 3 * RN + chunk, V[3], t);
     }
+    if (AHEAD && tid == 0) bulk_wait_read0();  // the previous tile's stores have left the buffer
     __syncthreads();  // native inputs are in registers; the buffer is free for long shifts
-    if (tid == 0 && tile + gridDim.x < p.tiles) {  // next tile towards L2 while this one is worked on
+    if (tid == 0 && tile + gridDim.x < p.tiles) {  // next tile into its buffer or towards L2 while this one is worked on
+      if (AHEAD) copy_ahead(tile + gridDim.x);
       const long long nrow0 = (tile + gridDim.x) * R;
       const int nrows = (int)min((long long)R, p.B - nrow0);
       const uint32_t bytes = (uint32_t)(nrows * N * sizeof(T));
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (q >= 2 || !tape) l2_prefetch(g_in[q] + nrow0 * N, bytes);
+        if (!AHEAD && (q >= 2 || !tape)) l2_prefetch(g_in[q] + nrow0 * N, bytes);
       for (uint32_t k = 0; k < n_ck; ++k) l2_prefetch(ckpt + (long long)k * BN + nrow0 * N, (uint32_t)(nrows * N * sizeof(float2)));
     }
 
     int s_cur = 0;
     StageRec rec_next = recs[L - 1];
+    if constexpr (ENDS) {  // (x, a are in the last stage's order)
+      lane_exchange<NG, G, 4, RAG, 2>(V, rec_next.s, p.ea_max, halo, lane, xrow, sh, m);
+      s_cur = rec_next.s;
+    }
     for (int l = L - 1; l >= 0; --l) {
       const StageRec rec = rec_next;
       if (l > 0) rec_next = recs[l - 1];
-      lane_exchange<NG, G, 4, RAG>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, sh, m);
+      if (INNER && rec.ck >= 0) lane_exchange<NG, G, 4, RAG, 2>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, sh, m);  // (x, a are in place)
+      else lane_exchange<NG, G, 4, RAG>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, sh, m);
       s_cur = rec.s;
       w.stage(rec.owi, rec.owj);
-      if (rec.ck >= 0) {  // a state saved after stage l replaces the rebuilt one
+      if (!AHEAD && rec.ck >= 0) {  // a state saved after stage l replaces the rebuilt one
         const float2* c = sck + rec.ck * RN + r * N + (sh.blk >> 1);
 #pragma unroll
         for (int s = 0; s < 2; ++s)
@@ -893,6 +944,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
         lane_backward<NG, ACT>(V[0][pp], V[1][pp], V[2][pp], V[3][pp], w, dwi, dwj);
         if (!sh.pair(pp)) { dwi = di; dwj = dj; }
       }
+      if (INNER && l > 0 && rec_next.ck >= 0 && active) load_state(tile, rec_next.ck);
       // ---- weight-gradient partial of this stage: fixed-order warp tree, one slot per warp
       {
         const float di = (dwi.x + dwi.y) * dsi, dj = (dwj.x + dwj.y) * dsj;
@@ -905,7 +957,14 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
         if ((lane & 15) == 0 && on_row) red[(l * nwarp + warp) * 2 + (hi ? 1 : 0)] += keep;
       }
     }
-    lane_exchange<NG, G, 4, RAG>(V, -s_cur, p.ea_max, halo, lane, xrow, sh, m);  // back to stride 0 = native order
+    if constexpr (AHEAD) {
+      if (ENDS && r < rows_of(tile + gridDim.x)) load_state(tile + gridDim.x, recs[L - 1].ck);  // (none beyond the last tile)
+      lane_exchange<NG, G, 4, RAG, 2>(V, -s_cur, p.ea_max, halo, lane, xrow, sh, m);
+      if (residual && !mbar_wait_bounded(&bar[1], phase ^ 1)) *abort_flag = 1;  // (seen at the next tile)
+      if (p.off_halo == p.off_work) __syncthreads();                             // the halo has been read; the buffer may take the results
+    } else {
+      lane_exchange<NG, G, 4, RAG>(V, -s_cur, p.ea_max, halo, lane, xrow, sh, m);  // back to stride 0 = native order
+    }
     if (active) {
       if (residual) {
         float2 gin[G / 2][NG];

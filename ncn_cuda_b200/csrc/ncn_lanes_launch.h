@@ -21,11 +21,17 @@ struct LaneParams {
   int ea_max;          // shifts of up to 2^ea_max blocks per offset use shuffles + halo, longer ones the tile buffer
   float alpha, oma;
   uint32_t off_work, off_res, off_ckpt, off_halo, off_red, off_w, off_bar;
+  uint32_t off_land;         // backward, ahead: buffer of the next tile's streams
   uint32_t halo_warp_bytes;  // halo bytes per warp and buffer
   uint32_t n_ckpt_slots;
   int test_short_wait;       // forward, tests of the give-up path only: expect 16 bytes that never come, poll 2^10 times
+  int ahead;                 // backward: LaneAhead
   int pipelined;             // backward, n = 4: the kernel of ncn_lanes_pipe.cuh (halo inside the tile buffer)
 };
+
+// Backward: what is fetched a tile ahead (lane_bwd_kernel): nothing; all four streams; with F_TAPE dy, dya and the last state, which is
+// the only stored one; the same with others behind it.
+enum LaneAhead : int { LANE_AHEAD_NONE = 0, LANE_AHEAD_OUTPUT = 1, LANE_AHEAD_TAPE = 2, LANE_AHEAD_TAPES = 3 };
 
 __host__ __device__ constexpr int lane_groups(int ng) { return ng == 2 ? 8 : ng == 4 ? 4 : 2; }
 // largest log2 |stride difference| the shuffle exchange is compiled for
