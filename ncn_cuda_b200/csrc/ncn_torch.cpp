@@ -12,6 +12,7 @@
 //
 // Saved tensors go through SavedVariable, so in-place changes, saved-tensor hooks and a second backward
 // without retain_graph behave as for any autograd operator.  Without gradients no state is stored.
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -588,6 +589,98 @@ Result py_net_list(const Tensor& x, const Tensor& xa, const variable_list& ws, d
   return chain_forward(x, xa, ws, Tensor(), ChainCfg{alpha, act, n, C, 0, L, keep, 0});
 }
 
+// ---------------------------------------------------------------- activations that live on the host
+// Forward and backward of a fused net, chunk of rows by chunk (host.py): copies in, kernels and copies out on a stream each, two
+// chunks of inputs and three of results on the device.  in: x, xa, dy, dya; out: y, ya, dx, dxa; dW [L, 2E] on the device gains the
+// weight gradient chunk after chunk.  Returns when the results are on the host.
+//
+// Native because a chunk's 8 copies, 3 launches and 4 events cost 220 us in Python against 75 here, which sets the smallest chunk and
+// with it how much of the first copy in and the last copy out nothing overlaps.
+void py_host_step(const variable_list& in, const variable_list& out, const Tensor& weights, const Tensor& dW, double alpha, int act, int n, int C,
+                  bool recompute, int every, bool tape, const std::vector<std::pair<int64_t, int64_t>>& chunks) {
+  py::gil_scoped_release nogil;
+  at::NoGradGuard no_grad;
+  const c10::cuda::CUDAGuard guard(weights.device());
+  const c10::DeviceIndex dev = weights.device().index();
+  using Stream = c10::cuda::CUDAStream;
+  const Stream s_in = c10::cuda::getStreamFromPool(false, dev), s_k = c10::cuda::getStreamFromPool(false, dev),
+               s_out = c10::cuda::getStreamFromPool(false, dev);
+  int64_t rows = 0;
+  for (const auto& c : chunks) rows = std::max(rows, c.second - c.first);
+  std::vector<int64_t> shape = in[0].sizes().vec();
+  if (!shape.empty()) shape[0] = rows;
+  const at::TensorOptions opt = in[0].options().device(weights.device()).pinned_memory(false);
+  constexpr int SI = 2, SO = 3;
+  // All memory comes from the caller's stream, which the others wait for: on streams of the pool, another three in every call, each
+  // would gather a cache of its own.
+  const int L = (int)weights.size(0);
+  Tensor bin[SI][4], bout[SO][4], ck, ws;
+  for (int k = 0; k < SO; ++k)
+    for (int q = 0; q < 4; ++q) {
+      if (k >= (int)chunks.size()) continue;
+      if (k < SI) bin[k][q] = at::empty(shape, opt);
+      bout[k][q] = at::empty(shape, opt);
+    }
+  if (chunks.empty()) return;
+  check_activations(bin[0][0], bin[0][1]);
+  const int64_t N = shape[1], E = shape[2];
+  const int dt = dtype_code(bin[0][0]);
+  const Tensor W = plain_weights(weights, (int64_t)L * 2 * E, weights.device());
+  ws = at::empty({(int64_t)ncn_bwd_workspace_bytes(rows, N, E, n, C, L, dt)}, opt.dtype(at::kByte));
+  if (const size_t bytes = ncn_ckpt_bytes(rows, N, E, L, every, tape ? NCN_TAPE : 0)) ck = at::empty({(int64_t)(bytes / 4)}, opt.dtype(at::kFloat));
+  at::cuda::CUDAEvent start;
+  start.record(c10::cuda::getCurrentCUDAStream(dev));
+  for (const Stream& s : {s_in, s_k, s_out}) start.block(s);
+
+  at::cuda::CUDAEvent ev_in[SI], ev_free[SI], ev_f[SO], ev_b[SO], ev_out[SO];
+  try {
+    int ci = 0;
+    for (const auto& c : chunks) {
+      const int ki = ci % SI, ko = ci % SO;
+      const int64_t B = c.second - c.first;
+      {
+        const c10::cuda::CUDAStreamGuard on(s_in);
+        if (ci >= SI) ev_free[ki].block(s_in);
+        for (int q = 0; q < 4; ++q) bin[ki][q].slice(0, 0, B).copy_(in[q].slice(0, c.first, c.second), true);
+        ev_in[ki].record(s_in);
+      }
+      {
+        const c10::cuda::CUDAStreamGuard on(s_k);
+        if (ci >= SO) ev_out[ko].block(s_k);
+        ev_in[ki].block(s_k);
+        void *const x = bin[ki][0].data_ptr(), *const xa = bin[ki][1].data_ptr(), *const y = bout[ko][0].data_ptr(), *const ya = bout[ko][1].data_ptr();
+        float* const ckp = ck.defined() ? ck.mutable_data_ptr<float>() : nullptr;
+        check_status("ncn_net_fwd", ncn_net_fwd(x, xa, W.const_data_ptr<float>(), y, ya, ckp, every, B, N, E, n, C, 0, L, alpha, act, dt,
+                                                tape ? NCN_TAPE : 0, s_k.stream()));
+        ev_f[ko].record(s_k);
+        const void *const s0 = tape ? nullptr : recompute ? x : y, *const s1 = tape ? nullptr : recompute ? xa : ya;
+        check_status("ncn_net_bwd",
+                     ncn_net_bwd(s0, s1, bin[ki][2].data_ptr(), bin[ki][3].data_ptr(), W.const_data_ptr<float>(), bout[ko][2].data_ptr(),
+                                 bout[ko][3].data_ptr(), nullptr, nullptr, dW.mutable_data_ptr<float>(), ckp, every, ws.data_ptr(),
+                                 (size_t)ws.numel(), B, N, E, n, C, 0, L, alpha, act, dt, (recompute ? NCN_RECOMPUTE : 0) | (tape ? NCN_TAPE : 0),
+                                 1, s_k.stream()));
+        ev_b[ko].record(s_k);
+        ev_free[ki].record(s_k);
+      }
+      {
+        const c10::cuda::CUDAStreamGuard on(s_out);
+        for (int q = 0; q < 4; ++q) {
+          if (q == 0) ev_f[ko].block(s_out);  // the outputs leave while the backward still runs
+          if (q == 2) ev_b[ko].block(s_out);
+          out[q].slice(0, c.first, c.second).copy_(bout[ko][q].slice(0, 0, B), true);
+        }
+        ev_out[ko].record(s_out);
+      }
+      ++ci;
+    }
+    s_out.synchronize();
+    s_k.synchronize();
+  } catch (...) {  // nothing may be on its way to or from buffers that are given back
+    for (const Stream& s : {s_in, s_k, s_out}) cudaStreamSynchronize(s.stream());
+    throw;
+  }
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_ncn_torch, m) {
@@ -596,4 +689,5 @@ PYBIND11_MODULE(_ncn_torch, m) {
   m.def("net_list", &py_net_list);
   m.def("stages", &py_stages);
   m.def("stage_ctx", &py_stage_ctx);
+  m.def("host_step", &py_host_step);
 }

@@ -1,18 +1,19 @@
 """Host-buffer entry: forward + backward of a fused net on tensors that live in (pinned) host memory.
 
 Rows are independent, so the batch is cut into chunks that flow through three streams
-(host->device copies, kernels, device->host copies) with two device slots per tensor; the
+(host->device copies, kernels, device->host copies; `host_step` of csrc/ncn_torch.cpp); the
 weight gradient is accumulated chunk after chunk in a fixed order, so it stays bitwise
 reproducible.  This is the call a host-side caller of the reference's operator would make
 when its activations are not resident on the GPU.
 """
 from __future__ import annotations
 
+import math
 from typing import Optional, Tuple
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from .ncn_pytorch_wrapper_v2 import plan_backward
 
 
@@ -37,14 +38,23 @@ def chunk_bounds(B: int, rows: int):
     return out
 
 
+def rows_per_chunk(B: int, tensor_bytes: int, chunk_rows: int) -> int:
+    """Rows of a chunk, at most `chunk_rows`.  c chunks leave 1/c of the copies without overlap and cost 75 us each (eight copies,
+    three launches, events), so the sum is smallest at c = sqrt(copies / 75 us); four tensors each way at 47 GB/s make that
+    sqrt(tensor / 0.9 MB).  Measured with 1, 2, 4, 8, 16 chunks, us: tensors of 2.1 MB 429 436 474 788 1134; 8.4 MB 1354 1149 1148 -
+    1623; 33.6 MB 5040 4050 3641 3662 4145; 134 MB 20045 15900 14225 13161 13033."""
+    c = max(1, round(math.sqrt(tensor_bytes / 0.9e6)))
+    return max(1, min(chunk_rows, B, -(-B // c)))
+
+
 def net_fwd_bwd_host(
     x: torch.Tensor, xa: torch.Tensor, W: torch.Tensor, dy: torch.Tensor, dya: torch.Tensor,
     alpha: float, activation, n_cache: int, n_head: int,
     out: Optional[Tuple[torch.Tensor, ...]] = None, chunk_rows: int = 4096, backward_mode: str = "auto",
     device: Optional[torch.device] = None,
 ):
-    """x, xa, dy, dya: CPU tensors [B, N, E] (pinned for full copy bandwidth); W: [L, 2E].
-    Returns (y, ya, dx, dxa, dW) on the host; `out` may supply the four pinned result tensors."""
+    """x, xa, dy, dya: CPU tensors [B, N, E] (pinned for full copy bandwidth); W: [L, 2E].  `chunk_rows`: most rows
+    on the device at a time per buffer.  Returns (y, ya, dx, dxa, dW) on the host; `out` may supply the four pinned result tensors."""
     device = device or torch.device("cuda", torch.cuda.current_device())
     B = x.shape[0]
     L = W.shape[0]
@@ -56,67 +66,9 @@ def net_fwd_bwd_host(
     recompute, every, tape = plan_backward(x.dtype, n_cache, L, False, backward_mode)
     act = ops.activation_code(activation)
 
-    main = torch.cuda.current_stream(device)
-    s_in, s_k, s_out = (torch.cuda.Stream(device) for _ in range(3))
-    for s in (s_in, s_k, s_out):
-        s.wait_stream(main)
-    nslot = 2
-    rows = min(chunk_rows, B)
-    with torch.cuda.stream(s_in):
-        slots = [[torch.empty((rows,) + tuple(x.shape[1:]), dtype=x.dtype, device=device) for _ in range(4)]
-                 for _ in range(nslot)]
-    slot_free = [None] * nslot  # event: kernels of the chunk that used the slot are done
-    done_out = []
-    for ci, (r0, r1) in enumerate(chunk_bounds(B, rows)):
-        k = ci % nslot
-        with torch.cuda.stream(s_in):
-            if slot_free[k] is not None:
-                s_in.wait_event(slot_free[k])
-            bufs = [b[: r1 - r0] for b in slots[k]]
-            for b, h in zip(bufs, (x, xa, dy, dya)):
-                b.copy_(h[r0:r1], non_blocking=True)
-            ev_in = torch.cuda.Event()
-            ev_in.record(s_in)
-        with torch.cuda.stream(s_k):
-            s_k.wait_event(ev_in)
-            y, ya, ckpt = ops.net_fwd(bufs[0], bufs[1], Wd, alpha, act, n_cache, n_head, 0, every, False, tape)
-            ev_f = torch.cuda.Event()
-            ev_f.record(s_k)
-            if tape:
-                res = ops.net_bwd(None, None, bufs[2], bufs[3], Wd, alpha, act, n_cache, n_head, 0, ckpt=ckpt,
-                                  ckpt_every=every, dW_out=dW, tape=True)
-            elif recompute:
-                res = ops.net_bwd(bufs[0], bufs[1], bufs[2], bufs[3], Wd, alpha, act, n_cache, n_head, 0,
-                                  recompute=True, dW_out=dW)
-            else:
-                res = ops.net_bwd(y, ya, bufs[2], bufs[3], Wd, alpha, act, n_cache, n_head, 0, ckpt=ckpt,
-                                  ckpt_every=every, dW_out=dW)
-            dx, dxa = res[0], res[1]
-            ev_k = torch.cuda.Event()
-            ev_k.record(s_k)
-            slot_free[k] = ev_k
-        with torch.cuda.stream(s_out):
-            s_out.wait_event(ev_f)  # the outputs leave while the backward still runs
-            for t, h in zip((y, ya), (y_h, ya_h)):
-                t.record_stream(s_out)
-                h[r0:r1].copy_(t, non_blocking=True)
-            s_out.wait_event(ev_k)
-            for t, h in zip((dx, dxa), (dx_h, dxa_h)):
-                t.record_stream(s_out)
-                h[r0:r1].copy_(t, non_blocking=True)
-            if ckpt is not None:
-                ckpt.record_stream(s_out)
-            ev_o = torch.cuda.Event()
-            ev_o.record(s_out)
-            done_out.append(ev_o)
-    with torch.cuda.stream(s_out):
-        s_out.wait_stream(s_k)
-        dW_h = dW.to("cpu", non_blocking=False)
-    main.wait_stream(s_out)
-    main.wait_stream(s_k)
-    main.wait_stream(s_in)
-    for b4 in slots:
-        for b in b4:
-            b.record_stream(s_k)
-            b.record_stream(main)
+    rows = rows_per_chunk(B, x.numel() * x.element_size(), chunk_rows)
+    _lib.native().host_step(
+        [x, xa, dy, dya], list(out), Wd, dW, alpha, act, n_cache, n_head, recompute, every, tape, chunk_bounds(B, rows)
+    )
+    dW_h = dW.to("cpu")
     return y_h, ya_h, dx_h, dxa_h, dW_h

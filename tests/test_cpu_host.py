@@ -182,6 +182,18 @@ def test_bench_reference_arm_prints_contract_line():
         assert line["cpu_reference_literal"]["kind"] == "reference" and line["cpu_reference_literal"]["value"] > 0
 
 
+@pytest.mark.parametrize("B,tensor_bytes,most", [(1, 4, 4096), (8192, 134 << 20, 4096), (256, 2 << 20, 4096), (65536, 1 << 30, 4096), (30, 400 << 20, 4), (7, 1 << 34, 4096)])
+def test_rows_per_chunk(B, tensor_bytes, most):
+    from ncn_cuda_b200.host import chunk_bounds, rows_per_chunk
+
+    rows = rows_per_chunk(B, tensor_bytes, most)
+    assert 1 <= rows <= min(B, most)
+    b = chunk_bounds(B, rows)
+    assert b[0][0] == 0 and b[-1][1] == B and all(p[1] == q[0] for p, q in zip(b, b[1:]))
+    if tensor_bytes < 2e6:  # a chunk costs more than it overlaps
+        assert len(b) == 1
+
+
 def test_host_pipeline_chunk_bounds():
     from ncn_cuda_b200.host import chunk_bounds
 
