@@ -47,9 +47,16 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
 #endif
 #endif
 #ifdef NCN_BWD
-  if (p.ahead == LANE_AHEAD_OUTPUT) return launch_form<ACT, T, false, LANE_AHEAD_OUTPUT>(p, grid, threads, smem, st, occ);
-  if (p.ahead == LANE_AHEAD_TAPES) return launch_form<ACT, T, false, LANE_AHEAD_TAPES>(p, grid, threads, smem, st, occ);
-  if (p.ahead == LANE_AHEAD_TAPE) return launch_form<ACT, T, false, LANE_AHEAD_TAPE>(p, grid, threads, smem, st, occ);
+#define NCN_AHEAD(A, OK)                                                                                \
+  if (p.ahead == A) {                                                                                   \
+    if (!p.ragged) return launch_form<ACT, T, false, A>(p, grid, threads, smem, st, occ);                \
+    if constexpr (OK) return launch_form<ACT, T, true, A>(p, grid, threads, smem, st, occ);              \
+    return cudaErrorNotSupported;                                                                       \
+  }
+  NCN_AHEAD(LANE_AHEAD_OUTPUT, true)
+  NCN_AHEAD(LANE_AHEAD_TAPE, lane_ahead_tape(NCN_NG, true))
+  NCN_AHEAD(LANE_AHEAD_TAPES, lane_ahead_tape(NCN_NG, true))
+#undef NCN_AHEAD
 #endif
   return p.ragged ? launch_form<ACT, T, true>(p, grid, threads, smem, st, occ) : launch_form<ACT, T, false>(p, grid, threads, smem, st, occ);
 }

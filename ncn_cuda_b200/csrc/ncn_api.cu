@@ -650,17 +650,24 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   // of 8, 4 stages 2126 -> 2065; 32768 x 4096 2295 -> 2203; 16384 x 8192, 3 stages 1960 -> 1770; groups of 2, 6 stages 1699 -> 1505.
   // fp32 from the output: 8192 x 8192, groups of 8, 3 stages 1305 -> 1214; 16384 x 4096, groups of 2, 8 stages 1139 -> 1085; groups of 8,
   // 4 stages 1437 -> 1428.  fp32 with all states stored, which then need no shared memory: 16384 x 4096, groups of 8 1880 -> 1414.
+  // Ragged rows: 20000 x 3000 fp32, groups of 4, 5 stages 1200 -> 1145; 5000 x 8176, groups of 8 861 -> 775; end state stored, 9000 x 5000
+  // fp32, groups of 2 888 -> 787, 10000 x 4000, groups of 4 615 -> 590; bf16 then, and groups of 8, only where that leaves room for more
+  // CTAs or there is one anyway (bf16 5000 x 8184 648 -> 630, but 20000 x 2000 400 -> 408; groups of 8, 4 stages 6000 x 5008 970 -> 897, but
+  // 3000 x 3008 249 -> 255).
   // The pipelined kernel of groups of 4 stays ahead of it (32768 x 4096, 5 stages bf16 1738 against 1810, fp32 2140 against 2328) unless its
   // stored states cost it a CTA (fp32, end state stored 2764 against 2195).
-  if (rc == NCN_OK && bwd && !rec && !shape.ragged && (!have_pipe || best.occ < want_occ)) {
-    const int enough = best.occ + (have_pipe ? 1 : 0);  // CTAs per SM that make it worth while
+  if (rc == NCN_OK && bwd && !rec && (!have_pipe || best.occ < want_occ) && (!(flags & F_TAPE) || lane_ahead_tape(n, shape.ragged))) {
+    // CTAs per SM that make it worth while
+    const bool even = shape.ragged && want_occ > 1 && (n == 8 || (dtype == DT_BF16 && (flags & F_TAPE)));  // (no gain at as many CTAs)
+    const int enough = best.occ + (have_pipe || even ? 1 : 0);
     const int ahead = !(flags & F_TAPE) ? LANE_AHEAD_OUTPUT : n_ck > 1 ? LANE_AHEAD_TAPES : LANE_AHEAD_TAPE;
-    for (int alias = 0; alias < 2 && best.ahead == LANE_AHEAD_NONE; ++alias) {
+    for (int alias = 0; alias < (shape.ragged ? 1 : 2) && best.ahead == LANE_AHEAD_NONE; ++alias) {
       LanePlan trial;
       if (!lane_layout(bwd, (int)N, n, L, dtype, flags, n_ck, R, tpr, ea_hi, e_need, terms, ahead, alias != 0, (uint32_t)dev.smem_optin, trial))
         continue;
       int occ = 0;
       LaneParams dummy{};
+      dummy.ragged = shape.ragged ? 1 : 0;
       dummy.tpr = tpr;
       dummy.ahead = ahead;
       cudaError_t e = lane_fn(n, bwd)(act, dtype, dummy, 0, trial.threads, trial.smem, nullptr, &occ);

@@ -32,6 +32,8 @@ struct LaneParams {
 // Backward: what is fetched a tile ahead (lane_bwd_kernel): nothing; all four streams; with F_TAPE dy, dya and the last state, which is
 // the only stored one; the same with others behind it.
 enum LaneAhead : int { LANE_AHEAD_NONE = 0, LANE_AHEAD_OUTPUT = 1, LANE_AHEAD_TAPE = 2, LANE_AHEAD_TAPES = 3 };
+// Ragged groups of 8 have neither of the last two: ptxas 12.9 fails on them (a segmentation fault).
+constexpr bool lane_ahead_tape(int ng, bool ragged) { return !(ragged && ng == 8); }
 
 __host__ __device__ constexpr int lane_groups(int ng) { return ng == 2 ? 8 : ng == 4 ? 4 : 2; }
 // largest log2 |stride difference| the shuffle exchange is compiled for
