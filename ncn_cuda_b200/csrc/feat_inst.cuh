@@ -12,8 +12,7 @@ template <int LD, int KF, int W, int ACT, typename T>
 static cudaError_t launch_one(const FeatParamsX& p, int grid, int threads, cudaStream_t st, int* occ) {
   auto go = [&](auto k, const auto& args) {
     if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, 0);
-    k<<<grid, threads, 0, st>>>(args);
-    return cudaGetLastError();
+    return launch_behind(k, dim3(grid), threads, 0, st, args);
   };
   constexpr int P = FeatGeom<NCN_NC, LD, KF, W>::P;
   constexpr bool SEVERAL = feat_groups_per_warp(NCN_NC, LD) > 1, BF16 = sizeof(T) != 4;

@@ -15,8 +15,7 @@ static cudaError_t launch_form(const LaneParams& p, int grid, int threads, size_
   cudaError_t e = grant_smem(granted, k, smem);
   if (e != cudaSuccess) return e;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, smem);
-  k<<<grid, threads, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_behind(k, dim3(grid), threads, smem, st, p);
 }
 
 template <int ACT, typename T>
@@ -29,8 +28,7 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
     cudaError_t ep = grant_smem(granted_p, kp, smem);
     if (ep != cudaSuccess) return ep;
     if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kp, threads, smem);
-    kp<<<grid, threads, smem, st>>>(p);
-    return cudaGetLastError();
+    return launch_behind(kp, dim3(grid), threads, smem, st, p);
   }
 #endif
 #else
@@ -41,8 +39,7 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
     cudaError_t ep = grant_smem(granted_pf, kp, smem);
     if (ep != cudaSuccess) return ep;
     if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kp, threads, smem);
-    kp<<<grid, threads, smem, st>>>(p);
-    return cudaGetLastError();
+    return launch_behind(kp, dim3(grid), threads, smem, st, p);
   }
 #endif
 #endif

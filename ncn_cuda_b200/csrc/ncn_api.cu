@@ -858,8 +858,7 @@ static int reduce_dw(const float* partials, float* dW, int rows, int cols, int a
     return NCN_OK;
   }
   const int warps = 4;
-  dw_reduce_kernel<<<(cols + warps - 1) / warps, warps * 32, 0, st>>>(partials, dW, rows, cols, accumulate);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_behind(dw_reduce_kernel, dim3((cols + warps - 1) / warps), warps * 32, 0, st, partials, dW, rows, cols, accumulate);
   return e == cudaSuccess ? NCN_OK : cuda_fail(e);
 }
 
@@ -1131,6 +1130,7 @@ struct ReduceParams {
   int cols;
 };
 __global__ void dw_reduce_stages_kernel(const __grid_constant__ ReduceParams p) {
+  wait_for_inputs();
   const int lane = threadIdx.x & 31, l = blockIdx.y;
   const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (col >= p.cols) return;
@@ -1785,10 +1785,10 @@ int ncn_reduce_partials(const float* const* partials, const int* rows, float* co
     }
     p.cols = (int)cols;
     const int warps = 4;
-    dw_reduce_stages_kernel<<<dim3((unsigned)((cols + warps - 1) / warps), (unsigned)cnt), warps * 32, 0, (cudaStream_t)stream>>>(p);
+    cudaError_t e = launch_behind(dw_reduce_stages_kernel, dim3((unsigned)((cols + warps - 1) / warps), (unsigned)cnt), warps * 32, 0, (cudaStream_t)stream, p);
+    if (e != cudaSuccess) return cuda_fail(e);
   }
-  cudaError_t e = cudaGetLastError();
-  return e == cudaSuccess ? NCN_OK : cuda_fail(e);
+  return NCN_OK;
 }
 
 }  // extern "C"

@@ -458,6 +458,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
   constexpr bool MID = NC >= 16 && (MODE == FM_ANY || MODE == FM_STORED);
   constexpr bool SC = feat_fwd_scaled(MODE, NC, P, W);
   __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
+  wait_for_inputs();
   const FeatThread<G, LD, W> th(p);
   const T* gx = static_cast<const T*>(p.in[0]);
   const T* ga = static_cast<const T*>(p.in[1]);
@@ -610,6 +611,7 @@ __global__ void __launch_bounds__(kFeatWarps * 32, FeatTune<FeatGeom<NC, LD, KF,
   __shared__ __align__(16) float xs[G::TEAMS][2][G::XS];
   __shared__ __align__(16) float cs[G::TEAMS][2][W][G::XS];
   __shared__ float sdw[kFeatWarps][2][D];
+  wait_for_inputs();
   const FeatThread<G, LD, W> th(p);
   const T* g_y = static_cast<const T*>(p.in[0]);
   const T* g_ya = static_cast<const T*>(p.in[1]);

@@ -335,6 +335,7 @@ __global__ void __launch_bounds__(256) stage_bwd_kernel(const StageParams p, con
 // rows in increasing order, then a shuffle tree.  out[c] = sum (+ out[c] when accumulate).
 __global__ void dw_reduce_kernel(const float* __restrict__ partials, float* __restrict__ out, int rows, int cols,
                                  int accumulate) {
+  wait_for_inputs();
   const int lane = threadIdx.x & 31;
   const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (col >= cols) return;

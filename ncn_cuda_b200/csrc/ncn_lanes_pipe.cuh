@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_fwd_kernel(const LaneParams 
     *abort_flag = 0;
     fence_mbar_init();
   }
+  wait_for_inputs();
   fill_stage_table(recs, p.W, p.oma, p.l0, p.m, p.L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr);
   __syncthreads();
 
@@ -402,6 +403,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
     *abort_flag = 0;
     fence_mbar_init();
   }
+  wait_for_inputs();
   fill_stage_table(recs, p.W, p.oma, p.l0, p.m, p.L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr);
   for (int i = tid; i < 2 * L * nwarp; i += nthr) red[i] = 0.0f;
   __syncthreads();

@@ -178,6 +178,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_fwd_kernel(const __grid_const
     *wild = 0;
     fence_mbar_init();
   }
+  wait_for_inputs();
   fill_stage_table(recs, p.W, p.oma, p.l0, m, L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr, &p.list);
   __syncthreads();
 
@@ -326,6 +327,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
     *abort_flag = 0;
     fence_mbar_init();
   }
+  wait_for_inputs();
   fill_stage_table(recs, p.W, p.oma, p.l0, m, L, p.ckpt_every, p.flags, ckpt != nullptr, tid, nthr);
   for (int i = tid; i < 2 * L * nwarp; i += nthr) red[i] = 0.0f;
   __syncthreads();

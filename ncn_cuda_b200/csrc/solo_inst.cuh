@@ -9,8 +9,7 @@ static cudaError_t launch_kernel(K k, SmemGrant& granted, const SoloParams& p, i
   cudaError_t e = grant_smem(granted, k, smem);
   if (e != cudaSuccess) return e;
   if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, k, threads, smem);
-  k<<<grid, threads, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_behind(k, dim3(grid), threads, smem, st, p);
 }
 
 template <int ACT, typename T>
