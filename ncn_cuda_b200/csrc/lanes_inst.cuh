@@ -23,12 +23,21 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
 #ifdef NCN_BWD
 #if NCN_NG == 4
   if (p.pipelined) {  // two half-rows per thread, half a stage apart (ncn_lanes_pipe.cuh)
-    auto kp = lanep_bwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads>;
-    static SmemGrant granted_p;
-    cudaError_t ep = grant_smem(granted_p, kp, smem);
-    if (ep != cudaSuccess) return ep;
-    if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kp, threads, smem);
-    return launch_behind(kp, dim3(grid), threads, smem, st, p);
+    static SmemGrant granted_p[4];
+    auto go = [&](auto kp, SmemGrant& granted) {
+      cudaError_t ep = grant_smem(granted, kp, smem);
+      if (ep != cudaSuccess) return ep;
+      if (occ) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kp, threads, smem);
+      return launch_behind(kp, dim3(grid), threads, smem, st, p);
+    };
+#define NCN_PIPE(A) go(lanep_bwd_kernel<NCN_NG, ACT, T, kLaneMaxThreads, kLaneBwdBlocks * kLaneThreads / kLaneMaxThreads, A>, granted_p[A])
+    switch (p.ahead) {
+      case LANE_AHEAD_OUTPUT: return NCN_PIPE(LANE_AHEAD_OUTPUT);
+      case LANE_AHEAD_TAPE: return NCN_PIPE(LANE_AHEAD_TAPE);
+      case LANE_AHEAD_TAPES: return NCN_PIPE(LANE_AHEAD_TAPES);
+      default: return NCN_PIPE(LANE_AHEAD_NONE);
+    }
+#undef NCN_PIPE
   }
 #endif
 #else

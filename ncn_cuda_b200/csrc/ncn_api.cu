@@ -530,7 +530,7 @@ static bool lane_layout(bool bwd, int N, int n, int L, int dtype, int flags, int
 // Pipelined backward (n = 4, ncn_lanes_pipe.cuh): a thread runs the two halves of its row half a
 // stage apart; every shift goes by shuffles + halo, and the halo lives in the tile buffer.  Needs
 // every change of stride to stay within a warp's reach: 3 * 2^e / 2 <= 24 lanes, i.e. e <= 4.
-static bool lanep_layout(bool bwd, int N, int L, int dtype, int flags, int n_ck, int R, int tpr, int e_need, uint32_t limit,
+static bool lanep_layout(bool bwd, int N, int L, int dtype, int flags, int n_ck, int R, int tpr, int e_need, int ahead, uint32_t limit,
                          LanePlan& pl) {
   if (e_need > 4) return false;
   const int NS = bwd ? 4 : 2;  // streams a thread holds
@@ -540,15 +540,16 @@ static bool lanep_layout(bool bwd, int N, int L, int dtype, int flags, int n_ck,
   const int threads = R * tpr;
   const int warps = threads / 32;
   pl.halo_warp_bytes = NS * 3 * kPipeSo;  // a region of kPipeSo bytes per (stream, offset): enough for shifts of 3 * 2^4 blocks
-  uint64_t work = NS * RN * w;
+  uint64_t work = (ahead ? 2 : NS) * RN * w;
   const uint64_t halo = (uint64_t)2 * warps * pl.halo_warp_bytes;  // two half-row "warps" per warp
   if (halo > work) work = halo;
   uint64_t off = 0;
   auto take = [&](uint64_t bytes) { uint64_t o = off; off = (off + bytes + 127) / 128 * 128; return (uint32_t)o; };
   pl.off_work = take(work);
   pl.off_halo = pl.off_work;
+  pl.off_land = ahead ? take((ahead == LANE_AHEAD_OUTPUT ? 4 : 2) * RN * w) : pl.off_work;
   pl.off_res = residual ? take(RN * w) : pl.off_work;
-  pl.off_ckpt = take(bwd && n_ck ? (uint64_t)n_ck * RN * 8 : 16);  // (the forward stores its states straight to global memory)
+  pl.off_ckpt = take(bwd && n_ck && !ahead ? (uint64_t)n_ck * RN * 8 : 16);  // (the forward stores its states straight to global memory)
   pl.off_red = take((uint64_t)2 * L * warps * 4);
   pl.off_w = take((uint64_t)16 * L);
   pl.off_bar = take(32);
@@ -556,6 +557,7 @@ static bool lanep_layout(bool bwd, int N, int L, int dtype, int flags, int n_ck,
   pl.threads = threads; pl.R = R; pl.tpr = tpr; pl.ea_max = 4; pl.smem = (size_t)off;
   pl.n_ckpt_slots = (uint32_t)n_ck;
   pl.pipelined = 1;
+  pl.ahead = ahead;
   return true;
 }
 
@@ -615,19 +617,26 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   LanePlan best;
   bool have_pipe = false;
   if (n == 4 && !shape.ragged && (bwd ? lanep_enabled() : env_switches().lanes_pipe_fwd)) {
-    LanePlan trial;
-    if (lanep_layout(bwd, (int)N, L, dtype, flags, n_ck, R, tpr, e_need, (uint32_t)dev.smem_optin, trial)) {
+    // The inputs a tile ahead, us without -> with: 32768 x 4096, 5 stages bf16 1738 -> 1682, fp32 from the output alone 2091 -> 2047; 16384 x 8192,
+    // 4 stages fp32 1948 -> 1840, bf16 1565 -> 1433.  Where states are stored inside a net and no CTA per SM is won by it, the copies of a
+    // stage with and without one cost what the rest wins (65536 x 4096, 6 stages 4976 either way; 4096 x 1024 103 -> 105).
+    const int fetch = !bwd || rec ? LANE_AHEAD_NONE : !(flags & F_TAPE) ? LANE_AHEAD_OUTPUT : n_ck > 1 ? LANE_AHEAD_TAPES : LANE_AHEAD_TAPE;
+    for (const int ahead : {(int)LANE_AHEAD_NONE, fetch}) {
+      LanePlan trial;
+      if (have_pipe && ahead == LANE_AHEAD_NONE) break;
+      if (!lanep_layout(bwd, (int)N, L, dtype, flags, n_ck, R, tpr, e_need, ahead, (uint32_t)dev.smem_optin, trial)) continue;
       int occ = 0;
       LaneParams dummy{};
       dummy.pipelined = 1;
+      dummy.ahead = ahead;
       cudaError_t e = lane_fn(n, bwd)(act, dtype, dummy, 0, trial.threads, trial.smem, nullptr, &occ);
       if (e != cudaSuccess) return cuda_fail(e);
-      if (occ >= 1) {
-        trial.occ = occ > want_occ ? want_occ : occ;
-        best = trial;
-        rc = NCN_OK;
-        have_pipe = true;
-      }
+      trial.occ = occ > want_occ ? want_occ : occ;
+      const bool inner = n_ck > ((flags & F_TAPE) ? 1 : 0) && want_occ > 1;
+      if (trial.occ < 1 || (have_pipe && trial.occ < best.occ + (inner ? 1 : 0))) continue;
+      best = trial;
+      rc = NCN_OK;
+      have_pipe = true;
     }
   }
   for (int ea = ea_hi; !have_pipe && ea >= ea_lo; --ea) {
@@ -654,8 +663,7 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   // fp32, groups of 2 888 -> 787, 10000 x 4000, groups of 4 615 -> 590; bf16 then, and groups of 8, only where that leaves room for more
   // CTAs or there is one anyway (bf16 5000 x 8184 648 -> 630, but 20000 x 2000 400 -> 408; groups of 8, 4 stages 6000 x 5008 970 -> 897, but
   // 3000 x 3008 249 -> 255).
-  // The pipelined kernel of groups of 4 stays ahead of it (32768 x 4096, 5 stages bf16 1738 against 1810, fp32 2140 against 2328) unless its
-  // stored states cost it a CTA (fp32, end state stored 2764 against 2195).
+  // The pipelined kernel of groups of 4 stays ahead of it (32768 x 4096, 5 stages bf16 1682 against 1810, fp32 2140 against 2328).
   if (rc == NCN_OK && bwd && !rec && (!have_pipe || best.occ < want_occ) && (!(flags & F_TAPE) || lane_ahead_tape(n, shape.ragged))) {
     // CTAs per SM that make it worth while
     const bool even = shape.ragged && want_occ > 1 && (n == 8 || (dtype == DT_BF16 && (flags & F_TAPE)));  // (no gain at as many CTAs)

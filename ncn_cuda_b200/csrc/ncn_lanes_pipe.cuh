@@ -69,9 +69,9 @@ __device__ __forceinline__ void lds32_io(bool on, uint32_t a, float& v) {
 // ---- publish: the values the neighbouring warp will want, before this set's registers are shuffled
 // UP = false: consumers take from higher blocks, so a warp publishes its FIRST k values per offset;
 // UP = true: its LAST k values.  k = o * ad (ad = |stride difference|).
-template <int NG, int NS, bool UP>
+template <int NG, int NS, bool UP, int S0 = 0>
 __device__ __forceinline__ void pipe_publish(const float2 (&V)[NS][NG], int ad, const PipeHalo& h, int lane) {
-  static_for<0, NS*(NG - 1)>([&](auto ic) {
+  static_for<S0*(NG - 1), NS*(NG - 1)>([&](auto ic) {
     constexpr int idx = decltype(ic)::value;
     constexpr int s = idx / (NG - 1), o = idx % (NG - 1) + 1;
     constexpr int OFF = idx * (int)kPipeSo;
@@ -87,10 +87,10 @@ __device__ __forceinline__ void pipe_publish(const float2 (&V)[NS][NG], int ad, 
 
 // ---- in-warp part of the shift (results for lanes whose source is in another warp are garbage
 // until pipe_fetch has run)
-template <int NG, int NS, bool UP, bool UNIT>
+template <int NG, int NS, bool UP, bool UNIT, int S0 = 0>
 __device__ __forceinline__ void pipe_shuffle(float2 (&V)[NS][NG], int ad) {
 #pragma unroll
-  for (int s = 0; s < NS; ++s) {
+  for (int s = S0; s < NS; ++s) {
 #pragma unroll
     for (int o = 1; o < NG; ++o) {
       const float2 v = V[s][o];
@@ -119,9 +119,9 @@ __device__ __forceinline__ void pipe_shuffle(float2 (&V)[NS][NG], int ad) {
 }
 
 // ---- halo part of the shift (after the barrier that follows the neighbours' pipe_publish)
-template <int NG, int NS, bool UP, bool UNIT>
+template <int NG, int NS, bool UP, bool UNIT, int S0 = 0>
 __device__ __forceinline__ void pipe_fetch(float2 (&V)[NS][NG], int ad, const PipeHalo& h, int lane) {
-  static_for<0, NS*(NG - 1)>([&](auto ic) {
+  static_for<S0*(NG - 1), NS*(NG - 1)>([&](auto ic) {
     constexpr int idx = decltype(ic)::value;
     constexpr int s = idx / (NG - 1), o = idx % (NG - 1) + 1;
     constexpr int OFF = idx * (int)kPipeSo;
@@ -148,33 +148,33 @@ __device__ __forceinline__ void pipe_fetch(float2 (&V)[NS][NG], int ad, const Pi
   });
 }
 
-// Whole shift of both sets with its own barriers (start and end of a tile, where nothing overlaps).
-template <int NG, int NS>
+// Whole shift of both sets, streams S0 .. NS-1, with its own barriers (start and end of a tile, where nothing overlaps).
+template <int NG, int NS, int S0 = 0>
 __device__ __forceinline__ void pipe_exchange_both(float2 (&VA)[NS][NG], float2 (&VB)[NS][NG], int delta, const PipeHalo& ha,
                                                    const PipeHalo& hb, int lane) {
   if (delta == 0) return;
   const int ad = delta < 0 ? -delta : delta;
   if (delta > 0) {
-    pipe_publish<NG, NS, false>(VA, ad, ha, lane);
-    pipe_publish<NG, NS, false>(VB, ad, hb, lane);
+    pipe_publish<NG, NS, false, S0>(VA, ad, ha, lane);
+    pipe_publish<NG, NS, false, S0>(VB, ad, hb, lane);
     __syncthreads();
     if (ad == 1) {
-      pipe_shuffle<NG, NS, false, true>(VA, ad); pipe_shuffle<NG, NS, false, true>(VB, ad);
-      pipe_fetch<NG, NS, false, true>(VA, ad, ha, lane); pipe_fetch<NG, NS, false, true>(VB, ad, hb, lane);
+      pipe_shuffle<NG, NS, false, true, S0>(VA, ad); pipe_shuffle<NG, NS, false, true, S0>(VB, ad);
+      pipe_fetch<NG, NS, false, true, S0>(VA, ad, ha, lane); pipe_fetch<NG, NS, false, true, S0>(VB, ad, hb, lane);
     } else {
-      pipe_shuffle<NG, NS, false, false>(VA, ad); pipe_shuffle<NG, NS, false, false>(VB, ad);
-      pipe_fetch<NG, NS, false, false>(VA, ad, ha, lane); pipe_fetch<NG, NS, false, false>(VB, ad, hb, lane);
+      pipe_shuffle<NG, NS, false, false, S0>(VA, ad); pipe_shuffle<NG, NS, false, false, S0>(VB, ad);
+      pipe_fetch<NG, NS, false, false, S0>(VA, ad, ha, lane); pipe_fetch<NG, NS, false, false, S0>(VB, ad, hb, lane);
     }
   } else {
-    pipe_publish<NG, NS, true>(VA, ad, ha, lane);
-    pipe_publish<NG, NS, true>(VB, ad, hb, lane);
+    pipe_publish<NG, NS, true, S0>(VA, ad, ha, lane);
+    pipe_publish<NG, NS, true, S0>(VB, ad, hb, lane);
     __syncthreads();
     if (ad == 1) {
-      pipe_shuffle<NG, NS, true, true>(VA, ad); pipe_shuffle<NG, NS, true, true>(VB, ad);
-      pipe_fetch<NG, NS, true, true>(VA, ad, ha, lane); pipe_fetch<NG, NS, true, true>(VB, ad, hb, lane);
+      pipe_shuffle<NG, NS, true, true, S0>(VA, ad); pipe_shuffle<NG, NS, true, true, S0>(VB, ad);
+      pipe_fetch<NG, NS, true, true, S0>(VA, ad, ha, lane); pipe_fetch<NG, NS, true, true, S0>(VB, ad, hb, lane);
     } else {
-      pipe_shuffle<NG, NS, true, false>(VA, ad); pipe_shuffle<NG, NS, true, false>(VB, ad);
-      pipe_fetch<NG, NS, true, false>(VA, ad, ha, lane); pipe_fetch<NG, NS, true, false>(VB, ad, hb, lane);
+      pipe_shuffle<NG, NS, true, false, S0>(VA, ad); pipe_shuffle<NG, NS, true, false, S0>(VB, ad);
+      pipe_fetch<NG, NS, true, false, S0>(VA, ad, ha, lane); pipe_fetch<NG, NS, true, false, S0>(VB, ad, hb, lane);
     }
   }
   __syncthreads();  // the halo may be overwritten again
@@ -373,7 +373,10 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_fwd_kernel(const LaneParams 
 // ------------------------------------------------------------------------------------------ backward
 // From the net output (reversible inverse), from stored states (checkpoints, F_TAPE), F_RESIDUAL; no
 // forward replay.
-template <int NG, int ACT, typename T, int MAXT, int MINB>
+//
+// AHEAD as in lane_bwd_kernel: the halo and the results share the tile buffer, the next tile's streams have one of their own, and stored
+// states go from global memory to x and a of a set as soon as it is done with them.
+template <int NG, int ACT, typename T, int MAXT, int MINB, int AHEAD>
 __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
@@ -392,14 +395,18 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
   const T* g_in[4] = {static_cast<const T*>(p.in[0]), static_cast<const T*>(p.in[1]), static_cast<const T*>(p.in[2]),
                       static_cast<const T*>(p.in[3])};
   const float2* ckpt = reinterpret_cast<const float2*>(p.ckpt);
-  const bool want_rec = p.out[2] != nullptr;
+  const bool want_rec = !AHEAD && p.out[2] != nullptr;
   const bool residual = (p.flags & F_RESIDUAL) != 0;
-  const bool tape = (p.flags & F_TAPE) != 0;  // the last stage's output state comes from its checkpoint
+  // the last stage's output state comes from its checkpoint
+  const bool tape = AHEAD ? AHEAD != LANE_AHEAD_OUTPUT : (p.flags & F_TAPE) != 0;
+  constexpr int Q0 = AHEAD > LANE_AHEAD_OUTPUT ? 2 : 0;  // AHEAD: native streams q >= Q0 at land + (q - Q0)*RN
+  T* const land = reinterpret_cast<T*>(smem + p.off_land);
   const long long BN = p.B * (long long)N;
   const uint32_t n_ck = p.n_ckpt_slots;
 
   if (tid == 0) {
     mbar_init(&bar[0], 1);
+    if (AHEAD) mbar_init(&bar[1], 1);  // F_RESIDUAL: dy of the tile once more, for its end
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -433,8 +440,22 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
   const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
+  auto copy_ahead = [&](long long tl) {
+    const uint32_t bytes = (uint32_t)((int)min((long long)R, p.B - tl * R) * N * sizeof(T));
+    mbar_expect_tx(&bar[0], (4 - Q0) * bytes);
+#pragma unroll
+    for (int q = Q0; q < 4; ++q) bulk_g2s(land + (q - Q0) * RN, g_in[q] + tl * R * N, bytes, &bar[0]);
+  };
+  if (AHEAD && tid == 0) copy_ahead(blockIdx.x);  // (there is a tile for every CTA)
+
   for (long long tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
-    if (tid == 0) {
+    if constexpr (AHEAD) {
+      if (tid == 0 && residual) {
+        const uint32_t bytes = (uint32_t)((int)min((long long)R, p.B - tile * R) * N * sizeof(T));
+        mbar_expect_tx(&bar[1], bytes);
+        bulk_g2s(sdy, g_in[2] + tile * R * N, bytes, &bar[1]);
+      }
+    } else if (tid == 0) {
       bulk_wait_read0();  // the previous tile's stores have left the buffer
       issue_load(tile);
     }
@@ -456,22 +477,34 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
 #pragma unroll
       for (int s = 0; s < 4; ++s)
         if (s >= 2 || !tape) {
-          pipe_ld_native<NG, T>(win + s * RN + chunkA, VA[s], t);
-          pipe_ld_native<NG, T>(win + s * RN + chunkA + NH, VB[s], t);
+          const T* c = (AHEAD ? land - Q0 * RN : win) + s * RN + chunkA;
+          pipe_ld_native<NG, T>(c, VA[s], t);
+          pipe_ld_native<NG, T>(c + NH, VB[s], t);
         }
     }
+    if (AHEAD && tid == 0) bulk_wait_read0();  // the previous tile's stores have left the buffer
     __syncthreads();  // native inputs are in registers; the buffer now serves as halo
-    if (tid == 0 && tile + gridDim.x < p.tiles) {  // next tile towards L2 while this one is worked on
+    if (tid == 0 && tile + gridDim.x < p.tiles) {  // next tile into its buffer or towards L2 while this one is worked on
+      if (AHEAD) copy_ahead(tile + gridDim.x);
       const long long nrow0 = (tile + gridDim.x) * R;
       const int nrows = (int)min((long long)R, p.B - nrow0);
       const uint32_t bytes = (uint32_t)(nrows * N * sizeof(T));
 #pragma unroll
       for (int q = 0; q < 4; ++q)
-        if (q >= 2 || !tape) l2_prefetch(g_in[q] + nrow0 * N, bytes);
+        if (!AHEAD && (q >= 2 || !tape)) l2_prefetch(g_in[q] + nrow0 * N, bytes);
       for (uint32_t k = 0; k < n_ck; ++k) l2_prefetch(ckpt + (long long)k * BN + nrow0 * N, (uint32_t)(nrows * N * sizeof(float2)));
     }
 
     auto load_ckpt = [&](float2 (&V)[4][NG], int ck, int set) {  // a state saved after a stage replaces the rebuilt one
+      if (AHEAD) {
+        if (!active) return;
+        const float2* c = ckpt + (long long)ck * BN + (row0 + r) * N + set * TPR + t;
+#pragma unroll
+        for (int s = 0; s < 2; ++s)
+#pragma unroll
+          for (int o = 0; o < NG; ++o) V[s][o] = __ldg(c + (s * NG + o) * (2 * TPR));
+        return;
+      }
       const float2* c = sck + ck * RN + r * N + set * TPR + t;
 #pragma unroll
       for (int s = 0; s < 2; ++s)
@@ -492,9 +525,10 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
 
     // ---- into the last stage's arrangement, then set A runs half a stage ahead of set B
     StageRec rec = recs[L - 1];
-    pipe_exchange_both<NG, 4>(VA, VB, rec.s, ha, hb, lane);
+    if (AHEAD && tape) { load_ckpt(VA, rec.ck, 0); load_ckpt(VB, rec.ck, 1); }
+    pipe_exchange_both<NG, 4, Q0>(VA, VB, rec.s, ha, hb, lane);
     set_w(rec);
-    if (rec.ck >= 0) { load_ckpt(VA, rec.ck, 0); load_ckpt(VB, rec.ck, 1); }
+    if (!AHEAD && rec.ck >= 0) { load_ckpt(VA, rec.ck, 0); load_ckpt(VB, rec.ck, 1); }
     float2 dwi = f2(0.0f), dwj = f2(0.0f);
     lane_backward<NG, ACT>(VA[0], VA[1], VA[2], VA[3], w, dwi, dwj);
     for (int l = L - 1; l > 0; --l) {
@@ -502,32 +536,40 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
       const int ad = rec.s - nxt.s;  // strides shrink: shifts towards lower blocks
       // One compile-time variant per kind of shift, each holding the exchange AND the arithmetic, so
       // that the two stay in one basic block.
-      auto stage = [&](auto unit_tag) {
+      auto stage = [&](auto unit_tag, auto state_tag) {
         constexpr bool UNIT = decltype(unit_tag)::value;
+        constexpr int S0 = decltype(state_tag)::value ? 2 : 0;  // a stored state replaces x, a
         // block A: A leaves stage l; B computes stage l
-        pipe_publish<NG, 4, true>(VA, ad, ha, lane);
-        pipe_shuffle<NG, 4, true, UNIT>(VA, ad);
+        if (S0) load_ckpt(VA, nxt.ck, 0);
+        pipe_publish<NG, 4, true, S0>(VA, ad, ha, lane);
+        pipe_shuffle<NG, 4, true, UNIT, S0>(VA, ad);
         lane_backward<NG, ACT>(VB[0], VB[1], VB[2], VB[3], w, dwi, dwj);
+        if (S0) load_ckpt(VB, nxt.ck, 1);
         reduce_dw(dwi, dwj, l);
-        pipe_publish<NG, 4, true>(VB, ad, hb, lane);
+        pipe_publish<NG, 4, true, S0>(VB, ad, hb, lane);
         __syncthreads();
         // block B: A enters stage l - 1; B leaves stage l
         set_w(nxt);
         dwi = f2(0.0f); dwj = f2(0.0f);
-        pipe_fetch<NG, 4, true, UNIT>(VA, ad, ha, lane);
-        if (nxt.ck >= 0) load_ckpt(VA, nxt.ck, 0);
-        pipe_shuffle<NG, 4, true, UNIT>(VB, ad);
+        pipe_fetch<NG, 4, true, UNIT, S0>(VA, ad, ha, lane);
+        if (!AHEAD && nxt.ck >= 0) load_ckpt(VA, nxt.ck, 0);
+        pipe_shuffle<NG, 4, true, UNIT, S0>(VB, ad);
         lane_backward<NG, ACT>(VA[0], VA[1], VA[2], VA[3], w, dwi, dwj);
-        pipe_fetch<NG, 4, true, UNIT>(VB, ad, hb, lane);
-        if (nxt.ck >= 0) load_ckpt(VB, nxt.ck, 1);
+        pipe_fetch<NG, 4, true, UNIT, S0>(VB, ad, hb, lane);
+        if (!AHEAD && nxt.ck >= 0) load_ckpt(VB, nxt.ck, 1);
         __syncthreads();
       };
-      if (ad == 1) stage(std::true_type{}); else stage(std::false_type{});
+      if (AHEAD && AHEAD != LANE_AHEAD_TAPE && nxt.ck >= 0) {
+        if (ad == 1) stage(std::true_type{}, std::true_type{}); else stage(std::false_type{}, std::true_type{});
+      } else {
+        if (ad == 1) stage(std::true_type{}, std::false_type{}); else stage(std::false_type{}, std::false_type{});
+      }
       rec = nxt;
     }
     lane_backward<NG, ACT>(VB[0], VB[1], VB[2], VB[3], w, dwi, dwj);
     reduce_dw(dwi, dwj, 0);
-    pipe_exchange_both<NG, 4>(VA, VB, -rec.s, ha, hb, lane);  // back to stride 0 = native order
+    pipe_exchange_both<NG, 4, AHEAD ? 2 : 0>(VA, VB, -rec.s, ha, hb, lane);  // back to stride 0 = native order
+    if (AHEAD && residual && !mbar_wait_bounded(&bar[1], phase ^ 1)) *abort_flag = 1;  // (seen at the next tile)
     if (active) {
       if (residual) {
         float2 gin[NG];
