@@ -90,9 +90,6 @@ __global__ void __launch_bounds__(THREADS, MINB) step_kernel(float* out, int ite
     }
   PairWB w;
   w.owi = f2(0.003f * wsc); w.owj = f2(-0.002f * wsc); w.owjs = f2(-0.002f * 2.885f * wsc); w.alpha = f2(0.9f); w.oma = f2(0.1f);
-  LaneWB<ACT> wl;
-  wl.alpha = f2(0.9f);
-  wl.stage(0.003f * wsc, -0.002f * wsc);
   PairW wf;
   wf.owi = f2(0.003f * wsc); wf.owj = f2(-0.002f * wsc); wf.alpha = f2(0.9f * 2.885f);
   float2 dwi = f2(0.f), dwj = f2(0.f);
@@ -100,7 +97,7 @@ __global__ void __launch_bounds__(THREADS, MINB) step_kernel(float* out, int ite
     for (int l = L - 1; l >= 0; --l) {
 #pragma unroll
       for (int p = 0; p < PAIRS; p++) {
-        if (VAR == 0) lane_backward<NG, ACT>(X[p], A[p], H[p], G[p], wl, dwi, dwj);
+        if (VAR == 0) lane_backward<NG, ACT>(X[p], A[p], H[p], G[p], w, dwi, dwj);
         if (VAR == 1) pair_backward<NG, ACT>(X[p], A[p], H[p], G[p], w, dwi, dwj);
         if (VAR == 2) lane_forward<NG, ACT>(X[p], A[p], wf);
         if (VAR == 3) pair_forward<NG, ACT>(X[p], A[p], wf);

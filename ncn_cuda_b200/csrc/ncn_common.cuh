@@ -386,12 +386,14 @@ struct ActForm<ACT_LINEAR> {
 // r = 1 / (1 + 2^ts) for all N values of an array at once (the positions of a group, or the features of a
 // position).
 // BATCH: reciprocals taken from one special-function reciprocal of the product of BATCH values
-// (4: 1.25, 2: 1.5 special-function instructions per position and step, one each 2; the smaller the batch
-// the fewer multiplies on the FMA pipe, and one each, ActForm::r, needs no cap).
+// (4: 1.25, 2: 1.5 special-function instructions per position and step; the smaller the batch
+// the fewer multiplies on the FMA pipe).
 // The exponent is capped at 30: beyond it r < 1e-9 (tanh = 1 to the last bit) and the product of four d stays a normal
 // fp32 number, as does its reciprocal.  A NaN reaches all values that share its reciprocal.  These would see it all the same
-// where they are the features of one position, through their dot product.  They would not in the forward steps of a group's
-// positions: a row with a NaN is taken again there (ncn_terms.cuh).
+// where they are the features of one position, through their dot product, and in the reverse sweep, where the sums for gx_j
+// bring a NaN in any x of a group to all of its cotangents (and to its rebuilt a; of the rebuilt x, those that share may have one
+// that a step of their own would not give, where an output holds a NaN that no forward leaves: in position 0 alone).  They would
+// not in the forward steps of a group's positions: a row with a NaN is taken again there (ncn_terms.cuh).
 template <int ACT, int NG, int BATCH>
 __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG]) {
   if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {

@@ -14,9 +14,9 @@
 //     the tile buffer (write, barrier, read at the shifted index).
 //   * Rows arrive and leave by 1-D TMA bulk copies through ONE tile buffer in native layout, which
 //     is idle while the stages run; a thread's G groups are G n contiguous positions at stride 0.
-//   * tanh / sigmoid need r = 1 / (1 + 2^t) per position and step.  The forward takes the n reciprocals of
-//     a group four at a time from ONE special-function reciprocal of their product (Montgomery's
-//     trick): 1.25 instead of 2 special-function instructions per position and step.  The backward takes one each.
+//   * tanh / sigmoid need r = 1 / (1 + 2^t) per position and step.  The n reciprocals of a group are
+//     taken four at a time from ONE special-function reciprocal of their product (Montgomery's
+//     trick): 1.25 instead of 2 special-function instructions per position and step.
 //
 // Two forms of each kernel: rows of a power of two of blocks that fill their warps, and any even number of blocks (RAG):
 // the last lanes of a warp may then hold nothing, and the length of a warp's share is a run-time value.
@@ -61,6 +61,19 @@ __device__ __forceinline__ void lds32_if(bool on, uint32_t a, float& v) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %2, 0;\n\t@p ld.shared.f32 %0, [%1];\n\t}" : "+f"(v) : "r"(a), "r"((int)on) : "memory");
 }
 
+// ------------------------------------------------------------------ activation, all positions of a group at once
+// Measured on the arithmetic alone (microbench.cu): the forward is bound by the special-function pipe
+// and wants the largest batch; the backward is bound by the FMA pipe, where groups of 8 do better
+// with batches of two (17.3 against 18.5 cycles per warp.position.step), groups of 4 with four.
+// One reciprocal per position would be faster in the backward of groups of 2 and 4 (32768 x 4096, groups of 4, 6 stages 2652 -> 2560 us),
+// but the walk back then no longer rounds as the forward did, and the two errors no longer cancel: dx further from fp64 in each of
+// 16 seeds, by 0.1 to 0.2 % where no walk exceeds 16 steps and by 1.2 % over 24.
+template <int NG>
+struct LaneBatch {
+  static constexpr int fwd = 4;
+  static constexpr int bwd = NG >= 8 ? 2 : 4;
+};
+
 // ------------------------------------------------------------------ step math (scaled variables of ncn_common.cuh)
 // The constants of a forward stage and those that undo it.
 template <int NG, int ACT>
@@ -94,7 +107,7 @@ struct LFwdSteps {
     float2 ts[NG], r[NG];
 #pragma unroll
     for (int i = 0; i < NG; ++i) ts[i] = ffma2(X[i], P, Q);
-    act_r_all<ACT, NG, 4>(ts, r);  // (two at a time: 65536 x 4096, groups of 4 3005 -> 3178 us, the special-function pipe)
+    act_r_all<ACT, NG, LaneBatch<NG>::fwd>(ts, r);
 #pragma unroll
     for (int i = 0; i < NG; ++i) {
       A[i] = ffma2(r[i], f2(cA), A[i]);
@@ -120,33 +133,13 @@ __device__ __forceinline__ void lane_forward(float2 (&X)[NG], float2 (&A)[NG], c
   }
 }
 
-// What a stage of the reverse sweep reads.  (kph folded into owi and alpha as well would save one more multiplication per step, but
-// the rounding of alpha kph comes back in every step the same way: dx 5 to 9 % further from fp64.)
-template <int ACT>
-struct LaneWB {
-  static constexpr float kph = (float)(kCd * ActForm<ACT>::ds / kMd), sT = (float)ActForm<ACT>::sT;  // kph = c ds / m
-  float2 owi, alpha;  // (1-alpha) wi, alpha
-  float2 hj, sj;      // 2 kph (1-alpha) wj, sT (1-alpha) wj
-  __device__ __forceinline__ void stage(float owi_, float owj) {
-    owi = f2(owi_);
-    hj = f2(owj * 2.0f * kph);
-    sj = f2(owj * sT);
-  }
-};
-
 // Reverse sweep as PBwdSteps (ncn_pairs.cuh) with the per-step scalars cut down: the sums for gx_j
 // and the weight gradients stay in raw units (dwi_raw = sum xj (aI + DX aS), dwj_raw = sum m^k xj^2 aS)
 // and take their constant factors once per stage.
-// One special-function reciprocal per position: the FMA pipe (a packed FMA of three registers takes 3.5 cycles, one with a
-// constant 2.2) is what the reverse sweep is short of, and sharing costs 2.25 multiplications and a cap each.  Backward, us,
-// reciprocals by fours (groups of 8: twos) -> one each, and the constants of gx_j in the weights: 65536 x 4096, groups of 4, 6 stages
-// 5207 -> 4980; 32768 x 4096, groups of 8 from the output, 4 stages 2972 -> 2892; 65536 x 1024, groups of 2, 9 stages 1362 -> 1273;
-// 20000 x 3000 (ragged), groups of 4, 5 stages 1278 -> 1199; 8192 x 8192, groups of 8, 3 stages 1311 -> 1306.  (Two of four by twos
-// 5147, all by twos 5097.)
 template <int NG, int ACT, int J>
 struct LBwdSteps {
   static __device__ __forceinline__ void run(float2 (&X)[NG], float2 (&A)[NG], float2 (&H)[NG], float2 (&G)[NG],
-                                             const LaneWB<ACT>& w, float2& dwi, float2& dwj) {
+                                             const PairWB& w, float2& dwi, float2& dwj) {
     using F = ActForm<ACT>;
     constexpr int k = NG - 1 - J;
     constexpr double mkd = cpow(kMd, k);
@@ -155,7 +148,9 @@ struct LBwdSteps {
     constexpr float imk1DX1 = (float)(bwd_DX(k + 1, F::f0) / cpow(kMd, k + 1));
     constexpr float cAr = (float)LaneStage<NG, ACT>::cAr(J);
     constexpr float sTimk1 = (float)(F::sT / cpow(kMd, k + 1));
-    constexpr float K1 = (float)(kCd * F::ds / kMd / cpow(kMd, k + 1));  // kph / m^(k+1)
+    constexpr float cdsm = (float)(kCd * F::ds / kMd);
+    constexpr float K1 = (float)(kCd * F::ds / kMd / cpow(kMd, k + 1));  // c ds / m^(k+2)
+    constexpr float twomk1 = (float)(2.0 * cpow(kMd, k + 1));
     constexpr float mk = (float)mkd;
 #pragma unroll
     for (int i = 0; i < NG; ++i) X[i] = ffma2(f2(-kC), A[i], X[i]);
@@ -163,15 +158,14 @@ struct LBwdSteps {
     if constexpr (imk1DX1 != 0.0f) xj = ffma2(X[J], f2(imk1), f2(imk1DX1)); else xj = fmul2(X[J], f2(imk1));
     const float2 pp = ffma2(w.owi, xj, w.alpha);  // p = alpha + (1-alpha) wi xj
     const float2 Ps = fmul2(pp, f2(sTimk1));
-    const float2 q0 = fmul2(fmul2(w.sj, xj), xj);
+    const float2 q0 = fmul2(fmul2(w.owjs, xj), xj);
     float2 Qs;
     if constexpr (DX1 != 0.0f) Qs = ffma2(Ps, f2(DX1), q0); else Qs = q0;
-    const float2 PH = fmul2(pp, f2(w.kph));
+    const float2 PH = fmul2(pp, f2(cdsm));
     float2 ts[NG], r[NG];
 #pragma unroll
     for (int i = 0; i < NG; ++i) ts[i] = ffma2(X[i], Ps, Qs);
-#pragma unroll
-    for (int i = 0; i < NG; ++i) r[i] = F::r(ts[i]);
+    act_r_all<ACT, NG, LaneBatch<NG>::bwd>(ts, r);
     float2 aI, aS;  // sums over the group's positions; the first term starts them (no zeroing, no add to zero)
 #pragma unroll
     for (int i = 0; i < NG; ++i) {
@@ -188,10 +182,11 @@ struct LBwdSteps {
       }
     }
     float2 u;
-    if constexpr (DX1 != 0.0f) u = ffma2(f2(DX1), aS, aI); else u = aI;  // sum gT x_i = kph u
-    const float2 v = fmul2(xj, aS);                                       // xj sum gT = kph m^(k+1) v
+    if constexpr (DX1 != 0.0f) u = ffma2(f2(DX1), aS, aI); else u = aI;  // sum gT x_i = (c ds / m) u
+    const float2 v = fmul2(xj, aS);                                       // xj sum gT = c ds m^k v
     // gx_j += (1-alpha) (wi sum gT x + 2 wj xj sum gT), in units of m^(k+1)
-    H[J] = ffma2(fmul2(w.owi, f2(K1)), u, ffma2(w.hj, v, H[J]));
+    const float2 t3 = ffma2(fmul2(w.owj, v), f2(twomk1), fmul2(w.owi, u));
+    H[J] = ffma2(t3, f2(K1), H[J]);
     dwi = ffma2(xj, u, dwi);
     dwj = ffma2(fmul2(xj, v), f2(mk), dwj);
     LBwdSteps<NG, ACT, J - 1>::run(X, A, H, G, w, dwi, dwj);
@@ -200,13 +195,13 @@ struct LBwdSteps {
 template <int NG, int ACT>
 struct LBwdSteps<NG, ACT, -1> {
   static __device__ __forceinline__ void run(float2 (&)[NG], float2 (&)[NG], float2 (&)[NG], float2 (&)[NG],
-                                             const LaneWB<ACT>&, float2&, float2&) {}
+                                             const PairWB&, float2&, float2&) {}
 };
 
 // dwi / dwj gain the RAW sums; their factors are lane_dw_scale_i/j below.
 template <int NG, int ACT>
 __device__ __forceinline__ void lane_backward(float2 (&X)[NG], float2 (&A)[NG], float2 (&H)[NG], float2 (&G)[NG],
-                                              const LaneWB<ACT>& w, float2& dwi, float2& dwj) {
+                                              const PairWB& w, float2& dwi, float2& dwj) {
   using F = ActForm<ACT>;
   LBwdSteps<NG, ACT, NG - 1>::run(X, A, H, G, w, dwi, dwj);
   using S = LaneStage<NG, ACT>;
@@ -833,8 +828,10 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
   const uint32_t xrow = smem_u32(smem + p.off_work) + (uint32_t)r * (uint32_t)(4 * N) * 4u;  // fp32 [4][NG][m] per row
   const LaneShare<G, RAG> sh(t, lane, wr, wpr, p.thr, m);
   const int chunk = r * N + sh.blk * NG;
-  LaneWB<ACT> w;
+  constexpr float sT = (float)F::sT;
+  PairWB w;
   w.alpha = f2(p.alpha);
+  w.oma = f2(p.oma);
   const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
@@ -927,7 +924,9 @@ __global__ void __launch_bounds__(MAXT, MINB) lane_bwd_kernel(const LaneParams p
       if (INNER && rec.ck >= 0) lane_exchange<NG, G, 4, RAG, 2>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, sh, m);  // (x, a are in place)
       else lane_exchange<NG, G, 4, RAG>(V, rec.s - s_cur, p.ea_max, halo, lane, xrow, sh, m);
       s_cur = rec.s;
-      w.stage(rec.owi, rec.owj);
+      w.owi = f2(rec.owi);
+      w.owj = f2(rec.owj);
+      w.owjs = f2(rec.owj * sT);
       if (!AHEAD && rec.ck >= 0) {  // a state saved after stage l replaces the rebuilt one
         const float2* c = sck + rec.ck * RN + r * N + (sh.blk >> 1);
 #pragma unroll

@@ -435,8 +435,10 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
   pipe_halo_init(ha, smem_u32(smem + p.off_work), p.halo_warp_bytes, wr, 2 * wpr, r * 2 * wpr, lane);
   pipe_halo_init(hb, smem_u32(smem + p.off_work), p.halo_warp_bytes, wpr + wr, 2 * wpr, r * 2 * wpr, lane);
   const int chunkA = r * N + t * (2 * NG);
-  LaneWB<ACT> w;
+  constexpr float sT = (float)F::sT;
+  PairWB w;
   w.alpha = f2(p.alpha);
+  w.oma = f2(p.oma);
   const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
@@ -511,7 +513,11 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
 #pragma unroll
         for (int o = 0; o < NG; ++o) V[s][o] = c[(s * NG + o) * (2 * TPR)];
     };
-    auto set_w = [&](const StageRec& rc) { w.stage(rc.owi, rc.owj); };
+    auto set_w = [&](const StageRec& rc) {
+      w.owi = f2(rc.owi);
+      w.owj = f2(rc.owj);
+      w.owjs = f2(rc.owj * sT);
+    };
     auto reduce_dw = [&](float2 dwi, float2 dwj, int l) {  // fixed-order warp tree, one slot per warp and stage
       const float di = (dwi.x + dwi.y) * dsi, dj = (dwj.x + dwj.y) * dsj;
       const bool hi = (lane & 16) != 0;

@@ -56,47 +56,28 @@ struct SoloFwd<NG, ACT, NG> {
   static __device__ __forceinline__ void run(float2 (&)[NG / 2], float2 (&)[NG / 2], float, float, float) {}
 };
 
-// Reciprocals of the reverse sweep: half of the pairs share by twos, the others take one each, which keeps the FMA pipe and the
-// special-function pipe equally busy.  Backward of fp32, groups of 16, 3 stages, us, all by twos / half / one each: 25000 x 2048
-// 1660 / 1604 / 1585; 8192 x 6000 1736 / 1702 / 1752; 8192 x 8192 2157 / 2128 / 2190 (one CTA of 512 threads per SM: its warps come to
-// the special-function pipe together).
-template <int ACT, int NP>
-__device__ __forceinline__ void solo_r_bwd(const float2 (&ts)[NP], float2 (&r)[NP]) {
-  constexpr int SH = ACT == ACT_TANH || ACT == ACT_SIGMOID ? NP / 2 : 0;
-  if constexpr (SH > 0) {
-    float2 t[SH], q[SH];
-#pragma unroll
-    for (int i = 0; i < SH; ++i) t[i] = ts[i];
-    act_r_all<ACT, SH, 2>(t, q);
-#pragma unroll
-    for (int i = 0; i < SH; ++i) r[i] = q[i];
-  }
-#pragma unroll
-  for (int i = SH; i < NP; ++i) r[i] = ActForm<ACT>::r(ts[i]);
-}
-
 template <int NG, int ACT, int J>
 struct SoloBwd {
   static __device__ __forceinline__ void run(float2 (&X)[NG / 2], float2 (&A)[NG / 2], float2 (&H)[NG / 2], float2 (&G)[NG / 2],
-                                             float owi, float alpha, float hj, float sj, float& dwi, float& dwj) {
+                                             float owi, float owj, float owjs, float alpha, float& dwi, float& dwj) {
     using F = ActForm<ACT>;
     using S = LaneStage<NG, ACT>;
     constexpr int k = NG - 1 - J;
     constexpr double mkd = cpow(kMd, k), DX = bwd_DX(k + 1, F::f0);
     constexpr float imk1 = (float)(1.0 / cpow(kMd, k + 1)), DX1 = (float)DX, imk1DX1 = (float)(DX / cpow(kMd, k + 1));
     constexpr float cAr = (float)S::cAr(J);
-    constexpr float sTimk1 = (float)(F::sT / cpow(kMd, k + 1));
-    constexpr float K1 = (float)(kCd * F::ds / kMd / cpow(kMd, k + 1));  // kph / m^(k+1)
+    constexpr float sTimk1 = (float)(F::sT / cpow(kMd, k + 1)), cdsm = (float)(kCd * F::ds / kMd);
+    constexpr float K1 = (float)(kCd * F::ds / kMd / cpow(kMd, k + 1)), K2 = (float)(2.0 * kCd * F::ds / kMd);
 #pragma unroll
     for (int i = 0; i < NG / 2; ++i) X[i] = __ffma2_rn(f2(-kC), A[i], X[i]);
     const float XJ = (J & 1) ? X[J / 2].y : X[J / 2].x;
     const float xj = fmaf(XJ, imk1, imk1DX1);
     const float pp = fmaf(owi, xj, alpha), ps = pp * sTimk1;
-    const float2 Ps = f2(ps), Qs = f2(fmaf(ps, DX1, (sj * xj) * xj)), PH = f2(pp * LaneWB<ACT>::kph);
+    const float2 Ps = f2(ps), Qs = f2(fmaf(ps, DX1, (owjs * xj) * xj)), PH = f2(pp * cdsm);
     float2 ts[NG / 2], r[NG / 2], aI, aS;
 #pragma unroll
     for (int i = 0; i < NG / 2; ++i) ts[i] = __ffma2_rn(X[i], Ps, Qs);
-    solo_r_bwd<ACT, NG / 2>(ts, r);
+    act_r_all<ACT, NG / 2, 2>(ts, r);
 #pragma unroll
     for (int i = 0; i < NG / 2; ++i) {
       A[i] = __ffma2_rn(r[i], f2(cAr), A[i]);
@@ -108,11 +89,11 @@ struct SoloBwd {
     }
     // sums in raw units (as LBwdSteps): dwi gains xj u, dwj m^k xj v; their factors are lane_dw_scale_i / _j
     const float sS = aS.x + aS.y, u = fmaf(DX1, sS, aI.x + aI.y), v = xj * sS;
-    const float add = fmaf(owi * K1, u, hj * v);
+    const float add = fmaf(owj * v, K2, (owi * u) * K1);
     if (J & 1) H[J / 2].y += add; else H[J / 2].x += add;
     dwi = fmaf(xj, u, dwi);
     dwj = fmaf(xj * v, (float)mkd, dwj);
-    SoloBwd<NG, ACT, J - 1>::run(X, A, H, G, owi, alpha, hj, sj, dwi, dwj);
+    SoloBwd<NG, ACT, J - 1>::run(X, A, H, G, owi, owj, owjs, alpha, dwi, dwj);
   }
 };
 template <int NG, int ACT>
@@ -335,7 +316,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
   const int r = tid / m, g = tid - r * m;
   const int base = r * N;
   const uint32_t row = smem_u32(smem) + 16u * (uint32_t)base;
-  constexpr float sT = (float)F::sT, kph = LaneWB<ACT>::kph;  // factors of the weights as in LaneWB
+  constexpr float sT = (float)F::sT;
   const float dsi = lane_dw_scale_i<ACT>(p.oma), dsj = lane_dw_scale_j<ACT>(p.oma);
   uint32_t phase = 0;
 
@@ -445,7 +426,7 @@ __global__ void __launch_bounds__(MAXT, MINB) solo_bwd_kernel(const SoloParams p
       // a state saved after stage l replaces the rebuilt one
       if (rec.ck >= 0 && active && (AHEAD != SOLO_AHEAD_TAPE || l < L - 1)) load_state(tile, rec.ck);
       float dwi = 0.0f, dwj = 0.0f;
-      SoloBwd<NG, ACT, NG - 1>::run(X, A, H, G, rec.owi, p.alpha, rec.owj * 2.0f * kph, rec.owj * sT, dwi, dwj);
+      SoloBwd<NG, ACT, NG - 1>::run(X, A, H, G, rec.owi, rec.owj, rec.owj * sT, p.alpha, dwi, dwj);
 #pragma unroll
       for (int i = 0; i < NG / 2; ++i) {
         X[i] = __ffma2_rn(X[i], f2((float)S::imN), f2((float)S::imNDX));
