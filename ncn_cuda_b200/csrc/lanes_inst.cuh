@@ -23,7 +23,7 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
 #ifdef NCN_BWD
 #if NCN_NG == 4
   if (p.pipelined) {  // two half-rows per thread, half a stage apart (ncn_lanes_pipe.cuh)
-    static SmemGrant granted_p[4];
+    static SmemGrant granted_p[5];
     auto go = [&](auto kp, SmemGrant& granted) {
       cudaError_t ep = grant_smem(granted, kp, smem);
       if (ep != cudaSuccess) return ep;
@@ -35,6 +35,7 @@ static cudaError_t launch_one(const LaneParams& p, int grid, int threads, size_t
       case LANE_AHEAD_OUTPUT: return NCN_PIPE(LANE_AHEAD_OUTPUT);
       case LANE_AHEAD_TAPE: return NCN_PIPE(LANE_AHEAD_TAPE);
       case LANE_AHEAD_TAPES: return NCN_PIPE(LANE_AHEAD_TAPES);
+      case LANE_STATES_GLOBAL: return NCN_PIPE(LANE_STATES_GLOBAL);
       default: return NCN_PIPE(LANE_AHEAD_NONE);
     }
 #undef NCN_PIPE

@@ -539,15 +539,16 @@ static bool lanep_layout(bool bwd, int N, int L, int dtype, int flags, int n_ck,
   const uint64_t RN = (uint64_t)R * N;
   const int threads = R * tpr;
   const int warps = threads / 32;
+  const bool fetch = ahead != LANE_AHEAD_NONE && ahead != LANE_STATES_GLOBAL;
   pl.halo_warp_bytes = NS * 3 * kPipeSo;  // a region of kPipeSo bytes per (stream, offset): enough for shifts of 3 * 2^4 blocks
-  uint64_t work = (ahead ? 2 : NS) * RN * w;
+  uint64_t work = (fetch ? 2 : NS) * RN * w;
   const uint64_t halo = (uint64_t)2 * warps * pl.halo_warp_bytes;  // two half-row "warps" per warp
   if (halo > work) work = halo;
   uint64_t off = 0;
   auto take = [&](uint64_t bytes) { uint64_t o = off; off = (off + bytes + 127) / 128 * 128; return (uint32_t)o; };
   pl.off_work = take(work);
   pl.off_halo = pl.off_work;
-  pl.off_land = ahead ? take((ahead == LANE_AHEAD_OUTPUT ? 4 : 2) * RN * w) : pl.off_work;
+  pl.off_land = fetch ? take((ahead == LANE_AHEAD_OUTPUT ? 4 : 2) * RN * w) : pl.off_work;
   pl.off_res = residual ? take(RN * w) : pl.off_work;
   pl.off_ckpt = take(bwd && n_ck && !ahead ? (uint64_t)n_ck * RN * 8 : 16);  // (the forward stores its states straight to global memory)
   pl.off_red = take((uint64_t)2 * L * warps * 4);
@@ -620,10 +621,12 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
     // The inputs a tile ahead, us without -> with: 32768 x 4096, 5 stages bf16 1738 -> 1682, fp32 from the output alone 2091 -> 2047; 16384 x 8192,
     // 4 stages fp32 1948 -> 1840, bf16 1565 -> 1433.  Where states are stored inside a net and no CTA per SM is won by it, the copies of a
     // stage with and without one cost what the rest wins (65536 x 4096, 6 stages 4976 either way; 4096 x 1024 103 -> 105).
-    const int fetch = !bwd || rec ? LANE_AHEAD_NONE : !(flags & F_TAPE) ? LANE_AHEAD_OUTPUT : n_ck > 1 ? LANE_AHEAD_TAPES : LANE_AHEAD_TAPE;
+    // rec: a forward that stored states counts on this family wherever the plan without rec is of it.  The states in global memory take
+    // no more room than the forms that fetch ahead, so that there is a plan with rec too.
+    const int fetch = !bwd || (rec && n_ck == 0) ? LANE_AHEAD_NONE : rec ? LANE_STATES_GLOBAL : !(flags & F_TAPE) ? LANE_AHEAD_OUTPUT : n_ck > 1 ? LANE_AHEAD_TAPES : LANE_AHEAD_TAPE;
     for (const int ahead : {(int)LANE_AHEAD_NONE, fetch}) {
       LanePlan trial;
-      if (have_pipe && ahead == LANE_AHEAD_NONE) break;
+      if (have_pipe && (ahead == LANE_AHEAD_NONE || ahead == LANE_STATES_GLOBAL)) break;
       if (!lanep_layout(bwd, (int)N, L, dtype, flags, n_ck, R, tpr, e_need, ahead, (uint32_t)dev.smem_optin, trial)) continue;
       int occ = 0;
       LaneParams dummy{};
@@ -1429,6 +1432,11 @@ static int net_bwd_impl(const void* s0, const void* s1, const void* dy, const vo
     bool lanes = plan_lanes(true, B, N, E, n_cache, n_head, first_module, L, dtype, flags, n_ck, x_rec != nullptr, dev, act, lp) == NCN_OK;
     if (lanes && n_ck > 0)
       lanes = plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, false, dev, act, lf) == NCN_OK;
+    // (states that a forward wrote in this family's order are never read in another)
+    if (!lanes && n_ck > 0 && x_rec != nullptr &&
+        plan_lanes(true, B, N, E, n_cache, n_head, first_module, L, dtype, flags, n_ck, false, dev, act, lp) == NCN_OK &&
+        plan_lanes(false, B, N, E, n_cache, n_head, first_module, L, dtype, flags, 0, false, dev, act, lf) == NCN_OK)
+      return NCN_ERR_SMEM;
     if (lanes) {
       if (lp.ragged || lp.tpr > kLaneThreads) {
         if ((rc = fit_grid(lp.grid)) != NCN_OK) return rc;

@@ -30,8 +30,9 @@ struct LaneParams {
 };
 
 // Backward: what is fetched a tile ahead (lane_bwd_kernel): nothing; all four streams; with F_TAPE dy, dya and the last state, which is
-// the only stored one; the same with others behind it.
-enum LaneAhead : int { LANE_AHEAD_NONE = 0, LANE_AHEAD_OUTPUT = 1, LANE_AHEAD_TAPE = 2, LANE_AHEAD_TAPES = 3 };
+// the only stored one; the same with others behind it.  LANE_STATES_GLOBAL (lanep_bwd_kernel): nothing, but stored states are read from
+// global memory as in the last three, for a backward that is asked for the rebuilt input where shared memory does not hold them all.
+enum LaneAhead : int { LANE_AHEAD_NONE = 0, LANE_AHEAD_OUTPUT = 1, LANE_AHEAD_TAPE = 2, LANE_AHEAD_TAPES = 3, LANE_STATES_GLOBAL = 4 };
 // Ragged groups of 8 have neither of the last two: ptxas 12.9 fails on them (a segmentation fault).
 constexpr bool lane_ahead_tape(int ng, bool ragged) { return !(ragged && ng == 8); }
 

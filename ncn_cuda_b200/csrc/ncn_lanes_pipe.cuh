@@ -374,13 +374,16 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_fwd_kernel(const LaneParams 
 // From the net output (reversible inverse), from stored states (checkpoints, F_TAPE), F_RESIDUAL; no
 // forward replay.
 //
-// AHEAD as in lane_bwd_kernel: the halo and the results share the tile buffer, the next tile's streams have one of their own, and stored
-// states go from global memory to x and a of a set as soon as it is done with them.
-template <int NG, int ACT, typename T, int MAXT, int MINB, int AHEAD>
+// FORM (LaneAhead) as in lane_bwd_kernel: the halo and the results share the tile buffer, the next tile's streams have one of their own, and stored
+// states go from global memory to x and a of a set as soon as it is done with them.  LANE_STATES_GLOBAL: as the plain form, but for where
+// the states are read.
+template <int NG, int ACT, typename T, int MAXT, int MINB, int FORM>
 __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   using F = ActForm<ACT>;
   static_assert(NG == 4, "two sets of one register pair per offset");
+  constexpr bool GLOBAL = FORM != LANE_AHEAD_NONE;                         // stored states are read from global memory
+  constexpr int AHEAD = FORM == LANE_STATES_GLOBAL ? LANE_AHEAD_NONE : FORM;  // what is fetched a tile ahead
   const int tid = threadIdx.x, nthr = blockDim.x;
   const int lane = tid & 31, warp = tid >> 5, nwarp = (nthr + 31) >> 5;
   const int N = p.N, R = p.R, L = p.L, TPR = p.tpr;
@@ -420,11 +423,11 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
     const int rows = (int)min((long long)R, p.B - row0);
     const uint32_t bytes = (uint32_t)(rows * N * sizeof(T));
     const uint32_t cbytes = (uint32_t)(rows * N * sizeof(float2));
-    mbar_expect_tx(&bar[0], (tape ? 2 : 4) * bytes + n_ck * cbytes + (residual ? bytes : 0));
+    mbar_expect_tx(&bar[0], (tape ? 2 : 4) * bytes + (GLOBAL ? 0 : n_ck * cbytes) + (residual ? bytes : 0));
 #pragma unroll
     for (int q = 0; q < 4; ++q)
       if (q >= 2 || !tape) bulk_g2s(win + q * RN, g_in[q] + row0 * N, bytes, &bar[0]);
-    for (uint32_t k = 0; k < n_ck; ++k)
+    for (uint32_t k = 0; !GLOBAL && k < n_ck; ++k)
       bulk_g2s(const_cast<float2*>(sck) + k * RN, ckpt + (long long)k * BN + row0 * N, cbytes, &bar[0]);
     if (residual) bulk_g2s(sdy, g_in[2] + row0 * N, bytes, &bar[0]);
   };
@@ -498,7 +501,7 @@ __global__ void __launch_bounds__(MAXT, MINB) lanep_bwd_kernel(const LaneParams 
     }
 
     auto load_ckpt = [&](float2 (&V)[4][NG], int ck, int set) {  // a state saved after a stage replaces the rebuilt one
-      if (AHEAD) {
+      if (GLOBAL) {
         if (!active) return;
         const float2* c = ckpt + (long long)ck * BN + (row0 + r) * N + set * TPR + t;
 #pragma unroll

@@ -125,6 +125,42 @@ def test_rows_a_tile_ahead(ncn, n, N, B, L, act, mode, dtype, first, ahead):
             assert O.rel_err(a, b) < 2e-2, name
 
 
+# A backward that is asked for the rebuilt input reads the states as the forward of the same arguments wrote them: where all of them fit
+# into shared memory, where they do not (groups of 4: read from global memory, form 4), behind an output and behind a stored end state.
+@pytest.mark.parametrize("n,N,L,tape,residual,dtype,form", [
+    (4, 512, 5, True, False, torch.float32, 0), (4, 512, 5, True, True, torch.float32, 4), (4, 512, 6, True, False, torch.float32, 4),
+    (4, 1024, 6, True, True, torch.bfloat16, 4), (4, 2048, 6, True, False, torch.float32, 4), (4, 2048, 5, True, True, torch.bfloat16, 0),
+    (4, 4096, 5, True, False, torch.float32, 0), (4, 4096, 5, True, True, torch.float32, 4), (4, 4096, 6, True, False, torch.float32, 4),
+    (4, 4096, 6, True, True, torch.float32, 4), (4, 4096, 6, True, False, torch.bfloat16, 4), (4, 8192, 2, True, False, torch.float32, 4),
+    (4, 8192, 4, True, True, torch.bfloat16, 4), (4, 8192, 4, False, False, torch.float32, 4), (4, 4096, 7, False, False, torch.float32, None),
+    (2, 1024, 9, True, False, torch.float32, None), (8, 4096, 4, True, True, torch.float32, None), (16, 1040, 3, True, False, torch.float32, None),
+])
+def test_rebuilt_input_from_the_same_states(ncn, n, N, L, tape, residual, dtype, form):
+    B = 37
+    x, xa, ws, dy, dya = _data(B, N, n, L, dtype, N + L)
+    W = torch.stack(ws).cuda()
+    xd, xad, dyd, dyad = (t.cuda().to(dtype) for t in (x, xa, dy, dya))
+    y, ya, ck = ncn.ops.net_fwd(xd, xad, W, 0.9, 0, n, 1, 0, 1, residual, tape)
+
+    def back(want):
+        return ncn.ops.net_bwd(None if tape else y, None if tape else ya, dyd, dyad, W, 0.9, 0, n, 1, 0, ckpt=ck, ckpt_every=1,
+                               residual=residual, tape=tape, want_inputs=want)
+
+    got, (rec, names) = back(False), kernels_of(lambda: back(True))
+    ncn.ops.device_status()
+    fp32 = dtype == torch.float32
+    for name, a, b in zip(("x", "xa"), rec[3:], (x, xa)):
+        assert O.rel_err(a.float(), b) < (1e-5 if fp32 else 2 ** -8), name
+    want = O.stack_fwd_bwd(x, xa, [ws], dy, dya, 0.9, "tanh", n, 1) if residual else O.net_fwd_bwd(x, xa, ws, dy, dya, 0.9, "tanh", n, 1)
+    dW = torch.stack(list(want[4][0] if residual else want[4]))
+    for res in (got, rec):
+        for name, a, b in zip(("dx", "dxa"), res, want[2:4]):
+            assert O.rel_err(a.float(), b) < (1e-5 if fp32 else 2e-2), name
+        assert O.rel_err(res[2], dW) < (2e-5 if fp32 else 2e-2), "dW"
+    if form is not None:
+        assert launched(names, rf"lanep_bwd_kernel<{n},.* {form}>"), names
+
+
 @pytest.mark.parametrize("n,N,B,act,mode", [
     (16, 240, 5003, "tanh", "checkpoint"), (16, 1840, 700, "sigmoid", "tape"), (8, 1048, 2001, "linear", "checkpoint"),
     (8, 1048, 2001, "tanh", "tape"), (16, 2048, 600, "relu", "checkpoint"),
