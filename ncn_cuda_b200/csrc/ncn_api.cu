@@ -22,7 +22,10 @@ __device__ int g_status_word = 0;
 
 static thread_local char tl_cuda_err[256] = "";
 
+// The error is reported here and nowhere else: what cudaGetLastError() still holds of it (cudaLaunchKernelEx and the attribute calls
+// leave it there) would be read as the failure of the next launch, of this library or of the caller.
 static int cuda_fail(cudaError_t e) {
+  cudaGetLastError();
   std::snprintf(tl_cuda_err, sizeof(tl_cuda_err), "%s: %s", cudaGetErrorName(e), cudaGetErrorString(e));
   return NCN_ERR_CUDA;
 }

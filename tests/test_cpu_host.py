@@ -204,3 +204,32 @@ def test_host_pipeline_chunk_bounds():
         assert all(0 < e - s <= rows for s, e in b)                  # fit the device slots
     long = chunk_bounds(65536, 4096)
     assert long[0] == (0, 1024) and long[-1] == (64512, 65536)       # short chunks at both ends
+
+
+FAKE_LAUNCHES = r"""
+static int last = 0;                                      /* the runtime's error state */
+int cudaLaunchKernelExC(const void *cfg, const void *f, void **args) { return last = 9; }  /* cudaErrorInvalidConfiguration */
+int cudaLaunchKernel() { return 0; }
+int cudaGetLastError(void) { int e = last; last = 0; return e; }
+"""
+A_FAILED_LAUNCH_THEN_ANOTHER = """
+import ctypes, sys
+lib = ctypes.CDLL(sys.argv[1])
+buf = (ctypes.c_float * 64)()
+ptrs = (ctypes.c_void_p * 1)(ctypes.addressof(buf))
+rows = (ctypes.c_int * 1)(4)
+first = lib.ncn_reduce_partials(ptrs, rows, ptrs, 1, ctypes.c_int64(2), None)
+print(first, lib.ncn_gather_weights(ptrs, 1, ctypes.c_int64(2), buf, None))
+"""
+
+
+def test_a_failed_launch_is_reported_once(tmp_path):
+    """The launches and the error state are fakes, so nothing runs: the first launch fails, the second does not."""
+    from ncn_cuda_b200 import _lib
+
+    src, so = tmp_path / "fake.c", tmp_path / "fake.so"
+    src.write_text(FAKE_LAUNCHES)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-w", "-o", str(so), str(src)], check=True)
+    res = subprocess.run([sys.executable, "-c", A_FAILED_LAUNCH_THEN_ANOTHER, _lib.LIB_PATH], capture_output=True, text=True,
+                         env=dict(os.environ, LD_PRELOAD=str(so)), timeout=300)
+    assert res.stdout.split() == ["7", "0"], res.stdout + res.stderr
