@@ -44,7 +44,7 @@ def rows_per_chunk(B: int, tensor_bytes: int, chunk_rows: int) -> int:
     sqrt(tensor / 0.9 MB).  Measured with 1, 2, 4, 8, 16 chunks, us: tensors of 2.1 MB 429 436 474 788 1134; 8.4 MB 1354 1149 1148 -
     1623; 33.6 MB 5040 4050 3641 3662 4145; 134 MB 20045 15900 14225 13161 13033."""
     c = max(1, round(math.sqrt(tensor_bytes / 0.9e6)))
-    return max(1, min(chunk_rows, B, -(-B // c)))
+    return min(chunk_rows, B, -(-B // c))
 
 
 def net_fwd_bwd_host(
@@ -55,8 +55,10 @@ def net_fwd_bwd_host(
 ):
     """x, xa, dy, dya: CPU tensors [B, N, E] (pinned for full copy bandwidth); W: [L, 2E].  `chunk_rows`: most rows
     on the device at a time per buffer.  Returns (y, ya, dx, dxa, dW) on the host; `out` may supply the four pinned result tensors."""
-    device = device or torch.device("cuda", torch.cuda.current_device())
     B = x.shape[0]
+    if B < 1 or chunk_rows < 1:
+        raise ValueError(f"no rows to take: {B} rows in chunks of {chunk_rows}")
+    device = device or torch.device("cuda", torch.cuda.current_device())
     L = W.shape[0]
     if out is None:
         out = tuple(torch.empty_like(x).pin_memory() for _ in range(4))

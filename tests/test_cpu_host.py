@@ -194,6 +194,15 @@ def test_rows_per_chunk(B, tensor_bytes, most):
         assert len(b) == 1
 
 
+@pytest.mark.parametrize("B,chunk_rows", [(0, 4096), (8, 0), (8, -3)])
+def test_host_call_without_rows_is_refused(B, chunk_rows):
+    from ncn_cuda_b200.host import net_fwd_bwd_host
+
+    x, dev = torch.zeros(B, 16, 1), torch.device("cuda", 0)
+    with pytest.raises(ValueError, match="no rows"):
+        net_fwd_bwd_host(x, x, torch.zeros(2, 2), x, x, 0.9, "tanh", 4, 1, chunk_rows=chunk_rows, device=dev)
+
+
 def test_host_pipeline_chunk_bounds():
     from ncn_cuda_b200.host import chunk_bounds
 
