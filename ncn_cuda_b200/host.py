@@ -41,7 +41,8 @@ def chunk_bounds(B: int, rows: int):
 def rows_per_chunk(B: int, tensor_bytes: int, chunk_rows: int) -> int:
     """Rows of a chunk, at most `chunk_rows`.  c chunks leave 1/c of the copies without overlap and cost 75 us each (eight copies,
     three launches, events), so the sum is smallest at c = sqrt(copies / 75 us); four tensors each way at 47 GB/s make that
-    sqrt(tensor / 0.9 MB).  Measured with 1, 2, 4, 8, 16 chunks, us: tensors of 2.1 MB 429 436 474 788 1134; 8.4 MB 1354 1149 1148 -
+    sqrt(tensor / 0.9 MB).  (From six on chunk_bounds cuts the first and the last up. That adds four, 300 us, and
+    takes three quarters off the first copy in and the last out, which at six chunks are 0.46 ms each.)  Measured with 1, 2, 4, 8, 16 chunks, us: tensors of 2.1 MB 429 436 474 788 1134; 8.4 MB 1354 1149 1148 -
     1623; 33.6 MB 5040 4050 3641 3662 4145; 134 MB 20045 15900 14225 13161 13033."""
     c = max(1, round(math.sqrt(tensor_bytes / 0.9e6)))
     return min(chunk_rows, B, -(-B // c))

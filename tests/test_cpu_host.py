@@ -182,16 +182,19 @@ def test_bench_reference_arm_prints_contract_line():
         assert line["cpu_reference_literal"]["kind"] == "reference" and line["cpu_reference_literal"]["value"] > 0
 
 
-@pytest.mark.parametrize("B,tensor_bytes,most", [(1, 4, 4096), (8192, 134 << 20, 4096), (256, 2 << 20, 4096), (65536, 1 << 30, 4096), (30, 400 << 20, 4), (7, 1 << 34, 4096)])
-def test_rows_per_chunk(B, tensor_bytes, most):
+@pytest.mark.parametrize("B,tensor_bytes,most,chunks", [
+    (1, 4, 4096, 1), (256, 1 << 20, 4096, 1), (256, 2 << 20, 4096, 2), (1000, 8 << 20, 4096, 3), (8192, 32 << 20, 4096, 6), (8192, 134 << 20, 4096, 12 + 4),
+    (65536, 1 << 30, 4096, 35 + 4), (30, 400 << 20, 4, 15), (7, 1 << 34, 4096, 7), (65536, 1 << 20, 4096, 16 + 4),
+])
+def test_rows_per_chunk(B, tensor_bytes, most, chunks):
+    """sqrt(tensor / 0.9 MB) chunks, at most `most` rows each; a batch of six of them or more has its first and last cut up (four chunks more)."""
     from ncn_cuda_b200.host import chunk_bounds, rows_per_chunk
 
     rows = rows_per_chunk(B, tensor_bytes, most)
     assert 1 <= rows <= min(B, most)
     b = chunk_bounds(B, rows)
     assert b[0][0] == 0 and b[-1][1] == B and all(p[1] == q[0] for p, q in zip(b, b[1:]))
-    if tensor_bytes < 2e6:  # a chunk costs more than it overlaps
-        assert len(b) == 1
+    assert len(b) == chunks
 
 
 @pytest.mark.parametrize("B,chunk_rows", [(0, 4096), (8, 0), (8, -3)])
