@@ -621,9 +621,9 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
   LanePlan best;
   bool have_pipe = false;
   if (n == 4 && !shape.ragged && (bwd ? lanep_enabled() : env_switches().lanes_pipe_fwd)) {
-    // The inputs a tile ahead, us without -> with: 32768 x 4096, 5 stages bf16 1738 -> 1682, fp32 from the output alone 2091 -> 2047; 16384 x 8192,
-    // 4 stages fp32 1948 -> 1840, bf16 1565 -> 1433.  Where states are stored inside a net and no CTA per SM is won by it, the copies of a
-    // stage with and without one cost what the rest wins (65536 x 4096, 6 stages 4976 either way; 4096 x 1024 103 -> 105).
+    // The inputs a tile ahead, us without -> with: 32768 x 4096, 5 stages bf16 1753 -> 1639, fp32 from the output alone 2191 -> 2138; 16384 x 8192,
+    // 4 stages fp32 1988 -> 1832, bf16 1559 -> 1407.  Where states are stored inside a net and no CTA per SM is won by it, the copies of a
+    // stage with and without one cost what the rest wins (65536 x 4096, 6 stages 5208 -> 5223; 4096 x 1024 111 -> 112).
     // rec: a forward that stored states counts on this family wherever the plan without rec is of it.  The states in global memory take
     // no more room than the forms that fetch ahead, so that there is a plan with rec too.
     const int fetch = !bwd || (rec && n_ck == 0) ? LANE_AHEAD_NONE : rec ? LANE_STATES_GLOBAL : !(flags & F_TAPE) ? LANE_AHEAD_OUTPUT : n_ck > 1 ? LANE_AHEAD_TAPES : LANE_AHEAD_TAPE;
@@ -662,14 +662,14 @@ static int plan_lanes(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, i
     if (occ >= want_occ) break;
   }
   // The inputs a tile ahead, where their buffer costs no CTA.  Backward, us, without -> with: bf16, end state stored: 65536 x 2048, groups
-  // of 8, 4 stages 2126 -> 2065; 32768 x 4096 2295 -> 2203; 16384 x 8192, 3 stages 1960 -> 1770; groups of 2, 6 stages 1699 -> 1505.
-  // fp32 from the output: 8192 x 8192, groups of 8, 3 stages 1305 -> 1214; 16384 x 4096, groups of 2, 8 stages 1139 -> 1085; groups of 8,
-  // 4 stages 1437 -> 1428.  fp32 with all states stored, which then need no shared memory: 16384 x 4096, groups of 8 1880 -> 1414.
-  // Ragged rows: 20000 x 3000 fp32, groups of 4, 5 stages 1200 -> 1145; 5000 x 8176, groups of 8 861 -> 775; end state stored, 9000 x 5000
-  // fp32, groups of 2 888 -> 787, 10000 x 4000, groups of 4 615 -> 590; bf16 then, and groups of 8, only where that leaves room for more
-  // CTAs or there is one anyway (bf16 5000 x 8184 648 -> 630, but 20000 x 2000 400 -> 408; groups of 8, 4 stages 6000 x 5008 970 -> 897, but
-  // 3000 x 3008 249 -> 255).
-  // The pipelined kernel of groups of 4 stays ahead of it (32768 x 4096, 5 stages bf16 1682 against 1810, fp32 2140 against 2328).
+  // of 8, 4 stages 2138 -> 2073; 32768 x 4096 2308 -> 2223; 16384 x 8192, 3 stages 1953 -> 1777; groups of 2, 6 stages 1722 -> 1502.
+  // fp32 from the output: 8192 x 8192, groups of 8, 3 stages 1286 -> 1168; 16384 x 4096, groups of 2, 8 stages 1236 -> 1222; groups of 8,
+  // 4 stages 1488 -> 1412.  fp32 with all states stored, which then need no shared memory: 16384 x 4096, groups of 8 1963 -> 1382.
+  // Ragged rows: 20000 x 3000 fp32, groups of 4, 5 stages 1272 -> 1249; end state stored, 9000 x 5000 fp32, groups of 2, 6 stages
+  // 946 -> 836, 10000 x 4000, groups of 4, 4 stages 645 -> 608; bf16 then, and groups of 8, only where that leaves room for more CTAs or
+  // there is one anyway (bf16, groups of 2, 6 stages 5000 x 8184 579 -> 539, but groups of 4 20000 x 2000 461 -> 461; groups of 8, 4
+  // stages 6000 x 5008 965 -> 885, 5000 x 8176 1084 -> 1083.  At as many CTAs groups of 8 would win little: 3000 x 3008 253 -> 246).
+  // The pipelined kernel of groups of 4 stays ahead of it (32768 x 4096, 5 stages bf16 1639 against 1811, fp32 2242 against 2437).
   if (rc == NCN_OK && bwd && !rec && (!have_pipe || best.occ < want_occ) && (!(flags & F_TAPE) || lane_ahead_tape(n, shape.ragged))) {
     // CTAs per SM that make it worth while
     const bool even = shape.ragged && want_occ > 1 && (n == 8 || (dtype == DT_BF16 && (flags & F_TAPE)));  // (no gain at as many CTAs)
@@ -793,9 +793,9 @@ static int plan_solo(bool bwd, int64_t B, int64_t N, int64_t E, int n, int C, in
     cudaError_t e = occupancy(p.smem, SOLO_AHEAD_NONE, p.occ);
     if (e != cudaSuccess) return cuda_fail(e);
     // Backward: the inputs a tile ahead, where their buffer costs no CTA.  Without -> with, us: 16384 x 8192 bf16, groups of 16, 4
-    // stages 4046 -> 3929; 8192 x 8192 fp32 with the end state stored 2158 -> 2048; 25000 x 2048 1650 -> 1562; 50000 x 2048 bf16
-    // 2963 -> 2934, 16384 x 4096 bf16 1932 -> 1925; 10000 x 2968 fp32, groups of 8, 3 stages 680 -> 613.  Where it does cost one (fp32
-    // from the output, 2048 and 4096 positions) the other CTAs cover the loads.
+    // stages 4070 -> 3931; 3 stages, fp32 with the end state stored 8192 x 8192 2180 -> 2091, 25000 x 2048 1703 -> 1615; 50000 x 2048
+    // bf16 2970 -> 2924, 16384 x 4096 bf16 1925 -> 1928; 10000 x 2968 fp32, groups of 8, 3 stages 690 -> 624.  Where it does cost one
+    // (fp32 from the output, 2048 and 4096 positions) the other CTAs cover the loads: 25000 x 2048 1668 -> 1895 with it.
     if (bwd && !rec && !(flags & F_RESIDUAL)) {
       const size_t more = ((size_t)(tape ? 2 : 4) * R * N * w + 127) / 128 * 128;
       const int ahead = tape ? SOLO_AHEAD_TAPE : SOLO_AHEAD_OUTPUT;

@@ -16,8 +16,8 @@
 // Any number of blocks up to 512 per row, any stride; R rows side by side in a CTA.
 //
 // Measured on a B200 (forward + backward, before = ncn_pairs.cuh forward and ncn_rows.cuh backward): 25000 x 2048 fp32, groups of
-// 16, 3 stages 1447 + 1947 -> 945 + 1604 us; 65536 x 8192 bf16, 4 stages 9.93 + 16.2 -> 9.23 + 15.6 ms.  Cycles per
-// warp, position and step: fp32 13.9 + 23.4, arithmetic alone 11.5 + 19.2; bf16 10.0 + 16.9, alone 8.3 + 12.6 (rows of 8192: one
+// 16, 3 stages 1447 + 1947 -> 945 + 1660 us; 65536 x 8192 bf16, 4 stages 9.93 + 16.2 -> 9.23 + 15.7 ms.  Cycles per
+// warp, position and step: fp32 13.9 + 24.2, arithmetic alone 11.5 + 19.2; bf16 10.0 + 17.0, alone 8.3 + 12.6 (rows of 8192: one
 // CTA of 512 threads per SM, whose boundaries nothing overlaps).
 #pragma once
 #include "ncn_lanes.cuh"
