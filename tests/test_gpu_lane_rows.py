@@ -147,12 +147,16 @@ def test_residual_layers_a_tile_ahead(ncn, n, N, B, L, dtype, ahead):
     W = torch.stack(ws).cuda()
     xd, xad, dyd, dyad = (t.cuda().to(dtype) for t in (x, xa, dy, dya))
     _, every, _ = plan_backward(dtype, n, L, True, "tape")
-    y, ya, ck = ncn.ops.net_fwd(xd, xad, W, 0.9, 0, n, 1, 0, every, True, True)
-    got, names = kernels_of(lambda: ncn.ops.net_bwd(None, None, dyd, dyad, W, 0.9, 0, n, 1, 0, ckpt=ck, ckpt_every=every, residual=True, tape=True))
+
+    def calls():
+        y, ya, ck = ncn.ops.net_fwd(xd, xad, W, 0.9, 0, n, 1, 0, every, True, True)
+        return y, ya, *ncn.ops.net_bwd(None, None, dyd, dyad, W, 0.9, 0, n, 1, 0, ckpt=ck, ckpt_every=every, residual=True, tape=True)
+
+    got, names = kernels_of(calls)
     ncn.ops.device_status()
     assert launched(names, rf"lane_bwd_kernel<{n},.* {ahead}, (true|false|0|1)>") or launched(names, rf"lanep_bwd_kernel<{n},.* {ahead}>"), names
     want = O.stack_fwd_bwd(x, xa, [ws], dy, dya, 0.9, "tanh", n, 1)
-    got, want = [t.float().cpu() for t in (y, ya, *got)], (*want[:4], want[4][0])
+    got, want = [t.float().cpu() for t in got], (*want[:4], want[4][0])
     if dtype == torch.bfloat16:
         _bf16_against_oracle(got, want)
     else:
@@ -177,13 +181,14 @@ def test_rebuilt_input_from_the_same_states(ncn, n, N, L, tape, residual, dtype,
     x, xa, ws, dy, dya = _data(B, N, n, L, dtype, N + L)
     W = torch.stack(ws).cuda()
     xd, xad, dyd, dyad = (t.cuda().to(dtype) for t in (x, xa, dy, dya))
-    y, ya, ck = ncn.ops.net_fwd(xd, xad, W, 0.9, 0, n, 1, 0, 1, residual, tape)
 
-    def back(want):
-        return ncn.ops.net_bwd(None if tape else y, None if tape else ya, dyd, dyad, W, 0.9, 0, n, 1, 0, ckpt=ck, ckpt_every=1,
-                               residual=residual, tape=tape, want_inputs=want)
+    def calls():
+        y, ya, ck = ncn.ops.net_fwd(xd, xad, W, 0.9, 0, n, 1, 0, 1, residual, tape)
+        s0, s1 = (None, None) if tape else (y, ya)
+        return [ncn.ops.net_bwd(s0, s1, dyd, dyad, W, 0.9, 0, n, 1, 0, ckpt=ck, ckpt_every=1, residual=residual, tape=tape, want_inputs=want)
+                for want in (False, True)]
 
-    got, (rec, names) = back(False), kernels_of(lambda: back(True))
+    (got, rec), names = kernels_of(calls)
     ncn.ops.device_status()
     fp32 = dtype == torch.float32
     for name, a, b in zip(("x", "xa"), rec[3:], (x, xa)):
