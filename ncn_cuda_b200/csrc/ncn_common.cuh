@@ -31,8 +31,8 @@ inline cudaError_t grant_smem(SmemGrant& g, K kernel, size_t smem) {
 
 // Kernels of this library in a row: a kernel is set up for launch while the one before it still runs (programmatic dependent launch), and
 // waits in wait_for_inputs(), before its first access to global memory, until that one is done and its writes are visible.  1 to 2 us
-// at each of the launches of a step: 1000 x 3000, groups of 4, 5 stages 128.0 -> 121.7 us; bf16 tokens 64 x 512 x 256, 4 stages 727 -> 709;
-// 64 padded rows, 3 stages 286 -> 270.  Nothing is let in earlier (griddepcontrol.launch_dependents): CTAs that take their places one by
+// at each of the launches of a step: 1000 x 3000, groups of 4, 5 stages 134.7 -> 128.3 us; bf16 tokens 64 x 512 x 256, 4 stages 727 -> 708;
+// 64 padded rows, 3 stages 269 -> 254.  (Small steps that the host bounds: no difference beyond their noise.)  Nothing is let in earlier (griddepcontrol.launch_dependents): CTAs that take their places one by
 // one, as those of the kernel before leave, are spread unevenly over the SMs (the first of these 127 -> 138, the last 284 -> 292).
 __device__ __forceinline__ void wait_for_inputs() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... Params, typename... Args>
