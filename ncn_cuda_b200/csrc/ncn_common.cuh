@@ -391,9 +391,9 @@ struct ActForm<ACT_LINEAR> {
 // The exponent is capped at 30: beyond it r < 1e-9 (tanh = 1 to the last bit) and the product of four d stays a normal
 // fp32 number, as does its reciprocal.  A NaN reaches all values that share its reciprocal.  These would see it all the same
 // where they are the features of one position, through their dot product, and in the reverse sweep, where the sums for gx_j
-// bring a NaN in any x of a group to all of its cotangents (and to its rebuilt a; of the rebuilt x, those that share may have one
-// that a step of their own would not give, where an output holds a NaN that no forward leaves: in position 0 alone).  They would
-// not in the forward steps of a group's positions: a row with a NaN is taken again there (ncn_terms.cuh).
+// bring a NaN in any x of a group to all of its cotangents, and the step at which that position is x_j to all of its rebuilt
+// a.  (The rebuilt x of positions that share with position 0 has one too many where an output is NaN in position 0 alone, as a NaN in
+// xa leaves it.)  They would not in the forward steps of a group's positions: a row with a NaN is taken again there (ncn_terms.cuh).
 template <int ACT, int NG, int BATCH>
 __device__ __forceinline__ void act_r_all(const float2 (&ts)[NG], float2 (&r)[NG]) {
   if constexpr (ACT == ACT_TANH || ACT == ACT_SIGMOID) {
